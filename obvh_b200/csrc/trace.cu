@@ -12,9 +12,14 @@
 // intersected after the next node is popped; triangles are tested in the
 // leaf's order and a hit replaces the closest one only if strictly nearer.
 // The reference's warp ballots only decide when a warp leaves its loops, so
-// the scheduling is free: persistent warps hand each lane a new ray as soon
-// as its ray is done (below), node records are read as 16-byte words through
-// the read-only path, and the 64-entry stack lives in local memory as in the
+// the scheduling is free, and what sets the time is how many lanes of a warp
+// step together: lane by lane, a warp of incoherent rays ran 7.7 of 32 lanes
+// wide.  Here a warp visits nodes only while most of its lanes stand at one
+// (25 lanes wide), tests the triangles of all waiting lanes as one dealt-out
+// batch, and finished lanes take new rays together.  2,000,003 probe rays into
+// the 2M-triangle soup: 6.71 -> 4.74 ms, now waiting for node rows (58 of 100
+// sectors miss L1); 1920 x 1080 camera rays into the 917K-triangle knot: 1.26
+// -> 0.31 ms.  The 64-entry stack lives in local memory as in the
 // reference.  Indices are checked: a node, leaf, primitive
 // slot or face outside its array, or a stack deeper than 64, stops that ray
 // with its miss record and sets the error word.
@@ -23,13 +28,18 @@
 #include <cstdint>
 #include <mutex>
 
+#include "device_common.cuh"
 #include "obvh_transforms.h"
 #include "runtime.h"
 
 namespace obvh {
 namespace trace {
 
-constexpr int kThreads = 128;
+// 32 warps an SM at 61 registers, no spills.  More warps do not help: the
+// probe rays wait for node rows from L2, and 36 warps (56 registers, spills)
+// or 24 (68) ran as fast within 1%.
+constexpr int kThreads = 512;
+constexpr int kBlocksPerSm = 2;
 constexpr int kStack = 64;
 constexpr int32_t kSentinel = 0x76543210;
 constexpr uint32_t kErrIndex = 1u;
@@ -57,9 +67,16 @@ __device__ __forceinline__ M43 load_m43(const kr_mat43* p) {
     return M43{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w}};
 }
 
-// (t0, t1) of the ray (rd, ro) against the unit cube [-0.5, 0.5]^3; (1, -1)
-// on a miss (kr_ray_unit_aabb_intersect).
-__device__ __forceinline__ float2 unit_slabs(V3 rd, V3 ro) {
+// A child's ray: the direction and origin in the frame where its box is the
+// unit cube.
+struct BoxRay {
+    V3 d, o;
+};
+
+// (t0, t1) of the ray against the unit cube [-0.5, 0.5]^3; (1, -1) on a miss
+// (kr_ray_unit_aabb_intersect).
+__device__ __forceinline__ float2 unit_slabs(const BoxRay& r) {
+    const V3 rd = r.d, ro = r.o;
     const float nx = (-0.5f - ro.x) / rd.x, ny = (-0.5f - ro.y) / rd.y, nz = (-0.5f - ro.z) / rd.z;
     const float fx = (0.5f - ro.x) / rd.x, fy = (0.5f - ro.y) / rd.y, fz = (0.5f - ro.z) / rd.z;
     const float t0 = kmax(kmax(kmin(nx, fx), kmin(ny, fy)), kmin(nz, fz));
@@ -68,15 +85,42 @@ __device__ __forceinline__ float2 unit_slabs(V3 rd, V3 ro) {
     return make_float2(t0, t1);
 }
 
-// (t0, t1) against the unit cube in the frame of `l` (kr_n43transform3p /
-// kr_v43transform3p, then kr_ray_unit_aabb_intersect).
-__device__ __forceinline__ float2 unit_box(const M43& l, V3 d, V3 o) {
+// The same (t0, t1), each within kSlabError of its size, before the hit test:
+// every quotient is the numerator times the hardware's reciprocal (at most
+// 2^-23 off, the product 2^-24, the exact quotient's own rounding 2^-24), and
+// min and max keep a relative bound.  A NaN reaches t0 and t1.  False where a
+// reciprocal is outside [2^-59, 2^59]: the bound needs products that neither
+// over- nor underflow (a numerator is zero or at least 2^-25).
+constexpr float kSlabError = 0x1p-20f;
+__device__ __forceinline__ bool near_slabs(const BoxRay& r, float& t0, float& t1) {
+    float yx, yy, yz;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yx) : "f"(r.d.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yy) : "f"(r.d.y));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yz) : "f"(r.d.z));
+    const float nx = (-0.5f - r.o.x) * yx, ny = (-0.5f - r.o.y) * yy, nz = (-0.5f - r.o.z) * yz;
+    const float fx = (0.5f - r.o.x) * yx, fy = (0.5f - r.o.y) * yy, fz = (0.5f - r.o.z) * yz;
+    asm("{\n\t.reg .f32 x, y, z;\n\tmin.NaN.f32 x, %1, %4;\n\tmin.NaN.f32 y, %2, %5;\n\tmin.NaN.f32 z, %3, %6;\n\t"
+        "max.NaN.f32 %0, x, y, z;\n\t}"
+        : "=f"(t0) : "f"(nx), "f"(ny), "f"(nz), "f"(fx), "f"(fy), "f"(fz));
+    asm("{\n\t.reg .f32 x, y, z;\n\tmax.NaN.f32 x, %1, %4;\n\tmax.NaN.f32 y, %2, %5;\n\tmax.NaN.f32 z, %3, %6;\n\t"
+        "min.NaN.f32 %0, x, y, z;\n\t}"
+        : "=f"(t1) : "f"(nx), "f"(ny), "f"(nz), "f"(fx), "f"(fy), "f"(fz));
+    return min3f(fabsf(yx), fabsf(yy), fabsf(yz)) > 0x1p-59f && max3f(fabsf(yx), fabsf(yy), fabsf(yz)) < 0x1p59f;
+}
+
+// Whether a < b (and a <= b) is decided although both may be off by
+// kSlabError of their size; false for a NaN or an infinity.
+__device__ __forceinline__ bool apart(float a, float b) {
+    return fabsf(a - b) > kSlabError * (fabsf(a) + fabsf(b));
+}
+
+// The ray in the frame of `l` (kr_n43transform3p / kr_v43transform3p).
+__device__ __forceinline__ BoxRay into_box(const M43& l, V3 d, V3 o) {
     const float* m = l.m;
-    const V3 rd = v3(m[0] * d.x + m[3] * d.y + m[6] * d.z, m[1] * d.x + m[4] * d.y + m[7] * d.z,
-                     m[2] * d.x + m[5] * d.y + m[8] * d.z);
-    const V3 ro = v3(m[0] * o.x + m[3] * o.y + m[6] * o.z + m[9], m[1] * o.x + m[4] * o.y + m[7] * o.z + m[10],
-                     m[2] * o.x + m[5] * o.y + m[8] * o.z + m[11]);
-    return unit_slabs(rd, ro);
+    return BoxRay{v3(m[0] * d.x + m[3] * d.y + m[6] * d.z, m[1] * d.x + m[4] * d.y + m[7] * d.z,
+                     m[2] * d.x + m[5] * d.y + m[8] * d.z),
+                  v3(m[0] * o.x + m[3] * o.y + m[6] * o.z + m[9], m[1] * o.x + m[4] * o.y + m[7] * o.z + m[10],
+                     m[2] * o.x + m[5] * o.y + m[8] * o.z + m[11])};
 }
 
 // kr_vrotate_angle_axis3 (vecmath.h:1178-1189): Rodrigues' formula, with the
@@ -92,8 +136,8 @@ __device__ __forceinline__ V3 rotate_angle_axis(V3 v, V3 axis, float radians) {
 // A child of the compressed SoA OBVH (intersectors.cu:1047-1071): the axis
 // and angle dequantised from the metadata word (byte / 127, the angle times
 // the reference's float pi), the ray rotated, offset by `min` and scaled by
-// `max`, then the unit cube.
-__device__ __forceinline__ float2 quant_box(const kr_aabb3* box, int32_t word, V3 d, V3 o) {
+// `max`.
+__device__ __forceinline__ BoxRay into_quant_box(const kr_aabb3* box, int32_t word, V3 d, V3 o) {
     const float* b = reinterpret_cast<const float*>(box);
     const V3 lo = v3(__ldg(b), __ldg(b + 1), __ldg(b + 2)), sc = v3(__ldg(b + 3), __ldg(b + 4), __ldg(b + 5));
     const uint32_t w = static_cast<uint32_t>(word);
@@ -103,26 +147,27 @@ __device__ __forceinline__ float2 quant_box(const kr_aabb3* box, int32_t word, V
     const float angle = (static_cast<float>(static_cast<int8_t>(w)) / 127.0f) * static_cast<float>(3.14159265359);
     const V3 rd0 = rotate_angle_axis(d, axis, angle);
     const V3 ro0 = rotate_angle_axis(sub(o, lo), axis, angle);
-    return unit_slabs(v3(rd0.x * sc.x, rd0.y * sc.y, rd0.z * sc.z), v3(ro0.x * sc.x, ro0.y * sc.y, ro0.z * sc.z));
+    return BoxRay{v3(rd0.x * sc.x, rd0.y * sc.y, rd0.z * sc.z), v3(ro0.x * sc.x, ro0.y * sc.y, ro0.z * sc.z)};
 }
 
-// Node tests of the two layouts: both children's (t0, t1) at internal node i
-// (m: its metadata).
+// Node tests of the two layouts: the ray in both children's frames at internal
+// node i (m: its metadata).
 struct SoaBoxes {
     const kr_mat43* __restrict__ left_t;
     const kr_mat43* __restrict__ right_t;
-    __device__ __forceinline__ void test(int32_t i, const int4& m, V3 d, V3 o, float2& li, float2& ri) const {
-        li = unit_box(load_m43(left_t + i), d, o);
-        ri = unit_box(load_m43(right_t + i), d, o);
+    __device__ __forceinline__ void rays(int32_t i, const int4& m, V3 d, V3 o, BoxRay& l, BoxRay& r) const {
+        const M43 lm = load_m43(left_t + i), rm = load_m43(right_t + i);
+        l = into_box(lm, d, o);
+        r = into_box(rm, d, o);
     }
 };
 
 struct QuantBoxes {
     const kr_aabb3* __restrict__ lbounds;
     const kr_aabb3* __restrict__ rbounds;
-    __device__ __forceinline__ void test(int32_t i, const int4& m, V3 d, V3 o, float2& li, float2& ri) const {
-        li = quant_box(lbounds + i, m.z, d, o);
-        ri = quant_box(rbounds + i, m.w, d, o);
+    __device__ __forceinline__ void rays(int32_t i, const int4& m, V3 d, V3 o, BoxRay& l, BoxRay& r) const {
+        l = into_quant_box(lbounds + i, m.z, d, o);
+        r = into_quant_box(rbounds + i, m.w, d, o);
     }
 };
 
@@ -136,7 +181,7 @@ struct RayState {
     V3 o, d;
     float hit_t, b1, b2;
     uint32_t hit, fail;
-    int32_t inode, leaf;
+    int32_t cur;  // the node to visit next: >= 0 internal, < 0 a leaf (~index), kSentinel when the ray is done
     int sp;
 };
 
@@ -166,141 +211,252 @@ __device__ __forceinline__ void finish(const RayState& st, const kr_vec3* verts,
     *out = rec;
 }
 
-// Persistent warps: warp w owns rays [w * per, (w + 1) * per) and hands a
-// lane the next of them as soon as that lane's ray is finished, at the top of
-// every outer step (one descent to a leaf plus the leaves found, the body of
-// the reference's outer loop), so lanes do not wait for the warp's slowest
-// ray.  A ray's own steps are those of the reference, in the same order.
+// One visit of an internal node: the nearer hit child next (ties to the
+// left), the farther pushed; neither hit: the next node of the stack.  Only
+// the outcome of the comparisons matters, so the slabs come from near_slabs
+// (3 reciprocals and 6 products a child instead of 6 IEEE divisions) and the
+// divisions are made where a comparison lies inside the error bound.
 template <class Boxes>
-__global__ void __launch_bounds__(kThreads)
+__device__ __forceinline__ void visit_node(const Boxes& boxes, const kr_ivec4* __restrict__ meta,
+                                           uint32_t internal_count, RayState& st, int32_t* stack) {
+    if (static_cast<uint32_t>(st.cur) >= internal_count) {
+        st.fail = kErrIndex;
+        st.cur = kSentinel;
+        return;
+    }
+    const int4 m = __ldg(reinterpret_cast<const int4*>(meta + st.cur));
+    BoxRay l, r;
+    boxes.rays(st.cur, m, st.d, st.o, l, r);
+    float l0, l1, r0, r1;
+    const bool sl = near_slabs(l, l0, l1), sr = near_slabs(r, r0, r1);
+    bool tl = l0 <= l1 && l1 > 0.0f && l0 <= st.hit_t;
+    bool tr = r0 <= r1 && r1 > 0.0f && r0 <= st.hit_t;
+    const bool sure_l = sl && apart(l0, l1) && apart(l0, st.hit_t);
+    const bool sure_r = sr && apart(r0, r1) && apart(r0, st.hit_t);
+    const bool close = (tl || !sure_l) && (tr || !sure_r) && !apart(l0, r0);
+    bool exact_l = !sure_l || close, exact_r = !sure_r || close;
+    while (exact_l || exact_r) {
+        const float2 e = unit_slabs(exact_l ? l : r);
+        const bool hit = e.y >= e.x && e.y >= 0.0f && e.x <= st.hit_t;
+        if (exact_l) {
+            tl = hit;
+            l0 = e.x;
+            exact_l = false;
+        } else {
+            tr = hit;
+            r0 = e.x;
+            exact_r = false;
+        }
+    }
+    const bool swap = r0 < l0;
+    if (tl && tr) {
+        if (st.sp + 1 >= kStack) {
+            st.fail = kErrStack;
+            st.cur = kSentinel;
+            return;
+        }
+        stack[++st.sp] = swap ? m.x : m.y;
+        st.cur = swap ? m.y : m.x;
+    } else if (tl || tr) {
+        st.cur = tl ? m.x : m.y;
+    } else {
+        st.cur = stack[st.sp--];
+    }
+}
+
+// t of the ray against one triangle, with its barycentrics; +inf on a miss
+// (kr_ray_triangle_intersect; its test against the closest hit so far is the
+// caller's strict t < hit_t).
+__device__ __forceinline__ float test_triangle(const kr_vec3* __restrict__ verts, uint4 f, V3 o, V3 d, float& c1,
+                                               float& c2) {
+    const V3 p1 = vertex(verts, f.x), p2 = vertex(verts, f.y), p3 = vertex(verts, f.z);
+    const V3 e1 = sub(p2, p1), e2 = sub(p3, p1);
+    const V3 s1 = cross(d, e2);
+    const float invd = 1.0f / dot(s1, e1);
+    const V3 dd = sub(o, p1);
+    c1 = dot(dd, s1) * invd;
+    const V3 s2 = cross(dd, e1);
+    c2 = dot(d, s2) * invd;
+    const float t = dot(e2, s2) * invd;
+    const bool miss = c1 < 0.0f || c1 > 1.0f || c2 < 0.0f || c1 + c2 > 1.0f || t < 0.0f;
+    return miss ? kInf : t;
+}
+
+// The leaves of the lanes that stand at one (st.cur < 0), by the whole warp:
+// their triangles are dealt out one to a lane, each tested against its
+// owner's ray, and the owner takes the first of the smallest t below its
+// closest hit -- what testing them in order with strict t < hit_t keeps.  A
+// leaf at a time and lane by lane, a warp ran about 3 lanes wide here, each
+// triangle behind its own chain of three loads.  Called by all 32 lanes.
+__device__ __forceinline__ void visit_leaves(const kr_ivec4* __restrict__ meta, uint32_t node_count,
+                                             const kr_vec3* __restrict__ verts, const kr_uvec4* __restrict__ faces,
+                                             uint32_t face_count, const kr_u32* __restrict__ prims,
+                                             uint32_t prim_slots, RayState& st, const int32_t* stack) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31;
+    const bool mine = st.cur < 0;
+    int32_t beg = 0;
+    uint32_t left = 0;  // triangles of this lane's leaf not yet dealt out
+    if (mine) {
+        const uint32_t li = static_cast<uint32_t>(~st.cur);
+        if (li >= node_count) {
+            st.fail = kErrIndex;
+        } else {
+            const int4 m = __ldg(reinterpret_cast<const int4*>(meta + li));
+            beg = m.x;
+            left = m.x < m.y ? static_cast<uint32_t>(m.y) - static_cast<uint32_t>(m.x) : 0u;
+        }
+    }
+    const bool single = left == 1;
+    for (;;) {
+        const uint32_t want = min(left, 32u);
+        uint32_t incl = want;
+#pragma unroll
+        for (int k = 1; k < 32; k <<= 1) {
+            const uint32_t v = __shfl_up_sync(kAll, incl, k);
+            if (lane >= static_cast<uint32_t>(k)) incl += v;
+        }
+        const uint32_t base = incl - want;
+        const uint32_t total = min(32u, __shfl_sync(kAll, incl, 31));
+        if (total == 0) break;
+        const uint32_t take = base < 32u ? min(want, 32u - base) : 0u;
+        // item `lane` belongs to the last lane whose base is at most `lane`
+        uint32_t owner = 0;
+#pragma unroll
+        for (int k = 16; k > 0; k >>= 1)
+            if (__shfl_sync(kAll, base, owner + k) <= lane) owner += k;
+        const uint32_t at = static_cast<uint32_t>(__shfl_sync(kAll, beg, owner)) + (lane - __shfl_sync(kAll, base, owner));
+        const bool one = __shfl_sync(kAll, static_cast<int>(single), owner) != 0;
+        const V3 o = v3(__shfl_sync(kAll, st.o.x, owner), __shfl_sync(kAll, st.o.y, owner), __shfl_sync(kAll, st.o.z, owner));
+        const V3 d = v3(__shfl_sync(kAll, st.d.x, owner), __shfl_sync(kAll, st.d.y, owner), __shfl_sync(kAll, st.d.z, owner));
+        bool bad = false;
+        float t = kInf, c1 = 0.0f, c2 = 0.0f;
+        uint32_t pid = at;
+        if (lane < total) {
+            if (!one) {
+                bad = static_cast<int32_t>(at) < 0 || at >= prim_slots;
+                if (!bad) pid = __ldg(prims + at);
+            }
+            bad = bad || pid >= face_count;
+            if (!bad) t = test_triangle(verts, __ldg(reinterpret_cast<const uint4*>(faces + pid)), o, d, c1, c2);
+        }
+        const unsigned wrong = __ballot_sync(kAll, bad);
+        const uint32_t most = __reduce_max_sync(kAll, take);
+        uint32_t who = lane;
+        bool better = false;
+        for (uint32_t j = 0; j < most; ++j) {
+            const float tj = __shfl_sync(kAll, t, (base + j) & 31u);
+            if (j < take && tj < st.hit_t) {
+                st.hit_t = tj;
+                who = base + j;
+                better = true;
+            }
+        }
+        c1 = __shfl_sync(kAll, c1, who);
+        c2 = __shfl_sync(kAll, c2, who);
+        pid = __shfl_sync(kAll, pid, who);
+        if (better) {
+            st.b1 = c1;
+            st.b2 = c2;
+            st.hit = pid;
+        }
+        beg += static_cast<int32_t>(take);
+        left -= take;
+        if (take && ((wrong >> base) & (take < 32u ? (1u << take) - 1u : kAll))) {
+            st.fail = kErrIndex;
+            left = 0;
+        }
+    }
+    if (mine) st.cur = (!st.fail && st.sp >= 0) ? stack[st.sp--] : kSentinel;
+}
+
+// A warp visits nodes while at least kNodeLanes of 32 lanes with a ray stand
+// at one; the lanes that meanwhile reached a leaf wait and test their leaves
+// together.  Finished lanes wait until kRefillLanes of them write their
+// records and take new rays together.  Measured (probe / camera, us): 20 of 32
+// 4,829 / 494, 24 4,808 / 505, 28 4,866 / 534; 4 or 8 finished lanes 5,044 /
+// 577 and 5,171 / 567 on an earlier form.
+constexpr int kNodeLanes = 24;
+constexpr int kRefillLanes = 4;
+
+// Persistent blocks: the rays lie in chunks of 32 and block b owns chunks b,
+// b + gridDim.x, ..., so that costly parts of the ray array (the object in a
+// camera's picture) spread over all blocks; a block's warps take its chunks
+// one after the other from a shared counter.  A ray's own steps are those of
+// the reference, in the same order; only which lanes step together differs.
+template <class Boxes>
+__global__ void __launch_bounds__(kThreads, kBlocksPerSm)
 trace_kernel(Boxes boxes, const kr_ivec4* __restrict__ meta, uint32_t internal_count, uint32_t node_count,
              const kr_vec3* __restrict__ verts, const kr_uvec4* __restrict__ faces, uint32_t face_count,
              const kr_u32* __restrict__ prims, uint32_t prim_slots, const kr_ray* __restrict__ rays,
-             kr_intersection* isects, uint32_t ray_count, uint32_t per_warp, uint32_t* err) {
+             kr_intersection* isects, uint32_t ray_count, uint32_t* err) {
+    constexpr unsigned kAll = 0xffffffffu;
+    __shared__ uint32_t s_taken;  // chunks of this block taken so far
+    if (threadIdx.x == 0) s_taken = 0;
+    __syncthreads();
     const uint32_t lane = threadIdx.x & 31;
-    const uint64_t warp = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t first = warp * per_warp;
-    const uint64_t last = first + per_warp;
-    const uint32_t end = last < ray_count ? static_cast<uint32_t>(last) : ray_count;
-    uint32_t next = first < ray_count ? static_cast<uint32_t>(first) : ray_count;  // next unassigned ray
+    const uint32_t chunks = (ray_count >> 5) + ((ray_count & 31u) != 0);
+    const uint32_t own = blockIdx.x < chunks ? (chunks - 1 - blockIdx.x) / gridDim.x + 1 : 0u;
+    uint32_t next = 0, stop = 0;  // the warp's unassigned rays
+    bool more = true;             // the block may have chunks left
     int32_t stack[kStack];
     RayState st;
+    st.cur = kSentinel;
+    st.fail = 0;
     uint32_t r = 0;
-    bool busy = false;
+    bool busy = false;  // this lane holds a ray (a finished one until its record is written)
     for (;;) {
-        // hand the warp's next rays to the idle lanes, in lane order
-        const uint32_t idle = __ballot_sync(0xffffffffu, !busy);
-        if (!busy) {
-            const uint32_t k = next + __popc(idle & ((1u << lane) - 1u));
-            if (k < end) {
-                r = k;
-                busy = true;
-                const float4* rp = reinterpret_cast<const float4*>(rays + r);
-                const float4 ra = __ldg(rp), rb = __ldg(rp + 1);
-                st.o = v3(ra.x, ra.y, ra.z);
-                st.d = v3(rb.x, rb.y, rb.z);
-                st.hit_t = rb.w;
-                st.hit = 0xFFFFFFFFu;
-                st.b1 = st.b2 = 0.0f;
-                st.fail = 0;
-                st.inode = 0;
-                st.leaf = 0;
-                st.sp = 0;
-                stack[0] = kSentinel;
+        const unsigned done = __ballot_sync(kAll, st.cur == kSentinel);
+        if (done == kAll || ((more || next < stop) && __popc(done) >= kRefillLanes)) {
+            if (busy && st.cur == kSentinel) {
+                finish(st, verts, faces, isects + r, err);
+                busy = false;
             }
-        }
-        next = min(end, next + __popc(idle));
-        if (!__any_sync(0xffffffffu, busy)) break;
-        if (!busy) continue;
-        const V3 o = st.o, d = st.d;
-        // descend until a leaf is found (the reference's inner loop)
-        bool searching = true;
-        while (searching && st.inode >= 0 && st.inode != kSentinel) {
-            if (static_cast<uint32_t>(st.inode) >= internal_count) {
-                st.fail = kErrIndex;
-                break;
-            }
-            const int4 m = __ldg(reinterpret_cast<const int4*>(meta + st.inode));
-            float2 li, ri;
-            boxes.test(st.inode, m, d, o, li, ri);
-            const bool tl = (li.y >= li.x) && (li.y >= 0.0f) && (li.x <= st.hit_t);
-            const bool tr = (ri.y >= ri.x) && (ri.y >= 0.0f) && (ri.x <= st.hit_t);
-            int32_t inode = m.x;
-            int32_t rnode = m.y;
-            if (tl != tr) {
-                if (tr) inode = rnode;
-            } else if (!tl) {
-                inode = stack[st.sp--];
-            } else {
-                if (ri.x < li.x) {
-                    const int32_t t = inode;
-                    inode = rnode;
-                    rnode = t;
-                }
-                if (st.sp + 1 >= kStack) {
-                    st.fail = kErrStack;
-                    break;
-                }
-                stack[++st.sp] = rnode;
-            }
-            if (inode < 0 && st.leaf >= 0) {
-                searching = false;
-                st.leaf = inode;
-                inode = st.sp >= 0 ? stack[st.sp--] : kSentinel;
-            }
-            st.inode = inode;
-        }
-        // the leaves found (the reference's leaf loop)
-        while (!st.fail && st.leaf < 0) {
-            const uint32_t li = static_cast<uint32_t>(~st.leaf);
-            if (li >= node_count) {
-                st.fail = kErrIndex;
-                break;
-            }
-            const int4 m = __ldg(reinterpret_cast<const int4*>(meta + li));
-            const int32_t num = m.y - m.x;
-            for (int32_t beg = m.x; beg < m.y; ++beg) {
-                uint32_t pid;
-                if (num == 1) {
-                    pid = static_cast<uint32_t>(beg);
-                } else {
-                    if (beg < 0 || static_cast<uint32_t>(beg) >= prim_slots) {
-                        st.fail = kErrIndex;
-                        break;
+            for (;;) {
+                if (next == stop && more) {
+                    uint32_t c = 0;
+                    if (lane == 0) c = atomicAdd(&s_taken, 1u);
+                    c = __shfl_sync(kAll, c, 0);
+                    more = c < own;
+                    if (more) {
+                        const uint64_t first = (static_cast<uint64_t>(c) * gridDim.x + blockIdx.x) * 32u;
+                        next = static_cast<uint32_t>(first);
+                        stop = ray_count - next > 32u ? next + 32u : ray_count;
                     }
-                    pid = __ldg(prims + beg);
                 }
-                if (pid >= face_count) {
-                    st.fail = kErrIndex;
-                    break;
+                const unsigned idle = __ballot_sync(kAll, !busy);
+                if (idle == 0 || next == stop) break;
+                const uint32_t k = __popc(idle & ((1u << lane) - 1u));
+                if (!busy && k < stop - next) {
+                    r = next + k;
+                    busy = true;
+                    const float4* rp = reinterpret_cast<const float4*>(rays + r);
+                    const float4 ra = __ldg(rp), rb = __ldg(rp + 1);
+                    st.o = v3(ra.x, ra.y, ra.z);
+                    st.d = v3(rb.x, rb.y, rb.z);
+                    st.hit_t = rb.w;
+                    st.hit = 0xFFFFFFFFu;
+                    st.b1 = st.b2 = 0.0f;
+                    st.fail = 0;
+                    st.cur = 0;
+                    st.sp = 0;
+                    stack[0] = kSentinel;
                 }
-                const uint4 f = __ldg(reinterpret_cast<const uint4*>(faces + pid));
-                const V3 p1 = vertex(verts, f.x), p2 = vertex(verts, f.y), p3 = vertex(verts, f.z);
-                // kr_ray_triangle_intersect
-                const V3 e1 = sub(p2, p1), e2 = sub(p3, p1);
-                const V3 s1 = cross(d, e2);
-                const float invd = 1.0f / dot(s1, e1);
-                const V3 dd = sub(o, p1);
-                const float c1 = dot(dd, s1) * invd;
-                const V3 s2 = cross(dd, e1);
-                const float c2 = dot(d, s2) * invd;
-                const float t = dot(e2, s2) * invd;
-                const bool miss = c1 < 0.0f || c1 > 1.0f || c2 < 0.0f || c1 + c2 > 1.0f || t < 0.0f || t > st.hit_t;
-                if (!miss && t < st.hit_t) {
-                    st.hit_t = t;
-                    st.hit = pid;
-                    st.b1 = c1;
-                    st.b2 = c2;
-                }
+                next += min(static_cast<uint32_t>(__popc(idle)), stop - next);
             }
-            if (st.fail) break;
-            st.leaf = st.inode;
-            if (st.inode < 0) st.inode = st.sp >= 0 ? stack[st.sp--] : kSentinel;
+            if (!__any_sync(kAll, busy)) break;
         }
-        if (st.fail || st.inode == kSentinel) {
-            finish(st, verts, faces, isects + r, err);
-            busy = false;
+        // nodes, while enough of the lanes with a ray stand at one
+        const int alive = __popc(__ballot_sync(kAll, st.cur != kSentinel));
+        const int enough = max(1, (alive * kNodeLanes) >> 5);
+        for (;;) {
+            const bool at_node = st.cur >= 0 && st.cur != kSentinel;
+            if (__popc(__ballot_sync(kAll, at_node)) < enough) break;
+            if (at_node) visit_node(boxes, meta, internal_count, st, stack);
+            __syncwarp();
         }
+        if (__any_sync(kAll, st.cur < 0))
+            visit_leaves(meta, node_count, verts, faces, face_count, prims, prim_slots, st, stack);
     }
 }
 
@@ -318,7 +474,7 @@ inline unsigned grid_for(uint32_t n) {
         k = 8;
     }
     if (k < 1) k = 1;
-    const unsigned want = (n + kThreads - 1) / kThreads;
+    const unsigned want = n / 32 + (n % 32 != 0);  // a chunk a block at least
     const unsigned cap = static_cast<unsigned>(dev.sm_count) * static_cast<unsigned>(k);
     return want < cap ? (want ? want : 1u) : cap;
 }
@@ -332,11 +488,9 @@ kr_error launch(const Boxes& boxes, const kr_ivec4* meta, uint32_t internal_coun
                 uint32_t prim_slots, const kr_ray* rays, kr_intersection* isects, uint32_t ray_count, uint32_t* err,
                 cudaStream_t s, const char* name) {
     const unsigned g = grid_for<Boxes>(ray_count);
-    const uint64_t warps = static_cast<uint64_t>(g) * (kThreads / 32);
-    const uint32_t per_warp = static_cast<uint32_t>((ray_count + warps - 1) / warps);
     ProfScope prof_scope_(name, s);
     trace_kernel<Boxes><<<g, kThreads, 0, s>>>(boxes, meta, internal_count, node_count, verts, faces, face_count,
-                                               prims, prim_slots, rays, isects, ray_count, per_warp, err);
+                                               prims, prim_slots, rays, isects, ray_count, err);
     OBVH_TRY_CUDA(cudaGetLastError());
     return kr_success;
 }

@@ -74,6 +74,36 @@ def test_traversal_matches_the_oracle(kind, n, collapse):
     assert (g["primitive"] != 0xFFFFFFFF).sum() > 0
 
 
+@pytest.mark.parametrize("count,ci", [(1, 1.2), (31, 1.2), (33, 0.1), (4093, 0.1), (70_001, 1.2)])
+def test_edges_of_warps_leaves_and_slab_ranges(count, ci):
+    """Ray counts around a chunk of 32 and past the grid, leaves of one and of
+    many triangles (a low ci collapses more), and rays whose slabs the
+    reciprocal form cannot decide: zero, denormal, tiny, huge and NaN
+    components, a finite and an infinite tmax."""
+    import torch
+    v, f = workloads.triangle_soup(5003, seed=21)
+    mesh = bvh.Mesh(v, f)
+    n = mesh.n_faces
+    b = bvh.ObvhBuilder()
+    o = b.build(mesh, flags=3, ci=ci)
+    s = bvh.obvh_pack(o["collapsed"], 2 * n - 1, n - 1, o["transforms"])
+    rays = _rays(count, seed=count)
+    odd = np.array([0.0, -0.0, 1e-42, 1e-30, -1e-19, 1e19, 1e30, np.nan, np.inf], np.float32)
+    rng = np.random.default_rng(count)
+    for k in range(0, count, 3):
+        rays["direction"][k, rng.integers(3)] = odd[rng.integers(odd.size)]
+        if k % 2:
+            rays["origin"][k, rng.integers(3)] = odd[rng.integers(odd.size)]
+    rays["tmax"][::5] = rng.uniform(0.0, 1.5, size=rays["tmax"][::5].shape)
+    rays["tmax"][1::7] = np.inf
+    got, err = bvh.soa_obvh_intersect(s, mesh, o["primitives"], _dev_rays(rays), 2 * n - 1, n - 1)
+    torch.cuda.synchronize()
+    lt, rt, meta = _soa_numpy(s, n - 1)
+    want = ref.soa_obvh_intersect(lt, rt, meta, v, f, o["primitives"].cpu().numpy().view(np.uint32), rays, threads=8)
+    assert int(err.item()) == 0
+    assert _isects(got, count).tobytes() == want.tobytes()
+
+
 def test_reference_entry_point_through_the_device_struct():
     """kr_cuda_obvh_persistent -> kr_cuda_soa_obvh -> kr_cuda_soa_obvh_intersect,
     the reference's own call sequence, against the stream form."""
