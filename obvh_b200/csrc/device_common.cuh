@@ -134,31 +134,42 @@ __device__ __forceinline__ bool better_max(float v, uint64_t i, float bv, uint64
     return v > bv || (v == bv && i < bi);
 }
 
-__device__ __forceinline__ void warp_argmin(float& v, uint64_t& i) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        float ov = __shfl_xor_sync(0xffffffffu, v, o);
-        uint64_t oi = __shfl_xor_sync(0xffffffffu, i, o);
-        if (better_min(ov, oi, v, i)) { v = ov; i = oi; }
-    }
-}
-__device__ __forceinline__ void warp_argmax(float& v, uint64_t& i) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        float ov = __shfl_xor_sync(0xffffffffu, v, o);
-        uint64_t oi = __shfl_xor_sync(0xffffffffu, i, o);
-        if (better_max(ov, oi, v, i)) { v = ov; i = oi; }
-    }
-}
+// Warp-wide min / max in one instruction (redux on floats, sm_100a; five
+// shuffle-and-compare steps before).  NaNs are skipped, as fminf skips them.
 __device__ __forceinline__ float warp_min(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
 }
 __device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// The smallest index among the lanes holding the value m.
+__device__ __forceinline__ uint32_t warp_first(bool holds, uint32_t i) {
+    return __reduce_min_sync(0xffffffffu, holds ? i : 0xffffffffu);
+}
+__device__ __forceinline__ uint64_t warp_first(bool holds, uint64_t i) {
+    const uint32_t hi = holds ? static_cast<uint32_t>(i >> 32) : 0xffffffffu;
+    const uint32_t top = __reduce_min_sync(0xffffffffu, hi);
+    return (static_cast<uint64_t>(top) << 32) | warp_first(holds && hi == top, static_cast<uint32_t>(i));
+}
+
+// (value, index) pairs over the warp: no lane's value is NaN.  Two redux
+// steps (three with 64-bit indices) instead of five of shuffles and compares.
+template <class Index>
+__device__ __forceinline__ void warp_argmin(float& v, Index& i) {
+    const float m = warp_min(v);
+    i = warp_first(v == m, i);
+    v = m;
+}
+template <class Index>
+__device__ __forceinline__ void warp_argmax(float& v, Index& i) {
+    const float m = warp_max(v);
+    i = warp_first(v == m, i);
+    v = m;
 }
 
 // Float <-> order-preserving unsigned key, for atomicMin/atomicMax on floats.

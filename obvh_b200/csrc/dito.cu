@@ -153,11 +153,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     // CTA reduction of (value, group) pairs: the first group reaching each extreme.
 #pragma unroll
     for (int k = 0; k < 7; ++k) {
-        uint64_t a = ex.gmn[k], b = ex.gmx[k];
-        warp_argmin(ex.mn[k], a);
-        warp_argmax(ex.mx[k], b);
-        ex.gmn[k] = static_cast<uint32_t>(a);
-        ex.gmx[k] = static_cast<uint32_t>(b);
+        warp_argmin(ex.mn[k], ex.gmn[k]);
+        warp_argmax(ex.mx[k], ex.gmx[k]);
     }
     if (lane == 0) {
 #pragma unroll
@@ -222,21 +219,18 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     }
     named_sync(1, kConsumers);
     if (warp == 0) {
-        CandidateInput in;
-        in.n = sp.n;
-        for (int k = 0; k < 14; ++k) in.val[k] = g_val[k];
-        if (sp.n > 0) {
-            for (int k = 0; k < 14; ++k) {
-                uint64_t i = g_idx[k];
-                if (i >= sp.n) {  // only when no finite projection exists (non-finite input)
-                    if (lane == 0) atomicOr(&ctl->error, kErrBadInput);
-                    i = 0;
-                }
-                const float* p = sp.xyz + 3 * i;
-                in.sel[k] = mk3(p[0], p[1], p[2]);
+        const float val = lane < 14 ? g_val[lane] : 0.f;
+        f3 sel = mk3(0, 0, 0);
+        if (sp.n > 0 && lane < 14) {
+            uint64_t i = g_idx[lane];
+            if (i >= sp.n) {  // only when no finite projection exists (non-finite input)
+                atomicOr(&ctl->error, kErrBadInput);
+                i = 0;
             }
+            const float* p = sp.xyz + 3 * i;
+            sel = mk3(p[0], p[1], p[2]);
         }
-        candidate_warp(in, sp.xyz, flags, ctl, out);
+        candidate_warp(sp.n, val, sel, sp.xyz, flags, ctl, out);
     }
     if (tid == 0) ctl->ticket[0] = 0;
 }

@@ -185,22 +185,16 @@ __device__ uint32_t resolve(const SetView& v, int e, float& val, uint32_t r, boo
 __device__ void candidate_from_lanes(const SetView& v, float val, uint32_t idx, uint32_t flags, Ctl* ctl,
                                      kr_obb3* out, uint32_t* err) {
     const int lane = threadIdx.x & 31;
-    CandidateInput in;
-    in.n = v.n;
-#pragma unroll
-    for (int e = 0; e < 14; ++e) {
-        in.val[e] = __shfl_sync(0xffffffffu, val, e);
-        uint32_t i = __shfl_sync(0xffffffffu, idx, e);
-        if (v.n > 0) {
-            if (i >= v.n) {  // only when no finite projection exists (non-finite input)
-                if (lane == 0) atomicOr(err, kErrBadInput);
-                i = 0;
-            }
-            const float* q = v.base + 3 * static_cast<uint64_t>(i);
-            in.sel[e] = mk3(q[0], q[1], q[2]);
+    f3 sel = mk3(0, 0, 0);
+    if (v.n > 0 && lane < 14) {
+        if (idx >= v.n) {  // only when no finite projection exists (non-finite input)
+            atomicOr(err, kErrBadInput);
+            idx = 0;
         }
+        const float* q = v.base + 3 * static_cast<uint64_t>(idx);
+        sel = mk3(q[0], q[1], q[2]);
     }
-    candidate_warp(in, v.base, flags, ctl, out);
+    candidate_warp(v.n, val, sel, v.base, flags, ctl, out);
 }
 
 struct Shared {
@@ -222,14 +216,13 @@ __device__ void cta_reduce_extremes(Extremes& ex, Shared& sh, float& val, uint32
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 #pragma unroll
     for (int k = 0; k < 7; ++k) {
-        uint64_t a = ex.gmn[k], b = ex.gmx[k];
-        warp_argmin(ex.mn[k], a);
-        warp_argmax(ex.mx[k], b);
+        warp_argmin(ex.mn[k], ex.gmn[k]);
+        warp_argmax(ex.mx[k], ex.gmx[k]);
         if (lane == 0) {
             sh.wval[warp][k] = ex.mn[k];
-            sh.widx[warp][k] = static_cast<uint32_t>(a);
+            sh.widx[warp][k] = ex.gmn[k];
             sh.wval[warp][7 + k] = ex.mx[k];
-            sh.widx[warp][7 + k] = static_cast<uint32_t>(b);
+            sh.widx[warp][7 + k] = ex.gmx[k];
         }
     }
     __syncthreads();
@@ -295,11 +288,10 @@ __device__ void warp_fit(const Params& p, uint32_t s, Ctl* ctl) {
     uint32_t r = kNoIndex;
 #pragma unroll
     for (int k = 0; k < 7; ++k) {
-        uint64_t a = ex.gmn[k], b = ex.gmx[k];
-        warp_argmin(ex.mn[k], a);
-        warp_argmax(ex.mx[k], b);
-        if (lane == k) { val = ex.mn[k]; r = static_cast<uint32_t>(a); }
-        if (lane == 7 + k) { val = ex.mx[k]; r = static_cast<uint32_t>(b); }
+        warp_argmin(ex.mn[k], ex.gmn[k]);
+        warp_argmax(ex.mx[k], ex.gmx[k]);
+        if (lane == k) { val = ex.mn[k]; r = ex.gmn[k]; }
+        if (lane == 7 + k) { val = ex.mx[k]; r = ex.gmx[k]; }
     }
     uint32_t idx = kNoIndex;
     if (lane < 14) idx = resolve(v, lane, val, r, true, true);

@@ -116,12 +116,6 @@ __device__ __forceinline__ void unpack4(const float4& a, const float4& b, const 
     x[3] = c.y; y[3] = c.z; z[3] = c.w;
 }
 
-struct CandidateInput {
-    uint64_t n;
-    float val[14];  // min of slab 0..6, then max of slab 0..6
-    f3 sel[14];     // first point reaching each of them
-};
-
 struct Mode {
     bool gpu;  // OBVH_DITO_REFERENCE_GPU semantics
     // dito.cpp:98-103 multiplies by the reciprocal length; kr_vnormalize3
@@ -170,27 +164,45 @@ __device__ __forceinline__ void store_from_bounds(kr_obb3* out, f3 b0, f3 b1, f3
     store_obb(out, mid, b0, b1, b2, scale3(0.5f, len), clamp);
 }
 
-// min/max of the projections of P[0..np) on dir; strict updates from P[0]
-// as in findExtremalProjs_OneDir (dito.cpp:193-206).
-__device__ __forceinline__ void extent_1d(const f3* P, int np, f3 dir, float& lo, float& hi) {
-    lo = hi = dot3(P[0], dir);
-    for (int i = 1; i < np; ++i) {
-        float q = dot3(P[i], dir);
-        if (q < lo) lo = q;
-        if (q > hi) hi = q;
-    }
+// Lane `src`'s point.
+__device__ __forceinline__ f3 shfl3(f3 p, int src) {
+    return mk3(__shfl_sync(0xffffffffu, p.x, src), __shfl_sync(0xffffffffu, p.y, src),
+               __shfl_sync(0xffffffffu, p.z, src));
+}
+
+// The lane a sequential scan with strict improvement ends at: lane 0 first,
+// a later lane only where its value is larger.  A NaN in lane 0 keeps lane 0,
+// a NaN elsewhere is never taken, equal values (zeros of either sign too) keep
+// the first.
+__device__ __forceinline__ int scan_argmax(float v) {
+    const uint32_t key = v == v ? f2key(v + 0.0f) : 0u;
+    const uint32_t best = __reduce_max_sync(0xffffffffu, key);
+    const int at = __ffs(__ballot_sync(0xffffffffu, key == best)) - 1;
+    return __shfl_sync(0xffffffffu, v, 0) == __shfl_sync(0xffffffffu, v, 0) ? at : 0;
+}
+__device__ __forceinline__ int scan_argmin(float v) {
+    const uint32_t key = v == v ? f2key(v + 0.0f) : 0xffffffffu;
+    const uint32_t best = __reduce_min_sync(0xffffffffu, key);
+    const int at = __ffs(__ballot_sync(0xffffffffu, key == best)) - 1;
+    return __shfl_sync(0xffffffffu, v, 0) == __shfl_sync(0xffffffffu, v, 0) ? at : 0;
 }
 
 // The candidate-axis search of DiTO-14 (dito.cpp:478-528, including
 // findBestObbAxesFromBaseTriangle :347-380 and the di-tetrahedron :382-418).
-// Called by all 32 lanes of one warp.  The sequential parts run redundantly
-// in every lane (uniform values, no divergence); the up to 21 candidate frames
-// are scored in parallel, lane f taking frame f in the reference's evaluation
-// order, and the reference's "strictly better than the best so far" scan is
-// reproduced as an argmin with the lowest frame index winning ties.
+// Called by all 32 lanes of one warp: lane e < 14 holds extreme e (min of slab
+// 0..6, then max of slab 0..6), its value and the first point reaching it.
+// The search is a chain of dependent steps that runs once per set, so what
+// counts is its latency: each scan over the points is one value per lane and
+// a redux, the up to 21 candidate frames are scored by 21 lanes at once, lane
+// f taking frame f in the reference's evaluation order, and the reference's
+// "strictly better than the best so far" scan is an argmin with the lowest
+// frame index winning ties.  No array is indexed at run time.  (With the
+// points in every lane's local memory and the scans run in turn by all lanes,
+// pass 1 of a 4,093-point fit took 21.7 us.)
 // Writes the plan for the extent pass into ctl, or the final box into out.
-inline __device__ void candidate_warp(const CandidateInput& in, const float* xyz, uint32_t flags, Ctl* ctl,
-                               kr_obb3* out) {
+inline __device__ void candidate_warp(uint64_t n, float val, f3 sel, const float* xyz, uint32_t flags, Ctl* ctl,
+                                      kr_obb3* out) {
+    constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const Mode md{(flags & OBVH_DITO_REFERENCE_GPU) != 0};
     const bool clamp = !md.gpu;
@@ -209,36 +221,35 @@ inline __device__ void candidate_warp(const CandidateInput& in, const float* xyz
     };
     const f3 I0 = mk3(1, 0, 0), I1 = mk3(0, 1, 0), I2 = mk3(0, 0, 1);
 
-    if (in.n == 0) {
+    if (n == 0) {
         if (lane == 0) store_aabb(out, mk3(0, 0, 0), mk3(0, 0, 0), clamp);
         publish(0, 0, I0, I1, I2, mk3(0, 0, 0), mk3(0, 0, 0), 0.f);
         return;
     }
 
     // AABB from slabs 0..2 (dito.cpp:507-510)
-    const f3 al_mid = mk3((in.val[0] + in.val[7]) * 0.5f, (in.val[1] + in.val[8]) * 0.5f, (in.val[2] + in.val[9]) * 0.5f);
-    const f3 al_len = mk3(in.val[7] - in.val[0], in.val[8] - in.val[1], in.val[9] - in.val[2]);
+    const f3 lo3 = mk3(__shfl_sync(kAll, val, 0), __shfl_sync(kAll, val, 1), __shfl_sync(kAll, val, 2));
+    const f3 hi3 = mk3(__shfl_sync(kAll, val, 7), __shfl_sync(kAll, val, 8), __shfl_sync(kAll, val, 9));
+    const f3 al_mid = mk3((lo3.x + hi3.x) * 0.5f, (lo3.y + hi3.y) * 0.5f, (lo3.z + hi3.z) * 0.5f);
+    const f3 al_len = sub3(hi3, lo3);
     const float al_val = half_area3(al_len);
 
-    // Selection set: the 14 extremal points, or every point when there are few.
-    f3 P[14];
-    int np;
-    if (in.n > 14) {
-        np = 14;
-        for (int k = 0; k < 14; ++k) P[k] = in.sel[k];
-    } else {
-        np = static_cast<int>(in.n);
-        for (int k = 0; k < np; ++k) P[k] = mk3(xyz[3 * k], xyz[3 * k + 1], xyz[3 * k + 2]);
+    // Selection set, a point per lane: the 14 extremal points, or every point
+    // when there are few; the lanes past it repeat its first point, which
+    // changes no extent and never wins a tie.
+    const int np = n > 14 ? 14 : static_cast<int>(n);
+    f3 P = sel;
+    if (n <= 14 && lane < np) P = mk3(xyz[3 * lane], xyz[3 * lane + 1], xyz[3 * lane + 2]);
+    {
+        const f3 p = shfl3(P, 0);
+        if (lane >= np) P = p;
     }
 
-    // Furthest (min, max) pair (dito.cpp:280-292)
-    int far = 0;
-    float far_d = len2_3(sub3(in.sel[0], in.sel[7]));
-    for (int k = 1; k < 7; ++k) {
-        float d = len2_3(sub3(in.sel[k], in.sel[7 + k]));
-        if (d > far_d) { far_d = d; far = k; }
-    }
-    const f3 p0 = in.sel[far], p1 = in.sel[7 + far];
+    // Furthest (min, max) pair (dito.cpp:280-292); lanes 7.. repeat pair 0
+    const f3 other = shfl3(sel, lane < 7 ? lane + 7 : 7);
+    const f3 first = shfl3(sel, lane < 7 ? lane : 0);
+    const int far = scan_argmax(len2_3(sub3(first, other)));
+    const f3 p0 = shfl3(sel, far), p1 = shfl3(sel, 7 + far);
     if (len2_3(sub3(p1, p0)) < eps) {
         if (lane == 0) store_aabb(out, al_mid, al_len, clamp);
         publish(1, 0, I0, I1, I2, al_mid, al_len, al_val);
@@ -247,22 +258,12 @@ inline __device__ void candidate_warp(const CandidateInput& in, const float* xyz
     const f3 e0 = md.unit(sub3(p0, p1));
 
     // Point furthest from the line through p0 along e0 (dito.cpp:230-258)
-    int far2 = 0;
-    float far2_d;
-    {
-        const float l2 = len2_3(e0);
-        f3 u = sub3(P[0], p0);
-        float t = dot3(e0, u);
-        far2_d = len2_3(u) - t * t / l2;
-        for (int i = 1; i < np; ++i) {
-            u = sub3(P[i], p0);
-            t = dot3(e0, u);
-            float d = len2_3(u) - t * t / l2;
-            if (d > far2_d) { far2_d = d; far2 = i; }
-        }
-    }
-    const f3 p2 = P[far2];
-    if (far2_d < eps) {
+    const f3 u = sub3(P, p0);
+    const float along = dot3(e0, u);
+    const float from_line = len2_3(u) - along * along / len2_3(e0);
+    const int far2 = scan_argmax(from_line);
+    const f3 p2 = shfl3(P, far2);
+    if (__shfl_sync(kAll, from_line, far2) < eps) {
         if (md.gpu) {
             if (lane == 0) store_aabb(out, al_mid, al_len, clamp);
             publish(2, 0, I0, I1, I2, al_mid, al_len, al_val);
@@ -285,57 +286,52 @@ inline __device__ void candidate_warp(const CandidateInput& in, const float* xyz
     const f3 nb = md.unit(md.cross(e1, e0));
 
     // Di-tetrahedron apexes (dito.cpp:294-307)
-    f3 q0 = P[0], q1 = P[0];
-    float qlo = dot3(P[0], nb), qhi = qlo;
-    for (int i = 1; i < np; ++i) {
-        float q = dot3(P[i], nb);
-        if (q < qlo) { qlo = q; q1 = P[i]; }
-        if (q > qhi) { qhi = q; q0 = P[i]; }
-    }
+    const float height = dot3(P, nb);
+    const int top = scan_argmax(height), bottom = scan_argmin(height);
+    const f3 q0 = shfl3(P, top), q1 = shfl3(P, bottom);
+    const float qhi = __shfl_sync(kAll, height, top), qlo = __shfl_sync(kAll, height, bottom);
     const float tri = dot3(p0, nb);
     const bool up = (qhi - eps > tri);
     const bool down = (qlo + eps < tri);
 
-    // Frames in the reference's evaluation order: triangle t = lane/3, edge lane%3.
-    const int t = lane / 3, k = lane % 3;
-    bool valid = false;
-    f3 tn = nb, te = e0;
-    if (lane < 21) {
-        if (t == 0) {
-            valid = true;
-            tn = nb;
-            te = k == 0 ? e0 : (k == 1 ? e1 : e2);
-        } else if (t <= 3 && up) {
-            const f3 f0 = md.unit(sub3(q0, p0)), f1 = md.unit(sub3(q0, p1)), f2 = md.unit(sub3(q0, p2));
-            valid = true;
-            if (t == 1) { tn = md.unit(md.cross(f1, e0)); te = k == 0 ? e0 : (k == 1 ? f1 : f0); }
-            else if (t == 2) { tn = md.unit(md.cross(f2, e1)); te = k == 0 ? e1 : (k == 1 ? f2 : f1); }
-            else { tn = md.unit(md.cross(f0, e2)); te = k == 0 ? e2 : (k == 1 ? f0 : f2); }
-        } else if (t >= 4 && down) {
-            const f3 g0 = md.unit(sub3(q1, p0)), g1 = md.unit(sub3(q1, p1)), g2 = md.unit(sub3(q1, p2));
-            valid = true;
-            if (t == 4) { tn = md.unit(md.cross(g1, e0)); te = k == 0 ? e0 : (k == 1 ? g1 : g0); }
-            else if (t == 5) { tn = md.unit(md.cross(g2, e1)); te = k == 0 ? e1 : (k == 1 ? g2 : g1); }
-            else { tn = md.unit(md.cross(g0, e2)); te = k == 0 ? e2 : (k == 1 ? g0 : g2); }
-        }
-    }
+    // Frames in the reference's evaluation order: triangle t = lane/3, edge
+    // k = lane%3.  Triangle 0 is the base (edges e0 e1 e2); triangle 1 + r has
+    // the upper apex, 4 + r the lower one, the base edge e_r, the apex edges
+    // a_{r+1} and a_r (a_i = unit(apex - p_i)) and the normal
+    // unit(a_{r+1} x e_r).  All lanes run the same instructions.
+    const int t = lane / 3, k = lane - 3 * t;
+    const bool lower = t >= 4;
+    const int r = t == 0 ? k : (lower ? t - 4 : t - 1);
+    const f3 er = r == 0 ? e0 : (r == 1 ? e1 : e2);
+    const f3 from0 = r == 0 ? p0 : (r == 1 ? p1 : p2);
+    const f3 from1 = r == 0 ? p1 : (r == 1 ? p2 : p0);
+    const f3 apex = lower ? q1 : q0;
+    const f3 a0 = md.unit(sub3(apex, from0)), a1 = md.unit(sub3(apex, from1));
+    const f3 na = md.unit(md.cross(a1, er));
+    const f3 tn = t == 0 ? nb : na;
+    const f3 te = t == 0 || k == 0 ? er : (k == 1 ? a1 : a0);
     const f3 tm = md.cross(te, tn);
-    float key = kInf;  // +inf: not a candidate
-    if (valid) {
-        float nlo, nhi, elo, ehi, mlo, mhi;
-        extent_1d(P, np, tn, nlo, nhi);
-        extent_1d(P, np, te, elo, ehi);
-        extent_1d(P, np, tm, mlo, mhi);
-        float q = half_area3(mk3(ehi - elo, nhi - nlo, mhi - mlo));
-        if (!(q != q)) key = q;  // NaN never wins (the reference's strict '<' skips it)
+    const bool valid = lane < 21 && (t == 0 || (lower ? down : up));
+
+    // Extents of the selection set along the three axes.  The reference's scan
+    // keeps a NaN of the first point, and such a frame never wins.
+    float nlo = kInf, nhi = -kInf, elo = kInf, ehi = -kInf, mlo = kInf, mhi = -kInf;
+    bool clean = true;
+#pragma unroll
+    for (int i = 0; i < 14; ++i) {
+        const f3 p = shfl3(P, i);
+        const float qn = dot3(p, tn), qe = dot3(p, te), qm = dot3(p, tm);
+        if (i == 0) clean = qn == qn && qe == qe && qm == qm;
+        nlo = fminf(nlo, qn); nhi = fmaxf(nhi, qn);
+        elo = fminf(elo, qe); ehi = fmaxf(ehi, qe);
+        mlo = fminf(mlo, qm); mhi = fmaxf(mhi, qm);
     }
-    uint64_t who = static_cast<uint64_t>(lane);
+    const float q = half_area3(mk3(ehi - elo, nhi - nlo, mhi - mlo));
+    float key = valid && clean && q == q ? q : kInf;  // +inf: not a candidate (NaN never wins a strict '<')
+    uint32_t who = static_cast<uint32_t>(lane);
     warp_argmin(key, who);
     const int src = static_cast<int>(who);
-    f3 b0, b1, b2;
-    b0.x = __shfl_sync(0xffffffffu, te.x, src); b0.y = __shfl_sync(0xffffffffu, te.y, src); b0.z = __shfl_sync(0xffffffffu, te.z, src);
-    b1.x = __shfl_sync(0xffffffffu, tn.x, src); b1.y = __shfl_sync(0xffffffffu, tn.y, src); b1.z = __shfl_sync(0xffffffffu, tn.z, src);
-    b2.x = __shfl_sync(0xffffffffu, tm.x, src); b2.y = __shfl_sync(0xffffffffu, tm.y, src); b2.z = __shfl_sync(0xffffffffu, tm.z, src);
+    const f3 b0 = shfl3(te, src), b1 = shfl3(tn, src), b2 = shfl3(tm, src);
 
     if (!(key < al_val)) {
         // No frame beats the AABB: its projections give the AABB back exactly,
