@@ -20,9 +20,13 @@
 // transactions; threads then read whole 4-point groups (3 x 16 B) from shared
 // memory without bank conflicts.  Pass 2 walks each CTA's slice backwards so
 // that the tail of pass 1, still in the 126 MB L2, is consumed first.
+//
+// Fits of up to 262,144 points run both passes in one launch of one
+// thread-block cluster instead (dito_cluster_fit).
 #include <cuda_runtime.h>
 
 #include <cfloat>
+#include <cstddef>
 #include <cstdint>
 #include <cstring>
 #include <mutex>
@@ -325,6 +329,172 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 }
 
 // ---------------------------------------------------------------------------
+// A whole fit in one launch, by one thread-block cluster of 1, 2, 4 or 8 CTAs
+// (the fits of up to kClusterMaxPoints points).
+//
+// At these sizes the two-launch form above is all latency: a second launch, a
+// ticket and per-CTA records through global memory in each pass.  Here CTA r
+// of the cluster scans groups [G r / size, G (r + 1) / size), writes its 14
+// extremes into every CTA's shared memory, and after a cluster barrier every
+// CTA runs the same merge and candidate search by itself, so the frame needs
+// no broadcast; the extents go to CTA 0, which writes the box.  The points are
+// read from global memory; the second pass finds them in L1.
+constexpr int kClusterThreads = 512;
+constexpr int kClusterWarps = kClusterThreads / 32;
+constexpr int kClusterMax = 8;  // the portable cluster size
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t cluster_size() {
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// Stores to the same shared-memory variable of CTA `rank`.
+__device__ __forceinline__ void cluster_store(uint32_t* at, uint32_t rank, uint32_t v) {
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(at)), "r"(rank));
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote), "r"(v) : "memory");
+}
+
+struct ClusterShared {
+    float wval[kClusterWarps][14];
+    uint32_t widx[kClusterWarps][14];
+    uint32_t val[kClusterMax][14];  // float bits, from every CTA of the cluster
+    uint32_t idx[kClusterMax][14];
+    float wlohi[kClusterWarps][6];
+    uint32_t lohi[kClusterMax][6];
+    Ctl ctl;
+    kr_obb3 spare;
+};
+
+__global__ void __launch_bounds__(kClusterThreads)
+    dito_cluster_fit(const float* xyz, uint32_t n, char* ws, kr_obb3* out, uint32_t flags) {
+    __shared__ ClusterShared sh;
+    cluster_arrive();  // matched before the first remote store: every CTA of the cluster has started
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t rank = cluster_rank(), size = cluster_size();
+    Ctl* ctl = reinterpret_cast<Ctl*>(ws);
+    const SetView v = view_of(xyz, n);
+    const uint32_t g0 = static_cast<uint32_t>(static_cast<uint64_t>(v.groups) * rank / size);
+    const uint32_t g1 = static_cast<uint32_t>(static_cast<uint64_t>(v.groups) * (rank + 1) / size);
+    const bool with_head = rank == 0, with_tail = rank == size - 1;
+
+    Extremes ex;
+    ex.init();
+    scan_extremes<2>(v, g0, g1, tid, kClusterThreads, ex);
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+        warp_argmin(ex.mn[k], ex.gmn[k]);
+        warp_argmax(ex.mx[k], ex.gmx[k]);
+        if (lane == 0) {
+            sh.wval[warp][k] = ex.mn[k];
+            sh.widx[warp][k] = ex.gmn[k];
+            sh.wval[warp][7 + k] = ex.mx[k];
+            sh.widx[warp][7 + k] = ex.gmx[k];
+        }
+    }
+    __syncthreads();
+    cluster_wait();
+    if (tid < 14) {
+        float val = sh.wval[0][tid];
+        uint32_t r = sh.widx[0][tid];
+        for (int w = 1; w < kClusterWarps; ++w) {
+            const float ov = sh.wval[w][tid];
+            const uint32_t orr = sh.widx[w][tid];
+            if (tid < 7 ? better_min(ov, orr, val, r) : better_max(ov, orr, val, r)) { val = ov; r = orr; }
+        }
+        const uint32_t i = resolve(v, tid, val, r, with_head, with_tail);
+        for (uint32_t c = 0; c < size; ++c) {
+            cluster_store(&sh.val[rank][tid], c, __float_as_uint(val));
+            cluster_store(&sh.idx[rank][tid], c, i);
+        }
+    }
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    if (warp == 0) {
+        float val = 0.f;
+        f3 sel = mk3(0, 0, 0);
+        if (lane < 14) {
+            uint32_t i = sh.idx[0][lane];
+            val = __uint_as_float(sh.val[0][lane]);
+            for (uint32_t c = 1; c < size; ++c) {
+                const float ov = __uint_as_float(sh.val[c][lane]);
+                const uint32_t oi = sh.idx[c][lane];
+                if (lane < 7 ? better_min(ov, oi, val, i) : better_max(ov, oi, val, i)) { val = ov; i = oi; }
+            }
+            if (n > 0) {
+                if (i >= n) {  // only when no finite projection exists (non-finite input)
+                    if (rank == 0) atomicOr(&ctl->error, kErrBadInput);
+                    i = 0;
+                }
+                const float* p = v.base + 3ull * i;
+                sel = mk3(p[0], p[1], p[2]);
+            }
+        }
+        candidate_warp(n, val, sel, v.base, flags, &sh.ctl, rank == 0 ? out : &sh.spare);
+    }
+    __syncthreads();
+    if (sh.ctl.plan != 0) {
+        Extents e2;
+        e2.init(sh.ctl.axes);
+        scan_extents<2>(v, g0, g1, tid, kClusterThreads, e2);
+        if (with_head && static_cast<uint32_t>(tid) < v.head) {
+            const float* q = v.base + 3 * tid;
+            e2.point(q[0], q[1], q[2]);
+        }
+        if (with_tail && static_cast<uint32_t>(tid) < n - v.tail0()) {
+            const float* q = v.base + 3ull * (v.tail0() + tid);
+            e2.point(q[0], q[1], q[2]);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            e2.lo[k] = warp_min(e2.lo[k]);
+            e2.hi[k] = warp_max(e2.hi[k]);
+        }
+        if (lane == 0)
+            for (int k = 0; k < 3; ++k) {
+                sh.wlohi[warp][k] = e2.lo[k];
+                sh.wlohi[warp][3 + k] = e2.hi[k];
+            }
+        __syncthreads();
+        if (tid < 6) {
+            float m = sh.wlohi[0][tid];
+            for (int w = 1; w < kClusterWarps; ++w) m = tid < 3 ? fminf(m, sh.wlohi[w][tid]) : fmaxf(m, sh.wlohi[w][tid]);
+            cluster_store(&sh.lohi[rank][tid], 0, __float_as_uint(m));
+        }
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        if (rank == 0 && warp == 0) {
+            float m = lane < 3 ? kInf : -kInf;
+            if (lane < 6)
+                for (uint32_t c = 0; c < size; ++c) {
+                    const float o = __uint_as_float(sh.lohi[c][lane]);
+                    m = lane < 3 ? fminf(m, o) : fmaxf(m, o);
+                }
+            float lohi[6];
+#pragma unroll
+            for (int k = 0; k < 6; ++k) lohi[k] = __shfl_sync(0xffffffffu, m, k);
+            if (lane == 0) finalize_extents(&sh.ctl, lohi, flags, out);
+            __syncwarp();
+        }
+    }
+    // the report (obvh_dito_workspace_report): everything but tickets and error word
+    if (rank == 0 && warp == 0) {
+        constexpr int kFirst = offsetof(Ctl, path) / 4, kLast = offsetof(Ctl, pad2) / 4;
+        if (kFirst + lane < kLast)
+            reinterpret_cast<uint32_t*>(ctl)[kFirst + lane] = reinterpret_cast<const uint32_t*>(&sh.ctl)[kFirst + lane];
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Host side.
 
 int grid_for(const Split& sp) {
@@ -351,12 +521,42 @@ kr_error configure_once() {
     return status == cudaSuccess ? kr_success : cuda_error(status);
 }
 
+// One launch up to kClusterMaxPoints, with a CTA per kClusterCtaPoints (8 at
+// most).  Measured (us a fit, two launches / one): 300 points 19.6 / 12.3,
+// 4,093 20.5 / 12.4, 30,011 21.6 / 14.8, 120,011 23.6 / 18.7, 200,011 26.7 /
+// 22.6, 300,011 26.7 / 26.7, 500,011 32.8 / 34.9: past a quarter million the
+// 296 CTAs of the two-launch form win.  Points per CTA at 16,111 points: 2,048
+// 14.4, 8,192 16.4, 16,384 19.1.
+constexpr uint64_t kClusterMaxPoints = 262144;
+constexpr uint64_t kClusterCtaPoints = 2048;
+
+kr_error enqueue_cluster(const kr_vec3* d_points, uint64_t count, uint32_t flags, kr_obb3* d_obb, void* ws,
+                         cudaStream_t stream) {
+    unsigned size = 1;
+    while (size < kClusterMax && size * kClusterCtaPoints < count) size *= 2;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = size;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(size);
+    cfg.blockDim = dim3(kClusterThreads);
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    ProfScope prof_scope_("dito_cluster_fit", stream);
+    OBVH_TRY_CUDA(cudaLaunchKernelEx(&cfg, dito_cluster_fit, reinterpret_cast<const float*>(d_points),
+                                     static_cast<uint32_t>(count), static_cast<char*>(ws), d_obb, flags));
+    return kr_success;
+}
+
 kr_error enqueue(const kr_vec3* d_points, uint64_t count, uint32_t flags, kr_obb3* d_obb, void* ws,
                  cudaStream_t stream, int passes) {
     if (!ws || !d_obb || (count > 0 && !d_points)) return "obvh_dito: null pointer argument";
     if (reinterpret_cast<uintptr_t>(d_points) & 3u) return "obvh_dito: points must be 4-byte aligned";
     if (reinterpret_cast<uintptr_t>(ws) & 255u) return "obvh_dito: workspace must be 256-byte aligned";
     OBVH_TRY(configure_once());
+    if (passes == 3 && count <= kClusterMaxPoints) return enqueue_cluster(d_points, count, flags, d_obb, ws, stream);
     Split sp = make_split(reinterpret_cast<const float*>(d_points), count);
     int grid = grid_for(sp);
     if (passes & 1) {

@@ -116,6 +116,104 @@ __device__ __forceinline__ void unpack4(const float4& a, const float4& b, const 
     x[3] = c.y; y[3] = c.z; z[3] = c.w;
 }
 
+// ---------------------------------------------------------------------------
+// A set of fewer than 2^32 points read straight from global memory (the batched
+// and the one-launch fits).
+constexpr uint32_t kNoIndex = 0xffffffffu;
+
+// One set: its points, and the split into an unaligned head (< 4 points), a
+// body of 16-byte-aligned 4-point groups and a tail.
+struct SetView {
+    const float* base;
+    uint32_t n, head, groups;
+    __device__ uint32_t tail0() const { return head + 4 * groups; }
+};
+
+__device__ __forceinline__ SetView view_of(const float* base, uint32_t n) {
+    SetView v;
+    v.base = base;
+    v.n = n;
+    // A point is 12 bytes: base misaligned by 4*m bytes becomes aligned after m points.
+    const uint32_t m = static_cast<uint32_t>((reinterpret_cast<uintptr_t>(v.base) & 15u) >> 2);
+    v.head = m < v.n ? m : v.n;
+    v.groups = (v.n - v.head) / 4;
+    return v;
+}
+
+__device__ __forceinline__ void load_group(const SetView& v, uint32_t g, float* x, float* y, float* z) {
+    const float4* q = reinterpret_cast<const float4*>(v.base + 3 * (v.head + 4ull * g));
+    unpack4(q[0], q[1], q[2], x, y, z);
+}
+
+// Groups g0 + t, g0 + t + stride, ... below g1, in increasing order, U at a
+// time (U groups' loads issued before any is used).
+template <int U>
+__device__ __forceinline__ void scan_extremes(const SetView& v, uint32_t g0, uint32_t g1, uint32_t t,
+                                              uint32_t stride, Extremes& ex) {
+    uint32_t g = g0 + t;
+    for (; g + (U - 1) * stride < g1; g += U * stride) {
+        float x[4 * U], y[4 * U], z[4 * U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) load_group(v, g + u * stride, x + 4 * u, y + 4 * u, z + 4 * u);
+#pragma unroll
+        for (int u = 0; u < U; ++u) ex.group(x + 4 * u, y + 4 * u, z + 4 * u, 4 * (g + u * stride));
+    }
+    for (; g < g1; g += stride) {
+        float x[4], y[4], z[4];
+        load_group(v, g, x, y, z);
+        ex.group(x, y, z, 4 * g);
+    }
+}
+
+template <int U>
+__device__ __forceinline__ void scan_extents(const SetView& v, uint32_t g0, uint32_t g1, uint32_t t, uint32_t stride,
+                                             Extents& ex) {
+    uint32_t g = g0 + t;
+    for (; g + (U - 1) * stride < g1; g += U * stride) {
+        float x[4 * U], y[4 * U], z[4 * U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) load_group(v, g + u * stride, x + 4 * u, y + 4 * u, z + 4 * u);
+#pragma unroll
+        for (int j = 0; j < 4 * U; ++j) ex.point(x[j], y[j], z[j]);
+    }
+    for (; g < g1; g += stride) {
+        float x[4], y[4], z[4];
+        load_group(v, g, x, y, z);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) ex.point(x[j], y[j], z[j]);
+    }
+}
+
+// Extreme e (0..6 min of slab e, 7..13 max of slab e-7): from the first
+// 4-point group reaching `val` (body offset r of its first point) to the first
+// point reaching it, then merged with the head points (which precede the
+// body) and the tail points (which follow it) when asked.
+inline __device__ uint32_t resolve(const SetView& v, int e, float& val, uint32_t r, bool with_head, bool with_tail) {
+    const int k = e < 7 ? e : e - 7;
+    const bool is_min = e < 7;
+    uint64_t best = ~0ull;
+    if (r != kNoIndex) {
+        for (int j = 3; j >= 0; --j) {
+            const float* q = v.base + 3 * (static_cast<uint64_t>(v.head) + r + j);
+            if (slab(k, q[0], q[1], q[2]) == val) best = v.head + r + j;
+        }
+    }
+    auto merge = [&](uint32_t i) {
+        const float* q = v.base + 3 * static_cast<uint64_t>(i);
+        const float s = slab(k, q[0], q[1], q[2]);
+        const bool b = is_min ? better_min(s, i, val, best) : better_max(s, i, val, best);
+        if (b) {
+            val = s;
+            best = i;
+        }
+    };
+    if (with_head)
+        for (uint32_t i = 0; i < v.head; ++i) merge(i);
+    if (with_tail)
+        for (uint32_t i = v.tail0(); i < v.n; ++i) merge(i);
+    return best == ~0ull ? kNoIndex : static_cast<uint32_t>(best);
+}
+
 struct Mode {
     bool gpu;  // OBVH_DITO_REFERENCE_GPU semantics
     // dito.cpp:98-103 multiplies by the reciprocal length; kr_vnormalize3

@@ -74,6 +74,36 @@ def test_sizes_around_tile_boundaries(torch, fitter, n):
     assert obb_contains(pts, out) == 0
 
 
+@pytest.mark.parametrize("n", [1, 14, 2048, 2049, 4097, 8192, 8193, 16385, 65536, 262144, 262145])
+@pytest.mark.parametrize("kind", ["cloud", "lattice", "nan"])
+def test_one_launch_fit_at_its_limits(torch, fitter, n, kind):
+    """Sizes around the cluster sizes (1, 2, 4, 8 CTAs) and the largest one-launch
+    fit, every alignment, ties that several CTAs share, NaN points after the
+    first; the two-launch form (by passes) gives the same box and report."""
+    rng = np.random.default_rng(n)
+    if kind == "lattice":
+        pts = rng.integers(-3, 4, size=(n, 3)).astype(np.float32)
+    else:
+        pts = (rng.normal(size=(n, 3)) * rng.uniform(0.1, 10, size=3) + rng.uniform(-9, 9, size=3)).astype(np.float32)
+    if kind == "nan" and n > 14:
+        pts[rng.integers(1, n, size=n // 7 + 1), rng.integers(3)] = np.nan
+    for pad in (0, 1, 2, 3):
+        out = _device_fit(torch, fitter, pts, pad=pad)
+        report = fitter.report()
+        if kind != "nan":
+            want, _, path = oracle.dito14(pts)
+            assert same_bits(out, want), (n, kind, pad)
+            assert report[0] == path and report[2] == 0
+        buf = torch.zeros((n + pad + 1, 3), dtype=torch.float32, device="cuda")
+        buf[pad:pad + n] = torch.from_numpy(pts).cuda()
+        two = torch.empty(15, dtype=torch.float32, device="cuda")
+        for p in (1, 2):
+            fitter.fit_pass(buf[pad:pad + n], two, p)
+        assert same_bits(out, two.cpu().numpy()), (n, kind, pad)
+        again = fitter.report()
+        assert again[0] == report[0] and again[2] == report[2] and same_bits(again[1], report[1])
+
+
 def test_first_index_ties_on_lattice(torch, fitter):
     """Millions of ties: the argmin/argmax must pick the first point like the CPU scan."""
     rng = np.random.default_rng(7)
