@@ -16,8 +16,8 @@
 //   6 bottom-up pass from every leaf (walk_up of the whole-GPU chain: bounds,
 //     costs, collapse marks, 7-direction summaries)
 //   7 candidate frames of the internal nodes
-//   8 extents over each node's leaf run (a thread per node of at most 32
-//     leaves, a warp per larger node) and the final boxes
+//   8 extents over each node's leaf run (a thread, 8 lanes or a warp by its
+//     size) and the final boxes
 //   9 collapse: roots, block scan of their sizes, primitive lists
 // Every per-element formula is the chain's own device code (lbvh_device.cuh,
 // up_device.cuh, tree_device.cuh, obb_device.cuh); results are the chain's
@@ -59,7 +59,6 @@ constexpr int kWarps = kThreads / 32;
 constexpr int kSmemCarveout = 32;
 constexpr uint32_t kMaxFaces = OBVH_BUILD_BATCH_CTA_MAX_FACES;
 constexpr uint32_t kMaxRounds = kMaxFaces / kThreads;  // sort rounds of kThreads keys
-constexpr uint32_t kThreadLeaves = 32;                  // extents: one thread per node up to this many leaves
 static_assert(kMaxFaces % kThreads == 0, "whole sort rounds");
 static_assert(kMaxFaces <= 65535, "sort ranks are 16-bit");
 
@@ -429,35 +428,57 @@ __device__ void build_mesh(const Args& a, const Job& J, char* slot, Smem& sm) {
         stage_sync();
 
         // ---- 8: extents over each node's leaf run; final boxes ---------------
-        for (uint32_t i = t; i < ni; i += kThreads) {
-            const uint32_t cnt = ld_own(counts + i);
-            if (cnt > kThreadLeaves) continue;
-            const obbtree::Cand c = load_cand_own(cand, i);
-            const obbtree::Axes ax = obbtree::make_axes(mk3(c.ax[0], c.ax[1], c.ax[2]), mk3(c.ax[3], c.ax[4], c.ax[5]),
-                                                        mk3(c.ax[6], c.ax[7], c.ax[8]), a.nz);
-            float lo[3] = {c.olo[0], c.olo[1], c.olo[2]}, hi[3] = {c.ohi[0], c.ohi[1], c.ohi[2]};
-            const float* tp = tris + 9 * static_cast<size_t>(ld_own(first + i));
-#pragma unroll 4
-            for (uint32_t k = 0; k < cnt; ++k) obbtree::project_tri_own(tp + 9 * k, ax, lo, hi);
-            obbtree::finalize_node(c, mk3(lo[0], lo[1], lo[2]), mk3(hi[0], hi[1], hi[2]), obbs + i, xfs + i);
-        }
-        for (uint32_t i = w; i < ni; i += kWarps) {
-            const uint32_t cnt = ld_own(counts + i);
-            if (cnt <= kThreadLeaves) continue;
-            const obbtree::Cand c = load_cand_own(cand, i);
-            const obbtree::Axes ax = obbtree::make_axes(mk3(c.ax[0], c.ax[1], c.ax[2]), mk3(c.ax[3], c.ax[4], c.ax[5]),
-                                                        mk3(c.ax[6], c.ax[7], c.ax[8]), a.nz);
-            float lo[3] = {kInf, kInf, kInf}, hi[3] = {-kInf, -kInf, -kInf};
-            const float* tp = tris + 9 * static_cast<size_t>(ld_own(first + i));
-#pragma unroll 4
-            for (uint32_t k = lane; k < cnt; k += 32) obbtree::project_tri_own(tp + 9 * k, ax, lo, hi);
+        // (kSoloLeaves) The larger nodes' extents are folded into their
+        // candidate records; every box is then built by a thread of its own.
+        const auto fold = [&](uint32_t i, const float* lo, const float* hi) {
+            obbtree::Cand& c = cand[i];
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                lo[k] = fminf(c.olo[k], warp_min(lo[k]));
-                hi[k] = fmaxf(c.ohi[k], warp_max(hi[k]));
+                c.olo[k] = fminf(c.olo[k], lo[k]);
+                c.ohi[k] = fmaxf(c.ohi[k], hi[k]);
             }
-            if (lane == 0)
-                obbtree::finalize_node(c, mk3(lo[0], lo[1], lo[2]), mk3(hi[0], hi[1], hi[2]), obbs + i, xfs + i);
+        };
+        for (uint32_t i0 = 4 * w; i0 < ni; i0 += 4 * kWarps) {
+            // a warp looks at 4 nodes at a time: 8 lanes for each of a size for a group ...
+            const uint32_t i = min(i0 + (lane >> 3), ni - 1);
+            const uint32_t cnt = i0 + (lane >> 3) < ni ? ld_own(counts + i) : 0u;
+            const bool group = cnt > obbtree::kSoloLeaves && cnt <= obbtree::kGroupLeaves;
+            if (__any_sync(0xffffffffu, group)) {
+                const obbtree::Axes ax = obbtree::cand_axes(load_cand_own(cand, i), a.nz);
+                float lo[3], hi[3];
+                obbtree::group_extents<obbtree::From::kShared>(tris + 9 * static_cast<size_t>(ld_own(first + i)),
+                                                              group ? cnt : 0u, ax, lo, hi);
+                if (group && (lane & 7) == 0) fold(i, lo, hi);
+            }
+            // ... then all 32 for each larger one
+            for (uint32_t big = __ballot_sync(0xffffffffu, cnt > obbtree::kGroupLeaves) & 0x01010101u; big; big &= big - 1) {
+                const uint32_t g = i0 + ((__ffs(big) - 1) >> 3), gc = ld_own(counts + g);
+                const obbtree::Axes ax = obbtree::cand_axes(load_cand_own(cand, g), a.nz);
+                float lo[3] = {kInf, kInf, kInf}, hi[3] = {-kInf, -kInf, -kInf};
+                const float* tp = tris + 9 * static_cast<size_t>(ld_own(first + g));
+#pragma unroll 4
+                for (uint32_t k = lane; k < gc; k += 32) obbtree::project_tri_own(tp + 9 * k, ax, lo, hi);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    lo[k] = warp_min(lo[k]);
+                    hi[k] = warp_max(hi[k]);
+                }
+                if (lane == 0) fold(g, lo, hi);
+                __syncwarp();
+            }
+        }
+        stage_sync();
+        for (uint32_t i = t; i < ni; i += kThreads) {
+            const uint32_t cnt = ld_own(counts + i);
+            const obbtree::Cand c = load_cand_own(cand, i);
+            float lo[3] = {c.olo[0], c.olo[1], c.olo[2]}, hi[3] = {c.ohi[0], c.ohi[1], c.ohi[2]};
+            if (cnt <= obbtree::kSoloLeaves) {
+                const obbtree::Axes ax = obbtree::cand_axes(c, a.nz);
+                const float* tp = tris + 9 * static_cast<size_t>(ld_own(first + i));
+#pragma unroll 4
+                for (uint32_t k = 0; k < cnt; ++k) obbtree::project_tri_own(tp + 9 * k, ax, lo, hi);
+            }
+            obbtree::finalize_node(c, mk3(lo[0], lo[1], lo[2]), mk3(hi[0], hi[1], hi[2]), obbs + i, xfs + i);
         }
     }
 

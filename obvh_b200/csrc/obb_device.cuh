@@ -113,5 +113,39 @@ __device__ __forceinline__ void project_tri_own(const float* t, const Axes& ax, 
     project_tri_from<From::kShared>(t, ax, lo, hi);
 }
 
+// Extents over a node's leaf run go by size: a thread alone for up to
+// kSoloLeaves leaves, 8 lanes for up to kGroupLeaves, a warp above.  A Karras
+// tree's nodes are mostly tiny (half have 2 or 3 leaves), and one thread per
+// node up to 32 leaves kept its warp in the loop for 32 rounds, 16 of 32 lanes
+// busy on average over the kernel.
+constexpr uint32_t kSoloLeaves = 8;
+constexpr uint32_t kGroupLeaves = 32;
+
+__device__ __forceinline__ Axes cand_axes(const Cand& c, float nz) {
+    return make_axes(mk3(c.ax[0], c.ax[1], c.ax[2]), mk3(c.ax[3], c.ax[4], c.ax[5]), mk3(c.ax[6], c.ax[7], c.ax[8]), nz);
+}
+
+// Extents of `cnt` consecutive triangles at tp by the 8 lanes of an aligned
+// group (every lane of the warp calls it, cnt 0 for a group without a node);
+// all 8 lanes get the result.
+template <From F>
+__device__ __forceinline__ void group_extents(const float* tp, uint32_t cnt, const Axes& ax, float lo[3], float hi[3]) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        lo[k] = kInf;
+        hi[k] = -kInf;
+    }
+    for (uint32_t i = threadIdx.x & 7; i < cnt; i += 8) project_tri_from<F>(tp + 9 * i, ax, lo, hi);
+    __syncwarp();
+#pragma unroll
+    for (int m = 4; m > 0; m >>= 1) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            lo[k] = fminf(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], m));
+            hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], m));
+        }
+    }
+}
+
 }  // namespace obbtree
 }  // namespace obvh

@@ -45,7 +45,6 @@ namespace obbtree {
 using namespace tree;
 
 constexpr int kThreads = 256;
-constexpr uint32_t kThreadMax = 32;  // leaves handled by one thread per node
 constexpr uint32_t kCollapseLeafMax = 8;  // MAX_LEAF_SIZE (transforms.cu:65)
 constexpr uint32_t kUnit = 1024;    // leaves per warp unit
 constexpr uint32_t kUnitRun = 4;   // consecutive units per warp visit
@@ -55,7 +54,10 @@ constexpr uint32_t kTile = 1u << kTileShift;
 // tie-break: each level lengthens the common prefix of the 62-bit (code,
 // index) keys, so there are at most 62.
 constexpr uint32_t kChain = 64;
-constexpr uint32_t kTileItems = 320;  // warp items per tile kept in shared memory
+// Extents items per tile kept in shared memory: of 8 lanes, and in all.  With
+// the triangles they fit the 48 KB of a static allocation.
+constexpr uint32_t kTileGroups = 160;
+constexpr uint32_t kTileItems = 320;
 
 struct Ctl {
     uint32_t error;
@@ -420,9 +422,9 @@ __device__ __forceinline__ void candidate_store(uint32_t a, const Summary& s, co
     uint32_t units;
     if (chain.parents) {  // tiles: 0 in one tile and small, 1 in one tile, 2 over several tiles
         const uint32_t f = __ldg(chain.first + a);
-        units = (f >> kTileShift) != ((f + cnt - 1) >> kTileShift) ? 2u : (cnt > kThreadMax ? 1u : 0u);
+        units = (f >> kTileShift) != ((f + cnt - 1) >> kTileShift) ? 2u : (cnt > kGroupLeaves ? 1u : 0u);
     } else {
-        units = cnt > kThreadMax ? (cnt + kUnit - 1) / kUnit : 0u;
+        units = cnt > kGroupLeaves ? (cnt + kUnit - 1) / kUnit : 0u;
     }
     nunits[a] = units;
     if (units > 1) {
@@ -485,7 +487,10 @@ __global__ void __launch_bounds__(kThreads, 2) candidate_kernel(const uint4* sum
     }
 }
 
-// Nodes of at most kThreadMax leaves: one thread each, finalised here.
+// Nodes of at most kGroupLeaves leaves: one thread each, finalised here.  (8
+// lanes for the nodes above kSoloLeaves, as in the tiles, was slower: 101 ->
+// 110 us on the 917K-triangle knot; here the triangles come from global memory
+// and the threads' loads in flight are what counts.)
 __global__ void __launch_bounds__(kThreads) extents_small_kernel(const Cand* cand, const uint32_t* counts,
                                                                  const uint32_t* first, const float* tris,
                                                                  uint32_t internal, kr_obb3* obbs, kr_mat4* xfs,
@@ -493,7 +498,7 @@ __global__ void __launch_bounds__(kThreads) extents_small_kernel(const Cand* can
     const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= internal || *err) return;
     const uint32_t cnt = counts[a];
-    if (cnt > kThreadMax) return;
+    if (cnt > kGroupLeaves) return;
     const Cand c = load_cand(cand, a);
     const f3 b0 = mk3(c.ax[0], c.ax[1], c.ax[2]), b1 = mk3(c.ax[3], c.ax[4], c.ax[5]), b2 = mk3(c.ax[6], c.ax[7], c.ax[8]);
     float lo[3] = {c.olo[0], c.olo[1], c.olo[2]}, hi[3] = {c.ohi[0], c.ohi[1], c.ohi[2]};
@@ -563,28 +568,41 @@ __global__ void __launch_bounds__(kThreads) extents_units_kernel(const Cand* can
 }
 
 // One tile of kTile consecutive leaves: their triangles are staged in shared
-// memory once, then every node over them is served from there.  Nodes inside
-// the tile with at most kThreadMax leaves: one thread each, finalised here.
-// Larger nodes inside the tile: a warp each, extents to the keys.  Nodes
-// crossing the tile's edges (the two chains): a warp each over their part in
-// the tile, combined in the keys with integer atomics.  Warps take items from
-// a shared counter; an item beyond the list's capacity is done by the thread
-// that found it.
+// memory once, then every node over them is served from there (kSoloLeaves).
+// The nodes of one thread are finalised by it; larger ones are items: 8 lanes
+// or a warp each compute the extents, and the boxes are built afterwards, a
+// thread per item (building them in the warp's first lane, 16 of 32 lanes were
+// busy over the kernel).  Nodes crossing the tile's edges (the two chains) are
+// warp items over their part in the tile, combined in the keys with integer
+// atomics.  Groups and warps take items from shared counters; an item beyond
+// the lists' capacity is done by the thread that found it.
 // A node over several tiles finishes in the last of them: each tile's part
 // folds its extents into the node's keys (atomics), fences them, and counts
 // itself in arrivals[a]; the part that completes the count reads the keys and
 // writes the box.
-__device__ __forceinline__ void part_done(const Cand* cand, const uint32_t* counts, const uint32_t* first,
-                                          const uint32_t* keys, uint32_t* arrivals, uint32_t a, kr_obb3* obbs,
-                                          kr_mat4* xfs) {
+__device__ __forceinline__ bool last_part(const uint32_t* counts, const uint32_t* first, uint32_t* arrivals,
+                                          uint32_t a) {
     const uint32_t f = __ldg(first + a), cnt = __ldg(counts + a);
     const uint32_t parts = ((f + cnt - 1) >> kTileShift) - (f >> kTileShift) + 1;
-    if (atomicAdd(arrivals + a, 1u) + 1u != parts) return;
+    if (atomicAdd(arrivals + a, 1u) + 1u != parts) return false;
     __threadfence();
+    return true;
+}
+__device__ __forceinline__ void finalize_keys(const Cand* cand, const uint32_t* keys, uint32_t a, kr_obb3* obbs,
+                                              kr_mat4* xfs) {
     const uint32_t* k = keys + 6 * static_cast<size_t>(a);
     finalize_node(load_cand(cand, a), mk3(key2f(__ldcg(k)), key2f(__ldcg(k + 1)), key2f(__ldcg(k + 2))),
                   mk3(key2f(__ldcg(k + 3)), key2f(__ldcg(k + 4)), key2f(__ldcg(k + 5))), obbs + a, xfs + a);
 }
+
+constexpr uint32_t kPart = 0x80000000u;   // item over part of its node
+constexpr uint32_t kIdle = 0xffffffffu;   // item with nothing left to finalise
+
+struct TileItems {
+    uint32_t node[kTileItems];
+    uint16_t b[kTileItems], e[kTileItems];
+    float ext[kTileItems][6];
+};
 
 __global__ void __launch_bounds__(kThreads) extents_tile_kernel(const Cand* cand, const uint32_t* counts,
                                                                 const uint32_t* first, const float* tris, uint32_t n,
@@ -592,9 +610,9 @@ __global__ void __launch_bounds__(kThreads) extents_tile_kernel(const Cand* cand
                                                                 uint32_t* keys, uint32_t* arrivals, kr_obb3* obbs,
                                                                 kr_mat4* xfs, const uint32_t* err, float nz) {
     __shared__ __align__(16) float tri[kTile * 9];
-    __shared__ uint32_t item_node[kTileItems];
-    __shared__ uint16_t item_b[kTileItems], item_e[kTileItems];
-    __shared__ uint32_t nitems, next_item;
+    // group items from the front, warp items from the back
+    __shared__ TileItems items;
+    __shared__ uint32_t ngroup, nwarp, next_group, next_warp;
     if (*err) return;
     const uint32_t t = threadIdx.x, lane = t & 31;
     const uint32_t t0 = blockIdx.x << kTileShift;
@@ -608,80 +626,64 @@ __global__ void __launch_bounds__(kThreads) extents_tile_kernel(const Cand* cand
         for (uint32_t i = t; i < n4; i += kThreads) dst[i] = __ldg(src + i);
         for (uint32_t i = 4 * n4 + t; i < 9 * tn; i += kThreads) tri[i] = __ldg(tris + 9 * static_cast<size_t>(t0) + i);
     }
-    if (t == 0) {
-        nitems = 0;
-        next_item = 0;
-    }
+    if (t == 0) ngroup = nwarp = next_group = next_warp = 0;
     __syncthreads();
-    const auto add_item = [&](uint32_t a, uint32_t b, uint32_t e, bool partial) {
-        const uint32_t idx = atomicAdd(&nitems, 1u);
-        if (idx < kTileItems) {
-            item_node[idx] = a | (partial ? 0x80000000u : 0u);
-            item_b[idx] = static_cast<uint16_t>(b);
-            item_e[idx] = static_cast<uint16_t>(e);
-            return;
-        }
-        // list full: this thread does the item alone
+    const auto alone = [&](uint32_t a, uint32_t b, uint32_t e, bool part) {
         const Cand c = load_cand(cand, a);
-        const Axes ax = make_axes(mk3(c.ax[0], c.ax[1], c.ax[2]), mk3(c.ax[3], c.ax[4], c.ax[5]),
-                                  mk3(c.ax[6], c.ax[7], c.ax[8]), nz);
+        const Axes ax = cand_axes(c, nz);
         float lo[3] = {kInf, kInf, kInf}, hi[3] = {-kInf, -kInf, -kInf};
         for (uint32_t i = b; i < e; ++i) project_tri_s(tri + 9 * i, ax, lo, hi);
-        if (partial) {
+        if (part) {
             uint32_t* kk = keys + 6 * static_cast<size_t>(a);
             for (int k = 0; k < 3; ++k) {
                 atomicMin(kk + k, f2key(lo[k]));
                 atomicMax(kk + 3 + k, f2key(hi[k]));
             }
             __threadfence();
-            part_done(cand, counts, first, keys, arrivals, a, obbs, xfs);
+            if (last_part(counts, first, arrivals, a)) finalize_keys(cand, keys, a, obbs, xfs);
         } else {
             finalize_node(c, mk3(fminf(c.olo[0], lo[0]), fminf(c.olo[1], lo[1]), fminf(c.olo[2], lo[2])),
                           mk3(fmaxf(c.ohi[0], hi[0]), fmaxf(c.ohi[1], hi[1]), fmaxf(c.ohi[2], hi[2])), obbs + a,
                           xfs + a);
         }
     };
-    // nodes inside the tile: their indices lie in the tile too
+    const auto add_item = [&](uint32_t a, uint32_t b, uint32_t e, bool part) -> bool {
+        const bool group = !part && e - b <= kGroupLeaves;
+        const uint32_t k = atomicAdd(group ? &ngroup : &nwarp, 1u);
+        if (k >= (group ? kTileGroups : kTileItems - kTileGroups)) return false;  // list full
+        const uint32_t at = group ? k : kTileItems - 1 - k;
+        items.node[at] = a | (part ? kPart : 0u);
+        items.b[at] = static_cast<uint16_t>(b);
+        items.e[at] = static_cast<uint16_t>(e);
+        return true;
+    };
+    // the nodes inside the tile (their indices lie in the tile too), then the
+    // nodes over its edges
     const uint32_t qn = t0 < internal ? min(tn, internal - t0) : 0u;
-    for (uint32_t i = t; i < qn; i += kThreads) {
-        const uint32_t a = t0 + i;
+    const uint32_t w0 = 2 * blockIdx.x;
+    const uint32_t c0 = min(chain_counts[w0], kChain), c1 = min(chain_counts[w0 + 1], kChain);
+    for (uint32_t i = t; i < qn + c0 + c1; i += kThreads) {
+        const bool part = i >= qn;
+        const uint32_t a = !part ? t0 + i
+                                 : chains[i < qn + c0 ? static_cast<size_t>(w0) * kChain + (i - qn)
+                                                      : static_cast<size_t>(w0 + 1) * kChain + (i - qn - c0)];
         const uint32_t f = __ldg(first + a), cnt = __ldg(counts + a);
-        if (f < t0 || f + cnt > t0 + tn) continue;
-        if (cnt <= kThreadMax) {
-            const Cand c = load_cand(cand, a);
-            float lo[3] = {c.olo[0], c.olo[1], c.olo[2]}, hi[3] = {c.ohi[0], c.ohi[1], c.ohi[2]};
-            const Axes ax = make_axes(mk3(c.ax[0], c.ax[1], c.ax[2]), mk3(c.ax[3], c.ax[4], c.ax[5]),
-                                      mk3(c.ax[6], c.ax[7], c.ax[8]), nz);
-            const float* tp = tri + 9 * (f - t0);
-            for (uint32_t k = 0; k < cnt; ++k) project_tri_s(tp + 9 * k, ax, lo, hi);
-            finalize_node(c, mk3(lo[0], lo[1], lo[2]), mk3(hi[0], hi[1], hi[2]), obbs + a, xfs + a);
-        } else {
-            add_item(a, f - t0, f - t0 + cnt, false);
-        }
-    }
-    // nodes over the tile's edges
-    for (uint32_t side = 0; side < 2; ++side) {
-        const uint32_t w = 2 * blockIdx.x + side;
-        const uint32_t cnt = min(chain_counts[w], kChain);
-        for (uint32_t i = t; i < cnt; i += kThreads) {
-            const uint32_t a = chains[static_cast<size_t>(w) * kChain + i];
-            const uint32_t f = __ldg(first + a), c = __ldg(counts + a);
-            add_item(a, max(f, t0) - t0, min(f + c, t0 + tn) - t0, true);
-        }
+        if (!part && (f < t0 || f + cnt > t0 + tn)) continue;
+        const uint32_t b = max(f, t0) - t0, e = min(f + cnt, t0 + tn) - t0;
+        if ((!part && cnt <= kSoloLeaves) || !add_item(a, b, e, part)) alone(a, b, e, part);
     }
     __syncthreads();
-    const uint32_t items = min(nitems, kTileItems);
-    for (;;) {
+    const uint32_t groups = min(ngroup, kTileGroups), warps = min(nwarp, kTileItems - kTileGroups);
+    for (;;) {  // warp items first: they are longer
         uint32_t it = 0;
-        if (lane == 0) it = atomicAdd(&next_item, 1u);
+        if (lane == 0) it = atomicAdd(&next_warp, 1u);
         it = __shfl_sync(0xffffffffu, it, 0);
-        if (it >= items) break;
-        const uint32_t a = item_node[it] & 0x7fffffffu;
-        const bool partial = item_node[it] >> 31;
-        const uint32_t b = item_b[it], e = item_e[it];
-        const Cand c = load_cand(cand, a);
-        const Axes ax = make_axes(mk3(c.ax[0], c.ax[1], c.ax[2]), mk3(c.ax[3], c.ax[4], c.ax[5]),
-                                  mk3(c.ax[6], c.ax[7], c.ax[8]), nz);
+        if (it >= warps) break;
+        const uint32_t at = kTileItems - 1 - it;
+        const uint32_t a = items.node[at] & ~kPart;
+        const bool part = (items.node[at] & kPart) != 0;
+        const uint32_t b = items.b[at], e = items.e[at];
+        const Axes ax = cand_axes(load_cand(cand, a), nz);
         float lo[3] = {kInf, kInf, kInf}, hi[3] = {-kInf, -kInf, -kInf};
         for (uint32_t i = b + lane; i < e; i += 32) project_tri_s(tri + 9 * i, ax, lo, hi);
 #pragma unroll
@@ -689,22 +691,50 @@ __global__ void __launch_bounds__(kThreads) extents_tile_kernel(const Cand* cand
             lo[k] = warp_min(lo[k]);
             hi[k] = warp_max(hi[k]);
         }
-        if (partial) {
+        const float v = lane == 0 ? lo[0] : lane == 1 ? lo[1] : lane == 2 ? lo[2] : lane == 3 ? hi[0] : lane == 4 ? hi[1] : hi[2];
+        if (part) {
             if (lane < 6) {
                 uint32_t* kk = keys + 6 * static_cast<size_t>(a) + lane;
-                if (lane < 3) atomicMin(kk, f2key(lo[lane])); else atomicMax(kk, f2key(hi[lane - 3]));
+                if (lane < 3) atomicMin(kk, f2key(v)); else atomicMax(kk, f2key(v));
                 __threadfence();
             }
             __syncwarp();
-            if (lane == 0) part_done(cand, counts, first, keys, arrivals, a, obbs, xfs);
-        } else if (lane == 0) {
-            // inside this tile: the box from the warp's extents (and the
-            // summary extremes the candidate holds), no keys
-            finalize_node(c, mk3(fminf(c.olo[0], lo[0]), fminf(c.olo[1], lo[1]), fminf(c.olo[2], lo[2])),
-                          mk3(fmaxf(c.ohi[0], hi[0]), fmaxf(c.ohi[1], hi[1]), fmaxf(c.ohi[2], hi[2])), obbs + a,
-                          xfs + a);
+            if (lane == 0 && !last_part(counts, first, arrivals, a)) items.node[at] = kIdle;
+        } else if (lane < 6) {
+            items.ext[at][lane] = v;
         }
         __syncwarp();
+    }
+    for (;;) {
+        uint32_t it = 0;
+        if (lane == 0) it = atomicAdd(&next_group, 4u);
+        it = __shfl_sync(0xffffffffu, it, 0);
+        if (it >= groups) break;
+        it += lane >> 3;
+        const bool live = it < groups;
+        const uint32_t a = live ? items.node[it] : items.node[0];
+        const uint32_t b = live ? items.b[it] : 0, e = live ? items.e[it] : 0;
+        const Axes ax = cand_axes(load_cand(cand, a), nz);
+        float lo[3], hi[3];
+        group_extents<From::kShared>(tri + 9 * b, e - b, ax, lo, hi);
+        const uint32_t sub = lane & 7;
+        if (live && sub < 6)
+            items.ext[it][sub] = sub == 0 ? lo[0] : sub == 1 ? lo[1] : sub == 2 ? lo[2] : sub == 3 ? hi[0] : sub == 4 ? hi[1] : hi[2];
+    }
+    __syncthreads();
+    for (uint32_t i = t; i < groups + warps; i += kThreads) {
+        const uint32_t at = i < groups ? i : kTileItems - 1 - (i - groups);
+        const uint32_t node = items.node[at];
+        if (node == kIdle) continue;
+        const uint32_t a = node & ~kPart;
+        if (node & kPart) {
+            finalize_keys(cand, keys, a, obbs, xfs);
+        } else {
+            const Cand c = load_cand(cand, a);
+            const float* x = items.ext[at];
+            finalize_node(c, mk3(fminf(c.olo[0], x[0]), fminf(c.olo[1], x[1]), fminf(c.olo[2], x[2])),
+                          mk3(fmaxf(c.ohi[0], x[3]), fmaxf(c.ohi[1], x[4]), fmaxf(c.ohi[2], x[5])), obbs + a, xfs + a);
+        }
     }
 }
 

@@ -102,13 +102,31 @@ struct M4 {
 
 // kr_minverse4 (vecmath.h:946-1076): each adjugate entry is a signed sum of
 // six triple products in the reference's order; then det and 1/det scaling.
+//
+// Shape says which entries are known: the frames and boxes inverted here have
+// the last row (0, 0, 0, 1), a pure frame (kFrame) a zero last column too.
+// With finite entries whose products do not overflow, a term with a zero
+// factor adds a zero and a factor 1 changes nothing, so those drop out and the
+// rest is evaluated in the same order: 150 operations a box instead of 560.
+enum class Shape { kAny, kAffine, kFrame };
+
+template <Shape S>
+__device__ __forceinline__ constexpr bool known_zero(int i) {
+    return (S != Shape::kAny && (i == 3 || i == 7 || i == 11)) || (S == Shape::kFrame && i >= 12 && i < 15);
+}
+
+template <Shape S>
 __device__ __forceinline__ float adj_term(const M4& m, int s, int a, int b, int c, float acc, bool first) {
-    float p = m.v[a] * m.v[b] * m.v[c];
+    if (known_zero<S>(a) || known_zero<S>(b) || known_zero<S>(c)) return acc;
+    // only the last factor of a term can be entry 15
+    const float p = S != Shape::kAny && c == 15 ? m.v[a] * m.v[b] : m.v[a] * m.v[b] * m.v[c];
     if (first) return s < 0 ? -p : p;
     return s < 0 ? acc - p : acc + p;
 }
 
-__device__ inline M4 minverse4(const M4& m) {
+// (*recip receives 1 / det, 1 where det is 0)
+template <Shape S>
+__device__ __forceinline__ M4 minverse4(const M4& m, float* recip = nullptr) {
     // sign, factor, factor, factor for the 6 terms of each of the 16 entries
     constexpr signed char T[16][6][4] = {
         {{1, 5, 10, 15}, {-1, 5, 11, 14}, {-1, 9, 6, 15}, {1, 9, 7, 14}, {1, 13, 6, 11}, {-1, 13, 7, 10}},
@@ -133,11 +151,13 @@ __device__ inline M4 minverse4(const M4& m) {
     for (int e = 0; e < 16; ++e) {
         float acc = 0.f;
 #pragma unroll
-        for (int t = 0; t < 6; ++t) acc = adj_term(m, T[e][t][0], T[e][t][1], T[e][t][2], T[e][t][3], acc, t == 0);
+        for (int t = 0; t < 6; ++t) acc = adj_term<S>(m, T[e][t][0], T[e][t][1], T[e][t][2], T[e][t][3], acc, t == 0);
         ret.v[e] = acc;
     }
-    float det = m.v[0] * ret.v[0] + m.v[1] * ret.v[4] + m.v[2] * ret.v[8] + m.v[3] * ret.v[12];
+    float det = m.v[0] * ret.v[0] + m.v[1] * ret.v[4] + m.v[2] * ret.v[8];
+    if (S == Shape::kAny) det = det + m.v[3] * ret.v[12];
     M4 inv;
+    if (recip) *recip = det == 0 ? 1.0f : 1.0f / det;
     if (det == 0) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) inv.v[i] = (i % 5 == 0) ? 1.0f : 0.0f;
@@ -173,6 +193,27 @@ __device__ __forceinline__ f3 mtransform(const M4& l, f3 r) {
                l.v[2] * r.x + l.v[6] * r.y + l.v[10] * r.z + l.v[14]);
 }
 
+// Whether the known zeros and ones of an affine matrix may drop out of its
+// inverse: every entry below 1e12 in size (a NaN fails), so that no product of
+// three overflows and zero times it is zero.
+__device__ __forceinline__ bool plain_entries(f3 a0, f3 a1, f3 a2, f3 t) {
+    const auto top = [](float a, float b, float c) {
+        float r;
+        asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(fabsf(a)), "f"(fabsf(b)), "f"(fabsf(c)));
+        return r;
+    };
+    return top(top(a0.x, a0.y, a0.z), top(a1.x, a1.y, a1.z), top(a2.x, a2.y, a2.z)) < 1e12f && top(t.x, t.y, t.z) < 1e12f;
+}
+
+// The inverse of T(mid) R(a0 a1 a2) S(2 ext), the matrices multiplied out in
+// full (entries that are not plain).
+static __device__ __noinline__ M4 box_inverse_any(f3 a0, f3 a1, f3 a2, f3 mid, f3 ext) {
+    const M4 r = mframe(a0, a1, a2);
+    const M4 s{{ext.x * 2.0f, 0, 0, 0, 0, ext.y * 2.0f, 0, 0, 0, 0, ext.z * 2.0f, 0, 0, 0, 0, 1}};
+    const M4 t{{1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 0, mid.x, mid.y, mid.z, 1}};
+    return minverse4<Shape::kAny>(mmul4(t, mmul4(r, s)));
+}
+
 // Writes obb (mid, axes, ext clamped to 0.001) and transform = inverse of
 // T(mid) R(axes) S(2 ext) for the box [lo, hi] in the frame's coordinates
 // (transforms.cu:826-834 and :928-963).
@@ -188,13 +229,26 @@ __device__ inline void write_box(kr_obb3* obb, kr_mat4* xf, f3 a0, f3 a1, f3 a2,
     o[6] = a1.x; o[7] = a1.y; o[8] = a1.z;
     o[9] = a2.x; o[10] = a2.y; o[11] = a2.z;
     o[12] = ext.x; o[13] = ext.y; o[14] = ext.z;
-    const M4 r = mframe(a0, a1, a2);
-    const M4 s{{ext.x * 2.0f, 0, 0, 0, 0, ext.y * 2.0f, 0, 0, 0, 0, ext.z * 2.0f, 0, 0, 0, 0, 1}};
-    const M4 t{{1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 0, mid.x, mid.y, mid.z, 1}};
-    const M4 inv = minverse4(mmul4(t, mmul4(r, s)));
+    // T R S: the axes scaled by twice the extents, then mid (finite factors:
+    // the products with zeros and ones change nothing)
+    const f3 c0 = mulv(a0, ext.x * 2.0f), c1 = mulv(a1, ext.y * 2.0f), c2 = mulv(a2, ext.z * 2.0f);
+    M4 inv;
+    if (plain_entries(c0, c1, c2, mid) && plain_entries(a0, a1, a2, ext)) {
+        inv = minverse4<Shape::kAffine>(M4{{c0.x, c0.y, c0.z, 0, c1.x, c1.y, c1.z, 0, c2.x, c2.y, c2.z, 0, mid.x, mid.y,
+                                            mid.z, 1}});
+    } else {
+        inv = box_inverse_any(a0, a1, a2, mid, ext);
+    }
     float4* x = reinterpret_cast<float4*>(xf);
 #pragma unroll
     for (int c = 0; c < 4; ++c) x[c] = make_float4(inv.v[4 * c], inv.v[4 * c + 1], inv.v[4 * c + 2], inv.v[4 * c + 3]);
+}
+
+// The inverse of the frame a0 a1 a2 applied to v0, v1, v2, the 4x4 form in
+// full (entries that are not plain).
+static __device__ __noinline__ void into_frame_any(f3 a0, f3 a1, f3 a2, f3* v) {
+    const M4 inv = minverse4<Shape::kAny>(mframe(a0, a1, a2));
+    for (int i = 0; i < 3; ++i) v[i] = mtransform(inv, v[i]);
 }
 
 // Leaf OBB from the triangle frame (refit_obbs_kernel_new, transforms.cu:794-834):
@@ -204,10 +258,21 @@ __device__ inline void leaf_box(f3 v0, f3 v1, f3 v2, kr_obb3* obb, kr_mat4* xf) 
     const f3 a2 = cross3(e0, e1);
     const f3 a0 = unit3(e0);
     const f3 a1 = unit3(cross3(a0, a2));
-    const M4 inv = minverse4(mframe(a0, a1, a2));
-    const f3 l0 = mtransform(inv, v0), l1 = mtransform(inv, v1), l2 = mtransform(inv, v2);
-    const f3 hi = vmax3(l0, vmax3(l1, l2));
-    const f3 lo = vmin3(l0, vmin3(l1, l2));
+    f3 l[3] = {v0, v1, v2};
+    float recip = kInf;
+    M4 inv;
+    if (plain_entries(a0, a1, a2, mk3(0, 0, 0))) inv = minverse4<Shape::kFrame>(mframe(a0, a1, a2), &recip);
+    if (fabsf(recip) < kInf) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i)  // mtransform without the zero translation (zero times a finite 1 / det)
+            l[i] = mk3(inv.v[0] * l[i].x + inv.v[4] * l[i].y + inv.v[8] * l[i].z,
+                       inv.v[1] * l[i].x + inv.v[5] * l[i].y + inv.v[9] * l[i].z,
+                       inv.v[2] * l[i].x + inv.v[6] * l[i].y + inv.v[10] * l[i].z);
+    } else {
+        into_frame_any(a0, a1, a2, l);
+    }
+    const f3 hi = vmax3(l[0], vmax3(l[1], l[2]));
+    const f3 lo = vmin3(l[0], vmin3(l[1], l[2]));
     write_box(obb, xf, a0, a1, a2, lo, hi);
 }
 
