@@ -52,18 +52,22 @@ namespace atrbvh {
 
 constexpr int kThreads = 256;
 constexpr int kTreeletThreads = 128;
+// 72 registers; 6, 8 and 10 blocks an SM were slower (917K-triangle knot:
+// 2,448, 2,418, 2,425 and 2,516 us a build with 6, 7, 8 and 10).
+constexpr int kTreeletBlocks = 7;
 constexpr int kTreeletWarps = kTreeletThreads / 32;
 constexpr int kMinTau = 3;
 constexpr int kMaxTau = 20;
 
-// One node of the working tree (48 bytes).
-struct TNode {
+// One node of the working tree (48 bytes).  A node carries its children's
+// areas, so that growing a treelet through it takes one 16-byte load (its
+// children) instead of a chain of two (the children, then their areas).
+struct __align__(16) TNode {
     float lo[3], hi[3];
-    int32_t left, right;
     float area;
     int32_t parent;
-    int32_t data;  // triangle of a leaf, -1 for an internal node
-    int32_t pad;
+    int32_t left, right;     // -1 in a leaf
+    float area_l, area_r;    // the children's areas; in a leaf area_r holds the triangle's index as bits
 };
 static_assert(sizeof(TNode) == 48, "TNode is 48 bytes");
 
@@ -117,6 +121,13 @@ __global__ void __launch_bounds__(kThreads) morton63_kernel(const kr_vec3* verts
     vals[i] = i;
 }
 
+__device__ __forceinline__ void set_triangle(TNode* leaf, int32_t tri) {
+    *reinterpret_cast<int32_t*>(&leaf->area_r) = tri;
+}
+__device__ __forceinline__ int32_t triangle_of(const TNode* leaf) {
+    return *reinterpret_cast<const int32_t*>(&leaf->area_r);
+}
+
 // longestCommonPrefix over 64-bit keys with the index tie-break (LBVH.cu:171-185).
 __device__ __forceinline__ int lcp64(const uint64_t* keys, uint32_t n, int i, int j, uint64_t ki) {
     if (j < 0 || j >= static_cast<int>(n)) return -1;
@@ -126,7 +137,7 @@ __device__ __forceinline__ int lcp64(const uint64_t* keys, uint32_t n, int i, in
 }
 
 __global__ void __launch_bounds__(kThreads) karras63_kernel(const uint64_t* keys, const uint32_t* order, uint32_t n,
-                                                            TNode* t, uint32_t* err) {
+                                                            TNode* t, int32_t* tris, uint32_t* err) {
     const int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
     const int internal = static_cast<int>(n) - 1;
     if (i >= internal) return;
@@ -155,46 +166,54 @@ __global__ void __launch_bounds__(kThreads) karras63_kernel(const uint64_t* keys
     int li = split, ri = split + 1;
     if (min(i, j) == split) {
         li = split + internal;
-        t[li].data = static_cast<int32_t>(__ldg(order + split));
+        set_triangle(t + li, static_cast<int32_t>(__ldg(order + split)));
     }
     if (max(i, j) == split + 1) {
         ri = split + 1 + internal;
-        t[ri].data = static_cast<int32_t>(__ldg(order + split + 1));
+        set_triangle(t + ri, static_cast<int32_t>(__ldg(order + split + 1)));
     }
     t[i].left = li;
     t[i].right = ri;
-    t[i].data = -1;
+    tris[i] = l + 1;  // a triangle per key of the node's range
     t[li].parent = i;
     t[ri].parent = i;
     if (i == 0) t[0].parent = -1;
 }
 
 __device__ __forceinline__ void store_box(TNode* t, int32_t i, const float* lo, const float* hi) {
-    float* d = t[i].lo;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        __stcg(d + k, lo[k]);
-        __stcg(d + 3 + k, hi[k]);
-    }
+    __stcg(reinterpret_cast<float4*>(t[i].lo), make_float4(lo[0], lo[1], lo[2], hi[0]));
+    __stcg(reinterpret_cast<float2*>(t[i].hi + 1), make_float2(hi[1], hi[2]));
     __stcg(&t[i].area, box_area(lo, hi));
 }
 
 __device__ __forceinline__ void load_box(const TNode* t, int32_t i, float* lo, float* hi) {
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        lo[k] = __ldcg(t[i].lo + k);
-        hi[k] = __ldcg(t[i].hi + k);
-    }
+    const float4 a = __ldcg(reinterpret_cast<const float4*>(t[i].lo));
+    const float2 b = __ldcg(reinterpret_cast<const float2*>(t[i].hi + 1));
+    lo[0] = a.x; lo[1] = a.y; lo[2] = a.z;
+    hi[0] = a.w; hi[1] = b.x; hi[2] = b.y;
 }
 
-// Leaf boxes, then node boxes bottom-up (the second thread to arrive merges).
+// A node's children and their areas.
+struct Kids {
+    int32_t left, right;
+    float area_l, area_r;
+};
+__device__ __forceinline__ Kids load_kids(const TNode* t, int32_t i) {
+    const int4 k = __ldcg(reinterpret_cast<const int4*>(&t[i].left));
+    return Kids{k.x, k.y, __int_as_float(k.z), __int_as_float(k.w)};
+}
+
+// Leaf boxes, then node boxes and SAHs bottom-up (the second thread to arrive
+// merges).  The SAH of a node is ci area + left + right, of a leaf ct area
+// (AgglomerativeTreelet.cu:405-570); the treelet passes start from them.
 __global__ void __launch_bounds__(kThreads) boxes_up_kernel(const kr_vec3* verts, const uint4* faces, uint32_t n,
-                                                            TNode* t, uint32_t* visits, uint32_t* err) {
+                                                            TNode* t, int32_t* tris, float* sah_arr, float ci,
+                                                            float ct, uint32_t* visits, uint32_t* err) {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const int32_t internal = static_cast<int32_t>(n) - 1;
     int32_t child = internal + static_cast<int32_t>(j);
-    const int32_t tri = t[child].data;
+    const int32_t tri = triangle_of(t + child);
     if (tri < 0 || tri >= static_cast<int32_t>(n)) {
         atomicOr(err, kErrBadInput);
         return;
@@ -205,7 +224,11 @@ __global__ void __launch_bounds__(kThreads) boxes_up_kernel(const kr_vec3* verts
     float hi[3] = {fmaxf(fmaxf(a.x, b.x), c.x), fmaxf(fmaxf(a.y, b.y), c.y), fmaxf(fmaxf(a.z, b.z), c.z)};
     t[child].left = -1;
     t[child].right = -1;
+    tris[child] = 1;
+    float area = box_area(lo, hi);
+    float sah = ct * area;
     store_box(t, child, lo, hi);
+    __stcg(sah_arr + child, sah);
     int32_t p = t[child].parent;
     for (uint32_t steps = 0; p >= 0; ++steps) {
         if (steps > n || p >= internal) {
@@ -224,12 +247,18 @@ __global__ void __launch_bounds__(kThreads) boxes_up_kernel(const kr_vec3* verts
         }
         float slo[3], shi[3];
         load_box(t, sib, slo, shi);
+        const float other_sah = __ldcg(sah_arr + sib);
+        const float other = box_area(slo, shi);
+        __stcg(reinterpret_cast<float2*>(&t[p].area_l), L == child ? make_float2(area, other) : make_float2(other, area));
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             lo[k] = fminf(lo[k], slo[k]);
             hi[k] = fmaxf(hi[k], shi[k]);
         }
+        area = box_area(lo, hi);
+        sah = ci * area + (L == child ? sah : other_sah) + (L == child ? other_sah : sah);
         store_box(t, p, lo, hi);
+        __stcg(sah_arr + p, sah);
         child = p;
         p = grand;
     }
@@ -239,29 +268,32 @@ __global__ void __launch_bounds__(kThreads) boxes_up_kernel(const kr_vec3* verts
 // Treelet optimisation.
 
 // Per-treelet shared state (one per segment of W lanes; a treelet has at most
-// W leaves, so the arrays are sized by W: 208 bytes a segment at W = 8, which
-// lets 12 CTAs of 128 threads share an SM where 32-entry arrays allowed 5).
+// W leaves).
 template <int W>
 struct SegSmem {
     int32_t internal[W];
-    int32_t leaves[W];
-    float areas[W];
     float dist[W * (W - 1) / 2];
 };
 
 // A treelet of tau <= W leaves is processed by a segment of W lanes (W = 8,
 // 16 or 32), so a warp works on 32 / W treelets at once.  The reference uses a
-// whole warp per treelet; its two reductions are replayed exactly:
+// whole warp per treelet; its two reductions give the same winners here:
 //   - the leaf to expand (Treelet.cuh:21-37): a shuffle-down over the first
-//     2 + it <= tau lanes, larger area wins, ties keep the lane's own value;
-//     within W lanes every shuffle source that matters exists, and a source
-//     past the segment returns the lane's own value, which never wins, as the
-//     reference's lanes past the count (area -FLT_MAX) do not;
-//   - the pair to merge (AgglomerativeTreelet.cu:59-90): 32 "virtual lanes"
-//     v scan the distance entries v, v + 32, ...; lane sl of the segment holds
-//     the virtual lanes sl + W q.  Shuffle steps of 16 and 8 that stay inside
-//     one physical lane (W <= 16) are folds of its own virtual lanes; the rest
-//     are segment-wide shuffles.  Same pairs, same order, same strict '<'.
+//     2 + it <= tau lanes in which a lane keeps its own value on ties.  Lane 0
+//     ends with the largest area, of equal ones the first in the order in
+//     which the tree's lanes reach it, which depends on the lane count alone
+//     (PickOrder);
+//   - the pair to merge (AgglomerativeTreelet.cu:59-90): 32 virtual lanes v
+//     scan the distance entries v, v + 32, ..., then a shuffle-down by 16, 8,
+//     4, 2, 1 with strict '<'.  The smallest distance wins, of equal ones that
+//     of the lane whose index has the smallest bit reversal (the last step
+//     prefers even lanes, the one before those divisible by 4, ...), and
+//     within a lane the first entry.
+// So each is one redux for the value and one for the tie.
+//
+// The kernel's time is the latency of one treelet, level after level up the
+// tree (about 23,000 cycles in an earlier form: 7 expansions behind two
+// dependent loads each, 8 merges with five-step reductions and 45 shuffles).
 template <int W>
 __device__ __forceinline__ int seg_lane() { return threadIdx.x & (W - 1); }
 
@@ -280,47 +312,71 @@ __device__ __forceinline__ void reduce_down_seg(int count, int& idx, float& val,
     }
 }
 
-// findMinimumDistance over `size` entries, the reference's 32-lane tree.
+// rank[c][lane]: the place of `lane` among c lanes in the reduction's order of
+// preference on ties: what lane 0 holds after the steps is its own candidates,
+// then those of the lane `amount` above, at every step.
+struct PickOrder {
+    uint8_t rank[kMaxTau + 1][32];
+    constexpr PickOrder() : rank{} {
+        for (int c = 1; c <= kMaxTau; ++c) {
+            int list[32][32] = {}, len[32] = {};
+            for (int l = 0; l < c; ++l) {
+                list[l][0] = l;
+                len[l] = 1;
+            }
+            int count = c, amount = c / 2;
+            while (count > 1) {
+                for (int l = 0; l + amount < c; ++l) {  // ascending: list[l + amount] is still the old one
+                    for (int k = 0; k < len[l + amount]; ++k) {
+                        bool known = false;
+                        for (int q = 0; q < len[l]; ++q) known = known || list[l][q] == list[l + amount][k];
+                        if (!known) list[l][len[l]++] = list[l + amount][k];
+                    }
+                }
+                count = (count + 1) / 2;
+                amount = count / 2;
+            }
+            for (int k = 0; k < len[0]; ++k) rank[c][list[0][k]] = static_cast<uint8_t>(k);
+        }
+    }
+};
+__constant__ PickOrder c_pick = PickOrder();
+
+// Reductions over the segments of a warp: one full-warp redux per segment, the
+// other lanes giving the neutral value.  (A redux with the segment's own mask
+// differs within the warp, and the mask of a redux is a uniform operand: the
+// treelet passes took 1.67 ms instead of 1.44.)
 template <int W>
-__device__ __forceinline__ int min_distance_seg(const float* dist, int size) {
-    constexpr int Q = 32 / W;
-    const int sl = seg_lane<W>();
-    float val[Q];
-    int idx[Q];
+__device__ __forceinline__ bool in_segment(int q) { return W == 32 || static_cast<int>(threadIdx.x & 31) / W == q; }
+template <int W>
+__device__ __forceinline__ float seg_min(float v) {
+    float mine = v;
 #pragma unroll
-    for (int q = 0; q < Q; ++q) {
-        val[q] = FLT_MAX;
-        idx[q] = 0;
-        for (int j = sl + W * q; j < size; j += 32) {
-            const float d = dist[j];
-            if (d < val[q]) {
-                val[q] = d;
-                idx[q] = j;
-            }
-        }
+    for (int q = 0; q < 32 / W; ++q) {
+        const float r = warp_min(in_segment<W>(q) ? v : kInf);
+        if (in_segment<W>(q)) mine = r;
     }
+    return mine;
+}
+template <int W>
+__device__ __forceinline__ uint32_t seg_min(uint32_t v) {
+    uint32_t mine = v;
 #pragma unroll
-    for (int amount = 16; amount >= W && amount >= 1; amount >>= 1) {
-        const int step = amount / W;  // virtual lanes v and v + amount share this physical lane
-#pragma unroll
-        for (int q = 0; q < Q; ++q)
-            if (q + step < Q && val[q + step] < val[q]) {
-                val[q] = val[q + step];
-                idx[q] = idx[q + step];
-            }
+    for (int q = 0; q < 32 / W; ++q) {
+        const uint32_t r = __reduce_min_sync(0xffffffffu, in_segment<W>(q) ? v : 0xffffffffu);
+        if (in_segment<W>(q)) mine = r;
     }
-    int i0 = idx[0];
-    float v0 = val[0];
+    return mine;
+}
+template <int W>
+__device__ __forceinline__ uint32_t seg_max(uint32_t v) {
+    uint32_t mine = v;
 #pragma unroll
-    for (int amount = W / 2; amount >= 1; amount >>= 1) {
-        const int oi = __shfl_down_sync(0xffffffffu, i0, amount, W);
-        const float ov = __shfl_down_sync(0xffffffffu, v0, amount, W);
-        if (ov < v0) {
-            v0 = ov;
-            i0 = oi;
-        }
+    for (int q = 0; q < 32 / W; ++q) {
+        const uint32_t r = __reduce_max_sync(0xffffffffu, in_segment<W>(q) ? v : 0u);
+        if (in_segment<W>(q)) mine = r;
     }
-    return __shfl_sync(0xffffffffu, i0, 0, W);
+    return mine;
 }
 
 __device__ __forceinline__ int trm_index(int row, int col) { return ((row - 1) * row) / 2 + col; }
@@ -332,12 +388,53 @@ __device__ __forceinline__ int trm_col(int index) {
     return index - (y * (y - 1)) / 2;
 }
 
-// (row, col) of every index of the distance matrices of treelets of up to
-// kMaxTau leaves, row << 8 | col, tabulated once per CTA with the functions
-// above (a shared-memory load instead of a square root per lookup)
+// Every index of the distance matrices of treelets of up to kMaxTau leaves as
+// one word, tabulated once per CTA: its place in the reduction's order of
+// preference on ties (bit-reversed virtual lane, then round) above its row and
+// column, so that the winning word says which pair it is.
 constexpr int kTrmEntries = (kMaxTau - 1) * kMaxTau / 2;
-__device__ __forceinline__ int lut_row(const uint16_t* lut, int index) { return lut[index] >> 8; }
-__device__ __forceinline__ int lut_col(const uint16_t* lut, int index) { return lut[index] & 0xff; }
+__device__ __forceinline__ uint32_t pair_word(int index) {
+    return ((__brev(static_cast<uint32_t>(index & 31)) >> 27) << 24) | (static_cast<uint32_t>(index >> 5) << 16) |
+           (static_cast<uint32_t>(trm_row(index)) << 8) | static_cast<uint32_t>(trm_col(index));
+}
+__device__ __forceinline__ int word_row(uint32_t w) { return (w >> 8) & 0xff; }
+__device__ __forceinline__ int word_col(uint32_t w) { return w & 0xff; }
+
+// The pair to merge among the first `size` entries (pair_word).
+template <int W>
+__device__ __forceinline__ uint32_t nearest_pair(const float* dist, int size, const uint32_t* words) {
+    float best = FLT_MAX;
+    uint32_t word = 0xffffffffu;
+    for (int j = seg_lane<W>(); j < size; j += W) {
+        const float d = dist[j];
+        const uint32_t e = words[j];
+        if (d < best || (d == best && e < word && word != 0xffffffffu)) {
+            best = d;
+            word = e;
+        }
+    }
+    const float least = seg_min<W>(best);
+    const uint32_t win = seg_min<W>(best == least ? word : 0xffffffffu);
+    return win == 0xffffffffu ? words[0] : win;  // no finite distance: the reference's index 0
+}
+
+// The leaf to expand among the segment's first `count` lanes (area -FLT_MAX:
+// not to be expanded).
+template <int W>
+__device__ __forceinline__ int largest_leaf(int count, float area, const uint8_t* rank) {
+    const int sl = seg_lane<W>();
+    const bool in = sl < count;
+    if (__any_sync(0xffffffffu, in && area != area)) {  // a NaN area: the reference's own steps
+        int idx = in ? sl : -1;
+        float a = in ? area : -FLT_MAX;
+        reduce_down_seg<W>(count, idx, a, true);
+        return __shfl_sync(0xffffffffu, idx, 0, W);
+    }
+    const uint32_t key = in ? f2key(area) : 0u;
+    const uint32_t most = seg_max<W>(key);
+    const uint32_t place = static_cast<uint32_t>(rank[32 * count + sl]) << 8 | static_cast<uint32_t>(sl);
+    return static_cast<int>(seg_min<W>(in && key == most ? place : 0xffffffffu) & 0xffu);
+}
 
 template <int W>
 __device__ __forceinline__ void shfl_box(const float* lo, const float* hi, int src, float* olo, float* ohi) {
@@ -348,244 +445,294 @@ __device__ __forceinline__ void shfl_box(const float* lo, const float* hi, int s
     }
 }
 
+// The arrays a treelet pass works on.  `rec` is each node's SAH as a bottom-up
+// pass over the tree as it stands would compute it: what the next pass takes
+// as the SAH of the subtrees below its gamma.  (A merged node's `sah` is summed
+// in another order, children first.)
+struct PassArgs {
+    TNode* t;
+    float* sah;
+    float* rec;
+    int32_t* tris;
+    int32_t n;
+    int tau;
+    int32_t gamma;
+    float ci;
+};
+
+// A treelet root on the way up: its record and its sums.
+struct Root {
+    int32_t node;
+    Kids kids;
+    float sah, rec;
+};
+
 // The treelet rooted at `root`, by a segment of W lanes.  Every lane of the
 // warp calls this together (the shuffles span the warp); a segment with
-// `active` false computes nothing that is stored.  Returns false (for the
-// segment) on a malformed tree.
-template <int W>
-__device__ bool process_treelet(TNode* t, float* sah_arr, int32_t n, int tau, float ci, int32_t root, bool active,
-                                SegSmem<W>& w, const uint16_t* lut) {
+// `active` false computes nothing that is stored.  Leaves the root's SAHs
+// after the pass in root.  Returns false (for the segment) on a malformed
+// tree.  kLast: no pass follows, rec and the counts are not kept up.
+template <int W, bool kLast>
+__device__ bool process_treelet(const PassArgs& a, Root& root, bool active, SegSmem<W>& w, const uint32_t* words,
+                                const uint8_t* rank) {
     const int sl = seg_lane<W>();
-    const int32_t internal_count = n - 1;
-    const int32_t node_count = 2 * n - 1;
+    const int tau = a.tau;
+    const int32_t internal_count = a.n - 1;
+    const int32_t node_count = 2 * a.n - 1;
     auto valid = [&](int32_t x) { return x >= 0 && x < node_count; };
 
-    // formTreelet: grow by the frontier node of largest area (Treelet.cuh:55-129)
-    int bad = active ? 0 : 1;
-    if (sl == 0 && active) {
-        const int32_t L = __ldcg(&t[root].left), R = __ldcg(&t[root].right);
-        if (!valid(L) || !valid(R)) {
-            bad = 1;
-        } else {
-            w.internal[0] = root;
-            w.leaves[0] = L;
-            w.leaves[1] = R;
-            w.areas[0] = __ldcg(&t[L].area);
-            w.areas[1] = __ldcg(&t[R].area);
-        }
-    }
-    bad = __shfl_sync(0xffffffffu, bad, 0, W);
-    __syncwarp();
+    // formTreelet: grow by the frontier node of largest area (Treelet.cuh:55-129);
+    // lane sl holds frontier node sl
+    bool bad = !active || !valid(root.kids.left) || !valid(root.kids.right);
+    int32_t node = sl == 0 ? root.kids.left : (sl == 1 ? root.kids.right : -1);
+    float area = sl == 0 ? root.kids.area_l : root.kids.area_r;
+    if (sl == 0) w.internal[0] = root.node;
     for (int it = 0; it < tau - 2; ++it) {
-        int idx = -1;
-        float a = -FLT_MAX;
-        if (!bad && sl < 2 + it) {
-            idx = sl;
-            a = w.areas[sl];
-            if (w.leaves[sl] >= internal_count) a = -FLT_MAX;
+        const bool grows = !bad && node >= 0 && node < internal_count;
+        const int idx = largest_leaf<W>(2 + it, grows ? area : -FLT_MAX, rank);
+        const int32_t rep = __shfl_sync(0xffffffffu, node, idx < 0 ? 0 : idx, W);
+        bad = bad || idx < 0 || rep < 0 || rep >= internal_count;
+        Kids k{-1, -1, 0.f, 0.f};
+        if (!bad) k = load_kids(a.t, rep);
+        bad = bad || !valid(k.left) || !valid(k.right);
+        if (sl == 0) w.internal[it + 1] = rep;
+        if (sl == idx) {
+            node = k.left;
+            area = k.area_l;
         }
-        reduce_down_seg<W>(2 + it, idx, a, true);
-        __syncwarp();
-        if (sl == 0 && !bad) {
-            const int32_t rep = idx >= 0 ? w.leaves[idx] : -1;
-            const bool internal_node = rep >= 0 && rep < internal_count;
-            const int32_t L = internal_node ? __ldcg(&t[rep].left) : -1;
-            const int32_t R = internal_node ? __ldcg(&t[rep].right) : -1;
-            if (!internal_node || !valid(L) || !valid(R)) {
-                bad = 1;
-            } else {
-                w.internal[it + 1] = rep;
-                w.leaves[idx] = L;
-                w.leaves[it + 2] = R;
-                w.areas[idx] = __ldcg(&t[L].area);
-                w.areas[it + 2] = __ldcg(&t[R].area);
-            }
+        if (sl == it + 2) {
+            node = k.right;
+            area = k.area_r;
         }
-        bad = __shfl_sync(0xffffffffu, bad, 0, W);
-        __syncwarp();
     }
 
-    // Lane sl < tau holds treelet leaf sl: its node, SAH and box.
-    int32_t node = -1;
-    float sah = 0.f, lo[3] = {0.f, 0.f, 0.f}, hi[3] = {0.f, 0.f, 0.f};
+    // Lane sl < tau holds treelet leaf sl: its node, area, SAH, box.
+    float sah = 0.f, rec = 0.f, lo[3] = {0.f, 0.f, 0.f}, hi[3] = {0.f, 0.f, 0.f};
+    int32_t count = 0;
     if (!bad && sl < tau) {
-        node = w.leaves[sl];
-        sah = __ldcg(sah_arr + node);
-        load_box(t, node, lo, hi);
+        sah = __ldcg(a.sah + node);
+        if (!kLast) {
+            rec = __ldcg(a.rec + node);
+            count = __ldcg(a.tris + node);
+        }
+        load_box(a.t, node, lo, hi);
     }
     const int nd = (tau - 1) * tau / 2;
     for (int k0 = 0; k0 < nd; k0 += W) {  // every pair row > col
         const int k = k0 + sl;
-        const int r = k < nd ? lut_row(lut, k) : 0, c = k < nd ? lut_col(lut, k) : 0;
+        const uint32_t e = words[min(k, nd - 1)];
         float rlo[3], rhi[3], clo[3], chi[3];
-        shfl_box<W>(lo, hi, r, rlo, rhi);
-        shfl_box<W>(lo, hi, c, clo, chi);
+        shfl_box<W>(lo, hi, word_row(e), rlo, rhi);
+        shfl_box<W>(lo, hi, word_col(e), clo, chi);
         if (k < nd) w.dist[k] = union_area(rlo, rhi, clo, chi);
     }
     __syncwarp();
 
+    // Merge the nearest pair (jr, jc), jr > jc, until one is left.  The merged
+    // node takes place jc, the last one place jr; lane `last` is then free and
+    // keeps the merge: its children (node, right), their areas, the box and
+    // the sums.
+    const int my_row = trm_index(sl, 0);
+    int32_t right = -1;
+    float area_l = 0.f, area_r = 0.f;
     for (int last = tau - 1; last > 0; --last) {
-        const int mi = min_distance_seg<W>(w.dist, last * (1 + last) / 2);
-        const int jr = lut_row(lut, mi), jc = lut_col(lut, mi);
+        const uint32_t e = nearest_pair<W>(w.dist, last * (1 + last) / 2, words);
+        const int jr = word_row(e), jc = word_col(e);
 
-        // updateState (AgglomerativeTreelet.cu:92-147)
-        const float s = __shfl_sync(0xffffffffu, sah, jr, W) + __shfl_sync(0xffffffffu, sah, jc, W);
-        const int32_t li = __shfl_sync(0xffffffffu, node, jr, W), ri = __shfl_sync(0xffffffffu, node, jc, W);
-        float alo[3], ahi[3], blo[3], bhi[3];
-        shfl_box<W>(lo, hi, jr, alo, ahi);
-        shfl_box<W>(lo, hi, jc, blo, bhi);
+        // updateState (AgglomerativeTreelet.cu:92-147).  One shuffle brings
+        // place jr's value to all lanes but jr, and the last place's to jr.
+        const bool is_jr = sl == jr;
+        const int from = is_jr ? last : jr;
+        const auto of_jr = [&](auto own, auto& moved) {
+            moved = __shfl_sync(0xffffffffu, own, from, W);
+            return is_jr ? own : moved;
+        };
+        int32_t mnode;
+        float msah, marea, mlo[3], mhi[3];
+        const int32_t li = of_jr(node, mnode), ri = __shfl_sync(0xffffffffu, node, jc, W);
+        const float s = of_jr(sah, msah) + __shfl_sync(0xffffffffu, sah, jc, W);
+        const float la = of_jr(area, marea), ra = __shfl_sync(0xffffffffu, area, jc, W);
+        float ulo[3], uhi[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            alo[k] = fminf(blo[k], alo[k]);
-            ahi[k] = fmaxf(bhi[k], ahi[k]);
+            ulo[k] = fminf(__shfl_sync(0xffffffffu, lo[k], jc, W), of_jr(lo[k], mlo[k]));
+            uhi[k] = fmaxf(__shfl_sync(0xffffffffu, hi[k], jc, W), of_jr(hi[k], mhi[k]));
         }
-        if (sl == jc) {
-            node = w.internal[last - 1];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) { lo[k] = alo[k]; hi[k] = ahi[k]; }
-            w.areas[last] = s + ci * box_area(alo, ahi);
-            sah = w.areas[last];
+        const float uarea = box_area(ulo, uhi);
+        float mrec = 0.f, urec = 0.f;
+        int32_t mcount = 0, ucount = 0;
+        if (!kLast) {
+            const float lrec = of_jr(rec, mrec);
+            urec = a.ci * uarea + lrec + __shfl_sync(0xffffffffu, rec, jc, W);
+            ucount = of_jr(count, mcount) + __shfl_sync(0xffffffffu, count, jc, W);
         }
-        const int32_t last_node = __shfl_sync(0xffffffffu, node, last, W);
-        const float last_sah = __shfl_sync(0xffffffffu, sah, last, W);
-        float llo[3], lhi[3];
-        shfl_box<W>(lo, hi, last, llo, lhi);
-        if (sl == jr) {
-            node = last_node;
-            sah = last_sah;
+        const bool merged = sl == jc || sl == last;
+        if (is_jr || merged) {
+            sah = merged ? s + a.ci * uarea : msah;
+            area = merged ? uarea : marea;
+            node = sl == last ? li : (sl == jc ? w.internal[last - 1] : mnode);
+            if (!kLast) {
+                rec = merged ? urec : mrec;
+                count = merged ? ucount : mcount;
+            }
 #pragma unroll
-            for (int k = 0; k < 3; ++k) { lo[k] = llo[k]; hi[k] = lhi[k]; }
+            for (int k = 0; k < 3; ++k) {
+                lo[k] = merged ? ulo[k] : mlo[k];
+                hi[k] = merged ? uhi[k] : mhi[k];
+            }
+            if (sl == last) {
+                right = ri;
+                area_l = la;
+                area_r = ra;
+            }
         }
-        if (sl == last) {
-            node = li;
-            w.leaves[last] = ri;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) { lo[k] = alo[k]; hi[k] = ahi[k]; }
+
+        // updateDistancesMatrix (AgglomerativeTreelet.cu:149-186): place jr's
+        // distances are the last one's, place jc's are new.  The two write
+        // different entries: (jr, jc) is left to lane jr's new distance.
+        if (sl < last && sl != jc) {
+            if (!is_jr) w.dist[sl > jr ? my_row + jr : trm_index(jr, sl)] = w.dist[trm_index(last, sl)];
+            w.dist[sl > jc ? my_row + jc : trm_index(jc, sl)] = union_area(lo, hi, ulo, uhi);
         }
         __syncwarp();
+    }
 
-        // updateDistancesMatrix (AgglomerativeTreelet.cu:149-186)
-        if (last > 1) {
-            float cp = 0.f;
-            int dst = -1;
-            if (sl < last && sl != jr) {
-                cp = w.dist[trm_index(last, sl)];
-                dst = trm_index(max(jr, sl), min(jr, sl));
+    // updateTreelet: keep the new topology if its SAH is lower.  Lane sl >= 1
+    // holds the new internal node sl - 1; lane 1 the root.
+    const float total = __shfl_sync(0xffffffffu, sah, 1, W);
+    const float total_rec = kLast ? 0.f : __shfl_sync(0xffffffffu, rec, 1, W);
+    if (!bad && total < root.sah) {
+        root.sah = total;
+        root.rec = total_rec;
+        if (sl >= 1 && sl < tau) {
+            const int32_t ni = w.internal[sl - 1];
+            __stcg(reinterpret_cast<int4*>(&a.t[ni].left),
+                   make_int4(node, right, __float_as_int(area_l), __float_as_int(area_r)));
+            __stcg(&a.t[node].parent, ni);
+            __stcg(&a.t[right].parent, ni);
+            __stcg(a.sah + ni, sah);
+            if (!kLast) {
+                __stcg(a.rec + ni, rec);
+                if (sl > 1) __stcg(a.tris + ni, count);  // the root's does not change
             }
-            __syncwarp();
-            if (dst >= 0) w.dist[dst] = cp;
-            __syncwarp();
-            int dr = sl, dc = sl;
-            const bool upd = sl < last && sl != jc;
-            if (upd) {
-                dr = max(jc, sl);
-                dc = min(jc, sl);
-            }
-            float rlo[3], rhi[3], clo[3], chi[3];
-            shfl_box<W>(lo, hi, dr, rlo, rhi);
-            shfl_box<W>(lo, hi, dc, clo, chi);
-            const float d = union_area(rlo, rhi, clo, chi);
-            if (upd) w.dist[trm_index(dr, dc)] = d;
-            __syncwarp();
+            store_box(a.t, ni, lo, hi);
         }
     }
-
-    // updateTreelet: keep the new topology if its SAH is lower
-    const bool better = !bad && w.areas[1] < __ldcg(sah_arr + w.internal[0]);
-    if (better && sl >= 1 && sl < tau) {
-        const int32_t ni = w.internal[sl - 1];
-        const int32_t right = w.leaves[sl];
-        __stcg(&t[ni].left, node);
-        __stcg(&t[ni].right, right);
-        __stcg(&t[node].parent, ni);
-        __stcg(&t[right].parent, ni);
-        __stcg(sah_arr + ni, w.areas[sl]);
-        store_box(t, ni, lo, hi);
-    }
-    __threadfence();
     __syncwarp();
     return !(active && bad);
 }
 
-template <int W>
-__global__ void __launch_bounds__(kTreeletThreads) treelet_kernel(TNode* t, float* sah_arr, int32_t* tris,
-                                                                  uint32_t* counters, int32_t n, int tau,
-                                                                  int32_t gamma, float ci, float ct, uint32_t* err) {
+// The lowest treelet roots: nodes of at least gamma triangles, both of whose
+// children have fewer.  count[0] receives their number.
+__global__ void __launch_bounds__(kThreads) treelet_starts_kernel(const TNode* t, const int32_t* tris, int32_t n,
+                                                                  int32_t gamma, int32_t* starts, uint32_t* count) {
+    const int32_t i = static_cast<int32_t>(blockIdx.x * blockDim.x + threadIdx.x);
+    bool start = false;
+    if (i < n - 1 && tris[i] >= gamma) {
+        const Kids k = load_kids(t, i);
+        start = tris[k.left] < gamma && tris[k.right] < gamma;
+    }
+    const uint32_t vote = __ballot_sync(0xffffffffu, start);
+    if (!vote) return;
+    const int lane = threadIdx.x & 31;
+    uint32_t base = 0;
+    if (lane == __ffs(vote) - 1) base = atomicAdd(count, __popc(vote));
+    base = __shfl_sync(0xffffffffu, base, __ffs(vote) - 1);
+    if (start) starts[base + __popc(vote & ((1u << lane) - 1u))] = i;
+}
+
+// One pass: each segment of W lanes takes a lowest root from the list, runs
+// its treelet and goes up.  At a parent whose other child has fewer than gamma
+// triangles nothing is waited for (that subtree has no treelet and does not
+// change); else the second child to arrive carries on.  So the subtrees below
+// gamma, nine tenths of the nodes, take no part: with a thread walking up from
+// every leaf, 515,260 warp rounds of arrivals took 17,600 cycles each against
+// 222,622 treelet rounds of 22,500 (917K-triangle knot).
+template <int W, bool kLast>
+__global__ void __launch_bounds__(kTreeletThreads, kTreeletBlocks)
+    treelet_kernel(PassArgs a, uint32_t* counters, const int32_t* starts, uint32_t* queue, uint32_t* err) {
     constexpr int S = 32 / W;  // segments (treelets in flight) per warp
     __shared__ SegSmem<W> smem[kTreeletWarps * S];
-    __shared__ uint16_t lut[kTrmEntries];
-    for (int k = threadIdx.x; k < kTrmEntries; k += kTreeletThreads)
-        lut[k] = static_cast<uint16_t>((trm_row(k) << 8) | trm_col(k));
+    __shared__ uint32_t words[kTrmEntries];
+    __shared__ uint8_t rank[(kMaxTau + 1) * 32];
+    for (int k = threadIdx.x; k < kTrmEntries; k += kTreeletThreads) words[k] = pair_word(k);
+    for (int k = threadIdx.x; k < (kMaxTau + 1) * 32; k += kTreeletThreads) rank[k] = c_pick.rank[k >> 5][k & 31];
     __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const int seg = lane / W;
-    SegSmem<W>& w = smem[(threadIdx.x >> 5) * S + seg];
-    const int32_t i = static_cast<int32_t>(blockIdx.x * blockDim.x + threadIdx.x);
-    const int32_t internal = n - 1;
-    int32_t cur = -1;
-    if (i < n) {
-        const int32_t leaf = internal + i;
-        __stcg(tris + leaf, 1);
-        __stcg(sah_arr + leaf, ct * __ldcg(&t[leaf].area));
-        cur = __ldcg(&t[leaf].parent);
-    }
-    uint32_t rounds = 0;
-    while (__ballot_sync(0xffffffffu, cur >= 0) != 0) {
-        if (++rounds > static_cast<uint32_t>(n) + 2) {  // deeper than any tree of n leaves
-            if (lane == 0) atomicOr(err, kErrCycle);
-            break;
-        }
-        // (the arrival's release orders this lane's writes; the lanes that
-        // rewrote a treelet fenced theirs before the warp synchronised)
-        int32_t count = 0;
-        int32_t up = -1;
-        if (cur >= 0) {
-            // cur's children and area change only in cur's own treelet (or an
-            // ancestor's), later: read them ahead of the arrival
-            int32_t L = -1, R = -1;
-            float area = 0.f;
-            if (cur < internal) {
-                L = __ldcg(&t[cur].left);
-                R = __ldcg(&t[cur].right);
-                area = __ldcg(&t[cur].area);
-                // cur's own parent link changes only in an ancestor's treelet
-                // (a treelet rewrites the links below its root)
-                up = __ldcg(&t[cur].parent);
-            }
-            if (cur >= internal) {
-                atomicOr(err, kErrCycle);
-                cur = -1;
-            } else if (tree::arrive(counters + cur) == 0) {
-                cur = -1;  // the first child to arrive stops; the second carries on
-            } else {
-                if (L < 0 || L >= 2 * n - 1 || R < 0 || R >= 2 * n - 1) {
-                    atomicOr(err, kErrCycle);
-                    cur = -1;
-                } else {
-                    // the four loads first, then the stores: one round of loads
-                    const int32_t tl = __ldcg(tris + L), tr = __ldcg(tris + R);
-                    const float sl_ = __ldcg(sah_arr + L), sr = __ldcg(sah_arr + R);
-                    count = tl + tr;
-                    __stcg(tris + cur, count);
-                    __stcg(sah_arr + cur, ci * area + sl_ + sr);
-                }
+    const int lane = threadIdx.x & 31, sl = seg_lane<W>();
+    SegSmem<W>& w = smem[(threadIdx.x >> 5) * S + lane / W];
+    const int32_t internal = a.n - 1, node_count = 2 * a.n - 1;
+    const uint32_t total = queue[0];  // queue: {starts listed, starts taken}
+    Root root{-1, {-1, -1, 0.f, 0.f}, 0.f, 0.f};
+    float area = 0.f;
+    int32_t up = -1;
+    uint32_t level = 0;
+    bool dry = false;
+    for (;;) {
+        // a segment without a walk takes the next start
+        const bool fresh = root.node < 0 && !dry;
+        uint32_t at = total;
+        if (fresh && sl == 0) at = atomicAdd(queue + 1, 1u);
+        at = __shfl_sync(0xffffffffu, at, 0, W);
+        if (fresh) {
+            dry = at >= total;
+            if (!dry) {
+                root.node = __ldg(starts + at);
+                root.kids = load_kids(a.t, root.node);
+                area = __ldcg(&a.t[root.node].area);
+                up = __ldcg(&a.t[root.node].parent);
+                root.sah = a.ci * area + __ldcg(a.sah + root.kids.left) + __ldcg(a.sah + root.kids.right);
+                if (!kLast)
+                    root.rec = a.ci * area + __ldcg(a.rec + root.kids.left) + __ldcg(a.rec + root.kids.right);
+                level = 0;
             }
         }
-        uint32_t vote = __ballot_sync(0xffffffffu, count >= gamma);
-        while (vote != 0) {
-            // the next S treelet roots of the warp, lowest lanes first, one per segment
-            int src = -1;
-#pragma unroll
-            for (int q = 0; q < S; ++q) {
-                const int b = vote ? __ffs(vote) - 1 : -1;
-                if (q == seg) src = b;
-                vote = vote ? (vote & (vote - 1)) : 0u;
-            }
-            const int32_t root = __shfl_sync(0xffffffffu, cur, src < 0 ? 0 : src);
-            if (!process_treelet<W>(t, sah_arr, n, tau, ci, root, src >= 0, w, lut) && (lane & (W - 1)) == 0)
-                atomicOr(err, kErrBadInput);
+        const bool live = root.node >= 0;
+        if (!__any_sync(0xffffffffu, live)) return;
+        // the parent's record does not change before its own treelet (its
+        // parent link not before an ancestor's): read it ahead
+        Kids pk{-1, -1, 0.f, 0.f};
+        float parea = 0.f;
+        int32_t pup = -1;
+        if (live && up >= 0 && up < internal) {
+            pk = load_kids(a.t, up);
+            parea = __ldcg(&a.t[up].area);
+            pup = __ldcg(&a.t[up].parent);
         }
-        if (cur >= 0) cur = up;
+        if (live && sl == 0) {
+            __stcg(a.sah + root.node, root.sah);
+            if (!kLast) __stcg(a.rec + root.node, root.rec);
+        }
+        __syncwarp();
+        const bool fine = process_treelet<W, kLast>(a, root, live, w, words, rank);
+        if (!fine && sl == 0) atomicOr(err, kErrBadInput);
+        // one level up: the first of two treelet children to arrive stops
+        const bool left = pk.left == root.node;
+        const int32_t sib = left ? pk.right : pk.left;
+        bool carry = live && fine && up >= 0;
+        if (carry && (up >= internal || sib < 0 || sib >= node_count || (!left && pk.right != root.node) ||
+                      ++level > static_cast<uint32_t>(a.n))) {
+            if (sl == 0) atomicOr(err, kErrCycle);
+            carry = false;
+        }
+        const bool meets = carry && __ldcg(a.tris + sib) >= a.gamma;
+        uint32_t before = 1;
+        if (meets && sl == 0) before = tree::arrive(counters + up);
+        before = __shfl_sync(0xffffffffu, before, 0, W);
+        __syncwarp();  // orders the segment's loads after lane 0's acquire
+        carry = carry && before != 0;
+        if (carry) {
+            const float other = __ldcg(a.sah + sib);
+            root.sah = a.ci * parea + (left ? root.sah : other) + (left ? other : root.sah);
+            if (!kLast) {
+                const float orec = __ldcg(a.rec + sib);
+                root.rec = a.ci * parea + (left ? root.rec : orec) + (left ? orec : root.rec);
+            }
+            root.node = up;
+            root.kids = pk;
+            up = pup;
+        } else {
+            root.node = -1;
+        }
     }
 }
 
@@ -609,7 +756,7 @@ __global__ void __launch_bounds__(kThreads) emit_kernel(const TNode* t, uint32_t
             w[k] = __float_as_uint(s.lo[k]);
             w[3 + k] = __float_as_uint(s.hi[k]);
         }
-        w[6] = static_cast<uint32_t>(s.data);
+        w[6] = static_cast<uint32_t>(triangle_of(&s));
         w[7] = 0u;
         w[8] = 1u;
     }
@@ -634,7 +781,7 @@ Layout layout(uint32_t n) {
     L.ctl = o;       o += align256(sizeof(Ctl));
     L.bounds_ws = o; o += align256(lbvh::layout(0).total);
     L.scene = o;     o += align256(2 * sizeof(kr_aabb3));
-    L.keys0 = o;     o += align256(8ull * n);
+    L.keys0 = o;     o += align256(8ull * n);  // later: recomputed SAHs, 4 (2n - 1)
     L.keys1 = o;     o += align256(8ull * n);
     L.vals0 = o;     o += align256(4ull * n);
     L.vals1 = o;     o += align256(4ull * n);
@@ -659,6 +806,19 @@ kr_error check_args(const kr_vec3* verts, const kr_uvec4* faces, uint32_t n, uin
     return kr_success;
 }
 
+// A segment per lowest root (at most n / gamma of them), as far as the blocks
+// are resident at once.
+template <int W>
+void launch_pass(const PassArgs& a, uint32_t* counters, const int32_t* starts, uint32_t* queue, uint32_t* err,
+                 bool last, cudaStream_t s) {
+    constexpr unsigned kPerBlock = kTreeletThreads / W;
+    const unsigned want = static_cast<unsigned>(a.n / a.gamma) / kPerBlock + 1;
+    const unsigned cap = kTreeletBlocks * static_cast<unsigned>(device_info().sm_count);
+    const unsigned g = want < cap ? want : cap;
+    if (last) treelet_kernel<W, true><<<g, kTreeletThreads, 0, s>>>(a, counters, starts, queue, err);
+    else treelet_kernel<W, false><<<g, kTreeletThreads, 0, s>>>(a, counters, starts, queue, err);
+}
+
 // refit false: the nodes are emitted with zero internal bounds, and counts
 // and costs are left to the caller's own bottom-up pass.
 kr_error enqueue_tree(const kr_vec3* verts, const kr_uvec4* faces, uint32_t n, uint32_t tau, uint32_t iterations,
@@ -674,6 +834,11 @@ kr_error enqueue_tree(const kr_vec3* verts, const kr_uvec4* faces, uint32_t n, u
     uint32_t* counters = reinterpret_cast<uint32_t*>(ws + L.counters);
     const unsigned grid_n = (n + kThreads - 1) / kThreads;
     const uint32_t internal = n - 1;
+    int32_t* tris = reinterpret_cast<int32_t*>(ws + L.tris);
+    float* sah = reinterpret_cast<float*>(ws + L.sah);
+    // free once the tree is built: the sort's keys (8n bytes) and values
+    float* rec = reinterpret_cast<float*>(ws + L.keys0);
+    int32_t* starts = reinterpret_cast<int32_t*>(ws + L.vals0);
 
     // the transform's and the collapse's control blocks start at zero on every
     // build, so the status reads zero for the steps that do not run
@@ -694,31 +859,35 @@ kr_error enqueue_tree(const kr_vec3* verts, const kr_uvec4* faces, uint32_t n, u
     const uint32_t* order = reinterpret_cast<const uint32_t*>(ws + (alt ? L.vals1 : L.vals0));
     {
         ProfScope prof_scope_("karras63_kernel", s);
-        karras63_kernel<<<(internal + kThreads - 1) / kThreads, kThreads, 0, s>>>(keys, order, n, t, err);
+        karras63_kernel<<<(internal + kThreads - 1) / kThreads, kThreads, 0, s>>>(keys, order, n, t, tris, err);
     }
     OBVH_TRY_CUDA(cudaGetLastError());
     OBVH_TRY_CUDA(cudaMemsetAsync(counters, 0, 4ull * internal, s));
     {
         ProfScope prof_scope_("boxes_up_kernel", s);
-        boxes_up_kernel<<<grid_n, kThreads, 0, s>>>(verts, reinterpret_cast<const uint4*>(faces), n, t, counters, err);
+        boxes_up_kernel<<<grid_n, kThreads, 0, s>>>(verts, reinterpret_cast<const uint4*>(faces), n, t, tris, rec, ci,
+                                                    ct, counters, err);
     }
     OBVH_TRY_CUDA(cudaGetLastError());
     int32_t gamma = static_cast<int32_t>(tau);
-    const unsigned grid_t = (n + kTreeletThreads - 1) / kTreeletThreads;
     for (uint32_t it = 0; it < iterations; ++it) {
-        OBVH_TRY_CUDA(cudaMemsetAsync(counters, 0, 4ull * internal, s));
+        // arrival counters, then the queue's two words behind them
+        uint32_t* queue = counters + internal;
+        OBVH_TRY_CUDA(cudaMemsetAsync(counters, 0, 4ull * (internal + 2), s));
+        OBVH_TRY_CUDA(cudaMemcpyAsync(sah, rec, 4ull * (2ull * n - 1), cudaMemcpyDeviceToDevice, s));
+        {
+            ProfScope prof_scope_("treelet_starts_kernel", s);
+            treelet_starts_kernel<<<(internal + kThreads - 1) / kThreads, kThreads, 0, s>>>(
+                t, tris, static_cast<int32_t>(n), gamma, starts, queue);
+        }
+        OBVH_TRY_CUDA(cudaGetLastError());
+        const PassArgs pa{t, sah, rec, tris, static_cast<int32_t>(n), static_cast<int>(tau), gamma, ci};
+        const bool last = it + 1 == iterations;
         {
             ProfScope prof_scope_("treelet_kernel", s);
-            float* sah = reinterpret_cast<float*>(ws + L.sah);
-            int32_t* tris = reinterpret_cast<int32_t*>(ws + L.tris);
-            const int32_t nn = static_cast<int32_t>(n);
-            const int tt = static_cast<int>(tau);
-            if (tau <= 8)
-                treelet_kernel<8><<<grid_t, kTreeletThreads, 0, s>>>(t, sah, tris, counters, nn, tt, gamma, ci, ct, err);
-            else if (tau <= 16)
-                treelet_kernel<16><<<grid_t, kTreeletThreads, 0, s>>>(t, sah, tris, counters, nn, tt, gamma, ci, ct, err);
-            else
-                treelet_kernel<32><<<grid_t, kTreeletThreads, 0, s>>>(t, sah, tris, counters, nn, tt, gamma, ci, ct, err);
+            if (tau <= 8) launch_pass<8>(pa, counters, starts, queue, err, last, s);
+            else if (tau <= 16) launch_pass<16>(pa, counters, starts, queue, err, last, s);
+            else launch_pass<32>(pa, counters, starts, queue, err, last, s);
         }
         OBVH_TRY_CUDA(cudaGetLastError());
         gamma = gamma > (1 << 29) ? gamma : 2 * gamma;

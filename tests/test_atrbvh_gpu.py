@@ -70,6 +70,25 @@ def test_lattice_ties(builder):
     _check_tree(o, ref.atrbvh_build(v, f, 7, 2), f.shape[0])
 
 
+@pytest.mark.parametrize("iters,tau", [(3, 3), (3, 8), (3, 9), (2, 16), (3, 17), (2, 20)])
+@pytest.mark.parametrize("kind", ["lattice", "soup"])
+def test_passes_over_every_segment_width(builder, kind, iters, tau):
+    """Treelets of 8, 16 and 32 lanes at the edges of their sizes, several
+    passes (each starts from the SAHs the one before kept up), ties."""
+    v, f = lattice_mesh(9) if kind == "lattice" else workloads.triangle_soup(5003, seed=77)
+    o, _ = _run(builder, v, f, flags=0, tau=tau, iters=iters)
+    r = ref.atrbvh_build(v, f, tau, iters)
+    _check_tree(o, r, f.shape[0])
+    assert same_bits(o["costs"].cpu().numpy(), r["costs"])
+
+
+@pytest.mark.parametrize("n", [1024, 1025, 400_000, 400_001])
+def test_seed_tree_at_sort_tile_edges(builder, n):
+    v, f = workloads.triangle_soup(n, seed=n)
+    o, _ = _run(builder, v, f, flags=0, iters=0)
+    _check_tree(o, ref.atrbvh_build(v, f, 9, 0), n)
+
+
 def _pin_mesh(kind):
     if kind == "soup":
         return workloads.triangle_soup(20_000, seed=1500)
