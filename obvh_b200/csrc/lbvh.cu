@@ -286,7 +286,7 @@ kr_error enqueue_codes(const kr_vec3* verts, const kr_uvec4* faces, uint32_t n, 
     kr_aabb3* boxes = reinterpret_cast<kr_aabb3*>(ws + L.boxes);
     // the sort's counts and status words are zeroed first; the codes kernel
     // counts the digits as it writes the keys
-    OBVH_TRY(radix_sort_prepare(ws + L.sort, n, 0, 30, s));
+    OBVH_TRY(radix_sort_prepare(ws + L.sort, n, 4, 0, 30, s));
     OBVH_TRY(enqueue_bounds(verts, faces, n, tri, ws, boxes, boxes + 1, true, s));
     {
         const sortdev::SortTemp st = sortdev::sort_temp(ws + L.sort);

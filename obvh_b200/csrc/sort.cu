@@ -72,8 +72,16 @@ using sortdev::kSortThreads;
 using sortdev::SortTemp;
 using sortdev::sort_temp;
 constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kRounds = 16;                       // keys per lane
-constexpr int kSortTile = kSortThreads * kRounds;  // 4096 keys per CTA
+// Keys per lane: 16 (tiles of 4,096 keys), or 4 (tiles of 1,024) for few keys,
+// where the passes are latency: a quarter of the ranking rounds, and four times
+// the CTAs.  The limits lie where the two meet (us a build, tiles of 4,096 /
+// 1,024): u32 keys, LBVH + OBB tree + collapse, 1,021 triangles 138.5 / 126.6,
+// 57,344 252 / 236, 200,003 328 / 330, 1,000,003 820 / 838; u64 keys, ATRBVH,
+// 14,336 697 / 639, 307,200 1,303 / 1,278, 917,504 2,417 / 2,445.
+constexpr int kRoundsLarge = 16, kRoundsSmall = 4;
+constexpr uint64_t kSmallSort32 = 150000, kSmallSort64 = 400000;
+constexpr bool is_small(uint64_t n, int key_bytes) { return n <= (key_bytes == 4 ? kSmallSort32 : kSmallSort64); }
+constexpr uint64_t sort_tile(bool small) { return kSortThreads * (small ? kRoundsSmall : kRoundsLarge); }
 
 // ---------------------------------------------------------------------------
 // Stable LSD radix sort, one sweep per 8-bit digit (the single-pass scheme of
@@ -114,8 +122,9 @@ __global__ void __launch_bounds__(kSortThreads) radix_digit_counts(const K* keys
     sortdev::finish_digit_counts(h, passes, digits, ticket);
 }
 
-template <typename K>
+template <typename K, int kRounds>
 struct ScatterSmem {
+    static constexpr int kSortTile = kSortThreads * kRounds;
     uint32_t wcount[kSortWarps][kRadix];
     uint32_t tstart[kRadix];
     uint32_t gbase[kRadix];
@@ -127,13 +136,15 @@ struct ScatterSmem {
 
 // 4 CTAs per SM for u32 keys (64 registers): every tile of 2M keys is
 // resident at once, so no tile waits for a slot; u64 keys keep 2.
-template <typename K>
-__global__ void __launch_bounds__(kSortThreads, sizeof(K) == 4 ? 4 : 2) radix_onesweep(const K* keys_in, const uint32_t* vals_in, K* keys_out,
+template <typename K, int kRounds>
+__global__ void __launch_bounds__(kSortThreads, sizeof(K) == 4 || kRounds == kRoundsSmall ? 4 : 2) radix_onesweep(const K* keys_in, const uint32_t* vals_in, K* keys_out,
                                                                uint32_t* vals_out, uint64_t n, int shift,
                                                                const uint32_t* offsets, uint32_t* status,
                                                                uint32_t* tile_counter, uint32_t* err) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    ScatterSmem<K>& sm = *reinterpret_cast<ScatterSmem<K>*>(smem_raw);
+    using Smem = ScatterSmem<K, kRounds>;
+    constexpr int kSortTile = Smem::kSortTile;
+    Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int i = threadIdx.x; i < kSortWarps * kRadix; i += kSortThreads) (&sm.wcount[0][0])[i] = 0;
     if (threadIdx.x == 0) sm.tile = atomicAdd(tile_counter, 1u);
@@ -244,8 +255,8 @@ __global__ void __launch_bounds__(kSortThreads, sizeof(K) == 4 ? 4 : 2) radix_on
     }
 }
 
-size_t prepared_bytes(uint64_t n, int begin_bit, int end_bit) {
-    const uint32_t ntiles = static_cast<uint32_t>(div_up(n, kSortTile));
+size_t prepared_bytes(uint64_t n, int key_bytes, int begin_bit, int end_bit) {
+    const uint32_t ntiles = static_cast<uint32_t>(div_up(n, sort_tile(is_small(n, key_bytes))));
     const int passes = (end_bit - begin_bit + 7) / 8;
     return kSortHeader + static_cast<size_t>(passes) * ntiles * kRadix * 4;
 }
@@ -255,21 +266,19 @@ kr_error sort_impl(K* keys, K* keys_alt, uint32_t* vals, uint32_t* vals_alt, uin
                    void* temp, cudaStream_t stream, bool* in_alt, uint32_t* err, bool counted) {
     *in_alt = false;
     if (n <= 1 || end_bit <= begin_bit) return kr_success;
-    const uint32_t ntiles = static_cast<uint32_t>(div_up(n, kSortTile));
+    const bool small = is_small(n, sizeof(K));
+    const uint32_t ntiles = static_cast<uint32_t>(div_up(n, sort_tile(small)));
     const int passes = (end_bit - begin_bit + 7) / 8;
     if (passes > kMaxPasses) return "radix_sort_pairs: at most 64 key bits";
     const SortTemp t = sort_temp(temp);
-    static bool configured = false;
-    if (!configured) {
-        OBVH_TRY_CUDA(cudaFuncSetAttribute(radix_onesweep<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           static_cast<int>(sizeof(ScatterSmem<K>))));
-        configured = true;
-    }
+    const auto pass = small ? radix_onesweep<K, kRoundsSmall> : radix_onesweep<K, kRoundsLarge>;
+    const size_t smem = small ? sizeof(ScatterSmem<K, kRoundsSmall>) : sizeof(ScatterSmem<K, kRoundsLarge>);
+    OBVH_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(pass), smem));
     // with counted, the key producer zeroed the header and the status words
     // (radix_sort_prepare) and wrote the digit offsets
     if (!counted) {
         // counts, tile counters, error word and this sort's status words start at zero
-        OBVH_TRY_CUDA(cudaMemsetAsync(temp, 0, prepared_bytes(n, begin_bit, end_bit), stream));
+        OBVH_TRY_CUDA(cudaMemsetAsync(temp, 0, prepared_bytes(n, sizeof(K), begin_bit, end_bit), stream));
         ProfScope prof_scope_("radix_digit_counts", stream);
         int grid = 2 * device_info().sm_count;
         const uint64_t need = div_up(n, kSortThreads);
@@ -284,7 +293,7 @@ kr_error sort_impl(K* keys, K* keys_alt, uint32_t* vals, uint32_t* vals_alt, uin
     for (int p = 0; p < passes; ++p) {
         {
             ProfScope prof_scope_("radix_onesweep", stream);
-            radix_onesweep<K><<<ntiles, kSortThreads, sizeof(ScatterSmem<K>), stream>>>(
+            pass<<<ntiles, kSortThreads, smem, stream>>>(
                 src_k, src_v, dst_k, dst_v, n, begin_bit + 8 * p, t.digits + p * kRadix,
                 t.status + static_cast<size_t>(p) * ntiles * kRadix, t.tiles + p, err ? err : t.err);
         }
@@ -340,7 +349,9 @@ kr_error exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint64_t n, uint3
 }
 
 size_t radix_sort_temp_bytes(uint64_t n) {
-    const uint64_t ntiles = div_up(n > 0 ? n : 1, kSortTile);
+    // the most that any count up to n needs (a workspace for n serves fewer)
+    const uint64_t few = std::min<uint64_t>(n > 0 ? n : 1, kSmallSort64);
+    const uint64_t ntiles = std::max(div_up(few, sort_tile(true)), div_up(n, sort_tile(false)));
     return kSortHeader + static_cast<size_t>(kMaxPasses) * ntiles * kRadix * 4;
 }
 
@@ -359,10 +370,10 @@ kr_error radix_sort_pairs(void* keys, void* keys_alt, uint32_t* vals, uint32_t* 
     return "radix_sort_pairs: key_bytes must be 4 or 8";
 }
 
-kr_error radix_sort_prepare(void* temp, uint64_t n, int begin_bit, int end_bit, cudaStream_t stream) {
+kr_error radix_sort_prepare(void* temp, uint64_t n, int key_bytes, int begin_bit, int end_bit, cudaStream_t stream) {
     if (n <= 1 || end_bit <= begin_bit) return kr_success;
     if ((end_bit - begin_bit + 7) / 8 > kMaxPasses) return "radix_sort_prepare: at most 64 key bits";
-    OBVH_TRY_CUDA(cudaMemsetAsync(temp, 0, prepared_bytes(n, begin_bit, end_bit), stream));
+    OBVH_TRY_CUDA(cudaMemsetAsync(temp, 0, prepared_bytes(n, key_bytes, begin_bit, end_bit), stream));
     return kr_success;
 }
 

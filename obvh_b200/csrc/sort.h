@@ -34,7 +34,7 @@ kr_error radix_sort_pairs(void* keys, void* keys_alt, uint32_t* vals, uint32_t* 
                           uint32_t* err = nullptr, bool counted = false);
 // Zeroes the digit counts, the tickets and the status words of a sort of n
 // keys by bits [begin_bit, end_bit), for a key producer that counts digits.
-kr_error radix_sort_prepare(void* temp, uint64_t n, int begin_bit, int end_bit, cudaStream_t stream);
+kr_error radix_sort_prepare(void* temp, uint64_t n, int key_bytes, int begin_bit, int end_bit, cudaStream_t stream);
 uint32_t* radix_sort_error_word(void* temp);
 
 }  // namespace obvh

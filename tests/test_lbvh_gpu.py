@@ -52,6 +52,13 @@ def test_soup_sizes(builder, n):
     _compare(_build(builder, v, f), obvh_oracle.lbvh_build(v, f), n)
 
 
+@pytest.mark.parametrize("n", [1023, 1024, 1025, 149_999, 150_000, 150_001])
+def test_sort_tile_edges(builder, n):
+    """Around a tile of the sort for few keys, and where it gives way to the larger tiles."""
+    v, f = workloads.triangle_soup(n, seed=n)
+    _compare(_build(builder, v, f), obvh_oracle.lbvh_build(v, f), n)
+
+
 def test_full_size_soup(builder):
     """The 2,000,000-triangle LBVH workload."""
     n = 2_000_000
