@@ -24,6 +24,7 @@
 #include <cstdint>
 
 #include "device_common.cuh"
+#include "lbvh_device.cuh"
 #include "lbvh_host.h"
 #include "obb_tree_host.h"
 #include "obvh_build.h"
@@ -46,7 +47,7 @@ struct Ctl {
     uint32_t error;
     uint32_t total_units;
     uint32_t total_slots;
-    uint32_t frontier;  // walks left for the cross-CTA pass
+    uint32_t spare;
     uint32_t across;    // nodes the cross-CTA pass completed (listed at Layout::across)
     uint32_t pad[59];
 };
@@ -73,14 +74,44 @@ __device__ __forceinline__ uint32_t* stage_at(uint32_t* stage, const void* dst, 
 // Sorted leaf j: node internal + j, its triangle at slot j, its own box.  The
 // CTA's leaves are consecutive, so every output is one contiguous run per CTA:
 // records are staged in shared memory and written out coalesced.
-__global__ void __launch_bounds__(kThreads) leaves_fused_kernel(const uint32_t* order,
+//
+// Odd CTAs build the Karras tree over the sorted codes instead (karras_node:
+// it needs the codes alone, so the two were one launch after the other; side
+// by side the tree's searches run while the leaves wait for memory).  The first
+// CTA also clears the chain's control block, which nothing reads before the
+// next kernel, and copies the scene and centroid boxes out.
+struct TreeArgs {
+    const uint32_t* codes;
+    uint32_t* parents;
+    uint32_t* first;
+    uint32_t* counts;
+    uint32_t* ctl;         // kCtlWords of them
+    const float* boxes;
+    float* bounds;         // nullable
+};
+constexpr uint32_t kCtlWords = sizeof(Ctl) / 4;
+
+__global__ void __launch_bounds__(kThreads) leaves_fused_kernel(TreeArgs tree_args, const uint32_t* order,
                                                                 const kr_vec3* verts, const uint4* faces, uint32_t n,
                                                                 kr_bvh_node* nodes, kr_bvh_node* collapsed,
                                                                 float* tris, kr_obb3* obbs, kr_mat4* xfs,
                                                                 uint32_t* visits, uint8_t* cflags) {
     __shared__ __align__(16) uint32_t stage_a[kThreads * 15 + 4];  // node (9), triangle (9) or box (15) records
     __shared__ __align__(16) uint32_t stage_x[kThreads * 16 + 4];  // transforms
-    const uint32_t j0 = blockIdx.x * blockDim.x;
+    const uint32_t j0 = (blockIdx.x >> 1) * blockDim.x;
+    if (blockIdx.x & 1) {
+        const uint32_t i = j0 + threadIdx.x;
+        if (n >= 2 && i < n - 1)
+            lbvh::karras_node(tree_args.codes, n, static_cast<int>(i), nodes, tree_args.parents, tree_args.first,
+                              tree_args.counts);
+        else if (n == 1 && i == 0)
+            tree_args.parents[0] = kNoParent;
+        return;
+    }
+    if (blockIdx.x == 0) {
+        for (uint32_t k = threadIdx.x; k < kCtlWords; k += kThreads) tree_args.ctl[k] = 0u;
+        if (tree_args.bounds && threadIdx.x < 12) tree_args.bounds[threadIdx.x] = tree_args.boxes[threadIdx.x];
+    }
     const uint32_t j = j0 + threadIdx.x;
     const uint32_t count = min(static_cast<uint32_t>(blockDim.x), n - j0);
     const bool live = j < n;
@@ -167,7 +198,7 @@ struct LocalSmem {
     uint8_t queue[3][kThreads]; // nodes ready in a round
     uint8_t local[kThreads], iflag[kThreads], lflag[kThreads], hidden[kThreads];
     uint32_t qn[3];
-    uint32_t nfront, front_base;
+    uint32_t nfront;
 };
 constexpr size_t kFusedSmemBytes = sizeof(LocalSmem);
 
@@ -231,7 +262,7 @@ __device__ __forceinline__ void leaf_vertices(const LocalSmem& sm, uint32_t q, f
 // memory, and the outputs are written at the end as contiguous runs.  The
 // leaves and local nodes whose parents are not local go to a list for part 2.
 __global__ void __launch_bounds__(kThreads, 4) fused_up_local_kernel(UpArgs a, uint32_t* frontier,
-                                                                     uint32_t* frontier_count) {
+                                                                     uint32_t* frontier_counts) {
     extern __shared__ __align__(16) unsigned char fused_smem[];
     LocalSmem& sm = *reinterpret_cast<LocalSmem*>(fused_smem);
     const uint32_t t = threadIdx.x;
@@ -451,46 +482,193 @@ __global__ void __launch_bounds__(kThreads, 4) fused_up_local_kernel(UpArgs a, u
     const bool node_walk = !bad && mine && parent != kNoParent && sm.up[t] == kNotLocal;
     const uint32_t nf = static_cast<uint32_t>(leaf_walk) + static_cast<uint32_t>(node_walk);
     const uint32_t at = nf ? atomicAdd(&sm.nfront, nf) : 0u;
+    if (nf && at + nf <= kThreads) {  // the roots of a forest over the CTA's leaves: at most kThreads
+        uint32_t* list = frontier + blockIdx.x * kThreads;
+        if (leaf_walk) list[at] = internal + j0 + t;
+        if (node_walk) list[at + (leaf_walk ? 1 : 0)] = p;
+    } else if (nf) {
+        atomicOr(a.err, kErrBadInput);
+    }
     __syncthreads();
-    if (t == 0) sm.front_base = sm.nfront ? atomicAdd(frontier_count, sm.nfront) : 0u;
-    __syncthreads();
-    if (leaf_walk) frontier[sm.front_base + at] = internal + j0 + t;
-    if (node_walk) frontier[sm.front_base + at + (leaf_walk ? 1 : 0)] = p;
+    if (t == 0) frontier_counts[blockIdx.x] = min(sm.nfront, static_cast<uint32_t>(kThreads));
+}
+
+// The listed node's carry and summary, then its walk.
+template <Src Sib, class Arrive>
+__device__ __forceinline__ void walk_listed(const UpArgs& a, uint32_t x, Arrive arrive_at) {
+    const uint32_t internal = a.n - 1;
+    Carry c;
+    {
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(a.nodes + x);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            c.lo[k] = __uint_as_float(__ldcg(w + k));
+            c.hi[k] = __uint_as_float(__ldcg(w + 3 + k));
+        }
+    }
+    c.cost = __ldcg(a.costs + x);
+    Summary s;
+    if (a.summary) {
+        if (x >= internal) {
+            const kr_vec3* pts = reinterpret_cast<const kr_vec3*>(a.tris);
+            f3 v[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) v[k] = load_vertex(pts, 3 * (x - internal) + k);
+#pragma unroll
+            for (int k = 0; k < 7; ++k) set_slab(s, k, leaf_slab(v, x - internal, k));
+        } else {
+            load_summary(a.summary + 7 * static_cast<size_t>(x), s);
+        }
+    }
+    walk_up<Src::kReadOnly, Sib>(a, x, c, s, arrive_at);
 }
 
 // Bottom-up pass, part 2 of 2: the walks from the listed nodes complete the
 // nodes whose leaf ranges cross a CTA's edge.  Part 1 has finished, so a
 // listed node's outputs are in memory.
+//
+// The walk is a chain of levels whose cost is their ordering, so CTA b takes
+// the lists of the part-1 CTAs over 2^kSuperShift consecutive leaves: a node
+// whose leaves lie inside them has both arrivals from this CTA, and a byte in
+// shared memory between CTA-scope fences counts them; only the nodes above pay
+// the GPU-scope release, atomic and acquire.  A walk belongs to 8 lanes: 7
+// merge a slab of the summary each, the last one completes the node (a thread
+// to a walk ran some 600 instructions a level, lanes diverging).  A group
+// whose walk ends takes the next one.  More leaves a CTA mean fewer levels
+// above but more walks to a CTA; us a build with a thread to a walk and global
+// arrivals / 2^10 / 2^11 / 2^12 leaves: 1,021 triangles 129 / 114 / 114 / 114,
+// 57,344 236 / 208 / 214 / 213, 200,003 336 / 307 / 316 / 317, 500,003 466 /
+// 467 / 467 / 469, 2,000,000 1,551 / 1,558 / 1,551 / 1,535.
+constexpr uint32_t kSuperShiftSmall = 10, kSuperShiftLarge = 12;
+constexpr uint32_t kSuperLarge = 1u << 20;
+
+template <uint32_t kSuperShift>
+struct SuperArrive {
+    uint32_t* bytes;  // one per node index of the superblock (a node's index lies in its leaf range)
+    __device__ __forceinline__ uint32_t operator()(const UpArgs& a, uint32_t p) const {
+        const uint32_t f = __ldg(a.first + p), l = f + __ldg(a.counts + p) - 1;
+        if ((f >> kSuperShift) != (l >> kSuperShift)) return arrive(a.visits + p);
+        const uint32_t q = p & ((1u << kSuperShift) - 1), shift = 8u * (q & 3u);
+        __threadfence_block();  // release: this thread's outputs before its arrival
+        const uint32_t old = atomicAdd(bytes + (q >> 2), 1u << shift);  // a byte counts at most 2: no carry
+        __threadfence_block();  // acquire: the sibling's outputs after it
+        return (old >> shift) & 0xffu;
+    }
+};
+
+template <uint32_t kSuperShift>
 __global__ void __launch_bounds__(kThreads) fused_up_cross_kernel(UpArgs a, const uint32_t* frontier,
-                                                                  const uint32_t* frontier_count) {
-    const uint32_t total = *frontier_count;
+                                                                  const uint32_t* frontier_counts, uint32_t blocks) {
+    constexpr uint32_t kSuperBlocks = 1u << (kSuperShift - kLocalShift);
+    __shared__ uint32_t bytes[(1u << kSuperShift) / 4];
+    __shared__ uint32_t start[kSuperBlocks + 1], next;
+    const uint32_t t = threadIdx.x, b0 = blockIdx.x * kSuperBlocks;
     const uint32_t internal = a.n - 1;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        const uint32_t x = frontier[i];
-        Carry c;
-        {
-            const uint32_t* w = reinterpret_cast<const uint32_t*>(a.nodes + x);
+    for (uint32_t i = t; i < (1u << kSuperShift) / 4; i += kThreads) bytes[i] = 0;
+    if (t < 32) {  // where each list starts among this CTA's walks
+        uint32_t run = 0;
+        for (uint32_t q0 = 0; q0 < kSuperBlocks; q0 += 32) {
+            const uint32_t q = q0 + t;
+            const uint32_t c = q < kSuperBlocks && b0 + q < blocks ? frontier_counts[b0 + q] : 0u;
+            uint32_t incl = c;
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                c.lo[k] = __uint_as_float(__ldcg(w + k));
-                c.hi[k] = __uint_as_float(__ldcg(w + 3 + k));
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
+                if (static_cast<int>(t) >= d) incl += v;
             }
+            if (q < kSuperBlocks) start[q] = run + incl - c;
+            run += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (t == 0) {
+            start[kSuperBlocks] = run;
+            next = 0;
+        }
+    }
+    __syncthreads();
+    const uint32_t lane = t & 7;  // of the walk's group
+    const uint32_t total = start[kSuperBlocks];
+    const SuperArrive<kSuperShift> arrive_at{bytes};
+    const kr_vec3* pts = reinterpret_cast<const kr_vec3*>(a.tris);
+    const bool slabs = a.summary != nullptr && lane < 7;
+    // slab `lane` of node x's summary; what was read may come from this kernel
+    const auto read_slab = [&](uint32_t x) -> Slab {
+        if (x >= internal) {
+            const f3 v[3] = {load_vertex(pts, 3 * (x - internal)), load_vertex(pts, 3 * (x - internal) + 1),
+                             load_vertex(pts, 3 * (x - internal) + 2)};
+            return leaf_slab(v, x - internal, static_cast<int>(lane));
+        }
+        const uint4 q = __ldcg(a.summary + 7 * static_cast<size_t>(x) + lane);
+        return Slab{__uint_as_float(q.x), __uint_as_float(q.y), q.z, q.w};
+    };
+    const auto read_carry = [&](uint32_t x) {
+        Carry c;
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(a.nodes + x);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            c.lo[k] = __uint_as_float(__ldcg(w + k));
+            c.hi[k] = __uint_as_float(__ldcg(w + 3 + k));
         }
         c.cost = __ldcg(a.costs + x);
-        Summary s;
-        if (a.summary) {
-            if (x >= internal) {
-                const kr_vec3* pts = reinterpret_cast<const kr_vec3*>(a.tris);
-                f3 v[3];
-#pragma unroll
-                for (int k = 0; k < 3; ++k) v[k] = load_vertex(pts, 3 * (x - internal) + k);
-#pragma unroll
-                for (int k = 0; k < 7; ++k) set_slab(s, k, leaf_slab(v, x - internal, k));
-            } else {
-                load_summary(a.summary + 7 * static_cast<size_t>(x), s);
+        return c;
+    };
+    bool live = false, dry = false;
+    uint32_t child = 0, p = kNoParent, steps = 0;
+    Slab own{0.f, 0.f, 0u, 0u};
+    Carry c{{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, 0.f};
+    for (;;) {
+        // a group whose walk has ended takes the next one
+        uint32_t i = total;
+        if (!live && !dry && lane == 0) i = atomicAdd(&next, 1u);
+        i = __shfl_sync(0xffffffffu, i, 0, 8);
+        if (!live && !dry) {
+            dry = i >= total;
+            if (!dry) {
+                uint32_t q = 0;  // the last list that starts at or before walk i
+                for (uint32_t step = kSuperBlocks / 2; step > 0; step >>= 1)
+                    if (start[q + step] <= i) q += step;
+                child = frontier[(b0 + q) * kThreads + (i - start[q])];
+                p = a.parents[child];
+                steps = 0;
+                live = true;
+                if (slabs) own = read_slab(child);
+                if (lane == 7) c = read_carry(child);
             }
         }
-        walk_up(a, x, c, s);
+        if (!__any_sync(0xffffffffu, live)) break;
+        if (live && (++steps > internal || p >= internal)) {
+            if (lane == 0 && p != kNoParent) atomicOr(a.err, kErrCycle);
+            live = false;
+        }
+        uint32_t L = 0, R = 0, grand = kNoParent, count = 0, before = 0;
+        if (live) {
+            // written before this kernel: read ahead of the arrival
+            const uint32_t* pw = reinterpret_cast<const uint32_t*>(a.nodes + p);
+            L = __ldg(pw + 6);
+            R = __ldg(pw + 7);
+            grand = __ldg(a.parents + p);
+            count = __ldg(a.counts + p);
+            if (lane == 0) before = arrive_at(a, p);
+        }
+        before = __shfl_sync(0xffffffffu, before, 0, 8);
+        __syncwarp();  // orders the group's loads after lane 0's acquire
+        live = live && before != 0;
+        if (live) {
+            const bool from_left = L == child;
+            const uint32_t other = from_left ? R : L;
+            if (lane == 7) {
+                const Carry o = read_carry(other);
+                c = complete_node(a, p, L, R, count, from_left ? c : o, from_left ? o : c);
+            }
+            if (slabs) {
+                const Slab sib = read_slab(other);
+                own = merge_slab(from_left ? own : sib, from_left ? sib : own);
+                store_slab(a.summary, p, static_cast<int>(lane), own);
+            }
+            if (lane == 0 && a.done_list) a.done_list[atomicAdd(a.done_count, 1u)] = p;
+            child = p;
+            p = grand;
+        }
+        __syncwarp();  // the group's outputs before lane 0's next release
     }
 }
 
@@ -576,7 +754,7 @@ Layout layout(uint32_t n) {
     L.sizes = o;    o += align256(4 * nn);
     L.offsets = o;  o += align256(4 * nn);
     L.scan = o;     o += align256(scan_temp_bytes(nn));
-    L.frontier = o; o += align256(4 * nn);
+    L.frontier = o; o += align256(4 * nn + 4 * kThreads);
     L.chains = o;   o += align256(obbtree::chain_bytes(n));
     L.chain_counts = o; o += align256(obbtree::chain_count_bytes(n));
     L.across = o;   o += align256(4 * ni);
@@ -619,18 +797,18 @@ kr_error enqueue(const kr_vec3* verts, const kr_uvec4* faces, uint32_t n, uint32
     uint8_t* cflags = reinterpret_cast<uint8_t*>(ws + L.flags);
     const unsigned gn = (n + kThreads - 1) / kThreads;
 
-    OBVH_TRY_CUDA(cudaMemsetAsync(ctl, 0, sizeof(Ctl), s));
     lbvh::Codes c;
     OBVH_TRY(lbvh::enqueue_codes(verts, faces, n, ws + L.lbvh, s, &c));
     {
         ProfScope prof_scope_("leaves_fused_kernel", s);
-        leaves_fused_kernel<<<gn, kThreads, 0, s>>>(c.order, verts, reinterpret_cast<const uint4*>(faces),
+        const TreeArgs ta{c.codes, parents, first, counts, reinterpret_cast<uint32_t*>(ctl),
+                          reinterpret_cast<const float*>(c.boxes), reinterpret_cast<float*>(bounds)};
+        leaves_fused_kernel<<<2 * gn, kThreads, 0, s>>>(ta, c.order, verts, reinterpret_cast<const uint4*>(faces),
                                                     n, nodes, want_collapse ? collapsed : nullptr, tris,
                                                     want_obbs ? obbs : nullptr, xfs, c.visits,
                                                     want_collapse ? cflags : nullptr);
     }
     OBVH_TRY_CUDA(cudaGetLastError());
-    OBVH_TRY(lbvh::enqueue_karras(c.codes, n, nodes, parents, first, counts, s));
     OBVH_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(fused_up_local_kernel), kFusedSmemBytes));
     // Two helper streams.  aux[0] (the highest priority, so that its CTAs
     // are placed first) takes the latency-bound walk up the top of the tree
@@ -664,10 +842,13 @@ kr_error enqueue(const kr_vec3* verts, const kr_uvec4* faces, uint32_t n, uint32
     {
         UpArgs a{nodes, want_collapse ? collapsed : nullptr, parents, first, tris, n, counts, costs,
                  want_collapse ? cflags : nullptr, ci, ct, want_obbs ? summary : nullptr, c.visits, &ctl->error};
+        // per part-1 CTA: the list of its walks, and its length (the collapse's
+        // sizes are written after the walk)
         uint32_t* frontier = reinterpret_cast<uint32_t*>(ws + L.frontier);
+        uint32_t* lists = reinterpret_cast<uint32_t*>(ws + L.sizes);
         {
             ProfScope prof_scope_("fused_up_local_kernel", s);
-            fused_up_local_kernel<<<gn, kThreads, kFusedSmemBytes, s>>>(a, frontier, &ctl->frontier);
+            fused_up_local_kernel<<<gn, kThreads, kFusedSmemBytes, s>>>(a, frontier, lists);
         }
         OBVH_TRY_CUDA(cudaGetLastError());
         OBVH_TRY(fork_to(*fk, 0, s));
@@ -676,13 +857,17 @@ kr_error enqueue(const kr_vec3* verts, const kr_uvec4* faces, uint32_t n, uint32
             a.done_list = across;
             a.done_count = &ctl->across;
         }
-        // at most one walk per leaf and per internal node; most of the grid
-        // finds nothing to do, so it is capped at a few CTAs per SM
-        const unsigned cap = 8u * static_cast<unsigned>(device_info().sm_count);
-        const unsigned gx = (nn + kThreads - 1) / kThreads;
         {
             ProfScope prof_scope_("fused_up_cross_kernel", ws0);
-            fused_up_cross_kernel<<<gx < cap ? gx : cap, kThreads, 0, ws0>>>(a, frontier, &ctl->frontier);
+            if (n <= kSuperLarge) {
+                constexpr unsigned kBlocks = 1u << (kSuperShiftSmall - kLocalShift);
+                fused_up_cross_kernel<kSuperShiftSmall>
+                    <<<(gn + kBlocks - 1) / kBlocks, kThreads, 0, ws0>>>(a, frontier, lists, gn);
+            } else {
+                constexpr unsigned kBlocks = 1u << (kSuperShiftLarge - kLocalShift);
+                fused_up_cross_kernel<kSuperShiftLarge>
+                    <<<(gn + kBlocks - 1) / kBlocks, kThreads, 0, ws0>>>(a, frontier, lists, gn);
+            }
         }
         OBVH_TRY_CUDA(cudaGetLastError());
         if (want_collapse) {
@@ -715,7 +900,6 @@ kr_error enqueue(const kr_vec3* verts, const kr_uvec4* faces, uint32_t n, uint32
     }
     if (frames) OBVH_TRY(obbtree::enqueue_extents(fb, internal, obbs, xfs, s));
     if (want_collapse) OBVH_TRY(join_from(*fk, 1, s));
-    if (bounds) OBVH_TRY_CUDA(cudaMemcpyAsync(bounds, c.boxes, 2 * sizeof(kr_aabb3), cudaMemcpyDeviceToDevice, s));
     return kr_success;
 }
 
