@@ -22,7 +22,7 @@
 //                one unit combine partial results, with 6 integer atomics per
 //                unit.  Nodes finished here are finalised in place (:903-964).
 //                For a Karras tree (the fused build), tiles instead: one CTA
-//                per 1,024 consecutive leaves stages their triangles in shared
+//                per 1,024 (256) consecutive leaves stages their triangles in shared
 //                memory once and serves every node over them from there.
 //   finalize     the nodes of more than one unit or tile.
 #include <cuda_runtime.h>
@@ -48,16 +48,24 @@ constexpr int kThreads = 256;
 constexpr uint32_t kCollapseLeafMax = 8;  // MAX_LEAF_SIZE (transforms.cu:65)
 constexpr uint32_t kUnit = 1024;    // leaves per warp unit
 constexpr uint32_t kUnitRun = 4;   // consecutive units per warp visit
-constexpr int kTileShift = 10;      // tiled extents: 1,024 leaves per tile
-constexpr uint32_t kTile = 1u << kTileShift;
+// Tiled extents: 1,024 leaves per tile, or 256 for up to kSmallTiles leaves, so
+// that a small tree spreads over more SMs (us a build, 1,024 / 256: 1,021
+// triangles 111 / 99, 10,007 157 / 141, 57,344 211 / 195, 200,003 299 / 274,
+// 500,003 466 / 473, 2,000,000 1,534 / 1,614).
+constexpr uint32_t kTileShiftLarge = 10, kTileShiftSmall = 8;
+constexpr uint32_t kSmallTiles = 300000;
+constexpr uint32_t tile_shift(uint32_t n) { return n <= kSmallTiles ? kTileShiftSmall : kTileShiftLarge; }
+constexpr uint32_t tiles_of(uint32_t n) {
+    return static_cast<uint32_t>((static_cast<uint64_t>(n) + (1u << tile_shift(n)) - 1) >> tile_shift(n));
+}
 // Ancestors of a leaf in a Karras tree over 30-bit codes with the index
 // tie-break: each level lengthens the common prefix of the 62-bit (code,
 // index) keys, so there are at most 62.
 constexpr uint32_t kChain = 64;
 // Extents items per tile kept in shared memory: of 8 lanes, and in all.  With
 // the triangles they fit the 48 KB of a static allocation.
-constexpr uint32_t kTileGroups = 160;
-constexpr uint32_t kTileItems = 320;
+constexpr uint32_t tile_groups(uint32_t shift) { return shift == kTileShiftLarge ? 160 : 48; }
+constexpr uint32_t tile_items(uint32_t shift) { return shift == kTileShiftLarge ? 320 : 224; }
 
 struct Ctl {
     uint32_t error;
@@ -371,6 +379,7 @@ struct ChainArgs {
     float nz;                 // -0.0f (tree::mul2)
     uint32_t which;           // FrameNodes: all nodes, or those inside / across aligned leaf blocks
     uint32_t block_shift;     // the blocks hold 2^block_shift leaves
+    uint32_t tile_shift;      // the tiles 2^tile_shift
     const uint32_t* list;     // kAcross: the nodes, list_count of them
     const uint32_t* list_count;
 };
@@ -379,10 +388,10 @@ struct ChainArgs {
 // leaf ranges are not inside the tile: the nodes the tile serves partially.
 // A node on both chains is listed on side 0 only.
 __device__ void walk_chain(const ChainArgs& c, const uint32_t* counts, uint32_t w) {
-    const uint32_t ntiles = (c.n + kTile - 1) >> kTileShift;
-    if (w >= 2 * ntiles) return;
+    const uint32_t tile = 1u << c.tile_shift;
+    if (w >= 2 * ((c.n + tile - 1) >> c.tile_shift)) return;
     const uint32_t tau = w >> 1, side = w & 1;
-    const uint32_t t0 = tau << kTileShift, tend = min(t0 + kTile, c.n);
+    const uint32_t t0 = tau << c.tile_shift, tend = min(t0 + tile, c.n);
     const uint32_t internal = c.n - 1;
     uint32_t* out = c.chains + static_cast<size_t>(w) * kChain;
     uint32_t count = 0;
@@ -422,7 +431,7 @@ __device__ __forceinline__ void candidate_store(uint32_t a, const Summary& s, co
     uint32_t units;
     if (chain.parents) {  // tiles: 0 in one tile and small, 1 in one tile, 2 over several tiles
         const uint32_t f = __ldg(chain.first + a);
-        units = (f >> kTileShift) != ((f + cnt - 1) >> kTileShift) ? 2u : (cnt > kGroupLeaves ? 1u : 0u);
+        units = (f >> chain.tile_shift) != ((f + cnt - 1) >> chain.tile_shift) ? 2u : (cnt > kGroupLeaves ? 1u : 0u);
     } else {
         units = cnt > kGroupLeaves ? (cnt + kUnit - 1) / kUnit : 0u;
     }
@@ -581,9 +590,9 @@ __global__ void __launch_bounds__(kThreads) extents_units_kernel(const Cand* can
 // itself in arrivals[a]; the part that completes the count reads the keys and
 // writes the box.
 __device__ __forceinline__ bool last_part(const uint32_t* counts, const uint32_t* first, uint32_t* arrivals,
-                                          uint32_t a) {
+                                          uint32_t a, uint32_t shift) {
     const uint32_t f = __ldg(first + a), cnt = __ldg(counts + a);
-    const uint32_t parts = ((f + cnt - 1) >> kTileShift) - (f >> kTileShift) + 1;
+    const uint32_t parts = ((f + cnt - 1) >> shift) - (f >> shift) + 1;
     if (atomicAdd(arrivals + a, 1u) + 1u != parts) return false;
     __threadfence();
     return true;
@@ -598,20 +607,23 @@ __device__ __forceinline__ void finalize_keys(const Cand* cand, const uint32_t* 
 constexpr uint32_t kPart = 0x80000000u;   // item over part of its node
 constexpr uint32_t kIdle = 0xffffffffu;   // item with nothing left to finalise
 
+template <uint32_t kTileItems>
 struct TileItems {
     uint32_t node[kTileItems];
     uint16_t b[kTileItems], e[kTileItems];
     float ext[kTileItems][6];
 };
 
+template <uint32_t kTileShift>
 __global__ void __launch_bounds__(kThreads) extents_tile_kernel(const Cand* cand, const uint32_t* counts,
                                                                 const uint32_t* first, const float* tris, uint32_t n,
                                                                 const uint32_t* chains, const uint32_t* chain_counts,
                                                                 uint32_t* keys, uint32_t* arrivals, kr_obb3* obbs,
                                                                 kr_mat4* xfs, const uint32_t* err, float nz) {
+    constexpr uint32_t kTile = 1u << kTileShift, kTileGroups = tile_groups(kTileShift), kTileItems = tile_items(kTileShift);
     __shared__ __align__(16) float tri[kTile * 9];
     // group items from the front, warp items from the back
-    __shared__ TileItems items;
+    __shared__ TileItems<kTileItems> items;
     __shared__ uint32_t ngroup, nwarp, next_group, next_warp;
     if (*err) return;
     const uint32_t t = threadIdx.x, lane = t & 31;
@@ -640,7 +652,7 @@ __global__ void __launch_bounds__(kThreads) extents_tile_kernel(const Cand* cand
                 atomicMax(kk + 3 + k, f2key(hi[k]));
             }
             __threadfence();
-            if (last_part(counts, first, arrivals, a)) finalize_keys(cand, keys, a, obbs, xfs);
+            if (last_part(counts, first, arrivals, a, kTileShift)) finalize_keys(cand, keys, a, obbs, xfs);
         } else {
             finalize_node(c, mk3(fminf(c.olo[0], lo[0]), fminf(c.olo[1], lo[1]), fminf(c.olo[2], lo[2])),
                           mk3(fmaxf(c.ohi[0], hi[0]), fmaxf(c.ohi[1], hi[1]), fmaxf(c.ohi[2], hi[2])), obbs + a,
@@ -699,7 +711,7 @@ __global__ void __launch_bounds__(kThreads) extents_tile_kernel(const Cand* cand
                 __threadfence();
             }
             __syncwarp();
-            if (lane == 0 && !last_part(counts, first, arrivals, a)) items.node[at] = kIdle;
+            if (lane == 0 && !last_part(counts, first, arrivals, a, kTileShift)) items.node[at] = kIdle;
         } else if (lane < 6) {
             items.ext[at][lane] = v;
         }
@@ -845,20 +857,25 @@ const uint32_t* dfs_prims(const void* workspace, uint32_t n) {
 }
 
 size_t cand_bytes(uint32_t internal) { return sizeof(Cand) * (internal > 0 ? internal : 1); }
-size_t chain_bytes(uint32_t n) { return 2ull * kChain * 4 * (((n > 0 ? n : 1) + kTile - 1) >> kTileShift); }
-size_t chain_count_bytes(uint32_t n) { return 2ull * 4 * (((n > 0 ? n : 1) + kTile - 1) >> kTileShift); }
+// (the most tiles of any count up to n: a workspace for n serves fewer)
+static size_t most_tiles(uint32_t n) {
+    const uint32_t few = n < kSmallTiles ? (n > 0 ? n : 1) : kSmallTiles;
+    return tiles_of(n) > tiles_of(few) ? tiles_of(n) : tiles_of(few);
+}
+size_t chain_bytes(uint32_t n) { return 2ull * kChain * 4 * most_tiles(n); }
+size_t chain_count_bytes(uint32_t n) { return 2ull * 4 * most_tiles(n); }
 
 namespace {
 ChainArgs chain_args(const FrameBuffers& b, uint32_t internal, FrameNodes which, uint32_t block_shift) {
     const uint32_t n = internal + 1;
     const bool tiled = b.chains != nullptr;
-    const uint32_t ntiles = (n + kTile - 1) >> kTileShift;
+    const uint32_t ntiles = tiles_of(n);
     // the chain walks ride along with the first (or only) candidate launch
     const bool walks = tiled && which != FrameNodes::kAcross;
     return ChainArgs{tiled ? b.parents : nullptr, b.first, n,
                      walks ? (2 * ntiles + kThreads - 1) / kThreads : 0u,
                      b.chains, b.chain_counts, b.err, b.ustart, -0.0f,
-                     static_cast<uint32_t>(which), block_shift, b.across_list, b.across_count};
+                     static_cast<uint32_t>(which), block_shift, tile_shift(n), b.across_list, b.across_count};
 }
 }  // namespace
 
@@ -898,13 +915,13 @@ kr_error enqueue_extents(const FrameBuffers& b, uint32_t internal, kr_obb3* obbs
     Cand* cand = static_cast<Cand*>(b.cand);
     const uint32_t n = internal + 1;
     const bool tiled = b.chains != nullptr;
-    const uint32_t ntiles = (n + kTile - 1) >> kTileShift;
     if (tiled) {
         {
             ProfScope prof_scope_("extents_tile_kernel", s);
-            extents_tile_kernel<<<ntiles, kThreads, 0, s>>>(cand, b.counts, b.first, b.tris, n, b.chains,
-                                                            b.chain_counts, b.keys, b.ustart, obbs, xfs, b.err,
-                                                            -0.0f);
+            const auto kernel = tile_shift(n) == kTileShiftSmall ? extents_tile_kernel<kTileShiftSmall>
+                                                                 : extents_tile_kernel<kTileShiftLarge>;
+            kernel<<<tiles_of(n), kThreads, 0, s>>>(cand, b.counts, b.first, b.tris, n, b.chains, b.chain_counts,
+                                                    b.keys, b.ustart, obbs, xfs, b.err, -0.0f);
         }
         OBVH_TRY_CUDA(cudaGetLastError());
         return kr_success;
