@@ -5,6 +5,8 @@
 //                for the leaves) and the scene and centroid AABBs (per-CTA
 //                records, the last CTA reduces; kr_cuda_bbox_calculate and
 //                kr_cuda_centroid_bbox_calculate, transforms.cu:1127-1250)
+//                (up to 2,048 triangles: one CTA does this, the codes and the
+//                sort, front_kernel)
 //   morton       30-bit codes of the centroids normalised by the centroid
 //                AABB (mortons_kernel, lbvh.cu:252-282)
 //   radix sort   stable (key, index) sort (sort.cu; thrust::stable_sort_by_key
@@ -232,6 +234,139 @@ __global__ void __launch_bounds__(kThreads) aabb_up_kernel(kr_bvh_node* nodes, c
     }
 }
 
+// Boxes, codes and the sort of up to kFrontMax triangles in one CTA: at these
+// sizes the six launches and the memset it replaces are latency only (us a
+// build, without / with it: 1,021 triangles 92 / 84, 1,500 106 / 100, 2,048 113
+// / 113; at 4,000, with larger buffers, 123 / 133).  Keys
+// and values stay in shared memory through the four 8-bit passes; warp w takes
+// the w-th run of 32 * rounds keys, ranks them in order (match_any), and the
+// counts are scanned digit by digit, warp by warp, so the order is stable.
+constexpr int kFrontThreads = 1024, kFrontWarps = kFrontThreads / 32;
+constexpr uint32_t kFrontMax = 2048;
+constexpr int kFrontRounds = kFrontMax / kFrontThreads;
+struct FrontSmem {
+    uint32_t keys[2][kFrontMax];
+    uint16_t vals[2][kFrontMax];
+    uint16_t count[kFrontWarps][256];
+    uint32_t warp_sum[kFrontWarps];
+    float red[kFrontWarps][12];
+    float box[12];
+};
+
+__global__ void __launch_bounds__(kFrontThreads) front_kernel(const kr_vec3* verts, const uint4* faces, uint32_t n,
+                                                              float* tri_boxes, kr_aabb3* boxes, uint32_t* keys_out,
+                                                              uint32_t* vals_out) {
+    extern __shared__ __align__(16) unsigned char front_smem[];
+    FrontSmem& sm = *reinterpret_cast<FrontSmem*>(front_smem);
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    float acc[12];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        acc[k] = kInf; acc[3 + k] = -kInf; acc[6 + k] = kInf; acc[9 + k] = -kInf;
+    }
+    for (uint32_t i = t; i < n; i += kFrontThreads) {
+        f3 lo, hi;
+        tri_box(verts, __ldg(faces + i), lo, hi);
+        float* b = tri_boxes + 6 * static_cast<size_t>(i);
+        b[0] = lo.x; b[1] = lo.y; b[2] = lo.z; b[3] = hi.x; b[4] = hi.y; b[5] = hi.z;
+        const f3 c = tree::mulv(add3(lo, hi), 0.5f);  // kr_aabb_center3
+        acc[0] = fminf(acc[0], lo.x); acc[1] = fminf(acc[1], lo.y); acc[2] = fminf(acc[2], lo.z);
+        acc[3] = fmaxf(acc[3], hi.x); acc[4] = fmaxf(acc[4], hi.y); acc[5] = fmaxf(acc[5], hi.z);
+        acc[6] = fminf(acc[6], c.x); acc[7] = fminf(acc[7], c.y); acc[8] = fminf(acc[8], c.z);
+        acc[9] = fmaxf(acc[9], c.x); acc[10] = fmaxf(acc[10], c.y); acc[11] = fmaxf(acc[11], c.z);
+    }
+#pragma unroll
+    for (int k = 0; k < 12; ++k) acc[k] = (k % 6) < 3 ? warp_min(acc[k]) : warp_max(acc[k]);
+    if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < 12; ++k) sm.red[w][k] = acc[k];
+    __syncthreads();
+    if (w < 12) {  // warp k folds value k of every warp
+        const float v = sm.red[lane][w];
+        const float r = (w % 6) < 3 ? warp_min(v) : warp_max(v);
+        if (lane == 0) {
+            sm.box[w] = r;
+            reinterpret_cast<float*>(boxes)[w] = r;
+        }
+    }
+    __syncthreads();
+    const uint32_t rounds = (n + kFrontThreads - 1) / kFrontThreads;
+    const uint32_t first = w * 32 * rounds;
+    for (uint32_t i = t; i < n; i += kFrontThreads) {  // the boxes this thread wrote
+        sm.keys[0][i] = morton_code(tri_boxes + 6 * static_cast<size_t>(i), sm.box + 6);
+        sm.vals[0][i] = static_cast<uint16_t>(i);
+    }
+    for (int pass = 0; pass < kMortonPasses; ++pass) {
+        const uint32_t* kin = sm.keys[pass & 1];
+        const uint16_t* vin = sm.vals[pass & 1];
+        uint32_t* kout = sm.keys[~pass & 1];
+        uint16_t* vout = sm.vals[~pass & 1];
+        reinterpret_cast<uint4*>(sm.count)[t] = make_uint4(0, 0, 0, 0);
+        __syncthreads();
+        uint32_t key[kFrontRounds];
+        uint32_t pos[kFrontRounds];
+#pragma unroll
+        for (int r = 0; r < kFrontRounds; ++r) {
+            if (r >= static_cast<int>(rounds)) break;
+            const uint32_t i = first + r * 32 + lane;
+            const bool ok = i < n;
+            key[r] = ok ? kin[i] : 0u;
+            const uint32_t d = ok ? (key[r] >> (8 * pass)) & 255u : 256u;
+            const uint32_t peers = __match_any_sync(0xffffffffu, d);
+            const uint32_t below = peers & ((1u << lane) - 1u);
+            const uint32_t before = sm.count[w][ok ? d : 0];
+            __syncwarp();
+            pos[r] = before + __popc(below);
+            if (ok && below == 0) sm.count[w][d] = static_cast<uint16_t>(before + __popc(peers));
+            __syncwarp();
+        }
+        __syncthreads();
+        // exclusive offsets, digits in order and within a digit the warps:
+        // thread t takes 8 warps of digit t / 4
+        const int d = t >> 2, w0 = (t & 3) * 8;
+        uint32_t c[8], sum = 0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            c[q] = sm.count[w0 + q][d];
+            sum += c[q];
+        }
+        uint32_t incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) sm.warp_sum[w] = incl;
+        __syncthreads();
+        uint32_t run = incl - sum;
+        {
+            const uint32_t mine = lane < w ? sm.warp_sum[lane] : 0u;
+            run += __reduce_add_sync(0xffffffffu, mine);
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            sm.count[w0 + q][d] = static_cast<uint16_t>(run);
+            run += c[q];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kFrontRounds; ++r) {
+            if (r >= static_cast<int>(rounds)) break;
+            const uint32_t i = first + r * 32 + lane;
+            if (i < n) {
+                const uint32_t at = sm.count[w][(key[r] >> (8 * pass)) & 255u] + pos[r];
+                kout[at] = key[r];
+                vout[at] = vin[i];
+            }
+        }
+        __syncthreads();
+    }
+    for (uint32_t i = t; i < n; i += kFrontThreads) {
+        keys_out[i] = sm.keys[kMortonPasses & 1][i];
+        vals_out[i] = sm.vals[kMortonPasses & 1][i];
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Host side.
 size_t align256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
@@ -284,6 +419,21 @@ kr_error enqueue_codes(const kr_vec3* verts, const kr_uvec4* faces, uint32_t n, 
     const Layout L = layout(n);
     float* tri = reinterpret_cast<float*>(ws + L.tri);
     kr_aabb3* boxes = reinterpret_cast<kr_aabb3*>(ws + L.boxes);
+    out->codes = reinterpret_cast<const uint32_t*>(ws + L.keys0);
+    out->order = reinterpret_cast<const uint32_t*>(ws + L.vals0);
+    out->tri_boxes = tri;
+    out->boxes = boxes;
+    out->visits = reinterpret_cast<uint32_t*>(ws + L.visits);
+    out->err = &reinterpret_cast<Ctl*>(ws + L.ctl)->error;
+    if (n <= kFrontMax) {
+        OBVH_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(front_kernel), sizeof(FrontSmem)));
+        ProfScope prof_scope_("front_kernel", s);
+        front_kernel<<<1, kFrontThreads, sizeof(FrontSmem), s>>>(
+            verts, reinterpret_cast<const uint4*>(faces), n, tri, boxes, reinterpret_cast<uint32_t*>(ws + L.keys0),
+            reinterpret_cast<uint32_t*>(ws + L.vals0));
+        OBVH_TRY_CUDA(cudaGetLastError());
+        return kr_success;
+    }
     // the sort's counts and status words are zeroed first; the codes kernel
     // counts the digits as it writes the keys
     OBVH_TRY(radix_sort_prepare(ws + L.sort, n, 4, 0, 30, s));
@@ -302,12 +452,10 @@ kr_error enqueue_codes(const kr_vec3* verts, const kr_uvec4* faces, uint32_t n, 
     OBVH_TRY(radix_sort_pairs(ws + L.keys0, ws + L.keys1, reinterpret_cast<uint32_t*>(ws + L.vals0),
                               reinterpret_cast<uint32_t*>(ws + L.vals1), n, 4, 0, 30, ws + L.sort, s, &alt,
                               &reinterpret_cast<Ctl*>(ws + L.ctl)->error, n >= 2));
-    out->codes = reinterpret_cast<const uint32_t*>(ws + (alt ? L.keys1 : L.keys0));
-    out->order = reinterpret_cast<const uint32_t*>(ws + (alt ? L.vals1 : L.vals0));
-    out->tri_boxes = tri;
-    out->boxes = boxes;
-    out->visits = reinterpret_cast<uint32_t*>(ws + L.visits);
-    out->err = &reinterpret_cast<Ctl*>(ws + L.ctl)->error;
+    if (alt) {
+        out->codes = reinterpret_cast<const uint32_t*>(ws + L.keys1);
+        out->order = reinterpret_cast<const uint32_t*>(ws + L.vals1);
+    }
     return kr_success;
 }
 

@@ -71,6 +71,26 @@ def test_fused_build_matches_the_three_steps(builder, n):
     _check(o, slots, _expect(v, f), n, 3)
 
 
+@pytest.mark.parametrize("n", [255, 256, 257, 1023, 1024, 1025, 2047, 2048, 2049, 4097, 8193, 300_000, 300_001])
+def test_fused_build_at_block_tile_and_sort_edges(builder, n):
+    """Around the bottom-up pass's blocks, the extents' tiles (256 leaves up to
+    300,000, then 1,024), the walk's superblocks and the one-CTA front end."""
+    v, f = workloads.triangle_soup(n, seed=700 + n)
+    o, slots = _run(builder, v, f, 3)
+    _check(o, slots, _expect(v, f), n, 3)
+
+
+def test_workspace_grows_with_the_face_count():
+    """A builder keeps the workspace of its largest mesh for smaller ones."""
+    from obvh_b200 import _native
+    lib = _native.lib()
+    edges = [2048, 8192, 131_072, 150_000, 262_144, 300_000, 400_000, 1 << 20]
+    sizes = sorted({1, 2, 1000, 10_007, 2_000_000} | {e + d for e in edges for d in (-1, 0, 1)})
+    for query in (lib.obvh_build_workspace_bytes, lib.obvh_atrbvh_workspace_bytes, lib.obvh_lbvh_workspace_bytes):
+        got = [query(n) for n in sizes]
+        assert got == sorted(got)
+
+
 def test_fused_build_full_size(builder):
     v, f = workloads.triangle_soup(2_000_000, seed=1)
     o, slots = _run(builder, v, f, 3)
