@@ -493,36 +493,6 @@ __global__ void __launch_bounds__(kThreads, 4) fused_up_local_kernel(UpArgs a, u
     if (t == 0) frontier_counts[blockIdx.x] = min(sm.nfront, static_cast<uint32_t>(kThreads));
 }
 
-// The listed node's carry and summary, then its walk.
-template <Src Sib, class Arrive>
-__device__ __forceinline__ void walk_listed(const UpArgs& a, uint32_t x, Arrive arrive_at) {
-    const uint32_t internal = a.n - 1;
-    Carry c;
-    {
-        const uint32_t* w = reinterpret_cast<const uint32_t*>(a.nodes + x);
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            c.lo[k] = __uint_as_float(__ldcg(w + k));
-            c.hi[k] = __uint_as_float(__ldcg(w + 3 + k));
-        }
-    }
-    c.cost = __ldcg(a.costs + x);
-    Summary s;
-    if (a.summary) {
-        if (x >= internal) {
-            const kr_vec3* pts = reinterpret_cast<const kr_vec3*>(a.tris);
-            f3 v[3];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) v[k] = load_vertex(pts, 3 * (x - internal) + k);
-#pragma unroll
-            for (int k = 0; k < 7; ++k) set_slab(s, k, leaf_slab(v, x - internal, k));
-        } else {
-            load_summary(a.summary + 7 * static_cast<size_t>(x), s);
-        }
-    }
-    walk_up<Src::kReadOnly, Sib>(a, x, c, s, arrive_at);
-}
-
 // Bottom-up pass, part 2 of 2: the walks from the listed nodes complete the
 // nodes whose leaf ranges cross a CTA's edge.  Part 1 has finished, so a
 // listed node's outputs are in memory.
