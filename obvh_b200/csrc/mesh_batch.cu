@@ -13,8 +13,8 @@
 //     __match_any_sync within a warp and a block scan across warps
 //   4 leaves: records, sorted triangles, leaf boxes and transforms
 //   5 Karras tree, first leaves and leaf counts
-//   6 bottom-up pass from every leaf (walk_up of the whole-GPU chain: bounds,
-//     costs, collapse marks, 7-direction summaries)
+//   6 bottom-up pass from every leaf (bounds, costs, collapse marks,
+//     7-direction summaries)
 //   7 candidate frames of the internal nodes
 //   8 extents over each node's leaf run (a thread, 8 lanes or a warp by its
 //     size) and the final boxes
@@ -29,7 +29,9 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <functional>
 #include <mutex>
+#include <queue>
 #include <vector>
 
 #include "device_common.cuh"
@@ -48,18 +50,15 @@ namespace meshbatch {
 
 using namespace tree;
 
-#ifndef OBVH_MESH_BATCH_THREADS
-#define OBVH_MESH_BATCH_THREADS 256
-#endif
-constexpr int kThreads = OBVH_MESH_BATCH_THREADS;  // one mesh per CTA of this many threads
-constexpr int kCtasPerSm = 512 / kThreads;           // the SM's registers at 128 per thread
-constexpr int kWarps = kThreads / 32;
-// Shared-memory carveout, in percent of the SM's maximum: room for kCtasPerSm
-// CTAs of static shared memory (33 KB each), the rest of the unified memory L1.
+// One mesh per CTA of kThreads threads: two CTAs of 256 to an SM, or one of
+// 512 (the SM's registers at 128 per thread either way).  See choose_threads.
+constexpr int kNarrow = 256, kWide = 512;
+constexpr int ctas_per_sm(int threads) { return kWide / threads; }
+// Shared-memory carveout, in percent of the SM's maximum: room for the
+// CTAs' static shared memory (33 KB each), the rest of the unified memory L1.
 constexpr int kSmemCarveout = 32;
 constexpr uint32_t kMaxFaces = OBVH_BUILD_BATCH_CTA_MAX_FACES;
-constexpr uint32_t kMaxRounds = kMaxFaces / kThreads;  // sort rounds of kThreads keys
-static_assert(kMaxFaces % kThreads == 0, "whole sort rounds");
+static_assert(kMaxFaces % kWide == 0, "whole sort rounds");
 static_assert(kMaxFaces <= 65535, "sort ranks are 16-bit");
 
 struct Job {
@@ -120,7 +119,10 @@ struct Args {
     float nz;              // -0.0f (tree::mul2)
 };
 
+template <int kThreads>
 struct Smem {
+    static constexpr int kWarps = kThreads / 32;
+    static constexpr uint32_t kMaxRounds = kMaxFaces / kThreads;  // sort rounds of kThreads keys
     uint16_t table[16 * kMaxRounds * kWarps];  // sort: digit counts per (digit, round, warp)
     uint32_t visits[kMaxFaces / 4];            // bottom-up arrivals: one byte per internal node
     float red[kWarps][12];
@@ -173,8 +175,9 @@ __device__ __forceinline__ void stage_sync() {
 
 // Exclusive scan of `len` values in place (u16 in shared memory or u32 in
 // global memory), by the whole CTA; returns the total to every thread.
-template <class T>
-__device__ uint32_t block_scan(T* data, uint32_t len, Smem& sm) {
+template <int kThreads, class T>
+__device__ uint32_t block_scan(T* data, uint32_t len, Smem<kThreads>& sm) {
+    constexpr uint32_t kWarps = kThreads / 32;
     const uint32_t t = threadIdx.x, lane = t & 31, w = t >> 5;
     const uint32_t chunk = (len + kThreads - 1) / kThreads;
     const uint32_t c0 = min(len, t * chunk), c1 = min(len, c0 + chunk);
@@ -214,8 +217,10 @@ __device__ uint32_t block_scan(T* data, uint32_t len, Smem& sm) {
 }
 
 // One stable pass of the LSD radix sort over 4 key bits.
+template <int kThreads>
 __device__ void sort_pass(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout, uint32_t n,
-                          int shift, Smem& sm) {
+                          int shift, Smem<kThreads>& sm) {
+    constexpr uint32_t kWarps = kThreads / 32;
     const uint32_t t = threadIdx.x, lane = t & 31, w = t >> 5;
     const uint32_t rounds = (n + kThreads - 1) / kThreads;
     const uint32_t cols = rounds * kWarps;
@@ -229,7 +234,7 @@ __device__ void sort_pass(const uint32_t* kin, const uint32_t* vin, uint32_t* ko
             sm.table[d * cols + r * kWarps + w] = static_cast<uint16_t>(__popc(same));
     }
     __syncthreads();
-    block_scan(sm.table, 16 * cols, sm);
+    block_scan<kThreads>(sm.table, 16 * cols, sm);
     const uint32_t below = (1u << lane) - 1u;
     for (uint32_t r = 0; r < rounds; ++r) {
         const uint32_t e = r * kThreads + t;
@@ -254,7 +259,9 @@ __device__ __forceinline__ obbtree::Cand load_cand_own(const obbtree::Cand* cand
     return c;
 }
 
-__device__ void build_mesh(const Args& a, const Job& J, char* slot, Smem& sm) {
+template <int kThreads>
+__device__ void build_mesh(const Args& a, const Job& J, char* slot, Smem<kThreads>& sm) {
+    constexpr int kWarps = kThreads / 32;
     const uint32_t t = threadIdx.x, lane = t & 31, w = t >> 5;
     const uint32_t n = J.n, ni = n - 1, nn = 2 * n - 1;
     JobBases B;
@@ -341,8 +348,8 @@ __device__ void build_mesh(const Args& a, const Job& J, char* slot, Smem& sm) {
     }
     stage_sync();
     for (int pass = 0; pass < 8; pass += 2) {
-        sort_pass(keys_a, vals_a, keys_b, vals_b, n, 4 * pass, sm);
-        sort_pass(keys_b, vals_b, keys_a, vals_a, n, 4 * pass + 4, sm);
+        sort_pass<kThreads>(keys_a, vals_a, keys_b, vals_b, n, 4 * pass, sm);
+        sort_pass<kThreads>(keys_b, vals_b, keys_a, vals_a, n, 4 * pass + 4, sm);
     }
 
     // ---- 4: leaves (leaves_fused_kernel) ---------------------------------------
@@ -374,33 +381,50 @@ __device__ void build_mesh(const Args& a, const Job& J, char* slot, Smem& sm) {
                                                                   first, counts);
     stage_sync();
 
-    // ---- 6: bottom-up pass from every leaf (walk_up of the chain) ------------
+    // ---- 6: bottom-up pass from every leaf -----------------------------------
+    // Thread t walks up from the leaves of its run [t R, (t + 1) R), in order.
+    // Each round every lane of a warp does one thing: the next leaf of its run
+    // where its last walk has ended, then one level.  (A loop over the leaves
+    // around a loop over the levels made the warp wait for its longest walk at
+    // every leaf: 7.22 -> 7.13 ms on the 2,048-mesh batch.)
     {
         pipeline::UpArgs ua{nodes,  collapsed, parents, first, tris, n, counts, costs, want_collapse ? flags : nullptr,
                             B.ci,   B.ct,      want_obbs ? summary : nullptr, nullptr, a.err};
-        // thread t walks up from the leaves of its run [t R, (t + 1) R), in order
         const uint32_t run = (n + kThreads - 1) / kThreads;
         const CtaArrive arrive{sm.visits, first, counts, run, t};
-        for (uint32_t j = t * run, jend = min(n, (t + 1) * run); j < jend; ++j) {
-            const uint32_t x = ni + j;
-            pipeline::Carry c;
-            const uint32_t* wd = reinterpret_cast<const uint32_t*>(nodes + x);
+        uint32_t j = t * run, child = 0, p = kNoParent, steps = 0;
+        const uint32_t jend = min(n, (t + 1) * run);
+        bool walking = false;
+        pipeline::Carry c{};
+        Summary s;
+        while (__any_sync(0xffffffffu, walking || j < jend)) {
+            if (!walking && j < jend) {
+                child = ni + j;
+                const uint32_t* wd = reinterpret_cast<const uint32_t*>(nodes + child);
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                c.lo[k] = __uint_as_float(ld_own(wd + k));
-                c.hi[k] = __uint_as_float(ld_own(wd + 3 + k));
+                for (int k = 0; k < 3; ++k) {
+                    c.lo[k] = __uint_as_float(ld_own(wd + k));
+                    c.hi[k] = __uint_as_float(ld_own(wd + 3 + k));
+                }
+                c.cost = leaf_ct * box_area(c.lo, c.hi);
+                if (want_obbs) {
+                    const kr_vec3* pts = reinterpret_cast<const kr_vec3*>(tris);
+                    f3 v[3];
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) v[k] = load_vertex_src<Src::kOwnCta>(pts, 3 * j + k);
+#pragma unroll
+                    for (int k = 0; k < 7; ++k) pipeline::set_slab(s, k, pipeline::leaf_slab(v, j, k));
+                }
+                p = ld_own(parents + child);
+                steps = 0;
+                walking = true;
+                ++j;
             }
-            c.cost = leaf_ct * box_area(c.lo, c.hi);
-            Summary s;
-            if (want_obbs) {
-                const kr_vec3* pts = reinterpret_cast<const kr_vec3*>(tris);
-                f3 v[3];
-#pragma unroll
-                for (int k = 0; k < 3; ++k) v[k] = load_vertex_src<Src::kOwnCta>(pts, 3 * j + k);
-#pragma unroll
-                for (int k = 0; k < 7; ++k) pipeline::set_slab(s, k, pipeline::leaf_slab(v, j, k));
-            }
-            pipeline::walk_up<Src::kOwnCta, Src::kOwnCta>(ua, x, c, s, arrive);
+            __syncwarp();
+            if (walking)
+                walking = p != kNoParent && ++steps <= n &&
+                          pipeline::walk_step<Src::kOwnCta, Src::kOwnCta>(ua, child, p, c, s, arrive);
+            __syncwarp();
         }
     }
     stage_sync();
@@ -492,7 +516,7 @@ __device__ void build_mesh(const Args& a, const Job& J, char* slot, Smem& sm) {
         stage_sync();
         for (uint32_t c = t; c < nn; c += kThreads) offsets[c] = ld_own(sizes + c);
         stage_sync();
-        const uint32_t total = block_scan(offsets, nn, sm);
+        const uint32_t total = block_scan<kThreads>(offsets, nn, sm);
         if (t == 0) a.mesh_slots[J.mesh] = total;
         stage_sync();
         uint32_t* prims = B.primitives;
@@ -535,8 +559,9 @@ __device__ void build_mesh(const Args& a, const Job& J, char* slot, Smem& sm) {
     stage_sync();
 }
 
-__global__ void __launch_bounds__(kThreads, kCtasPerSm) mesh_batch_kernel(Args a) {
-    __shared__ Smem sm;
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads, ctas_per_sm(kThreads)) mesh_batch_kernel(Args a) {
+    __shared__ Smem<kThreads> sm;
     char* slot = a.scratch + static_cast<size_t>(blockIdx.x) * a.slot_bytes;
     for (;;) {
         if (threadIdx.x == 0) sm.job = atomicAdd(a.next_job, 1u);
@@ -545,7 +570,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) mesh_batch_kernel(Args a
         __syncthreads();
         if (j >= a.njobs) return;
         const Job J = a.jobs[j];
-        build_mesh(a, J, slot, sm);
+        build_mesh<kThreads>(a, J, slot, sm);
     }
 }
 
@@ -563,6 +588,7 @@ struct Plan {
     std::vector<Job> cta_jobs;  // largest first
     std::vector<Job> chain_jobs;
     uint32_t chain_max = 0;
+    int threads = kNarrow;
     int grid = 0;
     SlotLayout slot{};
     DeviceBuffer jobs, scratch, chain_ws, status;  // status: [0] error, [1] job counter, [2..] slots
@@ -656,10 +682,39 @@ kr_error enqueue(Plan& P, const Buffers& b, cudaStream_t s) {
         a.mesh_slots = status + 2;
         a.nz = -0.0f;
         ProfScope prof_scope_("mesh_batch_kernel", s);
-        mesh_batch_kernel<<<P.grid, kThreads, 0, s>>>(a);
+        const auto kernel = P.threads == kWide ? mesh_batch_kernel<kWide> : mesh_batch_kernel<kNarrow>;
+        kernel<<<P.grid, P.threads, 0, s>>>(a);
         OBVH_TRY_CUDA(cudaGetLastError());
     }
     return kr_success;
+}
+
+// The larger of the CTAs' loads (faces) when each takes the next largest mesh
+// as it becomes free.
+uint64_t largest_load(const std::vector<Job>& jobs, size_t ctas) {
+    std::priority_queue<uint64_t, std::vector<uint64_t>, std::greater<uint64_t>> load;
+    uint64_t most = 0;
+    for (const Job& J : jobs) {
+        uint64_t l = J.n;
+        if (load.size() == ctas) {
+            l += load.top();
+            load.pop();
+        }
+        load.push(l);
+        most = std::max(most, l);
+    }
+    return most;
+}
+
+// Narrow or wide CTAs.  A wide one builds a mesh 1.85 times as fast as a narrow
+// one, so two narrow ones do 8% more work; but a batch lasts as long as its
+// most loaded CTA, and where a few large meshes set that, wide ones win.
+// Measured (ms, narrow / wide; 64..16,384 triangles): 100 meshes 3.24 / 2.40,
+// 300 4.76 / 2.54, 2,048 7.12 / 7.73; 600 of 64..4,096 1.30 / 0.89.
+int choose_threads(const std::vector<Job>& jobs, size_t sms) {
+    const double narrow = static_cast<double>(largest_load(jobs, sms * ctas_per_sm(kNarrow)));
+    const double wide = static_cast<double>(largest_load(jobs, sms * ctas_per_sm(kWide)));
+    return wide < 1.85 * narrow ? kWide : kNarrow;
 }
 
 kr_error plan(Plan& P, const kr_size* voff, const kr_size* foff, kr_size meshes) {
@@ -684,11 +739,13 @@ kr_error plan(Plan& P, const kr_size* voff, const kr_size* foff, kr_size meshes)
     std::stable_sort(P.cta_jobs.begin(), P.cta_jobs.end(), [](const Job& x, const Job& y) { return x.n > y.n; });
     P.slot = slot_layout(P.cta_max);
     const int sms = device_info().sm_count;
-    P.grid = static_cast<int>(std::min<size_t>(P.cta_jobs.size(), static_cast<size_t>(sms) * kCtasPerSm));
+    P.threads = choose_threads(P.cta_jobs, static_cast<size_t>(sms));
+    P.grid = static_cast<int>(std::min<size_t>(P.cta_jobs.size(), static_cast<size_t>(sms) * ctas_per_sm(P.threads)));
     // The kernel reads its own writes through L1: leave L1 the SM's unified
     // memory beyond the CTAs' static shared memory (a hint, per device).
-    OBVH_TRY_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(mesh_batch_kernel),
-                                       cudaFuncAttributePreferredSharedMemoryCarveout, kSmemCarveout));
+    for (const void* f : {reinterpret_cast<const void*>(mesh_batch_kernel<kNarrow>),
+                          reinterpret_cast<const void*>(mesh_batch_kernel<kWide>)})
+        OBVH_TRY_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, kSmemCarveout));
     OBVH_TRY(P.status.reserve(4ull * (2 + meshes)));
     OBVH_TRY_CUDA(cudaMemset(P.status.ptr, 0, 4ull * (2 + meshes)));
     if (!P.cta_jobs.empty()) {
@@ -730,7 +787,7 @@ kr_error make_runner(uint32_t capacity, Runner** out) {
     Runner* r = new Runner();
     r->capacity = capacity;
     r->slot = slot_layout(kMaxFaces);
-    r->grid = device_info().sm_count;  // one CTA per SM: a server round holds a few meshes
+    r->grid = device_info().sm_count;  // one wide CTA per SM: a server round holds a few meshes
     kr_error e = kr_success;
     if (cudaGetDevice(&r->device) != cudaSuccess) e = "make_runner: no current device";
     if (!e) e = r->scratch.reserve(r->slot.total * static_cast<size_t>(r->grid));
@@ -738,7 +795,7 @@ kr_error make_runner(uint32_t capacity, Runner** out) {
     if (!e) e = r->bases.reserve(sizeof(JobBases) * capacity);
     if (!e) e = r->status.reserve(4ull * (2 + capacity));
     if (!e) e = r->staging.reserve((sizeof(Job) + sizeof(JobBases)) * capacity);
-    if (!e && cudaFuncSetAttribute(reinterpret_cast<const void*>(mesh_batch_kernel),
+    if (!e && cudaFuncSetAttribute(reinterpret_cast<const void*>(mesh_batch_kernel<kWide>),
                                    cudaFuncAttributePreferredSharedMemoryCarveout, kSmemCarveout) != cudaSuccess)
         e = "make_runner: setting the kernel's carveout failed";
     if (e) {
@@ -795,7 +852,7 @@ kr_error run(Runner& r, const JobBases* bases, const uint32_t* faces, uint32_t c
     a.nz = -0.0f;
     const int grid = static_cast<int>(std::min<uint32_t>(count, static_cast<uint32_t>(r.grid)));
     ProfScope prof_scope_("mesh_batch_kernel", s);
-    mesh_batch_kernel<<<grid, kThreads, 0, s>>>(a);
+    mesh_batch_kernel<kWide><<<grid, kWide, 0, s>>>(a);
     OBVH_TRY_CUDA(cudaGetLastError());
     return kr_success;
 }

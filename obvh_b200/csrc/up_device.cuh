@@ -36,12 +36,6 @@ __device__ __forceinline__ void store_words(kr_bvh_node* nodes, uint32_t i, cons
     for (int k = 0; k < count; ++k) st_dst<S>(d + k, w[k]);
 }
 
-// Summary of sorted leaf j; its vertex ids are the triangle slots 3j..3j+2.
-__device__ __forceinline__ void slot_summary(const float* tris, uint32_t j, Summary& s) {
-    const kr_vec3* pts = reinterpret_cast<const kr_vec3*>(tris);
-    leaf_summary(pts, make_uint4(3 * j, 3 * j + 1, 3 * j + 2, 0), s);
-}
-
 // What a completed node passes to its parent: bounds and SAH cost.
 struct Carry {
     float lo[3], hi[3];
@@ -164,79 +158,66 @@ __device__ __forceinline__ Carry complete_node(const UpArgs& a, uint32_t p, uint
     return o;
 }
 
-// Leaf-to-root walk from node x (carry c, summary s) through nodes whose
-// leaf ranges cross a CTA's edge: the second thread to arrive at a node
-// (arrive_at: a GPU-scope acquire/release counter by default) completes it
-// from the sibling's outputs.
+// One level of a leaf-to-root walk: arrives at p, the parent of `child` (whose
+// carry and summary are c and s), and as the second to arrive completes p from
+// the sibling's outputs; child, p, c and s then stand at p.  False where the
+// walk ends here: the first of two children to arrive, or a malformed tree.
 //
-// Pre says where the node records' children, the parents, the counts and
-// the sorted triangles were written (before the kernel in the chain, by this
-// CTA in the one-CTA-per-mesh batch build), Sib where the sibling's outputs
-// were (in this kernel by any SM in the chain, by this CTA in the batch).
-// Arrival at internal node p through the global counters a.visits
-// (GPU-scope acquire/release): walks from any CTA.
-struct GlobalArrive {
-    __device__ __forceinline__ uint32_t operator()(const UpArgs& a, uint32_t p) const { return arrive(a.visits + p); }
-};
-
-template <Src Pre = Src::kReadOnly, Src Sib = Src::kL2, class Arrive = GlobalArrive>
-__device__ __forceinline__ void walk_up(const UpArgs& a, uint32_t x, Carry c, Summary s,
-                                        Arrive arrive_at = Arrive{}) {
+// Pre says where the node records' children, the parents, the counts and the
+// sorted triangles were written, Sib where the sibling's outputs were.
+template <Src Pre, Src Sib, class Arrive>
+__device__ __forceinline__ bool walk_step(const UpArgs& a, uint32_t& child, uint32_t& p, Carry& c, Summary& s,
+                                          const Arrive& arrive_at) {
     const uint32_t internal = a.n - 1;
-    uint32_t child = x;
-    uint32_t p = a.parents[x];
-    for (uint32_t steps = 0; p != kNoParent; ++steps) {
-        if (steps > internal || p >= internal) {
-            atomicOr(a.err, kErrCycle);
-            return;
-        }
-        // written before this kernel: read ahead of the arrival
-        const uint32_t* pw = reinterpret_cast<const uint32_t*>(a.nodes + p);
-        const uint32_t L = ld_src<Pre>(pw + 6), R = ld_src<Pre>(pw + 7);
-        const uint32_t grand = ld_src<Pre>(a.parents + p);
-        const uint32_t count = ld_src<Pre>(a.counts + p);
-        if (arrive_at(a, p) == 0) return;
-        const bool from_left = (L == child);
-        const uint32_t other = from_left ? R : L;
-        Carry o;
-        {
-            const uint32_t* sw = reinterpret_cast<const uint32_t*>(a.nodes + other);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                o.lo[k] = __uint_as_float(ld_src<Sib>(sw + k));
-                o.hi[k] = __uint_as_float(ld_src<Sib>(sw + 3 + k));
-            }
-        }
-        o.cost = ld_src<Sib>(a.costs + other);
-        c = from_left ? complete_node<Sib>(a, p, L, R, count, c, o) : complete_node<Sib>(a, p, L, R, count, o, c);
-        if (a.summary) {
-            const bool sleaf = other >= internal;
-            f3 v[3];
-            if (sleaf) {
-                const kr_vec3* pts = reinterpret_cast<const kr_vec3*>(a.tris);
-#pragma unroll
-                for (int i = 0; i < 3; ++i)
-                    v[i] = load_vertex_src<Pre>(pts, 3 * (other - internal) + i);
-            }
-#pragma unroll
-            for (int k = 0; k < 7; ++k) {
-                Slab sib;
-                if (sleaf) {
-                    sib = leaf_slab(v, other - internal, k);
-                } else {
-                    const uint4 q = ld_src<Sib>(a.summary + 7 * static_cast<size_t>(other) + k);
-                    sib = Slab{__uint_as_float(q.x), __uint_as_float(q.y), q.z, q.w};
-                }
-                const Slab own = slab_of(s, k);
-                const Slab m = from_left ? merge_slab(own, sib) : merge_slab(sib, own);
-                set_slab(s, k, m);
-                store_slab<Sib>(a.summary, p, k, m);
-            }
-        }
-        if (a.done_list) a.done_list[atomicAdd(a.done_count, 1u)] = p;
-        child = p;
-        p = grand;
+    if (p >= internal) {
+        atomicOr(a.err, kErrCycle);
+        return false;
     }
+    // read ahead of the arrival
+    const uint32_t* pw = reinterpret_cast<const uint32_t*>(a.nodes + p);
+    const uint32_t L = ld_src<Pre>(pw + 6), R = ld_src<Pre>(pw + 7);
+    const uint32_t grand = ld_src<Pre>(a.parents + p);
+    const uint32_t count = ld_src<Pre>(a.counts + p);
+    if (arrive_at(a, p) == 0) return false;
+    const bool from_left = (L == child);
+    const uint32_t other = from_left ? R : L;
+    Carry o;
+    {
+        const uint32_t* sw = reinterpret_cast<const uint32_t*>(a.nodes + other);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            o.lo[k] = __uint_as_float(ld_src<Sib>(sw + k));
+            o.hi[k] = __uint_as_float(ld_src<Sib>(sw + 3 + k));
+        }
+    }
+    o.cost = ld_src<Sib>(a.costs + other);
+    c = complete_node<Sib>(a, p, L, R, count, from_left ? c : o, from_left ? o : c);
+    if (a.summary) {
+        const bool sleaf = other >= internal;
+        f3 v[3];
+        if (sleaf) {
+            const kr_vec3* pts = reinterpret_cast<const kr_vec3*>(a.tris);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) v[i] = load_vertex_src<Pre>(pts, 3 * (other - internal) + i);
+        }
+#pragma unroll
+        for (int k = 0; k < 7; ++k) {
+            Slab sib;
+            if (sleaf) {
+                sib = leaf_slab(v, other - internal, k);
+            } else {
+                const uint4 q = ld_src<Sib>(a.summary + 7 * static_cast<size_t>(other) + k);
+                sib = Slab{__uint_as_float(q.x), __uint_as_float(q.y), q.z, q.w};
+            }
+            const Slab own = slab_of(s, k);
+            const Slab m = merge_slab(from_left ? own : sib, from_left ? sib : own);
+            set_slab(s, k, m);
+            store_slab<Sib>(a.summary, p, k, m);
+        }
+    }
+    child = p;
+    p = grand;
+    return true;
 }
 
 }  // namespace pipeline

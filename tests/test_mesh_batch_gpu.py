@@ -130,3 +130,10 @@ def test_chain_meshes_in_a_graph():
     become parallel branches and every result stays its lone build's."""
     batch = _check(_meshes([20000, 40000, 700, "knot"], seed=50), graph=True)
     assert batch.info()["chain_meshes"] >= 2
+
+
+@pytest.mark.parametrize("count,sizes", [(592, [61, 300]), (592, [2, 8, 9, 33]), (149, [257, 1025]), (3, [16_384, 513, 2])])
+def test_narrow_and_wide_ctas(count, sizes):
+    """592 meshes in equal halves fill two CTAs to an SM twice over (256 threads
+    each); fewer go to one CTA of 512 threads to an SM."""
+    _check(_meshes([sizes[k % len(sizes)] for k in range(count)], seed=4000))
