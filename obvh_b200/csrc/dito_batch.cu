@@ -7,7 +7,7 @@
 // sets of a batch are planned once on the host into a task queue, and one
 // kernel whose CTAs pull tasks from an atomic counter fits them all:
 //
-//   warp task   - up to 8 small sets, one warp each (both passes, the candidate
+//   warp task   - up to 8 (16) small sets, one warp each (both passes, the candidate
 //                 search and the final box by the same warp);
 //   CTA task    - one medium set, both passes by one CTA;
 //   pass-1 task - one chunk of a large set: extremal points of the chunk into a
@@ -29,10 +29,13 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <functional>
 #include <mutex>
 #include <numeric>
+#include <queue>
 #include <vector>
 
 #include "device_common.cuh"
@@ -47,8 +50,8 @@ namespace dito_batch {
 
 using namespace dito;
 
-constexpr int kThreads = 256;
-constexpr int kWarps = kThreads / 32;
+// CTAs of 256 threads, two to an SM, or of 512, one to an SM (choose_threads).
+constexpr int kNarrow = 256, kWide = 512;
 
 enum : uint32_t { kWarpTask = 0, kCtaTask = 1, kPass1 = 2, kPass2 = 3, kNoTask = 0xffffffffu };
 // Release states of a large set.
@@ -60,7 +63,7 @@ struct Params {
     const int64_t* first;       // [sets]: first coordinate of each set, in floats from xyz
     const uint64_t* count;      // [sets]: its points
     const uint4* tasks;         // {kind, set or first list slot, chunk or set count, large-set slot}
-    const uint32_t* warp_sets;  // sets of the warp tasks, 8 per task
+    const uint32_t* warp_sets;  // sets of the warp tasks, one per warp of a CTA
     const uint2* chunks;        // per large set: first record, chunk count
     uint32_t ntasks;
     uint32_t flags;
@@ -107,7 +110,9 @@ __device__ void candidate_from_lanes(const SetView& v, float val, uint32_t idx, 
     candidate_warp(v.n, val, sel, v.base, flags, ctl, out);
 }
 
+template <int kThreads>
 struct Shared {
+    static constexpr int kWarps = kThreads / 32;
     uint4 task;
     uint32_t flag;
     float wval[kWarps][14];
@@ -122,7 +127,8 @@ struct Shared {
 
 // CTA-wide (value, body offset) reduction of the per-thread extremes into
 // sh.val / sh.idx (threads 0..13 hold them afterwards too).
-__device__ void cta_reduce_extremes(Extremes& ex, Shared& sh, float& val, uint32_t& r) {
+template <int kThreads>
+__device__ void cta_reduce_extremes(Extremes& ex, Shared<kThreads>& sh, float& val, uint32_t& r) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 #pragma unroll
     for (int k = 0; k < 7; ++k) {
@@ -140,7 +146,7 @@ __device__ void cta_reduce_extremes(Extremes& ex, Shared& sh, float& val, uint32
         const bool is_min = tid < 7;
         val = sh.wval[0][tid];
         r = sh.widx[0][tid];
-        for (int w = 1; w < kWarps; ++w) {
+        for (int w = 1; w < sh.kWarps; ++w) {
             const float ov = sh.wval[w][tid];
             const uint32_t orr = sh.widx[w][tid];
             const bool b = is_min ? better_min(ov, orr, val, r) : better_max(ov, orr, val, r);
@@ -153,7 +159,8 @@ __device__ void cta_reduce_extremes(Extremes& ex, Shared& sh, float& val, uint32
 }
 
 // CTA-wide min/max of the per-thread extents into sh.glohi.
-__device__ void cta_reduce_extents(Extents& ex, Shared& sh) {
+template <int kThreads>
+__device__ void cta_reduce_extents(Extents& ex, Shared<kThreads>& sh) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -168,14 +175,15 @@ __device__ void cta_reduce_extents(Extents& ex, Shared& sh) {
     __syncthreads();
     if (tid < 6) {
         float v = sh.lohi[0][tid];
-        for (int w = 1; w < kWarps; ++w) v = tid < 3 ? fminf(v, sh.lohi[w][tid]) : fmaxf(v, sh.lohi[w][tid]);
+        for (int w = 1; w < sh.kWarps; ++w) v = tid < 3 ? fminf(v, sh.lohi[w][tid]) : fmaxf(v, sh.lohi[w][tid]);
         sh.glohi[tid] = v;
     }
     __syncthreads();
 }
 
 // True in exactly one CTA: the last of `count` to arrive on `ticket`.
-__device__ bool cta_last(uint32_t* ticket, uint32_t count, Shared& sh) {
+template <int kThreads>
+__device__ bool cta_last(uint32_t* ticket, uint32_t count, Shared<kThreads>& sh) {
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) sh.flag = (atomicAdd(ticket, 1u) == count - 1) ? 1u : 0u;
@@ -230,8 +238,8 @@ __device__ void warp_fit(const Params& p, uint32_t s, Ctl* ctl) {
 }
 
 // A whole set by one CTA.
-template <int U>
-__device__ void cta_fit(const Params& p, uint32_t s, Shared& sh) {
+template <int U, int kThreads>
+__device__ void cta_fit(const Params& p, uint32_t s, Shared<kThreads>& sh) {
     const int tid = threadIdx.x, warp = tid >> 5;
     const SetView v = set_view(p, s);
     Extremes ex;
@@ -274,8 +282,8 @@ __device__ __forceinline__ void chunk_range(const SetView& v, uint32_t c, uint32
     g1 = static_cast<uint32_t>(static_cast<uint64_t>(v.groups) * (c + 1) / nch);
 }
 
-template <int U>
-__device__ void chunk_pass1(const Params& p, uint32_t s, uint32_t c, uint32_t b, Shared& sh) {
+template <int U, int kThreads>
+__device__ void chunk_pass1(const Params& p, uint32_t s, uint32_t c, uint32_t b, Shared<kThreads>& sh) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const SetView v = set_view(p, s);
     const uint2 ch = p.chunks[b];  // first record, chunk count
@@ -296,7 +304,7 @@ __device__ void chunk_pass1(const Params& p, uint32_t s, uint32_t c, uint32_t b,
 
     // Last chunk: the set's extremes (the lowest index among equal values
     // wins), then the candidate search; the plan goes to the set's control block.
-    for (int e = warp; e < 14; e += kWarps) {
+    for (int e = warp; e < 14; e += sh.kWarps) {
         float bv = e < 7 ? kInf : -kInf;
         uint64_t bi = ~0ull;
         for (uint32_t k = lane; k < ch.y; k += 32) {
@@ -350,8 +358,8 @@ __device__ void chunk_pass1(const Params& p, uint32_t s, uint32_t c, uint32_t b,
     }
 }
 
-template <int U>
-__device__ void chunk_pass2(const Params& p, uint32_t s, uint32_t c, uint32_t b, Shared& sh) {
+template <int U, int kThreads>
+__device__ void chunk_pass2(const Params& p, uint32_t s, uint32_t c, uint32_t b, Shared<kThreads>& sh) {
     const int tid = threadIdx.x;
     if (tid == 0) {
         // Every pass-1 task of this set was taken before this task (queue
@@ -408,9 +416,9 @@ __device__ void chunk_pass2(const Params& p, uint32_t s, uint32_t c, uint32_t b,
     if (tid == 0) finalize_extents(&sh.ctl, sh.glohi, p.flags, p.out + s);
 }
 
-template <int U>
-__global__ void __launch_bounds__(kThreads, 2) dito_batch_kernel(Params p) {
-    __shared__ Shared sh;
+template <int U, int kThreads>
+__global__ void __launch_bounds__(kThreads, kWide / kThreads) dito_batch_kernel(Params p) {
+    __shared__ Shared<kThreads> sh;
     const int warp = threadIdx.x >> 5;
     for (;;) {
         if (threadIdx.x == 0) {
@@ -456,6 +464,7 @@ struct Batch {
     PinnedBuffer staging;  // the plan on its way up
     size_t off_tasks = 0, off_warp = 0, off_chunks = 0, off_ctl = 0, off_large = 0, off_r1v = 0, off_r1i = 0,
            off_r2 = 0, ctl_bytes = 0;
+    int threads = kNarrow;
     int grid = 0;
     // graph
     cudaGraph_t graph = nullptr;
@@ -500,6 +509,51 @@ kr_error check_tuning(const obvh_dito_batch_tuning& t) {
     return kr_success;
 }
 
+// Narrow or wide CTAs, by how long the most loaded one would run if each took
+// the next task as it became free.  In units of a point in one pass of a narrow
+// CTA: a wide CTA streams 1.65 times as fast, and a task costs 25,000 more in
+// either for its reductions, candidate search and boxes (8 us; a point 0.31
+// ns).  So a few sets go to wide CTAs, where the largest one sets the time, and
+// many to narrow ones, which overlap one set's serial steps with another's
+// points.  Measured (us, narrow / wide): 100 sets of 64..100,000 points 53 /
+// 39, 500 of 64..262,144 115 / 98, 1,000 of 64..60,000 54 / 72, 4,096 of
+// 64..262,144 499 / 606.
+double longest_cta(const Batch& B, const std::vector<uint32_t>& large, const std::vector<uint32_t>& cta,
+                   const std::vector<uint32_t>& warp, size_t ctas, int threads) {
+    const double speed = threads == kWide ? 1.65 : 1.0, fixed = 25000.0;
+    std::priority_queue<double, std::vector<double>, std::greater<double>> load;
+    double most = 0.0;
+    const auto add = [&](double cost) {
+        if (load.size() == ctas) {
+            cost += load.top();
+            load.pop();
+        }
+        load.push(cost);
+        most = std::max(most, cost);
+    };
+    const bool finisher = B.tuning.lag_tasks == 0;
+    for (const uint32_t s : large) {
+        const double n = static_cast<double>(B.size(s));
+        const double chunks = std::ceil(n / B.tuning.chunk_points);
+        // pass 1 in chunks, the last of which also runs pass 2 (or pass 2 in chunks too)
+        for (double c = 0; c < chunks; ++c) {
+            const double both = n / chunks * (finisher ? 1.0 : 2.0) / speed + fixed;
+            add(both + (finisher && c + 1 == chunks ? n / speed + fixed : 0.0));
+        }
+    }
+    for (const uint32_t s : cta) add(2.0 * static_cast<double>(B.size(s)) / speed + fixed);
+    const size_t per_task = static_cast<size_t>(threads) / 32;
+    for (size_t i = 0; i < warp.size(); i += per_task)  // one warp a set: a narrow CTA's eighth
+        add(2.0 * 8.0 * static_cast<double>(B.size(warp[i])) + fixed);
+    return most;
+}
+
+int choose_threads(const Batch& B, const std::vector<uint32_t>& large, const std::vector<uint32_t>& cta,
+                   const std::vector<uint32_t>& warp, size_t sms) {
+    return longest_cta(B, large, cta, warp, sms, kWide) < longest_cta(B, large, cta, warp, 2 * sms, kNarrow) ? kWide
+                                                                                                             : kNarrow;
+}
+
 // Orders the tasks: large sets' pass-1 chunks (largest set first), CTA sets,
 // then warp tasks (both largest first), with each large set's pass-2 chunks
 // inserted `lag` tasks after its last pass-1 chunk (or at the end).
@@ -521,8 +575,10 @@ kr_error plan(Batch& B, cudaStream_t s = nullptr, bool sync = true) {
     std::sort(cta_ids.begin(), cta_ids.end(), by_size);
     std::sort(large_ids.begin(), large_ids.end(), by_size);
 
-    const DeviceInfo& info = device_info();
-    B.grid = static_cast<int>(t.ctas_per_sm) * info.sm_count;
+    const size_t sms = static_cast<size_t>(device_info().sm_count);
+    B.threads = t.ctas_per_sm == 2 ? choose_threads(B, large_ids, cta_ids, warp_ids, sms) : kNarrow;
+    B.grid = static_cast<int>(B.threads == kWide ? sms : t.ctas_per_sm * sms);
+    const size_t per_task = static_cast<size_t>(B.threads) / 32;  // sets of a warp task
     // lag 0: no pass-2 tasks, the CTA completing a set's pass 1 runs its pass 2
     const bool finisher = t.lag_tasks == 0;
     const uint32_t lag = t.lag_tasks;
@@ -569,8 +625,8 @@ kr_error plan(Batch& B, cudaStream_t s = nullptr, bool sync = true) {
         }
     }
     for (uint32_t s : cta_ids) emit(make_uint4(kCtaTask, s, 0, 0));
-    for (size_t i = 0; i < warp_ids.size(); i += kWarps) {
-        const uint32_t cnt = static_cast<uint32_t>(std::min<size_t>(kWarps, warp_ids.size() - i));
+    for (size_t i = 0; i < warp_ids.size(); i += per_task) {
+        const uint32_t cnt = static_cast<uint32_t>(std::min<size_t>(per_task, warp_ids.size() - i));
         const uint32_t slot = static_cast<uint32_t>(B.warp_sets.size());
         for (uint32_t k = 0; k < cnt; ++k) B.warp_sets.push_back(warp_ids[i + k]);
         emit(make_uint4(kWarpTask, slot, cnt, 0));
@@ -620,7 +676,8 @@ template <int U>
 kr_error launch_u(const Batch& B, const Params& prm, cudaStream_t s) {
     {
         ProfScope prof_scope_("dito_batch_kernel", s);
-        dito_batch_kernel<U><<<B.grid, kThreads, 0, s>>>(prm);
+        if (B.threads == kWide) dito_batch_kernel<U, kWide><<<B.grid, kWide, 0, s>>>(prm);
+        else dito_batch_kernel<U, kNarrow><<<B.grid, kNarrow, 0, s>>>(prm);
     }
     OBVH_TRY_CUDA(cudaGetLastError());
     return kr_success;

@@ -171,3 +171,25 @@ def test_bad_arguments(torch):
     with pytest.raises(_native.ObvhError):
         DitoBatch(np.array([0, 5]), tuning=dict(points_per_thread=3, chunk_points=4096, warp_max_points=0,
                                                   cta_max_points=0, lag_tasks=0, ctas_per_sm=1))
+
+
+@pytest.mark.parametrize("sizes", [[70_000, 5_000, 300], [64, 4_097, 200, 4_096] * 400, [9_000] * 40])
+def test_narrow_and_wide_ctas(sizes):
+    """Few sets go to CTAs of 512 threads, many to two of 256 an SM: warp tasks of
+    16 or 8 sets, CTA tasks and chunked sets either way, each the lone fit."""
+    import torch
+    from obvh_b200 import DitoFitter
+    from obvh_b200.batch import DitoBatch
+    rng = np.random.default_rng(len(sizes))
+    offsets = np.concatenate([[0], np.cumsum(sizes)])
+    points = (rng.normal(size=(int(offsets[-1]), 3)) * [3.0, 1.0, 0.2]).astype(np.float32)
+    dev = torch.from_numpy(points).cuda()
+    boxes = torch.zeros((len(sizes), 15), device="cuda")
+    batch = DitoBatch(offsets)
+    batch.run(dev, boxes)
+    assert batch.status() == 0
+    got = boxes.cpu().numpy()
+    fitter = DitoFitter()
+    for s in list(range(0, len(sizes), 37)) + [len(sizes) - 1]:
+        want = fitter.fit(dev[int(offsets[s]):int(offsets[s + 1])].contiguous()).cpu().numpy()
+        assert np.array_equal((got[s] + 0).view(np.uint32), (want + 0).view(np.uint32)), s
