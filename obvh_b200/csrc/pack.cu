@@ -51,11 +51,23 @@ __device__ __forceinline__ void store_m43(kr_mat43* dst, const float4 c[4]) {
 // child's transform, and stores chunk q of the 64-byte record, column q of
 // both halves of the 128-byte pair and row-word q of the 48-byte SoA rows.
 // The chunks are assembled through a per-quad shared-memory stage.
-constexpr int kQuads = kThreads / 4;
+//
+// Bound by DRAM (1.24 GB for 4 M nodes, reads and writes mixed) as far as the
+// warps in flight cover its latency, and those are bound by registers: 32 a
+// thread for a full SM.  So nothing is looked ahead in registers, the one
+// load that depends on nothing and goes to cold memory (metadata.w) is issued
+// before the node's, and CTAs are small, so that the next starts as soon as
+// four warps are done.  2,000,000 triangles, all three outputs: 253 us with
+// the next nodes' words looked ahead and metadata.w read at the end; 254
+// without the look-ahead, 234 with metadata.w first, 229 with CTAs of 128
+// threads.  Inner and leaf nodes taken in turn cost 6 %, streaming stores 1
+// to 3 %, a lane instead of a quad for each leaf node 3 %.
+constexpr int kPackThreads = 128;
+constexpr int kQuads = kPackThreads / 4;
 constexpr int kStage = 48;  // words per quad: 14 box/count words, 32 column words
 
 template <bool kObb, bool kSoa>
-__global__ void __launch_bounds__(kThreads, 8)
+__global__ void __launch_bounds__(kPackThreads, 16)
 pack_kernel(const kr_bvh_node* __restrict__ nodes, const kr_mat4* __restrict__ xfs, kr_bvh_node_packed* packed,
             kr_bvh_transformation_pair* pairs, kr_mat43* left_t, kr_mat43* right_t, kr_ivec4* meta_out,
             uint32_t node_count, uint32_t internal_count, uint32_t* err) {
@@ -63,30 +75,20 @@ pack_kernel(const kr_bvh_node* __restrict__ nodes, const kr_mat4* __restrict__ x
     const uint32_t lane = threadIdx.x & 31, q = lane & 3;
     uint32_t* st = stage + (threadIdx.x >> 2) * kStage;
     float* cols = reinterpret_cast<float*>(st + 16);
-    const uint32_t warps = gridDim.x * (kThreads / 32);
-    // the node words of the next iteration are loaded while this one's
-    // children and transforms are on their way
-    auto node_words = [&](uint32_t b, uint32_t& wa, uint32_t& wb, uint32_t& w8) {
-        const uint64_t i = static_cast<uint64_t>(b) + (lane >> 2);
-        const bool ok = i < node_count;
-        const uint32_t* rec = reinterpret_cast<const uint32_t*>(nodes + (ok ? i : 0));
-        wa = ok ? __ldg(rec + q) : 0u;
-        wb = ok ? __ldg(rec + q + 4) : 0u;
-        w8 = ok && q == 0 ? __ldg(rec + 8) : 0u;
-    };
-    // the warp's first node and the stride in 64 bits, so that neither the
-    // loop step nor the look-ahead can wrap below node_count
-    const uint64_t stride = static_cast<uint64_t>(warps) * 8u;
-    uint64_t base = (static_cast<uint64_t>(blockIdx.x) * (kThreads / 32) + (threadIdx.x >> 5)) * 8u;
-    uint32_t na = 0, nb = 0, n8 = 0;
-    if (base < node_count) node_words(static_cast<uint32_t>(base), na, nb, n8);
-    for (; base < node_count; base += stride) {
-        const uint64_t i64 = base + (lane >> 2);
-        const bool valid = i64 < node_count;
-        const uint32_t i = static_cast<uint32_t>(valid ? i64 : 0);
-        const uint32_t wa = na, wb = nb;
-        const uint32_t w8 = __shfl_sync(0xffffffffu, n8, lane & ~3u);
-        if (base + stride < node_count) node_words(static_cast<uint32_t>(base + stride), na, nb, n8);
+    // chunks of eight nodes, counted so that no index passes 2^32
+    const uint32_t warps = gridDim.x * (kPackThreads / 32);
+    const uint32_t chunks = (node_count >> 3) + ((node_count & 7u) ? 1u : 0u);
+    for (uint32_t chunk = blockIdx.x * (kPackThreads / 32) + (threadIdx.x >> 5); chunk < chunks; chunk += warps) {
+        const bool valid = chunk * 8u + (lane >> 2) < node_count;
+        const uint32_t i = valid ? chunk * 8u + (lane >> 2) : 0u;
+        // metadata.w as found: the longest way to DRAM, so the first load
+        int old_w = 0;
+        if (kSoa && q == 3 && valid) old_w = *(reinterpret_cast<const int*>(packed + i) + 15);
+        const uint32_t* rec = reinterpret_cast<const uint32_t*>(nodes + i);
+        const uint32_t wa = __ldg(rec + q);
+        const uint32_t wb = __ldg(rec + q + 4);
+        uint32_t w8 = q == 0 ? __ldg(rec + 8) : 0u;
+        w8 = __shfl_sync(0xffffffffu, w8, lane & ~3u);
         const uint32_t left = __shfl_sync(0xffffffffu, wb, (lane & ~3u) + 2);   // word 6
         const uint32_t right = __shfl_sync(0xffffffffu, wb, (lane & ~3u) + 3);  // word 7
         const uint32_t np = w8 & 0xFFFFu, axis = (w8 >> 16) & 0xFFu;
@@ -130,7 +132,7 @@ pack_kernel(const kr_bvh_node* __restrict__ nodes, const kr_mat4* __restrict__ x
             reinterpret_cast<float4*>(cols)[4 + q] = rc;
         }
         __syncwarp();
-        char* out = reinterpret_cast<char*>(packed + (valid ? i : 0));
+        char* out = reinterpret_cast<char*>(packed + i);
         int2 lr = make_int2(0, 0);
         if (inner) {
             lr = make_int2((st[12] & 0xFFFFu) ? ~static_cast<int>(left) : static_cast<int>(left),
@@ -153,9 +155,9 @@ pack_kernel(const kr_bvh_node* __restrict__ nodes, const kr_mat4* __restrict__ x
         if (kSoa && valid) {
             if (q == 3) {
                 // metadata as it now stands: x, y, z as written, w as found
-                const int4 old = *reinterpret_cast<const int4*>(out + 48);
-                meta_out[i] = (inner || leafy) ? kr_ivec4{{lr.x, lr.y, static_cast<int>(axis), old.w}}
-                                               : kr_ivec4{{old.x, old.y, old.z, old.w}};
+                int4 now = make_int4(lr.x, lr.y, static_cast<int>(axis), old_w);
+                if (!inner && !leafy) now = *reinterpret_cast<const int4*>(out + 48);
+                reinterpret_cast<int4*>(meta_out)[i] = now;
             } else if (soa_row) {
                 // row-word q of each 4x3 (kr_m43from4): words 4q..4q+3 of
                 // (c0.xyz, c1.xyz, c2.xyz, c3.xyz)
@@ -202,10 +204,12 @@ inline unsigned grid_for(uint32_t n) {
 }
 
 // pack_kernel: one quad per node, eight nodes per warp; enough warps for
-// every node (up to 64 blocks per SM of grid-stride work).
+// every node (up to 256 blocks per SM of grid-stride work: 229 us for 4 M
+// nodes, 64 blocks 236, a chunk for each warp 237).
 inline unsigned pack_grid(uint32_t n) {
-    const unsigned want = (n + 8u * (kThreads / 32) - 1) / (8u * (kThreads / 32));
-    const unsigned cap = static_cast<unsigned>(device_info().sm_count) * 64u;
+    constexpr unsigned nodes = 8u * (kPackThreads / 32);
+    const unsigned want = n / nodes + (n % nodes ? 1u : 0u);
+    const unsigned cap = static_cast<unsigned>(device_info().sm_count) * 256u;
     return want < cap ? (want ? want : 1u) : cap;
 }
 
@@ -226,13 +230,13 @@ kr_error enqueue_pack(const kr_bvh_node* nodes, const kr_mat4* xfs, kr_bvh_node_
     const unsigned g = pack_grid(node_count);
     ProfScope prof_scope_("pack_kernel", s);
     if (!obb)
-        pack_kernel<false, false><<<g, kThreads, 0, s>>>(nodes, nullptr, packed, nullptr, nullptr, nullptr, nullptr,
+        pack_kernel<false, false><<<g, kPackThreads, 0, s>>>(nodes, nullptr, packed, nullptr, nullptr, nullptr, nullptr,
                                                           node_count, internal_count, err);
     else if (!soa)
-        pack_kernel<true, false><<<g, kThreads, 0, s>>>(nodes, xfs, packed, pairs, nullptr, nullptr, nullptr,
+        pack_kernel<true, false><<<g, kPackThreads, 0, s>>>(nodes, xfs, packed, pairs, nullptr, nullptr, nullptr,
                                                          node_count, internal_count, err);
     else
-        pack_kernel<true, true><<<g, kThreads, 0, s>>>(nodes, xfs, packed, pairs, left_t, right_t, meta, node_count,
+        pack_kernel<true, true><<<g, kPackThreads, 0, s>>>(nodes, xfs, packed, pairs, left_t, right_t, meta, node_count,
                                                         internal_count, err);
     OBVH_TRY_CUDA(cudaGetLastError());
     return kr_success;

@@ -114,6 +114,13 @@ def test_packing_equals_the_reference_functions(n, collapse, obbs):
         assert _host(f["metadata"], np.int32, (-1, 4))[:nn].tobytes() == rmeta.tobytes()
 
 
+@pytest.mark.parametrize("n", [4, 5, 17, 700_001])
+def test_packing_of_ragged_chunks_and_of_more_nodes_than_one_pass(n):
+    """Chunks of eight nodes: a last one of 1, 3 or 7 nodes, and more chunks
+    than warps (256 CTAs of 128 threads per SM cover 1.2 M nodes)."""
+    test_obvh_persistent_and_soa_match_the_oracle(n, True, True)
+
+
 def test_malformed_tree_is_reported():
     """A child index past the end is skipped and reported, not followed."""
     import torch
