@@ -83,38 +83,166 @@ __device__ __forceinline__ uint4 leaf_face(const kr_bvh_node* nodes, const kr_uv
 }
 
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kThreads) summary_up_kernel(const kr_bvh_node* nodes, const uint32_t* parents,
+// The walks of the two kernels below, a chain of dependent steps each: an
+// arrival (a fence and an atomic at GPU scope), the sibling's outputs from L2,
+// seven slabs merged one after another.  In three parts:
+//   - within the warp: leaves that are close in the tree are mostly close in
+//     number, so lanes that stand at one parent meet by a match and hand over
+//     by shuffles, without arrivals, until no two do;
+//   - across the GPU, a lane per walk, as long as more than kGroups are left
+//     (every arrival checks that its parent names the child, the first too:
+//     nodes whose children met in a warp have no arrivals to tell by);
+//   - then eight lanes per walk, lane k < 7 with slab k and lane 7 with
+//     everything else; the warp's fences stay as many as before.
+// Bound by the latency of those chains with 32 warps on an SM (64 registers:
+// 3 CTAs per SM 320 us where 4 take 314 and 5, spilling, 326).  Boxes and
+// transforms of a given 229,824-triangle tree: 332 us with lanes alone, 328
+// with groups, 323 with the meeting in the warp, 314 with the leaf boxes staged
+// and 4 CTAs per SM; the 917,504-triangle ATRBVH build 2,413 -> 2,363 us.
+constexpr uint32_t kGroups = 4;
+constexpr uint32_t kWalkCtas = 4;
+
+
+// The lane whose walk group `lane / 8` takes over (the group's own number
+// among the lanes of `going`), and that lane's slab `lane % 8` (7: none).
+__device__ __forceinline__ int source_lane(uint32_t going, uint32_t group) {
+    for (uint32_t k = 0; k < group; ++k) going &= going - 1;
+    return __ffs(static_cast<int>(going)) - 1;
+}
+
+__device__ __forceinline__ Slab take_slab(const Summary& s, int src, uint32_t sub) {
+    Slab o{0.f, 0.f, 0u, 0u};
+#pragma unroll
+    for (uint32_t k = 0; k < 7; ++k) {
+        const float lo = __shfl_sync(0xffffffffu, s.lo[k], src), hi = __shfl_sync(0xffffffffu, s.hi[k], src);
+        const uint32_t ilo = __shfl_sync(0xffffffffu, s.ilo[k], src), ihi = __shfl_sync(0xffffffffu, s.ihi[k], src);
+        if (sub == k) o = Slab{lo, hi, ilo, ihi};
+    }
+    return o;
+}
+
+__device__ __forceinline__ void store_slab(uint4* summary, uint32_t p, uint32_t k, const Slab& v) {
+    __stcg(summary + 7 * static_cast<size_t>(p) + k,
+           make_uint4(__float_as_uint(v.lo), __float_as_uint(v.hi), v.ilo, v.ihi));
+}
+
+// Slab k of node x's summary, x a leaf or a node that this kernel completed.
+__device__ __forceinline__ Slab load_slab(const kr_bvh_node* nodes, const kr_vec3* verts, const kr_uvec4* faces,
+                                          const uint4* summary, uint32_t x, uint32_t internal, uint32_t k) {
+    if (x >= internal) return face_slab(verts, leaf_face(nodes, faces, x), static_cast<int>(k));
+    const uint4 q = __ldcg(summary + 7 * static_cast<size_t>(x) + k);
+    return Slab{__uint_as_float(q.x), __uint_as_float(q.y), q.z, q.w};
+}
+
+__device__ __forceinline__ Slab slab_from(const Summary& s, int k, uint32_t lane) {
+    return Slab{__shfl_sync(0xffffffffu, s.lo[k], lane), __shfl_sync(0xffffffffu, s.hi[k], lane),
+                __shfl_sync(0xffffffffu, s.ilo[k], lane), __shfl_sync(0xffffffffu, s.ihi[k], lane)};
+}
+
+// Whether another lane of the warp stands at the same parent with its other
+// child, and which (else the lane itself).
+__device__ __forceinline__ bool paired(bool live, uint32_t p, uint32_t child, uint32_t L, uint32_t R, uint32_t lane,
+                                       uint32_t& partner) {
+    // p < internal < 2^31; lanes without a walk match no one
+    const uint32_t same = __match_any_sync(0xffffffffu, live ? p : 0x80000000u | lane);
+    partner = __popc(same) == 2 ? static_cast<uint32_t>(__ffs(static_cast<int>(same ^ (1u << lane))) - 1) : lane;
+    const uint32_t theirs = __shfl_sync(0xffffffffu, child, partner);
+    const bool pair = partner != lane && ((L == child && R == theirs) || (R == child && L == theirs));
+    if (!pair) partner = lane;
+    return pair;
+}
+
+// The boxes and transforms of a warp's leaves, consecutive records from obbs
+// and xfs on: staged in shared memory (rows of 15 and of 20 words: no two
+// lanes of an access in one bank) and written out in full sectors.
+struct LeafStage {
+    float4 xf[32 * 5];
+    float box[32 * 15];
+};
+
+__device__ __forceinline__ void leaf_boxes(LeafStage& st, bool live, const kr_vec3* verts, uint4 face, uint32_t lane,
+                                           kr_obb3* obbs, kr_mat4* xfs) {
+    const uint32_t m = __popc(__ballot_sync(0xffffffffu, live));  // the live lanes come first
+    if (live)
+        leaf_box(load_vertex(verts, face.x), load_vertex(verts, face.y), load_vertex(verts, face.z),
+                 reinterpret_cast<kr_obb3*>(st.box + 15 * lane), reinterpret_cast<kr_mat4*>(st.xf + 5 * lane));
+    __syncwarp();
+#pragma unroll
+    for (uint32_t k = lane; k < 32 * 15; k += 32)
+        if (k < 15 * m) reinterpret_cast<float*>(obbs)[k] = st.box[k];
+#pragma unroll
+    for (uint32_t k = lane; k < 32 * 4; k += 32)
+        if (k < 4 * m) reinterpret_cast<float4*>(xfs)[k] = st.xf[5 * (k >> 2) + (k & 3)];
+}
+
+__global__ void __launch_bounds__(kThreads, kWalkCtas) summary_up_kernel(const kr_bvh_node* nodes, const uint32_t* parents,
                                                               const kr_vec3* verts, const kr_uvec4* faces,
                                                               uint32_t n, uint32_t internal, uint4* summary,
                                                               uint32_t* counts, uint32_t* visits, kr_obb3* obbs,
                                                               kr_mat4* xfs, uint32_t* err) {
+    __shared__ LeafStage stage[kThreads / 32];
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const uint32_t leaf = internal + j;
+    const uint32_t lane = threadIdx.x & 31;
+    bool live = j < n;
+    const uint32_t leaf = internal + (live ? j : 0u);
     const uint4 face = leaf_face(nodes, faces, leaf);
-    leaf_box(load_vertex(verts, face.x), load_vertex(verts, face.y), load_vertex(verts, face.z), obbs + leaf,
-             xfs + leaf);
-    if (internal == 0) return;
+    const size_t first_leaf = static_cast<size_t>(internal) + (j - lane);
+    leaf_boxes(stage[threadIdx.x >> 5], live, verts, face, lane, obbs + first_leaf, xfs + first_leaf);
     Summary own;
     leaf_summary(verts, face, own);
-    uint32_t child = leaf;
-    uint32_t p = parents[leaf];
-    for (uint32_t steps = 0; p != kNoParent; ++steps) {
+    if (internal == 0) return;
+    uint32_t child = leaf, p = live ? parents[leaf] : kNoParent, grand = kNoParent;
+    uint32_t L = 0, R = 0, steps = 0, going, count = 1;
+    // p's children and its parent are final before this kernel
+    const auto at_parent = [&] {
+        if (!live) return;
         if (steps > internal || p >= internal) {
-            atomicOr(err, kErrCycle);
+            if (p != kNoParent) atomicOr(err, kErrCycle);
+            live = false;
             return;
         }
-        // p's children and its parent are final before this kernel: read them
-        // ahead of the arrival
         const uint32_t* w = reinterpret_cast<const uint32_t*>(nodes + p);
-        const uint32_t L = __ldg(w + 6), R = __ldg(w + 7);
-        const uint32_t grand = __ldg(parents + p);
-        if (arrive(visits + p) == 0) return;
-        const uint32_t other = (L == child) ? R : L;
-        if ((L != child && R != child) || other >= internal + n) {
-            atomicOr(err, kErrBadInput);
-            return;
+        L = __ldg(w + 6);
+        R = __ldg(w + 7);
+        grand = __ldg(parents + p);
+    };
+    at_parent();
+    for (;;) {
+        uint32_t partner;
+        const bool pair = paired(live, p, child, L, R, lane, partner);
+        if (!__any_sync(0xffffffffu, pair)) break;
+        const bool mine = pair && L == child;  // the left child's lane goes on
+        const uint32_t theirs = __shfl_sync(0xffffffffu, count, partner);
+#pragma unroll
+        for (int k = 0; k < 7; ++k) {
+            const Slab o = slab_from(own, k, partner);
+            if (mine) {
+                const Slab m = merge_slab(slab_of(own, k), o);
+                set_slab(own, k, m);
+                store_slab(summary, p, k, m);
+            }
         }
+        live = live && (mine || !pair);
+        if (mine) {
+            count += theirs;
+            __stcg(counts + p, count);
+            child = p;
+            p = grand;
+            ++steps;
+            at_parent();
+        }
+        __syncwarp();
+    }
+    for (;;) {
+        going = __ballot_sync(0xffffffffu, live);
+        if (__popc(going) <= kGroups) break;
+        if (!live) continue;
+        const bool second = arrive(visits + p) != 0;
+        const uint32_t other = (L == child) ? R : L;
+        const bool bad = (L != child && R != child) || other >= internal + n;
+        if (bad) atomicOr(err, kErrBadInput);
+        live = second && !bad;
+        if (!live) continue;
         Summary o;
         if (other >= internal) leaf_summary(verts, leaf_face(nodes, faces, other), o);
         else load_summary(summary + 7 * static_cast<size_t>(other), o);
@@ -125,9 +253,50 @@ __global__ void __launch_bounds__(kThreads) summary_up_kernel(const kr_bvh_node*
             own = o;
         }
         store_summary(summary + 7 * static_cast<size_t>(p), own);
-        __stcg(counts + p, count_of(counts, L, internal) + count_of(counts, R, internal));
+        count += count_of(counts, other, internal);
+        __stcg(counts + p, count);
         child = p;
         p = grand;
+        ++steps;
+        at_parent();
+    }
+    if (going == 0) return;
+    const uint32_t sub = lane & 7, group = lane >> 3;
+    live = group < __popc(going);
+    const int src = live ? source_lane(going, group) : 0;
+    Slab mine = take_slab(own, src, sub);
+    child = __shfl_sync(0xffffffffu, child, src);
+    p = __shfl_sync(0xffffffffu, p, src);
+    steps = __shfl_sync(0xffffffffu, steps, src);
+    L = __shfl_sync(0xffffffffu, L, src);
+    R = __shfl_sync(0xffffffffu, R, src);
+    grand = __shfl_sync(0xffffffffu, grand, src);
+    count = __shfl_sync(0xffffffffu, count, src);
+    __syncwarp();
+    while (__any_sync(0xffffffffu, live)) {
+        uint32_t before = 0;
+        if (live && sub == 0) before = arrive(visits + p);
+        before = __shfl_sync(0xffffffffu, before, 0, 8);
+        __syncwarp();  // orders the group's loads after lane 0's acquire
+        const uint32_t other = (L == child) ? R : L;
+        const bool bad = live && ((L != child && R != child) || other >= internal + n);
+        if (bad && sub == 0) atomicOr(err, kErrBadInput);
+        live = live && before != 0 && !bad;
+        if (live) {
+            if (sub < 7) {
+                const Slab sib = load_slab(nodes, verts, faces, summary, other, internal, sub);
+                mine = merge_slab(L == child ? mine : sib, L == child ? sib : mine);
+                store_slab(summary, p, sub, mine);
+            } else {
+                count += count_of(counts, other, internal);
+                __stcg(counts + p, count);
+            }
+            child = p;
+            p = grand;
+            ++steps;
+            at_parent();
+        }
+        __syncwarp();  // the group's outputs before lane 0's next release
     }
 }
 
@@ -157,147 +326,250 @@ struct WalkArgs {
     uint32_t* err;
 };
 
+// nPrimitives = 0xFFFF, the low half of word 8
 __device__ __forceinline__ void mark_hidden(kr_bvh_node* collapsed, uint32_t i) {
-    uint32_t* w = reinterpret_cast<uint32_t*>(collapsed + i) + 8;
-    __stcg(w, (__ldcg(w) & 0xffff0000u) | 0xffffu);
+    unsigned short* h = reinterpret_cast<unsigned short*>(reinterpret_cast<uint32_t*>(collapsed + i) + 8);
+    __stcg(h, static_cast<unsigned short>(0xffffu));
 }
 
-// 4 CTAs per SM (64 registers, a few spills): more walks in flight to hide
-// the chain of arrivals (0.44 -> 0.40 ms on the 917K-triangle knot)
-__global__ void __launch_bounds__(kThreads, 4) walk_kernel(WalkArgs a) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= a.n) return;
-    const uint32_t internal = a.n - 1;
-    const uint32_t leaf = internal + j;
-    const bool collapse = a.collapsed != nullptr;
-    uint32_t rec[9];
-    {
-        const uint32_t* lw = reinterpret_cast<const uint32_t*>(a.nodes + leaf);
-#pragma unroll
-        for (int k = 0; k < 9; ++k) rec[k] = __ldg(lw + k);
-    }
-    float olo[3], ohi[3];
+// A completed node as its parent's walk needs it: bounds, cost and count.
+struct Done {
+    float lo[3], hi[3], cost;
+    uint32_t count;
+};
+
+__device__ __forceinline__ Done done_from(const Done& d, uint32_t lane) {
+    Done o;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        olo[k] = __uint_as_float(rec[k]);
-        ohi[k] = __uint_as_float(rec[3 + k]);
+        o.lo[k] = __shfl_sync(0xffffffffu, d.lo[k], lane);
+        o.hi[k] = __shfl_sync(0xffffffffu, d.hi[k], lane);
+    }
+    o.cost = __shfl_sync(0xffffffffu, d.cost, lane);
+    o.count = __shfl_sync(0xffffffffu, d.count, lane);
+    return o;
+}
+
+__device__ __forceinline__ Done load_done(const WalkArgs& a, uint32_t x) {
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(a.nodes + x);
+    Done d;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        d.lo[k] = __uint_as_float(__ldcg(w + k));
+        d.hi[k] = __uint_as_float(__ldcg(w + 3 + k));
+    }
+    d.count = __ldcg(a.counts + x);
+    d.cost = __ldcg(a.costs + x);
+    return d;
+}
+
+// Node p (children L and R, word 8 of its record) from its children: bounds,
+// count, cost and collapse marks, all written here.
+__device__ __forceinline__ Done complete(const WalkArgs& a, uint32_t p, uint32_t L, uint32_t R, uint32_t w8,
+                                         const Done& l, const Done& r) {
+    Done o;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {  // kr_aabb_expand(left, right)
+        o.lo[k] = kmin(kmin(l.lo[k], r.lo[k]), r.hi[k]);
+        o.hi[k] = kmax(kmax(l.hi[k], r.lo[k]), r.hi[k]);
+    }
+    uint32_t* w = reinterpret_cast<uint32_t*>(a.nodes + p);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        __stcg(w + k, __float_as_uint(o.lo[k]));
+        __stcg(w + 3 + k, __float_as_uint(o.hi[k]));
+    }
+    if (a.collapsed) {
+        uint32_t* cw = reinterpret_cast<uint32_t*>(a.collapsed + p);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            __stcg(cw + k, __float_as_uint(o.lo[k]));
+            __stcg(cw + 3 + k, __float_as_uint(o.hi[k]));
+        }
+        __stcg(cw + 6, L);
+        __stcg(cw + 7, R);
+        __stcg(cw + 8, w8);
+    }
+    o.count = l.count + r.count;
+    __stcg(a.counts + p, o.count);
+    const float area = box_area(o.lo, o.hi);
+    if (a.collapsed) {
+        // bvh_mark_collapse_kernel (transforms.cu:111-133)
+        const float node_cost = a.ci * area + l.cost + r.cost;
+        const float leaf_cost = a.ct * area * static_cast<float>(o.count);
+        if (leaf_cost < node_cost && o.count <= kCollapseLeafMax) {
+            o.cost = leaf_cost;
+            a.flags[p] = 1;
+            a.flags[L] = 1;
+            a.flags[R] = 1;
+            mark_hidden(a.collapsed, L);
+            mark_hidden(a.collapsed, R);
+        } else {
+            o.cost = node_cost;
+        }
+    } else {
+        o.cost = 1.2f * area + r.cost + l.cost;  // calculate_aabbs_kernel (lbvh.cu:452)
+    }
+    __stcg(a.costs + p, o.cost);
+    return o;
+}
+
+__global__ void __launch_bounds__(kThreads, kWalkCtas) walk_kernel(WalkArgs a) {
+    __shared__ LeafStage stage[kThreads / 32];
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t internal = a.n - 1;
+    const bool collapse = a.collapsed != nullptr;
+    const bool slabs = a.summary != nullptr;
+    bool live = j < a.n;
+    const uint32_t leaf = internal + (live ? j : 0u);
+    Done own;
+    uint32_t prim;
+    {
+        // the warp's leaf records are consecutive: read, and copied to the
+        // collapsed array, as one run of words
+        LeafStage& st = stage[threadIdx.x >> 5];
+        const uint32_t first = j - lane, words = first < a.n ? 9 * min(32u, a.n - first) : 0u;
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(a.nodes + internal + first);
+        uint32_t* dst = collapse ? reinterpret_cast<uint32_t*>(a.collapsed + internal + first) : nullptr;
+        uint32_t* row = reinterpret_cast<uint32_t*>(st.box);
+#pragma unroll
+        for (uint32_t k = lane; k < 32 * 9; k += 32) {
+            const uint32_t v = k < words ? __ldg(src + k) : 0u;
+            row[k] = v;
+            if (collapse && k < words) __stcg(dst + k, v);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            own.lo[k] = __uint_as_float(row[9 * lane + k]);
+            own.hi[k] = __uint_as_float(row[9 * lane + 3 + k]);
+        }
+        prim = row[9 * lane + 6];
+        __syncwarp();
     }
     // leaf cost: ct * area in the collapse (transforms.cu:97), 1 * area in the LBVH (lbvh.cu:427)
-    float ocost = (collapse ? a.ct : 1.0f) * box_area(olo, ohi);
-    uint32_t ocount = 1;
-    __stcg(a.costs + leaf, ocost);
-    __stcg(a.counts + leaf, 1u);
-    if (collapse) {
-        uint32_t* cw = reinterpret_cast<uint32_t*>(a.collapsed + leaf);
-#pragma unroll
-        for (int k = 0; k < 9; ++k) __stcg(cw + k, rec[k]);
+    own.cost = (collapse ? a.ct : 1.0f) * box_area(own.lo, own.hi);
+    own.count = 1;
+    if (live) {
+        __stcg(a.costs + leaf, own.cost);
+        __stcg(a.counts + leaf, 1u);
     }
-    Summary own;
-    if (a.summary) {
-        const uint4 face = __ldg(a.faces + rec[6]);
-        leaf_box(load_vertex(a.verts, face.x), load_vertex(a.verts, face.y), load_vertex(a.verts, face.z),
-                 a.obbs + leaf, a.xfs + leaf);
-        leaf_summary(a.verts, face, own);
+    Summary sum;
+    if (slabs) {
+        const uint4 face = __ldg(a.faces + prim);
+        const size_t first_leaf = static_cast<size_t>(internal) + (j - lane);
+        leaf_boxes(stage[threadIdx.x >> 5], live, a.verts, face, lane, a.obbs + first_leaf, a.xfs + first_leaf);
+        leaf_summary(a.verts, face, sum);
     }
-    uint32_t child = leaf;
-    uint32_t p = a.parents[leaf];
-    for (uint32_t steps = 0; p != kNoParent; ++steps) {
+    const kr_uvec4* faces = reinterpret_cast<const kr_uvec4*>(a.faces);
+    uint32_t child = leaf, p = live ? a.parents[leaf] : kNoParent, grand = kNoParent;
+    uint32_t L = 0, R = 0, w8 = 0, steps = 0, going;
+    // p's children, its record's word 8 and its parent are final before this kernel
+    const auto at_parent = [&] {
+        if (!live) return;
         if (steps > internal || p >= internal) {
-            atomicOr(a.err, kErrCycle);
+            if (p != kNoParent) atomicOr(a.err, kErrCycle);
+            live = false;
             return;
         }
-        // written before this kernel: read ahead of the arrival
-        const uint32_t* pw = reinterpret_cast<const uint32_t*>(a.nodes + p);
-        const uint32_t L = __ldg(pw + 6), R = __ldg(pw + 7), w8 = __ldg(pw + 8);
-        const uint32_t grand = __ldg(a.parents + p);
-        if (arrive(a.visits + p) == 0) return;
-        const bool from_left = (L == child);
-        const uint32_t other = from_left ? R : L;
-        if ((L != child && R != child) || other >= internal + a.n) {
-            atomicOr(a.err, kErrBadInput);
-            return;
-        }
-        float slo[3], shi[3];
-        {
-            const uint32_t* sw = reinterpret_cast<const uint32_t*>(a.nodes + other);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                slo[k] = __uint_as_float(__ldcg(sw + k));
-                shi[k] = __uint_as_float(__ldcg(sw + 3 + k));
-            }
-        }
-        const uint32_t scount = __ldcg(a.counts + other);
-        const float scost = __ldcg(a.costs + other);
-        const float* llo = from_left ? olo : slo;
-        const float* lhi = from_left ? ohi : shi;
-        const float* rlo = from_left ? slo : olo;
-        const float* rhi = from_left ? shi : ohi;
-        float lo[3], hi[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {  // kr_aabb_expand(left, right)
-            lo[k] = kmin(kmin(llo[k], rlo[k]), rhi[k]);
-            hi[k] = kmax(kmax(lhi[k], rlo[k]), rhi[k]);
-        }
-        {
-            uint32_t* w = reinterpret_cast<uint32_t*>(a.nodes + p);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                __stcg(w + k, __float_as_uint(lo[k]));
-                __stcg(w + 3 + k, __float_as_uint(hi[k]));
-            }
-            if (collapse) {
-                uint32_t* cw = reinterpret_cast<uint32_t*>(a.collapsed + p);
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    __stcg(cw + k, __float_as_uint(lo[k]));
-                    __stcg(cw + 3 + k, __float_as_uint(hi[k]));
-                }
-                __stcg(cw + 6, L);
-                __stcg(cw + 7, R);
-                __stcg(cw + 8, w8);
-            }
-        }
-        const uint32_t count = ocount + scount;
-        __stcg(a.counts + p, count);
-        const float area = box_area(lo, hi);
-        const float cl = from_left ? ocost : scost, cr = from_left ? scost : ocost;
-        float cost;
-        if (collapse) {
-            // bvh_mark_collapse_kernel (transforms.cu:111-133)
-            const float node_cost = a.ci * area + cl + cr;
-            const float leaf_cost = a.ct * area * static_cast<float>(count);
-            if (leaf_cost < node_cost && count <= kCollapseLeafMax) {
-                cost = leaf_cost;
-                a.flags[p] = 1;
-                a.flags[L] = 1;
-                a.flags[R] = 1;
-                mark_hidden(a.collapsed, L);
-                mark_hidden(a.collapsed, R);
-            } else {
-                cost = node_cost;
-            }
-        } else {
-            cost = 1.2f * area + cr + cl;  // calculate_aabbs_kernel (lbvh.cu:452)
-        }
-        __stcg(a.costs + p, cost);
-        if (a.summary) {
-            Summary o;
-            if (other >= internal) leaf_summary(a.verts, __ldg(a.faces + __ldg(reinterpret_cast<const uint32_t*>(a.nodes + other) + 6)), o);
-            else load_summary(a.summary + 7 * static_cast<size_t>(other), o);
-            if (from_left) {
-                merge_right(own, o);
-            } else {
-                merge_right(o, own);
-                own = o;
-            }
-            store_summary(a.summary + 7 * static_cast<size_t>(p), own);
-        }
-#pragma unroll
-        for (int k = 0; k < 3; ++k) { olo[k] = lo[k]; ohi[k] = hi[k]; }
-        ocount = count;
-        ocost = cost;
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(a.nodes + p);
+        L = __ldg(w + 6);
+        R = __ldg(w + 7);
+        w8 = __ldg(w + 8);
+        grand = __ldg(a.parents + p);
+    };
+    const auto go_up = [&] {
         child = p;
         p = grand;
+        ++steps;
+        at_parent();
+    };
+    at_parent();
+    for (;;) {
+        uint32_t partner;
+        const bool pair = paired(live, p, child, L, R, lane, partner);
+        if (!__any_sync(0xffffffffu, pair)) break;
+        const bool mine = pair && L == child;  // the left child's lane goes on
+        const Done o = done_from(own, partner);
+        if (mine) own = complete(a, p, L, R, w8, own, o);
+        if (slabs) {
+#pragma unroll
+            for (int k = 0; k < 7; ++k) {
+                const Slab r = slab_from(sum, k, partner);
+                if (mine) {
+                    const Slab m = merge_slab(slab_of(sum, k), r);
+                    set_slab(sum, k, m);
+                    store_slab(a.summary, p, k, m);
+                }
+            }
+        }
+        live = live && (mine || !pair);
+        if (mine) go_up();
+        __syncwarp();  // this round's outputs before the next one's marks
+    }
+    for (;;) {
+        going = __ballot_sync(0xffffffffu, live);
+        if (__popc(going) <= kGroups) break;
+        if (!live) continue;
+        const bool second = arrive(a.visits + p) != 0;
+        const bool from_left = L == child;
+        const uint32_t other = from_left ? R : L;
+        const bool bad = (L != child && R != child) || other >= internal + a.n;
+        if (bad) atomicOr(a.err, kErrBadInput);
+        live = second && !bad;
+        if (!live) continue;
+        const Done o = load_done(a, other);
+        own = complete(a, p, L, R, w8, from_left ? own : o, from_left ? o : own);
+        if (slabs) {
+#pragma unroll
+            for (int k = 0; k < 7; ++k) {
+                const Slab sib = load_slab(a.nodes, a.verts, faces, a.summary, other, internal, k);
+                const Slab mine = slab_of(sum, k);
+                const Slab m = merge_slab(from_left ? mine : sib, from_left ? sib : mine);
+                set_slab(sum, k, m);
+                store_slab(a.summary, p, k, m);
+            }
+        }
+        go_up();
+    }
+    if (going == 0) return;
+    const uint32_t sub = lane & 7, group = lane >> 3;
+    live = group < __popc(going);
+    const int src = live ? source_lane(going, group) : 0;
+    Slab mine{0.f, 0.f, 0u, 0u};
+    if (slabs) mine = take_slab(sum, src, sub);
+    own = done_from(own, src);
+    child = __shfl_sync(0xffffffffu, child, src);
+    p = __shfl_sync(0xffffffffu, p, src);
+    steps = __shfl_sync(0xffffffffu, steps, src);
+    L = __shfl_sync(0xffffffffu, L, src);
+    R = __shfl_sync(0xffffffffu, R, src);
+    w8 = __shfl_sync(0xffffffffu, w8, src);
+    grand = __shfl_sync(0xffffffffu, grand, src);
+    __syncwarp();
+    while (__any_sync(0xffffffffu, live)) {
+        uint32_t before = 0;
+        if (live && sub == 0) before = arrive(a.visits + p);
+        before = __shfl_sync(0xffffffffu, before, 0, 8);
+        __syncwarp();  // orders the group's loads after lane 0's acquire
+        const bool from_left = L == child;
+        const uint32_t other = from_left ? R : L;
+        const bool bad = live && ((L != child && R != child) || other >= internal + a.n);
+        if (bad && sub == 0) atomicOr(a.err, kErrBadInput);
+        live = live && before != 0 && !bad;
+        if (live) {
+            if (sub == 7) {
+                const Done o = load_done(a, other);
+                own = complete(a, p, L, R, w8, from_left ? own : o, from_left ? o : own);
+            } else if (slabs) {
+                const Slab sib = load_slab(a.nodes, a.verts, faces, a.summary, other, internal, sub);
+                mine = merge_slab(from_left ? mine : sib, from_left ? sib : mine);
+                store_slab(a.summary, p, sub, mine);
+            }
+            go_up();
+        }
+        __syncwarp();  // the group's outputs before lane 0's next release
     }
 }
 

@@ -338,6 +338,54 @@ __device__ __forceinline__ void merge_right(Summary& a, const Summary& b) {
     }
 }
 
+// One slab of a 7-direction summary: extreme projections and their vertices.
+struct Slab {
+    float lo, hi;
+    uint32_t ilo, ihi;
+};
+
+// merge_right for one slab: the left child's values, the right child's where
+// strictly better.
+__device__ __forceinline__ Slab merge_slab(const Slab& l, const Slab& r) {
+    Slab o = l;
+    if (l.lo > r.lo) { o.lo = r.lo; o.ilo = r.ilo; }
+    if (l.hi < r.hi) { o.hi = r.hi; o.ihi = r.ihi; }
+    return o;
+}
+
+__device__ __forceinline__ Slab slab_of(const Summary& s, int k) { return Slab{s.lo[k], s.hi[k], s.ilo[k], s.ihi[k]}; }
+__device__ __forceinline__ void set_slab(Summary& s, int k, const Slab& v) {
+    s.lo[k] = v.lo; s.hi[k] = v.hi; s.ilo[k] = v.ilo; s.ihi[k] = v.ihi;
+}
+
+// slab7()[k] of one point, evaluated as slab7 does
+__device__ __forceinline__ float slab_at(f3 p, int k) {
+    switch (k) {
+        case 0: return p.x;
+        case 1: return p.y;
+        case 2: return p.z;
+        case 3: return p.x + p.y + p.z;
+        case 4: return p.x + p.y - p.z;
+        case 5: return p.x - p.y + p.z;
+        default: return p.x - p.y - p.z;
+    }
+}
+
+// Slab k of a triangle's summary (leaf_summary).
+__device__ __forceinline__ Slab face_slab(const kr_vec3* verts, uint4 face, int k) {
+    const uint32_t id[3] = {face.x, face.y, face.z};
+    Slab o;
+    o.lo = o.hi = slab_at(load_vertex(verts, id[0]), k);
+    o.ilo = o.ihi = id[0];
+#pragma unroll
+    for (int i = 1; i < 3; ++i) {
+        const float q = slab_at(load_vertex(verts, id[i]), k);
+        if (q < o.lo) { o.lo = q; o.ilo = id[i]; }
+        if (q > o.hi) { o.hi = q; o.ihi = id[i]; }
+    }
+    return o;
+}
+
 // ---------------------------------------------------------------------------
 // DiTO-14 candidate of one internal node (calculate_candidate_obb_kernel,
 // transforms.cu:676-756, with the helpers at :413-674) from the 14 extremal

@@ -42,39 +42,6 @@ struct Carry {
     float cost;
 };
 
-// One slab of a 7-direction summary: extreme projections and their vertices.
-struct Slab {
-    float lo, hi;
-    uint32_t ilo, ihi;
-};
-
-// merge_right for one slab: the left child's values, the right child's where
-// strictly better.
-__device__ __forceinline__ Slab merge_slab(const Slab& l, const Slab& r) {
-    Slab o = l;
-    if (l.lo > r.lo) { o.lo = r.lo; o.ilo = r.ilo; }
-    if (l.hi < r.hi) { o.hi = r.hi; o.ihi = r.ihi; }
-    return o;
-}
-
-__device__ __forceinline__ Slab slab_of(const Summary& s, int k) { return Slab{s.lo[k], s.hi[k], s.ilo[k], s.ihi[k]}; }
-__device__ __forceinline__ void set_slab(Summary& s, int k, const Slab& v) {
-    s.lo[k] = v.lo; s.hi[k] = v.hi; s.ilo[k] = v.ilo; s.ihi[k] = v.ihi;
-}
-
-// slab7()[k] of one point, evaluated as slab7 does
-__device__ __forceinline__ float slab_at(f3 p, int k) {
-    switch (k) {
-        case 0: return p.x;
-        case 1: return p.y;
-        case 2: return p.z;
-        case 3: return p.x + p.y + p.z;
-        case 4: return p.x + p.y - p.z;
-        case 5: return p.x - p.y + p.z;
-        default: return p.x - p.y - p.z;
-    }
-}
-
 // Slab k of sorted leaf j's summary (leaf_summary over vertex slots 3j..3j+2).
 __device__ __forceinline__ Slab leaf_slab(const f3* v, uint32_t j, int k) {
     Slab o;

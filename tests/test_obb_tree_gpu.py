@@ -124,6 +124,42 @@ def test_obb_tree_on_a_non_morton_tree():
     assert same_bits(xfs.cpu().numpy(), want_x)
 
 
+@pytest.mark.parametrize("n", [2, 31, 32, 33, 255, 257, 1000])
+@pytest.mark.parametrize("spread", [0, 3, 100])
+def test_obb_tree_where_siblings_meet_in_a_warp_and_across(n, spread):
+    """Neighbours in depth-first order `spread` leaf numbers apart on average:
+    from walks that all meet within a warp to walks that never do."""
+    import torch
+    rng = np.random.default_rng(1000 * spread + n)
+    v, f = workloads.triangle_soup(n, seed=n)
+    nodes, parents = _random_tree(n, rng)
+    # leaves renumbered: depth-first rank, jittered by `spread`
+    order, stack = [], [0]
+    while stack:
+        k = stack.pop()
+        if k >= n - 1:
+            order.append(k)
+        else:
+            stack += [int(nodes["right"][k]), int(nodes["left"][k])]
+    new = np.empty(n, np.int64)
+    rank = np.argsort(np.argsort(np.arange(n) + rng.uniform(0, spread, n), kind="stable"), kind="stable")
+    new[np.array(order) - (n - 1)] = n - 1 + rank
+    for side in ("left", "right"):
+        kids = nodes[side][:n - 1].astype(np.int64)
+        nodes[side][:n - 1] = np.where(kids >= n - 1, new[np.maximum(kids, n - 1) - (n - 1)], kids)
+    nodes["left"][n - 1:] = rng.permutation(n)
+    parents[:] = 0xFFFFFFFF
+    for k in range(n - 1):
+        parents[nodes["left"][k]] = parents[nodes["right"][k]] = k
+    mesh = bvh.Mesh(v, f)
+    tree = {"nodes": torch.from_numpy(nodes.view(np.uint8).copy()).cuda(),
+            "parents": torch.from_numpy(parents.view(np.int32).copy()).cuda()}
+    obbs, xfs = bvh.obb_tree(mesh, tree)
+    want_o, want_x, _ = ref.obb_tree(nodes, parents, v, f)
+    assert same_bits(obbs.cpu().numpy(), want_o)
+    assert same_bits(xfs.cpu().numpy(), want_x)
+
+
 def test_obb_tree_rejects_a_parent_cycle():
     """A malformed tree ends with an error from the bounded walks, not a hang."""
     import torch
