@@ -139,19 +139,6 @@ __device__ __forceinline__ Slab slab_from(const Summary& s, int k, uint32_t lane
                 __shfl_sync(0xffffffffu, s.ilo[k], lane), __shfl_sync(0xffffffffu, s.ihi[k], lane)};
 }
 
-// Whether another lane of the warp stands at the same parent with its other
-// child, and which (else the lane itself).
-__device__ __forceinline__ bool paired(bool live, uint32_t p, uint32_t child, uint32_t L, uint32_t R, uint32_t lane,
-                                       uint32_t& partner) {
-    // p < internal < 2^31; lanes without a walk match no one
-    const uint32_t same = __match_any_sync(0xffffffffu, live ? p : 0x80000000u | lane);
-    partner = __popc(same) == 2 ? static_cast<uint32_t>(__ffs(static_cast<int>(same ^ (1u << lane))) - 1) : lane;
-    const uint32_t theirs = __shfl_sync(0xffffffffu, child, partner);
-    const bool pair = partner != lane && ((L == child && R == theirs) || (R == child && L == theirs));
-    if (!pair) partner = lane;
-    return pair;
-}
-
 // The boxes and transforms of a warp's leaves, consecutive records from obbs
 // and xfs on: staged in shared memory (rows of 15 and of 20 words: no two
 // lanes of an access in one bank) and written out in full sectors.

@@ -28,6 +28,19 @@ __device__ __forceinline__ uint32_t arrive(uint32_t* counter) {
     return old;
 }
 
+// Whether another lane of the warp stands at the same parent with its other
+// child, and which (else the lane itself).
+__device__ __forceinline__ bool paired(bool live, uint32_t p, uint32_t child, uint32_t L, uint32_t R, uint32_t lane,
+                                       uint32_t& partner) {
+    // p < internal < 2^31; lanes without a walk match no one
+    const uint32_t same = __match_any_sync(0xffffffffu, live ? p : 0x80000000u | lane);
+    partner = __popc(same) == 2 ? static_cast<uint32_t>(__ffs(static_cast<int>(same ^ (1u << lane))) - 1) : lane;
+    const uint32_t theirs = __shfl_sync(0xffffffffu, child, partner);
+    const bool pair = partner != lane && ((L == child && R == theirs) || (R == child && L == theirs));
+    if (!pair) partner = lane;
+    return pair;
+}
+
 // kr_bvh_node field access through 4-byte words (the struct is 36 bytes,
 // 4-byte aligned): words 0..5 bounds, 6 left|primitivesOffset, 7 right,
 // 8 nPrimitives | axis << 16.
