@@ -180,11 +180,11 @@ __global__ void __launch_bounds__(kThreads) leaves_fused_kernel(TreeArgs tree_ar
 // kRow words (one word per node; the odd row length spreads a node's words
 // over the banks).  Internal node rows: bounds (6), cost, the 14 slab values,
 // then the 14 slab vertices as 16-bit offsets from 3 * j0, two per word (7).
-// Leaf rows: bounds (6) and the three vertices (9); a leaf's cost and slabs
-// are recomputed from them.
+// Leaf rows: bounds (6), the 14 slab values and which of the leaf's vertices
+// they are, two bits each (1); a leaf's cost is recomputed from its bounds.
 constexpr uint32_t kRow = kThreads + 1;
 constexpr int kSlotRows = 28;
-constexpr int kLeafRows = 15;
+constexpr int kLeafRows = 21;
 constexpr uint16_t kLeafKid = 0x8000u;  // child encoding: leaf j0 + q, else internal node j0 + q
 constexpr uint16_t kNotLocal = 0xffffu;
 
@@ -195,7 +195,7 @@ struct LocalSmem {
     uint16_t kid[2][kThreads];  // its children
     uint16_t cnt[kThreads];     // its primitive count
     uint16_t up[kThreads];      // its parent's local index, or kNotLocal
-    uint8_t queue[3][kThreads]; // nodes ready in a round
+    uint32_t queue[2][kThreads];  // nodes ready in a round (turn_of)
     uint8_t local[kThreads], iflag[kThreads], lflag[kThreads], hidden[kThreads];
     uint32_t qn[3];
     uint32_t nfront;
@@ -219,6 +219,14 @@ __device__ __forceinline__ void get_bounds(const uint32_t* slots, uint32_t q, Ca
     }
 }
 
+// Node j0 + q and its children in one word of the queue.
+constexpr uint32_t kLeftLeaf = 1u << 24, kRightLeaf = 1u << 25;
+__device__ __forceinline__ uint32_t turn_of(const LocalSmem& sm, uint32_t q) {
+    const uint32_t l = sm.kid[0][q], r = sm.kid[1][q];
+    return q | ((l & 0xffu) << 8) | ((r & 0xffu) << 16) | (l & kLeafKid ? kLeftLeaf : 0u) |
+           (r & kLeafKid ? kRightLeaf : 0u);
+}
+
 // carry of internal node j0 + q / of leaf j0 + q (its cost: leaf_ct * area)
 __device__ __forceinline__ Carry get_carry(const LocalSmem& sm, uint32_t q, bool leaf, float leaf_ct) {
     Carry c;
@@ -227,24 +235,18 @@ __device__ __forceinline__ Carry get_carry(const LocalSmem& sm, uint32_t q, bool
     return c;
 }
 
-__device__ __forceinline__ void put_slab(uint32_t* islot, uint32_t q, int k, const Slab& v, uint32_t base3) {
+// Slab k of internal node / leaf j0 + q; its vertices as offsets from 3 * j0.
+__device__ __forceinline__ void put_slab(uint32_t* islot, uint32_t q, uint32_t k, const Slab& v) {
     islot[(7 + 2 * k) * kRow + q] = __float_as_uint(v.lo);
     islot[(8 + 2 * k) * kRow + q] = __float_as_uint(v.hi);
-    islot[(21 + k) * kRow + q] = (v.ilo - base3) | ((v.ihi - base3) << 16);
+    islot[(21 + k) * kRow + q] = v.ilo | (v.ihi << 16);
 }
 
-__device__ __forceinline__ Slab get_slab(const uint32_t* islot, uint32_t q, int k, uint32_t base3) {
-    const uint32_t ids = islot[(21 + k) * kRow + q];
-    return Slab{__uint_as_float(islot[(7 + 2 * k) * kRow + q]), __uint_as_float(islot[(8 + 2 * k) * kRow + q]),
-                base3 + (ids & 0xffffu), base3 + (ids >> 16)};
-}
-
-// The vertices of leaf j0 + q, for its slabs (leaf_slab).
-__device__ __forceinline__ void leaf_vertices(const LocalSmem& sm, uint32_t q, f3* v) {
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-        v[i] = mk3(__uint_as_float(sm.lslot[(6 + 3 * i) * kRow + q]), __uint_as_float(sm.lslot[(7 + 3 * i) * kRow + q]),
-                   __uint_as_float(sm.lslot[(8 + 3 * i) * kRow + q]));
+__device__ __forceinline__ Slab get_slab(const LocalSmem& sm, uint32_t q, bool leaf, uint32_t k) {
+    const uint32_t* at = (leaf ? sm.lslot + 6 * kRow : sm.islot + 7 * kRow) + 2 * k * kRow + q;
+    const uint32_t ids = leaf ? sm.lslot[20 * kRow + q] >> (4 * k) : sm.islot[(21 + k) * kRow + q];
+    return Slab{__uint_as_float(at[0]), __uint_as_float(at[kRow]), leaf ? 3 * q + (ids & 3u) : ids & 0xffffu,
+                leaf ? 3 * q + ((ids >> 2) & 3u) : ids >> 16};
 }
 
 // Bottom-up pass, part 1 of 2: bounds, costs, collapse marks and summaries of
@@ -255,12 +257,20 @@ __device__ __forceinline__ void leaf_vertices(const LocalSmem& sm, uint32_t q, f
 // CTA b takes sorted leaves [j0, jend).  A Karras node lies at one end of its
 // own leaf range, so an internal node whose range lies within these leaves
 // ("local") has its index in [j0, jend) too.  The local nodes are completed
-// in rounds separated by CTA barriers: a round's ready nodes sit in a queue
-// and go to its first threads (to groups of 8 threads when few are ready); a
-// completed node's parent joins the next round's queue once both children
-// are done.  Children are read from shared
-// memory, and the outputs are written at the end as contiguous runs.  The
-// leaves and local nodes whose parents are not local go to a list for part 2.
+// in rounds separated by CTA barriers: a round's ready nodes sit in a queue;
+// a completed node's parent joins the next round's queue once both children
+// are done.  Children are read from shared memory, and the outputs are written
+// at the end as contiguous runs.  The leaves and local nodes whose parents are
+// not local go to a list for part 2.
+//
+// Bound by the length of a round, a chain of shared memory reads and compares
+// that few warps run: a random mesh takes about nine rounds.  So the work on a
+// node is dealt out by parts, its carry and each of its seven slabs to a warp
+// of its own with up to 32 nodes side by side, and the leaves' slabs are made
+// by all threads before the first round.  This kernel in a build of 2,000,000
+// triangles: 323 us with a thread for a whole node (eight where few were
+// ready), 274 with the parts dealt out, 255 with the children named in the
+// queue and the parts turning from warp to warp.
 __global__ void __launch_bounds__(kThreads, 4) fused_up_local_kernel(UpArgs a, uint32_t* frontier,
                                                                      uint32_t* frontier_counts) {
     extern __shared__ __align__(16) unsigned char fused_smem[];
@@ -276,9 +286,11 @@ __global__ void __launch_bounds__(kThreads, 4) fused_up_local_kernel(UpArgs a, u
     const float leaf_ct = a.flags ? a.ct : 1.0f;
     // The CTA's triangles (or, without summaries, its leaf records) are
     // contiguous runs of 9 words each: read word by word across the CTA
-    // (coalesced) into the leaf rows, every load in flight before the first
-    // store.  With the triangles at hand, a leaf's bounds are recomputed
-    // from its vertices below (exact min/max: the bits of its record).
+    // (coalesced), every load in flight before the first store: the records'
+    // bounds into the leaf rows, the triangles into rows of the internal
+    // nodes, which nothing else uses before the rounds.  With the triangles at
+    // hand, a leaf's bounds are recomputed from its vertices below (exact
+    // min/max: the bits of its record).
     {
         const uint32_t* src = with_summary ? reinterpret_cast<const uint32_t*>(a.tris + 9 * static_cast<size_t>(j0))
                                            : reinterpret_cast<const uint32_t*>(a.nodes + internal + j0);
@@ -293,7 +305,7 @@ __global__ void __launch_bounds__(kThreads, 4) fused_up_local_kernel(UpArgs a, u
             const uint32_t w = t + r * kThreads;
             if (w >= 9 * m) continue;
             const uint32_t q = w / 9, k = w - 9 * q;
-            if (with_summary) sm.lslot[(6 + k) * kRow + q] = vw[r];
+            if (with_summary) sm.islot[k * kRow + q] = vw[r];
             else if (k < 6) sm.lslot[k * kRow + q] = vw[r];
         }
     }
@@ -329,9 +341,12 @@ __global__ void __launch_bounds__(kThreads, 4) fused_up_local_kernel(UpArgs a, u
     if (t == 0) sm.nfront = 0;
     __syncthreads();
     if (t < m) {
-        if (with_summary) {  // the triangle's box (lbvh::tri_box) from its vertex rows
+        if (with_summary) {  // the triangle's box (lbvh::tri_box) and slabs from its vertices
             f3 v[3];
-            leaf_vertices(sm, t, v);
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+                v[i] = mk3(__uint_as_float(sm.islot[3 * i * kRow + t]), __uint_as_float(sm.islot[(3 * i + 1) * kRow + t]),
+                           __uint_as_float(sm.islot[(3 * i + 2) * kRow + t]));
             const f3 lo = vmin3(vmin3(v[0], v[1]), v[2]), hi = vmax3(vmax3(v[0], v[1]), v[2]);
             sm.lslot[0 * kRow + t] = __float_as_uint(lo.x);
             sm.lslot[1 * kRow + t] = __float_as_uint(lo.y);
@@ -339,6 +354,15 @@ __global__ void __launch_bounds__(kThreads, 4) fused_up_local_kernel(UpArgs a, u
             sm.lslot[3 * kRow + t] = __float_as_uint(hi.x);
             sm.lslot[4 * kRow + t] = __float_as_uint(hi.y);
             sm.lslot[5 * kRow + t] = __float_as_uint(hi.z);
+            uint32_t ids = 0;
+#pragma unroll
+            for (int k = 0; k < 7; ++k) {
+                const Slab o = leaf_slab(v, 0, k);
+                sm.lslot[(6 + 2 * k) * kRow + t] = __float_as_uint(o.lo);
+                sm.lslot[(7 + 2 * k) * kRow + t] = __float_as_uint(o.hi);
+                ids |= (o.ilo | (o.ihi << 2)) << (4 * k);
+            }
+            sm.lslot[20 * kRow + t] = ids;
         }
         Carry c;
         get_bounds(sm.lslot, t, c);
@@ -348,11 +372,11 @@ __global__ void __launch_bounds__(kThreads, 4) fused_up_local_kernel(UpArgs a, u
     const auto is_local = [&](uint32_t x) { return x != kNoParent && x - j0 < m && sm.local[x - j0]; };
     if (mine) {
         sm.up[t] = is_local(parent) ? static_cast<uint16_t>(parent - j0) : kNotLocal;
-        if (sm.deg[t] == 0) sm.queue[0][atomicAdd(&sm.qn[0], 1u)] = static_cast<uint8_t>(t);
+        if (sm.deg[t] == 0) sm.queue[0][atomicAdd(&sm.qn[0], 1u)] = turn_of(sm, t);
     }
     __syncthreads();
-    // Rounds.  Counters rotate over three slots: a round reads one, appends
-    // to the next and clears the one read the round before.
+    // Rounds.  The queue's counters rotate over three slots: a round reads one,
+    // appends to the next and clears the one read the round before.
     for (uint32_t r = 0;; ++r) {
         const uint32_t cur = r % 3, nxt = (r + 1) % 3, old = (r + 2) % 3;
         const uint32_t K = sm.qn[cur];
@@ -362,78 +386,62 @@ __global__ void __launch_bounds__(kThreads, 4) fused_up_local_kernel(UpArgs a, u
             break;
         }
         if (t == 0) sm.qn[old] = 0;
-        // Up to kThreads / 8 ready nodes: a group of 8 lanes per node (lanes
-        // 0..6 one summary slab each, lane 7 the rest).  More: a thread each.
-        const bool grouped = K <= kThreads / 8;
-        const uint32_t g = grouped ? t >> 3 : t;
-        const uint32_t sub = grouped ? (t & 7) : 8u;  // 8: the whole node
-        if (g < K) {
-            const uint32_t q = sm.queue[cur][g];
-            const uint32_t kl = sm.kid[0][q], kr = sm.kid[1][q];
-            const bool lleaf = kl & kLeafKid, rleaf = kr & kLeafKid;
-            const uint32_t lq = kl & 0xffu, rq = kr & 0xffu;
-            if (sub >= 7) {
-                const uint32_t count = sm.cnt[q];
-                const Carry l = get_carry(sm, lq, lleaf, leaf_ct);
-                const Carry rc = get_carry(sm, rq, rleaf, leaf_ct);
-                Carry o;
+        // Part 0 of a node is its carry (and its parent's turn), part 1 + k
+        // its slab k; the warps change parts from one 32 nodes to the next,
+        // since part 0 is the longest.  Without summaries there is part 0 only.
+        const uint32_t step = with_summary ? 32u : static_cast<uint32_t>(kThreads);
+        for (uint32_t s = t >> 5, i = t & (step - 1); i < K; ++s, i += step) {
+            const uint32_t part = with_summary ? s & 7u : 0u;
+            const uint32_t turn = sm.queue[r & 1][i], q = turn & 0xffu;
+            const bool lleaf = turn & kLeftLeaf, rleaf = turn & kRightLeaf;
+            const uint32_t lq = (turn >> 8) & 0xffu, rq = (turn >> 16) & 0xffu;
+            if (part > 0) {
+                put_slab(sm.islot, q, part - 1,
+                         merge_slab(get_slab(sm, lq, lleaf, part - 1), get_slab(sm, rq, rleaf, part - 1)));
+                continue;
+            }
+            const uint32_t count = sm.cnt[q];
+            const Carry l = get_carry(sm, lq, lleaf, leaf_ct);
+            const Carry rc = get_carry(sm, rq, rleaf, leaf_ct);
+            Carry o;
 #pragma unroll
-                for (int k = 0; k < 3; ++k) {  // kr_aabb_expand(left, right)
-                    o.lo[k] = kmin(kmin(l.lo[k], rc.lo[k]), rc.hi[k]);
-                    o.hi[k] = kmax(kmax(l.hi[k], rc.lo[k]), rc.hi[k]);
-                }
-                const float area = box_area(o.lo, o.hi);
-                if (a.flags) {
-                    // bvh_mark_collapse_kernel (transforms.cu:111-133)
-                    const float node_cost = a.ci * area + l.cost + rc.cost;
-                    const float leaf_cost = a.ct * area * static_cast<float>(count);
-                    if (leaf_cost < node_cost && count <= kMaxLeafSize) {
-                        o.cost = leaf_cost;
-                        sm.iflag[q] = 1;
-                        // collapsed children: marked, and nPrimitives = 0xFFFF (axis byte and pad are zero)
-                        if (lleaf) {
-                            sm.lflag[lq] = 1;
-                            __stcg(reinterpret_cast<uint32_t*>(a.collapsed + internal + j0 + lq) + 8, kHidden);
-                        } else {
-                            sm.iflag[lq] = 1;
-                            sm.hidden[lq] = 1;
-                        }
-                        if (rleaf) {
-                            sm.lflag[rq] = 1;
-                            __stcg(reinterpret_cast<uint32_t*>(a.collapsed + internal + j0 + rq) + 8, kHidden);
-                        } else {
-                            sm.iflag[rq] = 1;
-                            sm.hidden[rq] = 1;
-                        }
+            for (int k = 0; k < 3; ++k) {  // kr_aabb_expand(left, right)
+                o.lo[k] = kmin(kmin(l.lo[k], rc.lo[k]), rc.hi[k]);
+                o.hi[k] = kmax(kmax(l.hi[k], rc.lo[k]), rc.hi[k]);
+            }
+            const float area = box_area(o.lo, o.hi);
+            if (a.flags) {
+                // bvh_mark_collapse_kernel (transforms.cu:111-133)
+                const float node_cost = a.ci * area + l.cost + rc.cost;
+                const float leaf_cost = a.ct * area * static_cast<float>(count);
+                if (leaf_cost < node_cost && count <= kMaxLeafSize) {
+                    o.cost = leaf_cost;
+                    sm.iflag[q] = 1;
+                    // collapsed children: marked, and nPrimitives = 0xFFFF (axis byte and pad are zero)
+                    if (lleaf) {
+                        sm.lflag[lq] = 1;
+                        __stcg(reinterpret_cast<uint32_t*>(a.collapsed + internal + j0 + lq) + 8, kHidden);
                     } else {
-                        o.cost = node_cost;
+                        sm.iflag[lq] = 1;
+                        sm.hidden[lq] = 1;
+                    }
+                    if (rleaf) {
+                        sm.lflag[rq] = 1;
+                        __stcg(reinterpret_cast<uint32_t*>(a.collapsed + internal + j0 + rq) + 8, kHidden);
+                    } else {
+                        sm.iflag[rq] = 1;
+                        sm.hidden[rq] = 1;
                     }
                 } else {
-                    o.cost = 1.2f * area + rc.cost + l.cost;  // calculate_aabbs_kernel (lbvh.cu:452)
+                    o.cost = node_cost;
                 }
-                put_carry(sm.islot, q, o);
+            } else {
+                o.cost = 1.2f * area + rc.cost + l.cost;  // calculate_aabbs_kernel (lbvh.cu:452)
             }
-            if (with_summary && sub != 7) {
-                f3 lv[3], rv[3];
-                if (lleaf) leaf_vertices(sm, lq, lv);
-                if (rleaf) leaf_vertices(sm, rq, rv);
-                const auto slab = [&](int k) {
-                    const Slab ls = lleaf ? leaf_slab(lv, j0 + lq, k) : get_slab(sm.islot, lq, k, 3 * j0);
-                    const Slab rs = rleaf ? leaf_slab(rv, j0 + rq, k) : get_slab(sm.islot, rq, k, 3 * j0);
-                    put_slab(sm.islot, q, k, merge_slab(ls, rs), 3 * j0);
-                };
-                if (sub == 8) {
-#pragma unroll
-                    for (int k = 0; k < 7; ++k) slab(k);
-                } else {
-                    slab(static_cast<int>(sub));
-                }
-            }
-            if (sub >= 7) {
-                const uint32_t u = sm.up[q];
-                if (u != kNotLocal && atomicSub(&sm.deg[u], 1u) == 1u)
-                    sm.queue[nxt][atomicAdd(&sm.qn[nxt], 1u)] = static_cast<uint8_t>(u);
-            }
+            put_carry(sm.islot, q, o);
+            const uint32_t above = sm.up[q];
+            if (above != kNotLocal && atomicSub(&sm.deg[above], 1u) == 1u)
+                sm.queue[(r + 1) & 1][atomicAdd(&sm.qn[nxt], 1u)] = turn_of(sm, above);
         }
         __syncthreads();
     }

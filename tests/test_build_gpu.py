@@ -80,6 +80,16 @@ def test_fused_build_at_block_tile_and_sort_edges(builder, n):
     _check(o, slots, _expect(v, f), n, 3)
 
 
+@pytest.mark.parametrize("n", [33, 64, 97, 127, 191])
+@pytest.mark.parametrize("flags", [0, 3])
+def test_fused_build_around_rounds_of_one_warp(builder, n, flags):
+    """A block's first rounds with fewer and with more than 32 ready nodes,
+    with and without summaries."""
+    v, f = workloads.triangle_soup(n, seed=900 + n)
+    o, slots = _run(builder, v, f, flags)
+    _check(o, slots, _expect(v, f), n, flags)
+
+
 def test_workspace_grows_with_the_face_count():
     """A builder keeps the workspace of its largest mesh for smaller ones."""
     from obvh_b200 import _native
