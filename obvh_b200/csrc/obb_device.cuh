@@ -113,6 +113,24 @@ __device__ __forceinline__ void project_tri_own(const float* t, const Axes& ax, 
     project_tri_from<From::kShared>(t, ax, lo, hi);
 }
 
+// Whether some point of the box [lo, hi] can have a projection on one of the
+// axes beyond the extents [c.olo, c.ohi] that the node starts from.  Rounded
+// products and sums are monotonic, so dot3 evaluated as for the points, at the
+// box's corner furthest along the axis, bounds the computed projections of all
+// points in the box, not only the exact ones: where this is false they cannot
+// change a minimum or maximum.  A NaN bound counts as beyond.
+__device__ __forceinline__ bool may_extend(const float lo[3], const float hi[3], const Cand& c) {
+    bool inside = true;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const f3 d = mk3(c.ax[3 * k], c.ax[3 * k + 1], c.ax[3 * k + 2]);
+        const f3 far = mk3(d.x >= 0.f ? hi[0] : lo[0], d.y >= 0.f ? hi[1] : lo[1], d.z >= 0.f ? hi[2] : lo[2]);
+        const f3 near = mk3(d.x >= 0.f ? lo[0] : hi[0], d.y >= 0.f ? lo[1] : hi[1], d.z >= 0.f ? lo[2] : hi[2]);
+        inside = inside && dot3(far, d) <= c.ohi[k] && dot3(near, d) >= c.olo[k];
+    }
+    return !inside;
+}
+
 // Extents over a node's leaf run go by size: a thread alone for up to
 // kSoloLeaves leaves, 8 lanes for up to kGroupLeaves, a warp above.  A Karras
 // tree's nodes are mostly tiny (half have 2 or 3 leaves), and one thread per

@@ -90,6 +90,30 @@ def test_fused_build_around_rounds_of_one_warp(builder, n, flags):
     _check(o, slots, _expect(v, f), n, flags)
 
 
+def _shapes(kind, n, seed):
+    """Meshes whose blocks of leaves all touch their nodes' extents (a flat
+    sheet along the axes, one turned), few do (a shell), or all reach across
+    the whole mesh (large triangles)."""
+    rng = np.random.default_rng(seed)
+    c = rng.uniform(-1, 1, (n, 1, 3))
+    if kind == "shell":
+        c /= np.linalg.norm(c, axis=2, keepdims=True)
+    v = c + rng.uniform(-1, 1, (n, 3, 3)) * (1.0 if kind == "large" else 0.01)
+    if kind in ("sheet", "turned"):
+        v[..., 2] = 0.0
+    if kind == "turned":
+        v = v @ workloads.random_rotation(rng).T
+    return v.reshape(-1, 3).astype(np.float32), np.arange(3 * n, dtype=np.uint32).reshape(n, 3)
+
+
+@pytest.mark.parametrize("kind", ["sheet", "turned", "shell", "large"])
+@pytest.mark.parametrize("n", [300, 5000])
+def test_fused_build_extents_by_blocks(builder, kind, n):
+    v, f = _shapes(kind, n, n)
+    o, slots = _run(builder, v, f, 3)
+    _check(o, slots, _expect(v, f), n, 3)
+
+
 def test_workspace_grows_with_the_face_count():
     """A builder keeps the workspace of its largest mesh for smaller ones."""
     from obvh_b200 import _native
