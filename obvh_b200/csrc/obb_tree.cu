@@ -16,17 +16,21 @@
 //   candidate    node-parallel DiTO-14 candidate axes from the 14 summary
 //                vertices (:676-756) and the initial extents along them.
 //   extents      min/max of every subtree vertex on the node's axes, read
-//                from the contiguous run: one thread per node up to 32
-//                leaves, one warp per 1024-leaf unit above that (units dealt
-//                to the warps of a persistent grid); only nodes of more than
-//                one unit combine partial results, with 6 integer atomics per
-//                unit.  Nodes finished here are finalised in place (:903-964).
+//                from the contiguous run: the candidate's own thread for up
+//                to 8 leaves, 8 lanes for up to 32, one warp per 512-leaf unit
+//                above that (listed by the candidate kernel, dealt to the
+//                warps of a persistent grid); blocks of 32 leaves whose boxes
+//                lie within the node's extents so far are passed over; only
+//                nodes of more than one unit combine partial results, with 6
+//                integer atomics per unit.
 //                For a Karras tree (the fused build), tiles instead: one CTA
 //                per 1,024 (256) consecutive leaves stages their triangles in shared
 //                memory once and serves every node over them from there.
-//   finalize     the nodes of more than one unit or tile.
+//   finalize     the listed nodes' boxes (:903-964); others are finalised in
+//                place.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <mutex>
 #include <unordered_map>
@@ -46,8 +50,10 @@ using namespace tree;
 
 constexpr int kThreads = 256;
 constexpr uint32_t kCollapseLeafMax = 8;  // MAX_LEAF_SIZE (transforms.cu:65)
-constexpr uint32_t kUnit = 1024;    // leaves per warp unit
-constexpr uint32_t kUnitRun = 4;   // consecutive units per warp visit
+// Leaves per warp unit (us, 128 / 256 / 512 / 1,024 / 2,048: transform of 229,824
+// triangles 260 / 258 / 260 / 267 / 282, ATRBVH of 917,504 2,300 / 2,278 /
+// 2,270 / 2,280 / 2,299; four 1,024s in a row for a warp 281 and 2,311).
+constexpr uint32_t kUnit = 512;
 // Tiled extents: 1,024 leaves per tile, or 256 for up to kSmallTiles leaves, so
 // that a small tree spreads over more SMs (us a build, 1,024 / 256: 1,021
 // triangles 111 / 99, 10,007 157 / 141, 57,344 211 / 195, 200,003 299 / 274,
@@ -69,8 +75,9 @@ constexpr uint32_t tile_items(uint32_t shift) { return shift == kTileShiftLarge 
 
 struct Ctl {
     uint32_t error;
-    uint32_t total_units;
-    uint32_t pad[62];
+    uint32_t groups;             // PlanArgs
+    unsigned long long units;
+    uint32_t pad[60];
 };
 
 __device__ __forceinline__ uint32_t count_of(const uint32_t* counts, uint32_t node, uint32_t internal) {
@@ -626,11 +633,16 @@ __global__ void __launch_bounds__(kThreads) dfs_rank_kernel(const kr_bvh_node* n
 
 // `points` is the packed xyz array the summary's vertex ids index: the mesh
 // vertices, or the depth-first triangle slots of the fused build.
+// Tiled: a thread per node, extents in tiles; listed: those of chain.list
+// (FrameNodes::kAcross), extents in tiles; planned: a thread per node, extents
+// by plan_node's lists.
+enum class Nodes { kTiled, kListed, kPlanned };
+
 struct ChainArgs {
     const uint32_t* parents;  // null: per-node extents, no chains
     const uint32_t* first;
     uint32_t n;
-    uint32_t walker_blocks;   // leading CTAs that walk the tile chains
+    uint32_t walker_blocks;   // leading CTAs that walk the tile chains, or box the blocks of leaves
     uint32_t* chains;
     uint32_t* chain_counts;
     uint32_t* err;
@@ -639,6 +651,18 @@ struct ChainArgs {
     uint32_t which;           // FrameNodes: all nodes, or those inside / across aligned leaf blocks
     uint32_t block_shift;     // the blocks hold 2^block_shift leaves
     uint32_t tile_shift;      // the tiles 2^tile_shift
+    // Without tiles: the leaves' triangles in depth-first order, the boxes of
+    // each 32 of them (block_box), the outputs for the nodes of up to
+    // kSoloLeaves leaves (finished by their candidate's thread) and the plan
+    // of the others (plan_node).
+    const float* tris;
+    float* boxes;
+    kr_obb3* obbs;
+    kr_mat4* xfs;
+    uint32_t* plan;
+    uint32_t* plan_start;
+    uint32_t* groups;
+    unsigned long long* units;
     const uint32_t* list;     // kAcross: the nodes, list_count of them
     const uint32_t* list_count;
 };
@@ -668,11 +692,68 @@ __device__ void walk_chain(const ChainArgs& c, const uint32_t* counts, uint32_t 
     c.chain_counts[w] = count;
 }
 
-// The candidate of internal node a and its extents plan (nunits, keys, the
-// finalize list).
-__device__ __forceinline__ void candidate_store(uint32_t a, const Summary& s, const Candidate& c,
-                                                const uint32_t* counts, Cand* cand, uint32_t* nunits, uint32_t* keys,
-                                                const ChainArgs& chain) {
+// The box of leaves 32k to 32k + 31 (of n, in depth-first order), for
+// may_extend: six rows of one float per block.
+__device__ void block_box(const float* tris, uint32_t n, uint32_t k, uint32_t lane, float* boxes) {
+    const uint32_t blocks = (n + 31) / 32;
+    if (k >= blocks) return;
+    float lo[3] = {kInf, kInf, kInf}, hi[3] = {-kInf, -kInf, -kInf};
+    if (32 * k + lane < n) {
+        const float* v = tris + 9 * static_cast<size_t>(32 * k + lane);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const float a = __ldg(v + d), b = __ldg(v + 3 + d), c = __ldg(v + 6 + d);
+            lo[d] = min3f(a, b, c);
+            hi[d] = max3f(a, b, c);
+        }
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const float l = warp_min(lo[d]), h = warp_max(hi[d]);
+        if (lane == 0) {
+            boxes[static_cast<size_t>(d) * blocks + k] = l;
+            boxes[static_cast<size_t>(3 + d) * blocks + k] = h;
+        }
+    }
+}
+
+// Lists node a for extents_units_kernel (every lane of a warp calls it): nodes
+// of up to kGroupLeaves leaves from the back of chain.plan, groups of them in
+// all; larger ones from the front, with the number of the first of their units
+// of kUnit leaves.  *units holds the nodes listed in front in its high word and
+// their units in the low one, so that both grow by one addition and the starts
+// ascend.  A warp adds once.
+__device__ __forceinline__ void plan_node(const ChainArgs& c, bool valid, uint32_t a, uint32_t cnt) {
+    const uint32_t lane = threadIdx.x & 31, below = (1u << lane) - 1u, internal = c.n - 1;
+    const bool big = valid && cnt > kGroupLeaves, mid = valid && cnt > kSoloLeaves && !big;
+    const uint32_t mids = __ballot_sync(0xffffffffu, mid), bigs = __ballot_sync(0xffffffffu, big);
+    if (mids) {
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(c.groups, static_cast<uint32_t>(__popc(mids)));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (mid) c.plan[internal - 1 - (base + __popc(mids & below))] = a;
+    }
+    if (bigs) {
+        const uint32_t own = big ? (cnt + kUnit - 1) / kUnit : 0u;
+        uint32_t incl = own;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
+            if (static_cast<int>(lane) >= d) incl += v;
+        }
+        const uint32_t sum = __shfl_sync(0xffffffffu, incl, 31);
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd(c.units, (static_cast<unsigned long long>(__popc(bigs)) << 32) + sum);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        const uint32_t at = static_cast<uint32_t>(base >> 32) + __popc(bigs & below);
+        if (big && at < internal) {
+            c.plan[at] = a;
+            c.plan_start[at] = static_cast<uint32_t>(base) + incl - own;
+        }
+    }
+}
+
+__device__ __forceinline__ Cand cand_of(const Summary& s, const Candidate& c) {
     Cand out;
     out.ax[0] = c.b0.x; out.ax[1] = c.b0.y; out.ax[2] = c.b0.z;
     out.ax[3] = c.b1.x; out.ax[4] = c.b1.y; out.ax[5] = c.b1.z;
@@ -682,44 +763,53 @@ __device__ __forceinline__ void candidate_store(uint32_t a, const Summary& s, co
 #pragma unroll
     for (int k = 0; k < 3; ++k) { out.alo[k] = s.lo[k]; out.ahi[k] = s.hi[k]; }
     out.pad[0] = out.pad[1] = out.pad[2] = 0.f;
+    return out;
+}
+
+// The candidate of internal node a, stored for the extents kernels with the
+// initial keys of a node that several units or tiles share.  Without tiles a
+// node of up to kSoloLeaves leaves is finished here.
+template <Nodes kNodes>
+__device__ __forceinline__ void candidate_node(uint32_t a, const uint4* summary, const kr_vec3* verts,
+                                               const uint32_t* counts, Cand* cand, uint32_t* keys, const ChainArgs& chain) {
+    Summary s;
+    const Candidate c = summary_candidate<Src::kL2, Src::kReadOnly>(summary, verts, a, chain.nz, s);
+    const Cand out = cand_of(s, c);
+    const uint32_t cnt = counts[a];  // (not held over the search)
+    if (kNodes == Nodes::kPlanned && cnt <= kSoloLeaves) {
+        float lo[3] = {c.lo.x, c.lo.y, c.lo.z}, hi[3] = {c.hi.x, c.hi.y, c.hi.z};
+        const float* t = chain.tris + 9 * static_cast<size_t>(__ldg(chain.first + a));
+        const Axes ax = cand_axes(out, chain.nz);
+        for (uint32_t i = 0; i < cnt; ++i) project_tri(t + 9 * i, ax, lo, hi);
+        finalize_node(out, mk3(lo[0], lo[1], lo[2]), mk3(hi[0], hi[1], hi[2]), chain.obbs + a, chain.xfs + a);
+        return;
+    }
     float4* dst = reinterpret_cast<float4*>(cand + a);
     const float4* src = reinterpret_cast<const float4*>(&out);
 #pragma unroll
     for (int q = 0; q < 6; ++q) dst[q] = src[q];
-    const uint32_t cnt = counts[a];
-    uint32_t units;
-    if (chain.parents) {  // tiles: 0 in one tile and small, 1 in one tile, 2 over several tiles
+    bool shared;
+    if (kNodes != Nodes::kPlanned) {
         const uint32_t f = __ldg(chain.first + a);
-        units = (f >> chain.tile_shift) != ((f + cnt - 1) >> chain.tile_shift) ? 2u : (cnt > kGroupLeaves ? 1u : 0u);
+        shared = (f >> chain.tile_shift) != ((f + cnt - 1) >> chain.tile_shift);
+        if (shared) chain.arrivals[a] = 0u;  // counted up by extents_tile_kernel
     } else {
-        units = cnt > kGroupLeaves ? (cnt + kUnit - 1) / kUnit : 0u;
+        shared = cnt > kUnit;
     }
-    nunits[a] = units;
-    if (units > 1) {
+    if (shared) {
         uint32_t* k = keys + 6 * static_cast<size_t>(a);
         k[0] = f2key(c.lo.x); k[1] = f2key(c.lo.y); k[2] = f2key(c.lo.z);
         k[3] = f2key(c.hi.x); k[4] = f2key(c.hi.y); k[5] = f2key(c.hi.z);
     }
-    if (chain.parents && units == 2) chain.arrivals[a] = 0u;  // counted up by extents_tile_kernel
 }
 
-__device__ __forceinline__ void candidate_node(uint32_t a, const uint4* summary, const kr_vec3* verts,
-                                               const uint32_t* counts, Cand* cand, uint32_t* nunits, uint32_t* keys,
-                                               const ChainArgs& chain) {
-    Summary s;
-    const Candidate c = summary_candidate<Src::kL2, Src::kReadOnly>(summary, verts, a, chain.nz, s);
-    candidate_store(a, s, c, counts, cand, nunits, keys, chain);
-}
-
-// kList: the nodes of chain.list (FrameNodes::kAcross); else one thread per
-// node (kAll, kInside).  Two instantiations, so that each holds one inlined
-// copy of the search (fewer spills).
-template <bool kList>
+// One instantiation for each kind of nodes, so that each holds one inlined copy
+// of the search and nothing of the others (fewer spills).
+template <Nodes kNodes>
 __global__ void __launch_bounds__(kThreads, 2) candidate_kernel(const uint4* summary, const kr_vec3* verts,
                                                              const uint32_t* counts, uint32_t internal, Cand* cand,
-                                                             uint32_t* nunits, uint32_t* keys, const uint32_t* err,
-                                                             ChainArgs chain) {
-    if constexpr (kList) {
+                                                             uint32_t* keys, const uint32_t* err, ChainArgs chain) {
+    if constexpr (kNodes == Nodes::kListed) {
         // the listed nodes (written by the walk that completed them), a
         // grid-stride loop so that warps stay full
         const uint32_t total = min(*chain.list_count, internal);
@@ -729,29 +819,28 @@ __global__ void __launch_bounds__(kThreads, 2) candidate_kernel(const uint4* sum
                 atomicOr(chain.err, kErrBadInput);
                 continue;
             }
-            if (*err) {
-                nunits[a] = 0;
-                continue;
-            }
-            candidate_node(a, summary, verts, counts, cand, nunits, keys, chain);
+            if (*err) continue;
+            candidate_node<kNodes>(a, summary, verts, counts, cand, keys, chain);
         }
         return;
     } else {
         if (blockIdx.x < chain.walker_blocks) {
-            if (!*err) walk_chain(chain, counts, blockIdx.x * blockDim.x + threadIdx.x);
+            const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
+            if (*err) return;
+            if constexpr (kNodes == Nodes::kTiled) walk_chain(chain, counts, w);
+            else block_box(chain.tris, chain.n, w >> 5, threadIdx.x & 31, chain.boxes);
             return;
         }
         const uint32_t a = (blockIdx.x - chain.walker_blocks) * blockDim.x + threadIdx.x;
-        if (a >= internal) return;
+        // malformed tree: no summaries to read; nothing is planned after this
+        const bool valid = a < internal && !*err;
+        if constexpr (kNodes == Nodes::kPlanned) plan_node(chain, valid, a, valid ? counts[a] : 0u);
+        if (!valid) return;
         if (chain.which == static_cast<uint32_t>(FrameNodes::kInside)) {
             const uint32_t f = __ldg(chain.first + a), cnt = __ldg(counts + a);
             if ((f >> chain.block_shift) != ((f + cnt - 1) >> chain.block_shift)) return;
         }
-        if (*err) {  // malformed tree: no summaries to read; nothing is scheduled after this
-            nunits[a] = 0;
-            return;
-        }
-        candidate_node(a, summary, verts, counts, cand, nunits, keys, chain);
+        candidate_node<kNodes>(a, summary, verts, counts, cand, keys, chain);
     }
 }
 
@@ -759,77 +848,100 @@ __global__ void __launch_bounds__(kThreads, 2) candidate_kernel(const uint4* sum
 // lanes for the nodes above kSoloLeaves, as in the tiles, was slower: 101 ->
 // 110 us on the 917K-triangle knot; here the triangles come from global memory
 // and the threads' loads in flight are what counts.)
-__global__ void __launch_bounds__(kThreads) extents_small_kernel(const Cand* cand, const uint32_t* counts,
-                                                                 const uint32_t* first, const float* tris,
-                                                                 uint32_t internal, kr_obb3* obbs, kr_mat4* xfs,
-                                                                 const uint32_t* err, float nz) {
-    const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= internal || *err) return;
-    const uint32_t cnt = counts[a];
-    if (cnt > kGroupLeaves) return;
-    const Cand c = load_cand(cand, a);
-    const f3 b0 = mk3(c.ax[0], c.ax[1], c.ax[2]), b1 = mk3(c.ax[3], c.ax[4], c.ax[5]), b2 = mk3(c.ax[6], c.ax[7], c.ax[8]);
-    float lo[3] = {c.olo[0], c.olo[1], c.olo[2]}, hi[3] = {c.ohi[0], c.ohi[1], c.ohi[2]};
-    const float* t = tris + 9 * static_cast<size_t>(first[a]);
-    const Axes ax = make_axes(b0, b1, b2, nz);
-    for (uint32_t i = 0; i < cnt; ++i) project_tri(t + 9 * i, ax, lo, hi);
-    finalize_node(c, mk3(lo[0], lo[1], lo[2]), mk3(hi[0], hi[1], hi[2]), obbs + a, xfs + a);
-}
-
-// Larger nodes: warp-sized units of kUnit leaves taken from a counter.
+// The planned nodes (plan_node): eight lanes per node of up to kGroupLeaves
+// leaves, then units of kUnit leaves of the larger ones, a warp each, dealt
+// round-robin so that big and small nodes spread over the warps.  In a unit,
+// only the blocks of 32 leaves that could extend the node are projected
+// (may_extend).  All extents go to the keys; finalize_multi_kernel builds the
+// boxes, a thread per node.
+//
+// Bound by the latency of a unit: its search, its node's records, its blocks.
+// (Before, the units were found by a search among all nodes' starts and a step
+// for every node without units in between, after a scan over all nodes; nodes
+// of up to 32 leaves were a thread's.  Boxes and transforms of 229,824
+// triangles 314 -> 260 us, the 917,504-triangle ATRBVH 2,353 -> 2,270 us.)
 __global__ void __launch_bounds__(kThreads) extents_units_kernel(const Cand* cand, const uint32_t* counts,
                                                                  const uint32_t* first, const float* tris,
-                                                                 const uint32_t* nunits, const uint32_t* unit_start,
+                                                                 const uint32_t* plan, const uint32_t* plan_start,
                                                                  uint32_t internal, const uint32_t* err,
-                                                                 const uint32_t* total_units, uint32_t* keys,
-                                                                 kr_obb3* obbs, kr_mat4* xfs, float nz) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t total = *err ? 0u : *total_units;
-    // Warps take runs of kUnitRun consecutive units round-robin: one binary
-    // search per run, and big and small nodes spread evenly over the warps.
+                                                                 const uint32_t* group_count,
+                                                                 const unsigned long long* unit_count, uint32_t* keys,
+                                                                 const float* boxes, float nz) {
+    if (*err) return;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t nblocks = (internal + 1 + 31) / 32;
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
     const uint32_t w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    for (uint32_t u0 = w * kUnitRun; u0 < total; u0 += warps * kUnitRun) {
-        const uint32_t u1 = min(total, u0 + kUnitRun);
-        uint32_t a;
-        {
-            uint32_t lo_i = 0, hi_i = internal;  // the last node whose first unit is <= u0 owns it
-            while (hi_i - lo_i > 1) {
-                const uint32_t mid = (lo_i + hi_i) >> 1;
-                if (__ldg(unit_start + mid) <= u0) lo_i = mid; else hi_i = mid;
-            }
-            a = lo_i;
+    const uint32_t groups = min(*group_count, internal);
+    for (uint32_t g0 = 4 * w; g0 < groups; g0 += 4 * warps) {
+        const uint32_t g = g0 + (lane >> 3), sub = lane & 7;
+        const bool live = g < groups;
+        const uint32_t a = __ldg(plan + (internal - 1 - (live ? g : g0)));
+        const Cand c = load_cand(cand, a);
+        float lo[3], hi[3];
+        group_extents<From::kGlobal>(tris + 9 * static_cast<size_t>(__ldg(first + a)), live ? __ldg(counts + a) : 0u,
+                                     cand_axes(c, nz), lo, hi);
+        if (live && sub < 6) {
+            const float v = sub == 0 ? fminf(c.olo[0], lo[0]) : sub == 1 ? fminf(c.olo[1], lo[1])
+                          : sub == 2 ? fminf(c.olo[2], lo[2]) : sub == 3 ? fmaxf(c.ohi[0], hi[0])
+                          : sub == 4 ? fmaxf(c.ohi[1], hi[1]) : fmaxf(c.ohi[2], hi[2]);
+            keys[6 * static_cast<size_t>(a) + sub] = f2key(v);
         }
-        for (uint32_t u = u0; u < u1; ++u) {
-            while (__ldg(unit_start + a) + __ldg(nunits + a) <= u) ++a;
-            const uint32_t chunk = u - __ldg(unit_start + a);
-            const uint32_t cnt = __ldg(counts + a);
-            const uint32_t units = __ldg(nunits + a);
-            const uint32_t begin = chunk * kUnit;
-            const uint32_t end = min(cnt, begin + kUnit);
-            const Cand c = load_cand(cand, a);
-            const f3 b0 = mk3(c.ax[0], c.ax[1], c.ax[2]), b1 = mk3(c.ax[3], c.ax[4], c.ax[5]),
-                     b2 = mk3(c.ax[6], c.ax[7], c.ax[8]);
-            float lo[3] = {kInf, kInf, kInf}, hi[3] = {-kInf, -kInf, -kInf};
-            const float* t = tris + 9 * static_cast<size_t>(__ldg(first + a));
-            const Axes ax = make_axes(b0, b1, b2, nz);
-            for (uint32_t i = begin + lane; i < end; i += 32) project_tri(t + 9 * static_cast<size_t>(i), ax, lo, hi);
+    }
+    const uint32_t listed = min(static_cast<uint32_t>(*unit_count >> 32), internal);
+    const uint32_t total = static_cast<uint32_t>(*unit_count);
+    for (uint64_t u = w; u < total; u += warps) {
+        uint32_t at = 0, end_at = listed;  // the last node whose first unit is <= u owns it
+        while (end_at - at > 1) {
+            const uint32_t step = (end_at - at + 31) / 32, probe = at + step * lane;
+            const uint32_t in = __ballot_sync(0xffffffffu, probe < end_at && __ldg(plan_start + probe) <= u);
+            at += step * (31 - __clz(static_cast<int>(in | 1u)));
+            end_at = min(end_at, at + step);
+        }
+        const uint32_t a = __ldg(plan + at);
+        const uint32_t cnt = __ldg(counts + a), f = __ldg(first + a);
+        const Cand c = load_cand(cand, a);
+        const uint32_t begin = (static_cast<uint32_t>(u) - __ldg(plan_start + at)) * kUnit;
+        if (begin >= cnt) continue;  // more than 2^32 units: the starts wrapped
+        // leaves [b, e); of the blocks of 32 those that could extend the node
+        const uint32_t b = f + begin, e = f + min(cnt, begin + kUnit);
+        const Axes ax = cand_axes(c, nz);
+        float lo[3] = {kInf, kInf, kInf}, hi[3] = {-kInf, -kInf, -kInf};
+        for (uint32_t k0 = b / 32; 32 * k0 < e; k0 += 32) {
+            const uint32_t k = k0 + lane;
+            bool beyond = 32 * k < e;
+            if (beyond) {
+                float blo[3], bhi[3];
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                lo[k] = warp_min(lo[k]);
-                hi[k] = warp_max(hi[k]);
-            }
-            if (units == 1) {
-                // the whole node in this unit: its extents go straight to the
-                // keys; finalize_multi_kernel builds the box, one thread per node
-                if (lane < 6) {
-                    const float v = lane < 3 ? fminf(c.olo[lane], lo[lane]) : fmaxf(c.ohi[lane - 3], hi[lane - 3]);
-                    __stcg(keys + 6 * static_cast<size_t>(a) + lane, f2key(v));
+                for (int d = 0; d < 3; ++d) {
+                    blo[d] = __ldg(boxes + static_cast<size_t>(d) * nblocks + k);
+                    bhi[d] = __ldg(boxes + static_cast<size_t>(3 + d) * nblocks + k);
                 }
-            } else if (lane < 6) {
-                const float v = lane < 3 ? lo[lane] : hi[lane - 3];
-                uint32_t* k = keys + 6 * static_cast<size_t>(a) + lane;
-                if (lane < 3) atomicMin(k, f2key(v)); else atomicMax(k, f2key(v));
+                beyond = may_extend(blo, bhi, c);
+            }
+            for (uint32_t some = __ballot_sync(0xffffffffu, beyond); some; some &= some - 1) {
+                const uint32_t i = 32 * (k0 + __ffs(static_cast<int>(some)) - 1) + lane;
+                if (i >= b && i < e) project_tri(tris + 9 * static_cast<size_t>(i), ax, lo, hi);
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            lo[k] = warp_min(lo[k]);
+            hi[k] = warp_max(hi[k]);
+        }
+        if (lane < 6) {
+            uint32_t* k = keys + 6 * static_cast<size_t>(a) + lane;
+            const float v = lane == 0 ? lo[0] : lane == 1 ? lo[1] : lane == 2 ? lo[2] : lane == 3 ? hi[0]
+                          : lane == 4 ? hi[1] : hi[2];
+            if (cnt <= kUnit) {  // the whole node in this unit
+                const float o = lane == 0 ? c.olo[0] : lane == 1 ? c.olo[1] : lane == 2 ? c.olo[2]
+                              : lane == 3 ? c.ohi[0] : lane == 4 ? c.ohi[1] : c.ohi[2];
+                *k = f2key(lane < 3 ? fminf(o, v) : fmaxf(o, v));
+            } else if (lane < 3) {
+                atomicMin(k, f2key(v));
+            } else {
+                atomicMax(k, f2key(v));
             }
         }
     }
@@ -1049,14 +1161,16 @@ __global__ void __launch_bounds__(kThreads) extents_tile_kernel(const Cand* cand
 
 // Nodes handled in warp units: the box from the extents in the keys (one unit:
 // written by it; several: the atomic min/max over the units).
-__global__ void __launch_bounds__(kThreads) finalize_multi_kernel(const Cand* cand, const uint32_t* nunits,
+__global__ void __launch_bounds__(kThreads) finalize_multi_kernel(const Cand* cand, const uint32_t* plan,
+                                                                  const uint32_t* group_count,
+                                                                  const unsigned long long* unit_count,
                                                                   const uint32_t* keys, uint32_t internal,
                                                                   kr_obb3* obbs, kr_mat4* xfs, const uint32_t* err) {
-    const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= internal || *err || nunits[a] == 0) return;
-    const uint32_t* k = keys + 6 * static_cast<size_t>(a);
-    finalize_node(load_cand(cand, a), mk3(key2f(k[0]), key2f(k[1]), key2f(k[2])),
-                  mk3(key2f(k[3]), key2f(k[4]), key2f(k[5])), obbs + a, xfs + a);
+    if (*err) return;
+    const uint32_t listed = min(static_cast<uint32_t>(*unit_count >> 32), internal);
+    const uint32_t all = min(listed + min(*group_count, internal), internal);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < all; i += gridDim.x * blockDim.x)
+        finalize_keys(cand, keys, i < listed ? plan[i] : plan[internal - 1 - (i - listed)], obbs, xfs);
 }
 
 // ---------------------------------------------------------------------------
@@ -1075,10 +1189,9 @@ Layout layout(uint32_t n) {
     L.tris = o;     o += align256(36ull * (n > 0 ? n : 1));
     L.rank_prims = o; o += align256(4ull * (n > 0 ? n : 1));
     L.cand = o;     o += align256(sizeof(Cand) * ni);
-    L.nunits = o;   o += align256(4 * ni);
+    L.plan = o;     o += align256(4 * ni);
     L.ustart = o;   o += align256(4 * ni);
     L.keys = o;     o += align256(24 * ni);
-    L.scan = o;     o += align256(scan_temp_bytes(ni));
     L.total = o;
     return L;
 }
@@ -1119,7 +1232,6 @@ kr_error enqueue_ranks_frames(const kr_bvh_node* nodes, const uint32_t* parents,
     uint32_t* first = reinterpret_cast<uint32_t*>(ws + L.first);
     float* tris = reinterpret_cast<float*>(ws + L.tris);
     Cand* cand = reinterpret_cast<Cand*>(ws + L.cand);
-    uint32_t* nunits = reinterpret_cast<uint32_t*>(ws + L.nunits);
     uint32_t* ustart = reinterpret_cast<uint32_t*>(ws + L.ustart);
     uint32_t* keys = reinterpret_cast<uint32_t*>(ws + L.keys);
     const unsigned gl = (n + kThreads - 1) / kThreads;
@@ -1137,12 +1249,14 @@ kr_error enqueue_ranks_frames(const kr_bvh_node* nodes, const uint32_t* parents,
     fb.first = first;
     fb.tris = tris;
     fb.cand = cand;
-    fb.nunits = nunits;
+    fb.plan = reinterpret_cast<uint32_t*>(ws + L.plan);
     fb.ustart = ustart;
     fb.keys = keys;
-    fb.scan = ws + L.scan;
     fb.err = &ctl->error;
-    fb.total_units = &ctl->total_units;
+    fb.groups = &ctl->groups;
+    fb.units = &ctl->units;
+    // the walk's counters are no longer needed (24 bytes per 32 leaves)
+    fb.boxes = reinterpret_cast<float*>(ws + L.visits);
     return enqueue_frames(fb, internal, obbs, xfs, s);
 }
 
@@ -1163,21 +1277,24 @@ size_t chain_bytes(uint32_t n) { return 2ull * kChain * 4 * most_tiles(n); }
 size_t chain_count_bytes(uint32_t n) { return 2ull * 4 * most_tiles(n); }
 
 namespace {
-ChainArgs chain_args(const FrameBuffers& b, uint32_t internal, FrameNodes which, uint32_t block_shift) {
+ChainArgs chain_args(const FrameBuffers& b, uint32_t internal, FrameNodes which, uint32_t block_shift, kr_obb3* obbs,
+                     kr_mat4* xfs) {
     const uint32_t n = internal + 1;
     const bool tiled = b.chains != nullptr;
     const uint32_t ntiles = tiles_of(n);
-    // the chain walks ride along with the first (or only) candidate launch
-    const bool walks = tiled && which != FrameNodes::kAcross;
+    // the chain walks, or the leaves' boxes, ride along with the first (or only) candidate launch
+    const uint32_t walkers = which == FrameNodes::kAcross ? 0u : tiled ? 2 * ntiles : n;
     return ChainArgs{tiled ? b.parents : nullptr, b.first, n,
-                     walks ? (2 * ntiles + kThreads - 1) / kThreads : 0u,
+                     static_cast<uint32_t>((static_cast<uint64_t>(walkers) + kThreads - 1) / kThreads),
                      b.chains, b.chain_counts, b.err, b.ustart, -0.0f,
-                     static_cast<uint32_t>(which), block_shift, tile_shift(n), b.across_list, b.across_count};
+                     static_cast<uint32_t>(which), block_shift, tile_shift(n), b.tris, b.boxes, obbs, xfs, b.plan, b.ustart, b.groups,
+                     b.units, b.across_list, b.across_count};
 }
 }  // namespace
 
-kr_error enqueue_candidates(const FrameBuffers& b, uint32_t internal, FrameNodes which, uint32_t block_shift,
-                            cudaStream_t s) {
+namespace {
+kr_error launch_candidates(const FrameBuffers& b, uint32_t internal, FrameNodes which, uint32_t block_shift,
+                           kr_obb3* obbs, kr_mat4* xfs, cudaStream_t s) {
     if (internal == 0) return kr_success;
     const bool tiled = b.chains != nullptr;
     if (tiled && !b.parents) return "enqueue_frames: tiled extents need the parents";
@@ -1185,24 +1302,30 @@ kr_error enqueue_candidates(const FrameBuffers& b, uint32_t internal, FrameNodes
         return "enqueue_candidates: node classes need the tiled path and a block shift below 32";
     if (which == FrameNodes::kAcross && (!b.across_list || !b.across_count))
         return "enqueue_candidates: the nodes across blocks come as a list";
-    const ChainArgs chain = chain_args(b, internal, which, block_shift);
+    const ChainArgs chain = chain_args(b, internal, which, block_shift, obbs, xfs);
     // kAcross loops over its list: two CTAs per SM
     const unsigned gi = which == FrameNodes::kAcross ? 2u * static_cast<unsigned>(device_info().sm_count)
                                                      : (internal + kThreads - 1) / kThreads;
-    // the chain walks go first, so that they overlap the candidate search
+    // the leading CTAs' work overlaps the candidate search
     ProfScope prof_scope_("candidate_kernel", s);
-    if (which == FrameNodes::kAcross)
-        candidate_kernel<true><<<gi + chain.walker_blocks, kThreads, 0, s>>>(
-            b.summary, b.points, b.counts, internal, static_cast<Cand*>(b.cand), b.nunits, b.keys, b.err, chain);
-    else
-        candidate_kernel<false><<<gi + chain.walker_blocks, kThreads, 0, s>>>(
-            b.summary, b.points, b.counts, internal, static_cast<Cand*>(b.cand), b.nunits, b.keys, b.err, chain);
+    const auto kernel = !tiled ? candidate_kernel<Nodes::kPlanned>
+                        : which == FrameNodes::kAcross ? candidate_kernel<Nodes::kListed>
+                                                       : candidate_kernel<Nodes::kTiled>;
+    kernel<<<gi + chain.walker_blocks, kThreads, 0, s>>>(b.summary, b.points, b.counts, internal,
+                                                         static_cast<Cand*>(b.cand), b.keys, b.err, chain);
     OBVH_TRY_CUDA(cudaGetLastError());
     return kr_success;
 }
+}  // namespace
+
+kr_error enqueue_candidates(const FrameBuffers& b, uint32_t internal, FrameNodes which, uint32_t block_shift,
+                            cudaStream_t s) {
+    if (internal > 0 && !b.chains) return "enqueue_candidates: the tiled path only";
+    return launch_candidates(b, internal, which, block_shift, nullptr, nullptr, s);
+}
 
 kr_error enqueue_frames(const FrameBuffers& b, uint32_t internal, kr_obb3* obbs, kr_mat4* xfs, cudaStream_t s) {
-    OBVH_TRY(enqueue_candidates(b, internal, FrameNodes::kAll, 0, s));
+    OBVH_TRY(launch_candidates(b, internal, FrameNodes::kAll, 0, obbs, xfs, s));
     return enqueue_extents(b, internal, obbs, xfs, s);
 }
 
@@ -1223,23 +1346,17 @@ kr_error enqueue_extents(const FrameBuffers& b, uint32_t internal, kr_obb3* obbs
         OBVH_TRY_CUDA(cudaGetLastError());
         return kr_success;
     }
-    {
-        ProfScope prof_scope_("extents_small_kernel", s);
-        extents_small_kernel<<<gi, kThreads, 0, s>>>(cand, b.counts, b.first, b.tris, internal, obbs, xfs, b.err,
-                                                     -0.0f);
-    }
-    OBVH_TRY_CUDA(cudaGetLastError());
-    OBVH_TRY(exclusive_scan_u32(b.nunits, b.ustart, internal, b.total_units, b.scan, s));
     const int grid = 4 * device_info().sm_count;
     {
         ProfScope prof_scope_("extents_units_kernel", s);
-        extents_units_kernel<<<grid, kThreads, 0, s>>>(cand, b.counts, b.first, b.tris, b.nunits, b.ustart, internal,
-                                                       b.err, b.total_units, b.keys, obbs, xfs, -0.0f);
+        extents_units_kernel<<<grid, kThreads, 0, s>>>(cand, b.counts, b.first, b.tris, b.plan, b.ustart, internal,
+                                                       b.err, b.groups, b.units, b.keys, b.boxes, -0.0f);
     }
     OBVH_TRY_CUDA(cudaGetLastError());
     {
         ProfScope prof_scope_("finalize_multi_kernel", s);
-        finalize_multi_kernel<<<gi, kThreads, 0, s>>>(cand, b.nunits, b.keys, internal, obbs, xfs, b.err);
+        finalize_multi_kernel<<<std::min(gi, 2u * static_cast<unsigned>(grid)), kThreads, 0, s>>>(
+            cand, b.plan, b.groups, b.units, b.keys, internal, obbs, xfs, b.err);
     }
     OBVH_TRY_CUDA(cudaGetLastError());
     return kr_success;

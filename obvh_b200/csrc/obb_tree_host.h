@@ -13,7 +13,7 @@ namespace obbtree {
 
 // Byte offsets inside a transform workspace for n primitives.
 struct Layout {
-    size_t ctl, visits, counts, summary, first, tris, rank_prims, cand, nunits, ustart, keys, scan, total;
+    size_t ctl, visits, counts, summary, first, tris, rank_prims, cand, plan, ustart, keys, total;
 };
 Layout layout(uint32_t n);
 
@@ -55,12 +55,15 @@ struct FrameBuffers {
     const uint32_t* first;
     const float* tris;         // 9 floats per leaf, depth-first
     void* cand;                // cand_bytes(internal)
-    uint32_t* nunits;          // internal entries each
-    uint32_t* ustart;          // (tiles: the nodes finished through the keys, total_units of them)
+    uint32_t* ustart;          // internal entries (tiles: parts that have arrived)
     uint32_t* keys;            // 6 per internal node
-    void* scan;                // scan_temp_bytes(internal)
     uint32_t* err;
-    uint32_t* total_units;
+    // Per-node path: 6 floats per 32 leaves, the plan of the nodes above a few
+    // leaves (internal entries) and its two counts, zero before the candidates.
+    float* boxes = nullptr;
+    uint32_t* plan = nullptr;
+    uint32_t* groups = nullptr;
+    unsigned long long* units = nullptr;
     // Tiled extents, for a Karras tree over sorted leaves (internal node a's
     // leaves are [first[a], first[a] + counts[a]) and no leaf has more than
     // 62 ancestors): null chains selects the per-node path.

@@ -45,7 +45,7 @@ static_assert((1 << kLocalShift) == kThreads, "CTA leaf blocks are aligned power
 
 struct Ctl {
     uint32_t error;
-    uint32_t total_units;
+    uint32_t spare0;
     uint32_t total_slots;
     uint32_t spare;
     uint32_t across;    // nodes the cross-CTA pass completed (listed at Layout::across)
@@ -710,7 +710,7 @@ __global__ void __launch_bounds__(kThreads) gather_kernel(const uint32_t* sizes,
 size_t align256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
 
 struct Layout {
-    size_t lbvh, ctl, first, tris, summary, flags, cand, nunits, ustart, keys, sizes, offsets, scan, frontier, chains,
+    size_t lbvh, ctl, first, tris, summary, flags, cand, ustart, keys, sizes, offsets, scan, frontier, chains,
         chain_counts, across, total;
 };
 
@@ -726,7 +726,6 @@ Layout layout(uint32_t n) {
     L.summary = o;  o += align256(112 * ni);
     L.flags = o;    o += align256(nn);
     L.cand = o;     o += align256(obbtree::cand_bytes(static_cast<uint32_t>(ni)));
-    L.nunits = o;   o += align256(4 * ni);
     L.ustart = o;   o += align256(4 * ni);
     L.keys = o;     o += align256(24 * ni);
     L.sizes = o;    o += align256(4 * nn);
@@ -805,12 +804,9 @@ kr_error enqueue(const kr_vec3* verts, const kr_uvec4* faces, uint32_t n, uint32
         fb.first = first;
         fb.tris = tris;
         fb.cand = ws + L.cand;
-        fb.nunits = reinterpret_cast<uint32_t*>(ws + L.nunits);
         fb.ustart = reinterpret_cast<uint32_t*>(ws + L.ustart);
         fb.keys = reinterpret_cast<uint32_t*>(ws + L.keys);
-        fb.scan = ws + L.scan;
         fb.err = &ctl->error;
-        fb.total_units = &ctl->total_units;
         fb.parents = parents;
         fb.chains = reinterpret_cast<uint32_t*>(ws + L.chains);
         fb.chain_counts = reinterpret_cast<uint32_t*>(ws + L.chain_counts);

@@ -7,6 +7,7 @@ import pytest
 from conftest import contained, same_bits, uncontained_leaves
 from oracle import bvh as ref
 from obvh_b200 import bvh, workloads
+from test_build_gpu import _shapes
 
 pytestmark = pytest.mark.gpu
 
@@ -155,6 +156,19 @@ def test_obb_tree_where_siblings_meet_in_a_warp_and_across(n, spread):
     tree = {"nodes": torch.from_numpy(nodes.view(np.uint8).copy()).cuda(),
             "parents": torch.from_numpy(parents.view(np.int32).copy()).cuda()}
     obbs, xfs = bvh.obb_tree(mesh, tree)
+    want_o, want_x, _ = ref.obb_tree(nodes, parents, v, f)
+    assert same_bits(obbs.cpu().numpy(), want_o)
+    assert same_bits(xfs.cpu().numpy(), want_x)
+
+
+@pytest.mark.parametrize("kind", ["sheet", "turned", "shell", "large"])
+@pytest.mark.parametrize("n", [8, 9, 32, 33, 511, 513, 5000])
+def test_obb_tree_extents_by_groups_units_and_blocks(builder, kind, n):
+    """Around the sizes of a thread's, a group's and a unit's nodes."""
+    v, f = _shapes(kind, n, n)
+    mesh, tree = _lbvh(builder, v, f)
+    obbs, xfs = bvh.obb_tree(mesh, tree)
+    nodes, parents = _tree_numpy(tree)
     want_o, want_x, _ = ref.obb_tree(nodes, parents, v, f)
     assert same_bits(obbs.cpu().numpy(), want_o)
     assert same_bits(xfs.cpu().numpy(), want_x)
