@@ -17,15 +17,16 @@
 //                vertices (:676-756) and the initial extents along them.
 //   extents      min/max of every subtree vertex on the node's axes, read
 //                from the contiguous run: the candidate's own thread for up
-//                to 8 leaves, 8 lanes for up to 32, one warp per 512-leaf unit
+//                to 12 leaves, 8 lanes for up to 32, one warp per 512-leaf unit
 //                above that (listed by the candidate kernel, dealt to the
 //                warps of a persistent grid); blocks of 32 leaves whose boxes
 //                lie within the node's extents so far are passed over; only
 //                nodes of more than one unit combine partial results, with 6
 //                integer atomics per unit.
 //                For a Karras tree (the fused build), tiles instead: one CTA
-//                per 1,024 (256) consecutive leaves stages their triangles in shared
-//                memory once and serves every node over them from there.
+//                per 1,024 (256) consecutive leaves stages their triangles in
+//                shared memory once and serves every larger node over them
+//                from there.
 //   finalize     the listed nodes' boxes (:903-964); others are finalised in
 //                place.
 #include <cuda_runtime.h>
@@ -54,6 +55,13 @@ constexpr uint32_t kCollapseLeafMax = 8;  // MAX_LEAF_SIZE (transforms.cu:65)
 // triangles 260 / 258 / 260 / 267 / 282, ATRBVH of 917,504 2,300 / 2,278 /
 // 2,270 / 2,280 / 2,299; four 1,024s in a row for a warp 281 and 2,311).
 constexpr uint32_t kUnit = 512;
+// A node of up to kOwnLeaves leaves is finished by the thread that finds its
+// candidate: its axes are at hand, and its 96-byte record is neither written
+// nor read again.  (us with the nodes of up to 8 done by the extents kernels /
+// with 5, 8, 12 and 16 here: builds of 200,003 triangles 257 / 255, 247, 245,
+// 245, of 500,003 438 / 438, 427, 421, -, of 2,000,000 1,446 / 1,483, 1,444,
+// 1,437, 1,441; transform of 229,824 - / 266, 264, 260, 262.)
+constexpr uint32_t kOwnLeaves = 12;
 // Tiled extents: 1,024 leaves per tile, or 256 for up to kSmallTiles leaves, so
 // that a small tree spreads over more SMs (us a build, 1,024 / 256: 1,021
 // triangles 111 / 99, 10,007 157 / 141, 57,344 211 / 195, 200,003 299 / 274,
@@ -653,7 +661,7 @@ struct ChainArgs {
     uint32_t tile_shift;      // the tiles 2^tile_shift
     // Without tiles: the leaves' triangles in depth-first order, the boxes of
     // each 32 of them (block_box), the outputs for the nodes of up to
-    // kSoloLeaves leaves (finished by their candidate's thread) and the plan
+    // kOwnLeaves leaves (finished by their candidate's thread) and the plan
     // of the others (plan_node).
     const float* tris;
     float* boxes;
@@ -725,7 +733,7 @@ __device__ void block_box(const float* tris, uint32_t n, uint32_t k, uint32_t la
 // ascend.  A warp adds once.
 __device__ __forceinline__ void plan_node(const ChainArgs& c, bool valid, uint32_t a, uint32_t cnt) {
     const uint32_t lane = threadIdx.x & 31, below = (1u << lane) - 1u, internal = c.n - 1;
-    const bool big = valid && cnt > kGroupLeaves, mid = valid && cnt > kSoloLeaves && !big;
+    const bool big = valid && cnt > kGroupLeaves, mid = valid && cnt > kOwnLeaves && !big;
     const uint32_t mids = __ballot_sync(0xffffffffu, mid), bigs = __ballot_sync(0xffffffffu, big);
     if (mids) {
         uint32_t base = 0;
@@ -768,7 +776,7 @@ __device__ __forceinline__ Cand cand_of(const Summary& s, const Candidate& c) {
 
 // The candidate of internal node a, stored for the extents kernels with the
 // initial keys of a node that several units or tiles share.  Without tiles a
-// node of up to kSoloLeaves leaves is finished here.
+// node of up to kOwnLeaves leaves is finished here.
 template <Nodes kNodes>
 __device__ __forceinline__ void candidate_node(uint32_t a, const uint4* summary, const kr_vec3* verts,
                                                const uint32_t* counts, Cand* cand, uint32_t* keys, const ChainArgs& chain) {
@@ -776,7 +784,7 @@ __device__ __forceinline__ void candidate_node(uint32_t a, const uint4* summary,
     const Candidate c = summary_candidate<Src::kL2, Src::kReadOnly>(summary, verts, a, chain.nz, s);
     const Cand out = cand_of(s, c);
     const uint32_t cnt = counts[a];  // (not held over the search)
-    if (kNodes == Nodes::kPlanned && cnt <= kSoloLeaves) {
+    if (cnt <= kOwnLeaves) {
         float lo[3] = {c.lo.x, c.lo.y, c.lo.z}, hi[3] = {c.hi.x, c.hi.y, c.hi.z};
         const float* t = chain.tris + 9 * static_cast<size_t>(__ldg(chain.first + a));
         const Axes ax = cand_axes(out, chain.nz);
@@ -844,10 +852,6 @@ __global__ void __launch_bounds__(kThreads, 2) candidate_kernel(const uint4* sum
     }
 }
 
-// Nodes of at most kGroupLeaves leaves: one thread each, finalised here.  (8
-// lanes for the nodes above kSoloLeaves, as in the tiles, was slower: 101 ->
-// 110 us on the 917K-triangle knot; here the triangles come from global memory
-// and the threads' loads in flight are what counts.)
 // The planned nodes (plan_node): eight lanes per node of up to kGroupLeaves
 // leaves, then units of kUnit leaves of the larger ones, a warp each, dealt
 // round-robin so that big and small nodes spread over the warps.  In a unit,
@@ -948,11 +952,10 @@ __global__ void __launch_bounds__(kThreads) extents_units_kernel(const Cand* can
 }
 
 // One tile of kTile consecutive leaves: their triangles are staged in shared
-// memory once, then every node over them is served from there (kSoloLeaves).
-// The nodes of one thread are finalised by it; larger ones are items: 8 lanes
-// or a warp each compute the extents, and the boxes are built afterwards, a
-// thread per item (building them in the warp's first lane, 16 of 32 lanes were
-// busy over the kernel).  Nodes crossing the tile's edges (the two chains) are
+// memory once, then every node of more than kOwnLeaves leaves over them is
+// served from there as an item: 8 lanes or a warp each compute the extents,
+// and the boxes are built afterwards, a thread per item (building them in the
+// warp's first lane, 16 of 32 lanes were busy over the kernel).  Nodes crossing the tile's edges (the two chains) are
 // warp items over their part in the tile, combined in the keys with integer
 // atomics.  Groups and warps take items from shared counters; an item beyond
 // the lists' capacity is done by the thread that found it.
@@ -962,8 +965,7 @@ __global__ void __launch_bounds__(kThreads) extents_units_kernel(const Cand* can
 // item tests the boxes of its blocks of 32 leaves, a lane each, and projects
 // those that could (may_extend; about 3.4 of 8 in a random mesh, fewer the
 // larger the node).  What bounds the kernel is issue and the latency of the
-// candidates' records, a third of it in the nodes of one thread.  2,000,000
-// triangles: 298 us with every block projected and each part fenced by its
+// candidates' records.  2,000,000 triangles, with the smallest nodes here too: 298 us with every block projected and each part fenced by its
 // warp, 283 with the test, 274 with the parts' atomics and fences a lane each
 // at the end (a build 1,482 -> 1,456 us).
 // A node over several tiles finishes in the last of them: each tile's part
@@ -1080,9 +1082,9 @@ __global__ void __launch_bounds__(kThreads) extents_tile_kernel(const Cand* cand
                                  : chains[i < qn + c0 ? static_cast<size_t>(w0) * kChain + (i - qn)
                                                       : static_cast<size_t>(w0 + 1) * kChain + (i - qn - c0)];
         const uint32_t f = __ldg(first + a), cnt = __ldg(counts + a);
-        if (!part && (f < t0 || f + cnt > t0 + tn)) continue;
+        if (cnt <= kOwnLeaves || (!part && (f < t0 || f + cnt > t0 + tn))) continue;
         const uint32_t b = max(f, t0) - t0, e = min(f + cnt, t0 + tn) - t0;
-        if ((!part && cnt <= kSoloLeaves) || !add_item(a, b, e, part)) alone(a, b, e, part);
+        if (!add_item(a, b, e, part)) alone(a, b, e, part);
     }
     __syncthreads();
     const uint32_t groups = min(ngroup, kTileGroups), warps = min(nwarp, kTileItems - kTileGroups);
@@ -1319,9 +1321,9 @@ kr_error launch_candidates(const FrameBuffers& b, uint32_t internal, FrameNodes 
 }  // namespace
 
 kr_error enqueue_candidates(const FrameBuffers& b, uint32_t internal, FrameNodes which, uint32_t block_shift,
-                            cudaStream_t s) {
+                            kr_obb3* obbs, kr_mat4* xfs, cudaStream_t s) {
     if (internal > 0 && !b.chains) return "enqueue_candidates: the tiled path only";
-    return launch_candidates(b, internal, which, block_shift, nullptr, nullptr, s);
+    return launch_candidates(b, internal, which, block_shift, obbs, xfs, s);
 }
 
 kr_error enqueue_frames(const FrameBuffers& b, uint32_t internal, kr_obb3* obbs, kr_mat4* xfs, cudaStream_t s) {

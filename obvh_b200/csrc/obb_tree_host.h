@@ -86,7 +86,7 @@ kr_error enqueue_frames(const FrameBuffers& b, uint32_t internal, kr_obb3* obbs,
 // the list b.across_list, e.g. written by the walk that completes them).
 enum class FrameNodes : uint32_t { kAll = 0, kInside = 1, kAcross = 2 };
 kr_error enqueue_candidates(const FrameBuffers& b, uint32_t internal, FrameNodes which, uint32_t block_shift,
-                            cudaStream_t s);
+                            kr_obb3* obbs, kr_mat4* xfs, cudaStream_t s);
 // The extents and final boxes, after the candidates of every node.
 kr_error enqueue_extents(const FrameBuffers& b, uint32_t internal, kr_obb3* obbs, kr_mat4* xfs, cudaStream_t s);
 

@@ -866,9 +866,10 @@ kr_error enqueue(const kr_vec3* verts, const kr_uvec4* faces, uint32_t n, uint32
             OBVH_TRY_CUDA(cudaGetLastError());
         }
         if (frames) {
-            OBVH_TRY(obbtree::enqueue_candidates(fb, internal, obbtree::FrameNodes::kAcross, kLocalShift, ws0));
+            OBVH_TRY(obbtree::enqueue_candidates(fb, internal, obbtree::FrameNodes::kAcross, kLocalShift, obbs, xfs,
+                                                 ws0));
             // a node is completed by fused_up_local iff its leaves lie inside one CTA's kThreads leaves
-            OBVH_TRY(obbtree::enqueue_candidates(fb, internal, obbtree::FrameNodes::kInside, kLocalShift, s));
+            OBVH_TRY(obbtree::enqueue_candidates(fb, internal, obbtree::FrameNodes::kInside, kLocalShift, obbs, xfs, s));
         }
         OBVH_TRY(join_from(*fk, 0, s));
     }
