@@ -131,12 +131,11 @@ __device__ __forceinline__ bool may_extend(const float lo[3], const float hi[3],
     return !inside;
 }
 
-// Extents over a node's leaf run go by size: a thread alone for the smallest
-// (up to kSoloLeaves leaves in a batch's CTA), 8 lanes for up to kGroupLeaves,
-// a warp above.  A Karras tree's nodes are mostly tiny (half have 2 or 3
+// Extents over a node's leaf run go by size: the thread of its candidate for
+// the smallest (kOwnLeaves), 8 lanes for up to kGroupLeaves leaves, a warp
+// above.  A Karras tree's nodes are mostly tiny (half have 2 or 3
 // leaves), and one thread per node up to 32 leaves kept its warp in the loop
 // for 32 rounds, 16 of 32 lanes busy on average over the kernel.
-constexpr uint32_t kSoloLeaves = 8;
 constexpr uint32_t kGroupLeaves = 32;
 
 __device__ __forceinline__ Axes cand_axes(const Cand& c, float nz) {

@@ -137,3 +137,9 @@ def test_narrow_and_wide_ctas(count, sizes):
     """592 meshes in equal halves fill two CTAs to an SM twice over (256 threads
     each); fewer go to one CTA of 512 threads to an SM."""
     _check(_meshes([sizes[k % len(sizes)] for k in range(count)], seed=4000))
+
+
+@pytest.mark.parametrize("sizes", [[12, 13, 20, 21], [19, 22, 32, 33], [64, 100]])
+def test_nodes_finished_by_their_candidates_thread(sizes):
+    """Around the sizes that a candidate's thread, 8 lanes and a warp take."""
+    _check(_meshes(sizes, seed=sum(sizes)))
