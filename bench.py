@@ -278,14 +278,16 @@ def tree_bytes_per_launch(n):
         # faces + vertices in, leaf boxes + transforms out, summaries out and read once
         "summary_up_kernel": 52 * n + 124 * n + 112 * ni * 2 + 4 * ni,
         "dfs_rank_kernel": 52 * n + 36 * n + 4 * ni,   # faces + vertices in; ordered triangles + firsts out
-        "candidate_kernel": 112 * ni + 168 * ni + 96 * ni + 8 * ni,  # summary + 14 vertices in; frame out
-        "extents_small_kernel": 96 * ni + 124 * ni,    # frame in; box + transform out
+        # summary + 14 vertices + count in; a box + transform (most nodes, finished here) or a larger node's frame
+        # out: the smaller of the two
+        "candidate_kernel": 112 * ni + 168 * ni + 96 * ni + 8 * ni,
         "extents_units_kernel": 36 * n,                # ordered triangles in
-        # tiles: ordered triangles, frames, first leaves and counts in; boxes + transforms (or extent keys) out
-        "extents_tile_kernel": 36 * n + 104 * ni + 124 * ni,
+        # tiles: ordered triangles, first leaves and counts in (and the few larger nodes' frames and boxes)
+        "extents_tile_kernel": 36 * n + 8 * ni,
         "mark_up_kernel": 36 * nn + 16 * nn + 36 * n,
-        # fused build: order, face, vertices in; leaf node (x2), ordered triangle, leaf box + transform out
-        "leaves_fused_kernel": 4 * n + 52 * n + 72 * n + 36 * n + 124 * n,
+        # fused build: order, face, vertices in; leaf node (x2), ordered triangle, leaf box + transform out; beside
+        # them the Karras tree: codes in; internal nodes, parents, first leaves, spans out
+        "leaves_fused_kernel": 4 * n + 52 * n + 72 * n + 36 * n + 124 * n + 4 * n + 36 * ni + 16 * ni,
         # fused leaf-to-root pass over the CTA-local nodes: triangles in (the leaf bounds are recomputed from
         # them), leaf costs + counts out; children, first leaf, count in; bounds, collapsed node, cost, summary
         # out; collapse marks
@@ -1125,6 +1127,9 @@ def bench_dito_ours(a, dist):
     }
     if dist.rank == 0 and dist.world == 1:
         import oracle
+        if not oracle.ref_available():
+            line["cpu_baseline"] = {"unavailable": "oracle/_ref/libref_dito.so was not built"}
+            return line
         oracle.ref_dito14(host_np[:1000])
         t0 = time.perf_counter()
         for _ in range(3):
@@ -1266,6 +1271,9 @@ def bench_batch_ours(a, dist):
     }
     if dist.rank == 0 and dist.world == 1:
         import oracle
+        if not oracle.ref_available():
+            line["cpu_baseline"] = {"unavailable": "oracle/_ref/libref_dito.so was not built"}
+            return line
         threads = os.cpu_count() or 1
         off = np.asarray(offsets, np.int64)
         oracle.ref_dito14_batch(host_np, off[:65], threads)
