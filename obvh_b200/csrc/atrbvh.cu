@@ -11,6 +11,7 @@
 //                    split search (LBVH.cu:156-300)
 //   boxes_up_kernel  leaf boxes and bottom-up node boxes and areas
 //                    (LBVH.cu:414-447,551-648)
+//   treelet_starts_kernel  the nodes where a pass begins
 //   treelet_kernel   one bottom-up pass per iteration (gamma = tau, 2 tau,
 //                    ...): at every node whose subtree holds at least gamma
 //                    triangles, the warp forms a treelet of tau leaves by

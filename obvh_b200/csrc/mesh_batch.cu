@@ -15,9 +15,9 @@
 //   5 Karras tree, first leaves and leaf counts
 //   6 bottom-up pass from every leaf (bounds, costs, collapse marks,
 //     7-direction summaries)
-//   7 candidate frames of the internal nodes
-//   8 extents over each node's leaf run (a thread, 8 lanes or a warp by its
-//     size) and the final boxes
+//   7 candidate frames of the internal nodes, and the smaller nodes' boxes
+//   8 extents over each larger node's leaf run (8 lanes or a warp by its size)
+//     and its box
 //   9 collapse: roots, block scan of their sizes, primitive lists
 // Every per-element formula is the chain's own device code (lbvh_device.cuh,
 // up_device.cuh, tree_device.cuh, obb_device.cuh); results are the chain's

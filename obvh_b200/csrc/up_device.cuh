@@ -76,7 +76,7 @@ struct UpArgs {
     uint4* summary;  // null: no summaries
     uint32_t* visits;
     uint32_t* err;
-    // null, or the nodes walk_up completes are appended here (done_count of
+    // null, or the nodes the walk completes are appended here (done_count of
     // them; at most the internal nodes)
     uint32_t* done_list = nullptr;
     uint32_t* done_count = nullptr;
