@@ -233,7 +233,8 @@ __device__ __forceinline__ void visit_node(const Boxes& boxes, const kr_ivec4* _
     bool tr = r0 <= r1 && r1 > 0.0f && r0 <= st.hit_t;
     const bool sure_l = sl && apart(l0, l1) && apart(l0, st.hit_t);
     const bool sure_r = sr && apart(r0, r1) && apart(r0, st.hit_t);
-    const bool close = (tl || !sure_l) && (tr || !sure_r) && !apart(l0, r0);
+    // which child is nearer: decided only where both distances have the bound
+    const bool close = (tl || !sure_l) && (tr || !sure_r) && !(sl && sr && apart(l0, r0));
     bool exact_l = !sure_l || close, exact_r = !sure_r || close;
     while (exact_l || exact_r) {
         const float2 e = unit_slabs(exact_l ? l : r);

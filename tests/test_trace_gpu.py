@@ -104,6 +104,37 @@ def test_edges_of_warps_leaves_and_slab_ranges(count, ci):
     assert _isects(got, count).tobytes() == want.tobytes()
 
 
+@pytest.mark.parametrize("mirrored", [False, True])
+def test_nearer_child_where_one_reciprocal_is_out_of_range(mirrored):
+    """Two boxes entered at the same distance a / b (the left child first), one
+    of them in a frame scaled by 2^120, where 1 / direction leaves the range in
+    which the approximate slabs hold: the other's approximate a * (1 / b) must
+    not decide the order against its exact distance.  Both leaves hold the same
+    triangle, so the primitive hit says which was visited first."""
+    import torch
+    n = 4096
+    rng = np.random.default_rng(11)
+    v = np.array([[0, -10, -10], [0, 10, -10], [0, 0, 20]], np.float32)
+    f = np.array([[0, 1, 2, 0], [0, 1, 2, 0]], np.uint32)
+    near = np.array([[1, 0, 0, 0, 1, 0, 0, 0, 1, -0.5, 0, 0]], np.float32)
+    scaled = np.array([[2.0 ** 120, 0, 0, 0, 1, 0, 0, 0, 1, 0, 0, 0]], np.float32)
+    lt, rt = (near, scaled) if mirrored else (scaled, near)
+    meta = np.array([[~1, ~2, 0, 0], [0, 1, 0, 0], [1, 2, 0, 0]], np.int32)
+    rays = np.zeros(n, workloads.RAY)
+    rays["origin"][:, 0] = -rng.integers(1 << 19, 1 << 22, n) / 2.0 ** 22
+    rays["direction"] = 2.0 ** -10
+    rays["direction"][:, 0] = rng.uniform(64, 128, n)
+    rays["tmax"] = 1e30
+    soa = {"left_T": torch.from_numpy(lt).cuda(), "right_T": torch.from_numpy(rt).cuda(),
+           "metadata": torch.from_numpy(meta).cuda()}
+    got, err = bvh.soa_obvh_intersect(soa, bvh.Mesh(v, f), None, _dev_rays(rays), 3, 1)
+    torch.cuda.synchronize()
+    want = ref.soa_obvh_intersect(lt, rt, meta, v, f, None, rays, threads=4)
+    assert int(err.item()) == 0
+    assert (want["primitive"] == 0).all()
+    assert _isects(got, n).tobytes() == want.tobytes()
+
+
 def test_reference_entry_point_through_the_device_struct():
     """kr_cuda_obvh_persistent -> kr_cuda_soa_obvh -> kr_cuda_soa_obvh_intersect,
     the reference's own call sequence, against the stream form."""
