@@ -43,6 +43,7 @@
 #include "runtime.h"
 #include "sort.h"
 #include "tree_device.cuh"
+#include "unit_plan.h"
 
 namespace obvh {
 namespace obbtree {
@@ -51,10 +52,6 @@ using namespace tree;
 
 constexpr int kThreads = 256;
 constexpr uint32_t kCollapseLeafMax = 8;  // MAX_LEAF_SIZE (transforms.cu:65)
-// Leaves per warp unit (us, 128 / 256 / 512 / 1,024 / 2,048: transform of 229,824
-// triangles 260 / 258 / 260 / 267 / 282, ATRBVH of 917,504 2,300 / 2,278 /
-// 2,270 / 2,280 / 2,299; four 1,024s in a row for a warp 281 and 2,311).
-constexpr uint32_t kUnit = 512;
 // A node of up to kOwnLeaves leaves is finished by the thread that finds its
 // candidate: its axes are at hand, and its 96-byte record is neither written
 // nor read again.  (us with the nodes of up to 8 done by the extents kernels /
@@ -668,7 +665,8 @@ struct ChainArgs {
     kr_obb3* obbs;
     kr_mat4* xfs;
     uint32_t* plan;
-    uint32_t* plan_start;
+    unsigned long long* plan_start;
+    UnitPlan units_of;
     uint32_t* groups;
     unsigned long long* units;
     const uint32_t* list;     // kAcross: the nodes, list_count of them
@@ -727,10 +725,10 @@ __device__ void block_box(const float* tris, uint32_t n, uint32_t k, uint32_t la
 
 // Lists node a for extents_units_kernel (every lane of a warp calls it): nodes
 // of up to kGroupLeaves leaves from the back of chain.plan, groups of them in
-// all; larger ones from the front, with the number of the first of their units
-// of kUnit leaves.  *units holds the nodes listed in front in its high word and
-// their units in the low one, so that both grow by one addition and the starts
-// ascend.  A warp adds once.
+// all; larger ones from the front, with the number of the first of their
+// units.  *units holds their units in its low bits and the nodes listed in
+// front above them (unit_plan), so that both grow by one addition and the
+// starts ascend.  A warp adds once.
 __device__ __forceinline__ void plan_node(const ChainArgs& c, bool valid, uint32_t a, uint32_t cnt) {
     const uint32_t lane = threadIdx.x & 31, below = (1u << lane) - 1u, internal = c.n - 1;
     const bool big = valid && cnt > kGroupLeaves, mid = valid && cnt > kOwnLeaves && !big;
@@ -742,21 +740,22 @@ __device__ __forceinline__ void plan_node(const ChainArgs& c, bool valid, uint32
         if (mid) c.plan[internal - 1 - (base + __popc(mids & below))] = a;
     }
     if (bigs) {
-        const uint32_t own = big ? (cnt + kUnit - 1) / kUnit : 0u;
-        uint32_t incl = own;
+        const uint32_t own = big ? ((cnt - 1) >> c.units_of.unit_shift) + 1 : 0u;
+        uint64_t incl = own;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
+            const uint64_t v = __shfl_up_sync(0xffffffffu, incl, d);
             if (static_cast<int>(lane) >= d) incl += v;
         }
-        const uint32_t sum = __shfl_sync(0xffffffffu, incl, 31);
+        const uint64_t sum = __shfl_sync(0xffffffffu, incl, 31);
         unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(c.units, (static_cast<unsigned long long>(__popc(bigs)) << 32) + sum);
+        if (lane == 0)
+            base = atomicAdd(c.units, (static_cast<unsigned long long>(__popc(bigs)) << c.units_of.unit_bits) + sum);
         base = __shfl_sync(0xffffffffu, base, 0);
-        const uint32_t at = static_cast<uint32_t>(base >> 32) + __popc(bigs & below);
+        const uint32_t at = static_cast<uint32_t>(base >> c.units_of.unit_bits) + __popc(bigs & below);
         if (big && at < internal) {
             c.plan[at] = a;
-            c.plan_start[at] = static_cast<uint32_t>(base) + incl - own;
+            c.plan_start[at] = (base & ((1ull << c.units_of.unit_bits) - 1)) + incl - own;
         }
     }
 }
@@ -802,7 +801,7 @@ __device__ __forceinline__ void candidate_node(uint32_t a, const uint4* summary,
         shared = (f >> chain.tile_shift) != ((f + cnt - 1) >> chain.tile_shift);
         if (shared) chain.arrivals[a] = 0u;  // counted up by extents_tile_kernel
     } else {
-        shared = cnt > kUnit;
+        shared = cnt > (1u << chain.units_of.unit_shift);
     }
     if (shared) {
         uint32_t* k = keys + 6 * static_cast<size_t>(a);
@@ -860,7 +859,7 @@ __global__ void __launch_bounds__(kCandThreads, kCandCtas) candidate_kernel(cons
 }
 
 // The planned nodes (plan_node): eight lanes per node of up to kGroupLeaves
-// leaves, then units of kUnit leaves of the larger ones, a warp each, dealt
+// leaves, then the units (unit_plan) of the larger ones, a warp each, dealt
 // round-robin so that big and small nodes spread over the warps.  In a unit,
 // only the blocks of 32 leaves that could extend the node are projected
 // (may_extend).  All extents go to the keys; finalize_multi_kernel builds the
@@ -873,7 +872,8 @@ __global__ void __launch_bounds__(kCandThreads, kCandCtas) candidate_kernel(cons
 // triangles 314 -> 260 us, the 917,504-triangle ATRBVH 2,353 -> 2,270 us.)
 __global__ void __launch_bounds__(kThreads) extents_units_kernel(const Cand* cand, const uint32_t* counts,
                                                                  const uint32_t* first, const float* tris,
-                                                                 const uint32_t* plan, const uint32_t* plan_start,
+                                                                 const uint32_t* plan,
+                                                                 const unsigned long long* plan_start, UnitPlan units_of,
                                                                  uint32_t internal, const uint32_t* err,
                                                                  const uint32_t* group_count,
                                                                  const unsigned long long* unit_count, uint32_t* keys,
@@ -899,8 +899,8 @@ __global__ void __launch_bounds__(kThreads) extents_units_kernel(const Cand* can
             keys[6 * static_cast<size_t>(a) + sub] = f2key(v);
         }
     }
-    const uint32_t listed = min(static_cast<uint32_t>(*unit_count >> 32), internal);
-    const uint32_t total = static_cast<uint32_t>(*unit_count);
+    const uint32_t listed = static_cast<uint32_t>(min(*unit_count >> units_of.unit_bits, static_cast<unsigned long long>(internal)));
+    const uint64_t total = *unit_count & ((1ull << units_of.unit_bits) - 1);
     for (uint64_t u = w; u < total; u += warps) {
         uint32_t at = 0, end_at = listed;  // the last node whose first unit is <= u owns it
         while (end_at - at > 1) {
@@ -912,10 +912,9 @@ __global__ void __launch_bounds__(kThreads) extents_units_kernel(const Cand* can
         const uint32_t a = __ldg(plan + at);
         const uint32_t cnt = __ldg(counts + a), f = __ldg(first + a);
         const Cand c = load_cand(cand, a);
-        const uint32_t begin = (static_cast<uint32_t>(u) - __ldg(plan_start + at)) * kUnit;
-        if (begin >= cnt) continue;  // more than 2^32 units: the starts wrapped
+        const uint32_t begin = static_cast<uint32_t>(u - __ldg(plan_start + at)) << units_of.unit_shift;
         // leaves [b, e); of the blocks of 32 those that could extend the node
-        const uint32_t b = f + begin, e = f + min(cnt, begin + kUnit);
+        const uint32_t b = f + begin, e = f + min(cnt, begin + (1u << units_of.unit_shift));
         const Axes ax = cand_axes(c, nz);
         float lo[3] = {kInf, kInf, kInf}, hi[3] = {-kInf, -kInf, -kInf};
         for (uint32_t k0 = b / 32; 32 * k0 < e; k0 += 32) {
@@ -945,7 +944,7 @@ __global__ void __launch_bounds__(kThreads) extents_units_kernel(const Cand* can
             uint32_t* k = keys + 6 * static_cast<size_t>(a) + lane;
             const float v = lane == 0 ? lo[0] : lane == 1 ? lo[1] : lane == 2 ? lo[2] : lane == 3 ? hi[0]
                           : lane == 4 ? hi[1] : hi[2];
-            if (cnt <= kUnit) {  // the whole node in this unit
+            if (cnt <= (1u << units_of.unit_shift)) {  // the whole node in this unit
                 const float o = lane == 0 ? c.olo[0] : lane == 1 ? c.olo[1] : lane == 2 ? c.olo[2]
                               : lane == 3 ? c.ohi[0] : lane == 4 ? c.ohi[1] : c.ohi[2];
                 *k = f2key(lane < 3 ? fminf(o, v) : fmaxf(o, v));
@@ -1172,11 +1171,11 @@ __global__ void __launch_bounds__(kThreads) extents_tile_kernel(const Cand* cand
 // written by it; several: the atomic min/max over the units).
 __global__ void __launch_bounds__(kThreads) finalize_multi_kernel(const Cand* cand, const uint32_t* plan,
                                                                   const uint32_t* group_count,
-                                                                  const unsigned long long* unit_count,
+                                                                  const unsigned long long* unit_count, uint32_t unit_bits,
                                                                   const uint32_t* keys, uint32_t internal,
                                                                   kr_obb3* obbs, kr_mat4* xfs, const uint32_t* err) {
     if (*err) return;
-    const uint32_t listed = min(static_cast<uint32_t>(*unit_count >> 32), internal);
+    const uint32_t listed = static_cast<uint32_t>(min(*unit_count >> unit_bits, static_cast<unsigned long long>(internal)));
     const uint32_t all = min(listed + min(*group_count, internal), internal);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < all; i += gridDim.x * blockDim.x)
         finalize_keys(cand, keys, i < listed ? plan[i] : plan[internal - 1 - (i - listed)], obbs, xfs);
@@ -1199,7 +1198,7 @@ Layout layout(uint32_t n) {
     L.rank_prims = o; o += align256(4ull * (n > 0 ? n : 1));
     L.cand = o;     o += align256(sizeof(Cand) * ni);
     L.plan = o;     o += align256(4 * ni);
-    L.ustart = o;   o += align256(4 * ni);
+    L.plan_start = o; o += align256(8 * ni);
     L.keys = o;     o += align256(24 * ni);
     L.total = o;
     return L;
@@ -1241,7 +1240,6 @@ kr_error enqueue_ranks_frames(const kr_bvh_node* nodes, const uint32_t* parents,
     uint32_t* first = reinterpret_cast<uint32_t*>(ws + L.first);
     float* tris = reinterpret_cast<float*>(ws + L.tris);
     Cand* cand = reinterpret_cast<Cand*>(ws + L.cand);
-    uint32_t* ustart = reinterpret_cast<uint32_t*>(ws + L.ustart);
     uint32_t* keys = reinterpret_cast<uint32_t*>(ws + L.keys);
     const unsigned gl = (n + kThreads - 1) / kThreads;
     {
@@ -1259,7 +1257,7 @@ kr_error enqueue_ranks_frames(const kr_bvh_node* nodes, const uint32_t* parents,
     fb.tris = tris;
     fb.cand = cand;
     fb.plan = reinterpret_cast<uint32_t*>(ws + L.plan);
-    fb.ustart = ustart;
+    fb.plan_start = reinterpret_cast<unsigned long long*>(ws + L.plan_start);
     fb.keys = keys;
     fb.err = &ctl->error;
     fb.groups = &ctl->groups;
@@ -1295,8 +1293,9 @@ ChainArgs chain_args(const FrameBuffers& b, uint32_t internal, FrameNodes which,
     const uint32_t walkers = which == FrameNodes::kAcross ? 0u : tiled ? 2 * ntiles : n;
     return ChainArgs{tiled ? b.parents : nullptr, b.first, n,
                      static_cast<uint32_t>((static_cast<uint64_t>(walkers) + kCandThreads - 1) / kCandThreads),
-                     b.chains, b.chain_counts, b.err, b.ustart, -0.0f,
-                     static_cast<uint32_t>(which), block_shift, tile_shift(n), b.tris, b.boxes, obbs, xfs, b.plan, b.ustart, b.groups,
+                     b.chains, b.chain_counts, b.err, b.arrivals, -0.0f,
+                     static_cast<uint32_t>(which), block_shift, tile_shift(n), b.tris, b.boxes, obbs, xfs, b.plan, b.plan_start,
+                     unit_plan(n), b.groups,
                      b.units, b.across_list, b.across_count};
 }
 }  // namespace
@@ -1350,7 +1349,7 @@ kr_error enqueue_extents(const FrameBuffers& b, uint32_t internal, kr_obb3* obbs
             const auto kernel = tile_shift(n) == kTileShiftSmall ? extents_tile_kernel<kTileShiftSmall>
                                                                  : extents_tile_kernel<kTileShiftLarge>;
             kernel<<<tiles_of(n), kThreads, 0, s>>>(cand, b.counts, b.first, b.tris, n, b.chains, b.chain_counts,
-                                                    b.keys, b.ustart, obbs, xfs, b.err, -0.0f);
+                                                    b.keys, b.arrivals, obbs, xfs, b.err, -0.0f);
         }
         OBVH_TRY_CUDA(cudaGetLastError());
         return kr_success;
@@ -1358,14 +1357,15 @@ kr_error enqueue_extents(const FrameBuffers& b, uint32_t internal, kr_obb3* obbs
     const int grid = 4 * device_info().sm_count;
     {
         ProfScope prof_scope_("extents_units_kernel", s);
-        extents_units_kernel<<<grid, kThreads, 0, s>>>(cand, b.counts, b.first, b.tris, b.plan, b.ustart, internal,
-                                                       b.err, b.groups, b.units, b.keys, b.boxes, -0.0f);
+        extents_units_kernel<<<grid, kThreads, 0, s>>>(cand, b.counts, b.first, b.tris, b.plan, b.plan_start,
+                                                       unit_plan(n), internal, b.err, b.groups, b.units, b.keys,
+                                                       b.boxes, -0.0f);
     }
     OBVH_TRY_CUDA(cudaGetLastError());
     {
         ProfScope prof_scope_("finalize_multi_kernel", s);
         finalize_multi_kernel<<<std::min(gi, 2u * static_cast<unsigned>(grid)), kThreads, 0, s>>>(
-            cand, b.plan, b.groups, b.units, b.keys, internal, obbs, xfs, b.err);
+            cand, b.plan, b.groups, b.units, unit_plan(n).unit_bits, b.keys, internal, obbs, xfs, b.err);
     }
     OBVH_TRY_CUDA(cudaGetLastError());
     return kr_success;

@@ -13,7 +13,7 @@ namespace obbtree {
 
 // Byte offsets inside a transform workspace for n primitives.
 struct Layout {
-    size_t ctl, visits, counts, summary, first, tris, rank_prims, cand, plan, ustart, keys, total;
+    size_t ctl, visits, counts, summary, first, tris, rank_prims, cand, plan, plan_start, keys, total;
 };
 Layout layout(uint32_t n);
 
@@ -55,13 +55,14 @@ struct FrameBuffers {
     const uint32_t* first;
     const float* tris;         // 9 floats per leaf, depth-first
     void* cand;                // cand_bytes(internal)
-    uint32_t* ustart;          // internal entries (tiles: parts that have arrived)
     uint32_t* keys;            // 6 per internal node
     uint32_t* err;
     // Per-node path: 6 floats per 32 leaves, the plan of the nodes above a few
-    // leaves (internal entries) and its two counts, zero before the candidates.
+    // leaves and the first units of the larger ones (internal entries each) and
+    // its two counts, zero before the candidates.
     float* boxes = nullptr;
     uint32_t* plan = nullptr;
+    unsigned long long* plan_start = nullptr;
     uint32_t* groups = nullptr;
     unsigned long long* units = nullptr;
     // Tiled extents, for a Karras tree over sorted leaves (internal node a's
@@ -70,6 +71,7 @@ struct FrameBuffers {
     const uint32_t* parents = nullptr;
     uint32_t* chains = nullptr;        // chain_bytes(n)
     uint32_t* chain_counts = nullptr;  // chain_count_bytes(n)
+    uint32_t* arrivals = nullptr;      // internal entries: parts that have arrived
     // FrameNodes::kAcross: those nodes, as a list of across_count entries
     const uint32_t* across_list = nullptr;
     const uint32_t* across_count = nullptr;

@@ -710,7 +710,7 @@ __global__ void __launch_bounds__(kThreads) gather_kernel(const uint32_t* sizes,
 size_t align256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
 
 struct Layout {
-    size_t lbvh, ctl, first, tris, summary, flags, cand, ustart, keys, sizes, offsets, scan, frontier, chains,
+    size_t lbvh, ctl, first, tris, summary, flags, cand, arrivals, keys, sizes, offsets, scan, frontier, chains,
         chain_counts, across, total;
 };
 
@@ -726,7 +726,7 @@ Layout layout(uint32_t n) {
     L.summary = o;  o += align256(112 * ni);
     L.flags = o;    o += align256(nn);
     L.cand = o;     o += align256(obbtree::cand_bytes(static_cast<uint32_t>(ni)));
-    L.ustart = o;   o += align256(4 * ni);
+    L.arrivals = o; o += align256(4 * ni);
     L.keys = o;     o += align256(24 * ni);
     L.sizes = o;    o += align256(4 * nn);
     L.offsets = o;  o += align256(4 * nn);
@@ -804,7 +804,7 @@ kr_error enqueue(const kr_vec3* verts, const kr_uvec4* faces, uint32_t n, uint32
         fb.first = first;
         fb.tris = tris;
         fb.cand = ws + L.cand;
-        fb.ustart = reinterpret_cast<uint32_t*>(ws + L.ustart);
+        fb.arrivals = reinterpret_cast<uint32_t*>(ws + L.arrivals);
         fb.keys = reinterpret_cast<uint32_t*>(ws + L.keys);
         fb.err = &ctl->error;
         fb.parents = parents;
