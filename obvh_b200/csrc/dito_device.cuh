@@ -325,6 +325,15 @@ inline __device__ void candidate_warp(uint64_t n, float val, f3 sel, const float
         return;
     }
 
+    // The axis extremes as their own points have them: of zeros of both signs a
+    // reduction may have returned either, depending on how the points were
+    // split over warps and CTAs (the scan from the first point keeps its own).
+    {
+        const int k = lane < 7 ? lane : lane - 7;
+        const float own = k == 0 ? sel.x : (k == 1 ? sel.y : sel.z);
+        if (lane < 14 && k < 3 && own == val) val = own;
+    }
+
     // AABB from slabs 0..2 (dito.cpp:507-510)
     const f3 lo3 = mk3(__shfl_sync(kAll, val, 0), __shfl_sync(kAll, val, 1), __shfl_sync(kAll, val, 2));
     const f3 hi3 = mk3(__shfl_sync(kAll, val, 7), __shfl_sync(kAll, val, 8), __shfl_sync(kAll, val, 9));

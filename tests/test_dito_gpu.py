@@ -82,7 +82,7 @@ def test_one_launch_fit_at_its_limits(torch, fitter, n, kind):
     first; the two-launch form (by passes) gives the same box and report."""
     rng = np.random.default_rng(n)
     if kind == "lattice":
-        pts = rng.integers(-3, 4, size=(n, 3)).astype(np.float32)
+        pts = rng.integers(-2, 3, size=(n, 3)).astype(np.float32)
     else:
         pts = (rng.normal(size=(n, 3)) * rng.uniform(0.1, 10, size=3) + rng.uniform(-9, 9, size=3)).astype(np.float32)
     if kind == "nan" and n > 14:
@@ -146,3 +146,32 @@ def test_empty_and_tiny_inputs(torch, fitter):
         pts = np.arange(3 * n, dtype=np.float32).reshape(n, 3) ** 1.5
         want, _, _ = oracle.dito14(pts)
         assert same_bits(_device_fit(torch, fitter, pts), want), n
+
+
+@pytest.mark.parametrize("n", [15, 40, 300, 5000, 40_000, 300_000])
+def test_zero_signs_of_an_axis_aligned_box(torch, fitter, n):
+    """Points of a flat lattice hexagon with zeros of both signs: where the axis-aligned box
+    wins, its centre has the zeros that a scan from the first point keeps,
+    whichever way the fit is made (one launch, two launches, batched)."""
+    from obvh_b200.batch import DitoBatch
+    checked = 0
+    for seed in range(24):
+        rng = np.random.default_rng(1000 * seed + n)
+        pts = np.zeros((n, 3), np.float32)
+        pts[:, 0], pts[:, 1] = rng.integers(-8, 9, n), rng.integers(-4, 5, n)
+        pts[np.abs(pts[:, 0]) / 8 + np.abs(pts[:, 1]) / 4 > 1.3, 0] = 0.0
+        pts[pts == 0] *= np.where(rng.random(int((pts == 0).sum())) < 0.5, 1, -1)
+        want, _, _ = oracle.dito14(pts)
+        if not np.array_equal(want[3:12], np.eye(3, dtype=np.float32).reshape(-1)):
+            continue
+        checked += 1
+        dev = torch.from_numpy(pts).cuda()
+        two = torch.empty(15, device="cuda")
+        fitter.fit_pass(dev, two, 1)
+        fitter.fit_pass(dev, two, 2)
+        batched = torch.empty((1, 15), device="cuda")
+        DitoBatch(np.array([0, n])).run(dev, batched)
+        for box in (fitter.fit(dev), two, batched[0]):
+            got = box.cpu().numpy()
+            assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), (seed, got[:3], want[:3])
+    assert checked > 0
