@@ -25,6 +25,7 @@
 // with its miss record and sets the error word.
 #include <cuda_runtime.h>
 
+#include <cfloat>
 #include <cstdint>
 #include <mutex>
 
@@ -231,10 +232,14 @@ __device__ __forceinline__ void visit_node(const Boxes& boxes, const kr_ivec4* _
     const bool sl = near_slabs(l, l0, l1), sr = near_slabs(r, r0, r1);
     bool tl = l0 <= l1 && l1 > 0.0f && l0 <= st.hit_t;
     bool tr = r0 <= r1 && r1 > 0.0f && r0 <= st.hit_t;
-    const bool sure_l = sl && apart(l0, l1) && apart(l0, st.hit_t);
-    const bool sure_r = sr && apart(r0, r1) && apart(r0, st.hit_t);
+    // Of an infinite limit (a ray's that has none) apart() decides nothing, so
+    // FLT_MAX stands in: it compares with a finite distance alike, and
+    // apart(l0, l1) lets no other pass.
+    const float limit = fminf(st.hit_t, FLT_MAX);
+    const bool sure_l = sl && apart(l0, l1) && apart(l0, limit);
+    const bool sure_r = sr && apart(r0, r1) && apart(r0, limit);
     // which child is nearer: decided only where both distances have the bound
-    const bool close = (tl || !sure_l) && (tr || !sure_r) && !(sl && sr && apart(l0, r0));
+    const bool close = (tl || !sure_l) && (tr || !sure_r) && (sl != sr || !apart(l0, r0));
     bool exact_l = !sure_l || close, exact_r = !sure_r || close;
     while (exact_l || exact_r) {
         const float2 e = unit_slabs(exact_l ? l : r);
