@@ -44,6 +44,7 @@
 #include "runtime.h"
 #include "tree_device.cuh"
 #include "up_device.cuh"
+#include "walk_limit.h"
 
 namespace obvh {
 namespace meshbatch {
@@ -428,9 +429,11 @@ __device__ void build_mesh(const Args& a, const Job& J, char* slot, Smem<kThread
                 ++j;
             }
             __syncwarp();
-            if (walking)
-                walking = p != kNoParent && ++steps <= n &&
-                          pipeline::walk_step<Src::kOwnCta, Src::kOwnCta>(ua, child, p, c, s, arrive);
+            if (walking) {
+                const pipeline::Climb next = pipeline::climb(p, steps++, ni);
+                if (next == pipeline::Climb::kCycle) atomicOr(a.err, kErrCycle);
+                walking = next == pipeline::Climb::kLevel && pipeline::walk_step(ua, child, p, c, s, arrive);
+            }
             __syncwarp();
         }
     }

@@ -125,26 +125,21 @@ __device__ __forceinline__ Carry complete_node(const UpArgs& a, uint32_t p, uint
     return o;
 }
 
-// One level of a leaf-to-root walk: arrives at p, the parent of `child` (whose
-// carry and summary are c and s), and as the second to arrive completes p from
-// the sibling's outputs; child, p, c and s then stand at p.  False where the
-// walk ends here: the first of two children to arrive, or a malformed tree.
-//
-// Pre says where the node records' children, the parents, the counts and the
-// sorted triangles were written, Sib where the sibling's outputs were.
-template <Src Pre, Src Sib, class Arrive>
+// One level of a leaf-to-root walk within a CTA that wrote the tree itself:
+// arrives at p, the parent of `child` (whose carry and summary are c and s; p
+// an internal node, climb()), and as the second to arrive completes p from the
+// sibling's outputs; child, p, c and s then stand at p.  False where the walk
+// ends here: the first of two children to arrive.
+template <class Arrive>
 __device__ __forceinline__ bool walk_step(const UpArgs& a, uint32_t& child, uint32_t& p, Carry& c, Summary& s,
                                           const Arrive& arrive_at) {
+    constexpr Src kOwn = Src::kOwnCta;
     const uint32_t internal = a.n - 1;
-    if (p >= internal) {
-        atomicOr(a.err, kErrCycle);
-        return false;
-    }
     // read ahead of the arrival
     const uint32_t* pw = reinterpret_cast<const uint32_t*>(a.nodes + p);
-    const uint32_t L = ld_src<Pre>(pw + 6), R = ld_src<Pre>(pw + 7);
-    const uint32_t grand = ld_src<Pre>(a.parents + p);
-    const uint32_t count = ld_src<Pre>(a.counts + p);
+    const uint32_t L = ld_src<kOwn>(pw + 6), R = ld_src<kOwn>(pw + 7);
+    const uint32_t grand = ld_src<kOwn>(a.parents + p);
+    const uint32_t count = ld_src<kOwn>(a.counts + p);
     if (arrive_at(a, p) == 0) return false;
     const bool from_left = (L == child);
     const uint32_t other = from_left ? R : L;
@@ -153,19 +148,19 @@ __device__ __forceinline__ bool walk_step(const UpArgs& a, uint32_t& child, uint
         const uint32_t* sw = reinterpret_cast<const uint32_t*>(a.nodes + other);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            o.lo[k] = __uint_as_float(ld_src<Sib>(sw + k));
-            o.hi[k] = __uint_as_float(ld_src<Sib>(sw + 3 + k));
+            o.lo[k] = __uint_as_float(ld_src<kOwn>(sw + k));
+            o.hi[k] = __uint_as_float(ld_src<kOwn>(sw + 3 + k));
         }
     }
-    o.cost = ld_src<Sib>(a.costs + other);
-    c = complete_node<Sib>(a, p, L, R, count, from_left ? c : o, from_left ? o : c);
+    o.cost = ld_src<kOwn>(a.costs + other);
+    c = complete_node<kOwn>(a, p, L, R, count, from_left ? c : o, from_left ? o : c);
     if (a.summary) {
         const bool sleaf = other >= internal;
         f3 v[3];
         if (sleaf) {
             const kr_vec3* pts = reinterpret_cast<const kr_vec3*>(a.tris);
 #pragma unroll
-            for (int i = 0; i < 3; ++i) v[i] = load_vertex_src<Pre>(pts, 3 * (other - internal) + i);
+            for (int i = 0; i < 3; ++i) v[i] = load_vertex_src<kOwn>(pts, 3 * (other - internal) + i);
         }
 #pragma unroll
         for (int k = 0; k < 7; ++k) {
@@ -173,13 +168,13 @@ __device__ __forceinline__ bool walk_step(const UpArgs& a, uint32_t& child, uint
             if (sleaf) {
                 sib = leaf_slab(v, other - internal, k);
             } else {
-                const uint4 q = ld_src<Sib>(a.summary + 7 * static_cast<size_t>(other) + k);
+                const uint4 q = ld_src<kOwn>(a.summary + 7 * static_cast<size_t>(other) + k);
                 sib = Slab{__uint_as_float(q.x), __uint_as_float(q.y), q.z, q.w};
             }
             const Slab own = slab_of(s, k);
             const Slab m = merge_slab(from_left ? own : sib, from_left ? sib : own);
             set_slab(s, k, m);
-            store_slab<Sib>(a.summary, p, k, m);
+            store_slab<kOwn>(a.summary, p, k, m);
         }
     }
     child = p;
