@@ -174,6 +174,49 @@ def test_obb_tree_extents_by_groups_units_and_blocks(builder, kind, n):
     assert same_bits(xfs.cpu().numpy(), want_x)
 
 
+def _chain(n):
+    """A tree as deep as it has leaves: internal node k holds leaf k and node k + 1."""
+    nodes = np.zeros(2 * n - 1, ref.NODE)
+    parents = np.full(2 * n - 1, 0xFFFFFFFF, np.uint32)
+    k = np.arange(n - 1)
+    nodes["left"][:n - 1], nodes["right"][:n - 1] = n - 1 + k, np.append(k[1:], 2 * n - 2)
+    nodes["left"][n - 1:], nodes["n_prims"][n - 1:] = np.arange(n), 1
+    parents[nodes["left"][:n - 1]] = parents[nodes["right"][:n - 1]] = k
+    return nodes, parents
+
+
+def test_obb_tree_of_a_chain_costs_little_more_than_its_collapse():
+    """One walk a level all the way up, every sibling a leaf.  The collapse of the
+    same tree is such a walk too, without slabs: the transform took 1.19 times
+    its time with a lane for a walk, and 1.50 where a group's lanes took turns
+    at a leaf's slabs."""
+    import torch
+    n = 5000
+    v, f = workloads.triangle_soup(n, seed=8)
+    nodes, parents = _chain(n)
+    tri = v[bvh.as_faces4(f)[:, :3]]
+    nodes["b"][n - 1:] = np.concatenate([tri.min(1), tri.max(1)], 1)
+    mesh = bvh.Mesh(v, f)
+    tree = {"nodes": torch.from_numpy(nodes.view(np.uint8).copy()).cuda(),
+            "parents": torch.from_numpy(parents.view(np.int32).copy()).cuda(),
+            "counts": torch.zeros(2 * n - 1, dtype=torch.int32, device="cuda"),
+            "costs": torch.zeros(2 * n - 1, device="cuda")}
+    obbs, xfs = bvh.obb_tree(mesh, tree)
+    want_o, want_x, _ = ref.obb_tree(nodes, parents, v, f)
+    assert same_bits(obbs.cpu().numpy(), want_o)
+    assert same_bits(xfs.cpu().numpy(), want_x)
+    times = ([], [])
+    for _ in range(7):  # in turn, the medians compared
+        for k, call in enumerate((lambda: bvh.obb_tree(mesh, tree, obbs, xfs), lambda: bvh.collapse(tree))):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            call()
+            b.record()
+            b.synchronize()
+            times[k].append(a.elapsed_time(b))
+    assert np.median(times[0]) < 1.35 * np.median(times[1]), (np.median(times[0]), np.median(times[1]))
+
+
 def test_obb_tree_rejects_a_parent_cycle():
     """A malformed tree ends with an error from the bounded walks, not a hang."""
     import torch
