@@ -35,7 +35,8 @@ typedef struct obvh_dito_batch_tuning {
     kr_u32 cta_max_points;    /* sets up to this size by one CTA; larger ones in chunks */
     kr_u32 lag_tasks;         /* 0: the CTA completing a large set's pass 1 runs its pass 2 (from L2);
                                  n > 0: pass 2 in chunk tasks queued n tasks after the set's pass 1 */
-    kr_u32 ctas_per_sm;       /* 1 or 2 */
+    kr_u32 ctas_per_sm;       /* 1: one CTA of 256 threads per SM; 2: the SM filled, by two CTAs of 256 threads or, where
+                                 a few sets set the batch's time, by one of 512 (chosen from the sets' sizes) */
 } obvh_dito_batch_tuning;
 
 /* Plans a batch; `offsets` is a HOST array of sets + 1 values starting at 0.

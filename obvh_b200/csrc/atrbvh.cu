@@ -27,9 +27,10 @@
 // The reference runs its treelet kernel with __syncthreads() inside
 // warp-divergent loops; every shared array it touches there is per warp, so
 // here each warp synchronises only itself (__syncwarp).  The two warp
-// reductions that pick the leaf to expand and the pair to merge use the
-// reference's shuffle-down order and strict comparisons, so ties resolve as
-// there.  Node data written by other warps is read through L2 (__ldcg) after
+// reductions that pick the leaf to expand and the pair to merge are a redux for
+// the value and one for the place that the reference's shuffle-down order and
+// strict comparisons prefer among equals, so ties resolve as there (a NaN area
+// takes the reference's own steps).  Node data written by other warps is read through L2 (__ldcg) after
 // the arrival counter's acquire.
 #include <cuda_runtime.h>
 
@@ -339,12 +340,12 @@ template <int W>
 __device__ __forceinline__ int seg_lane() { return threadIdx.x & (W - 1); }
 
 template <int W>
-__device__ __forceinline__ void reduce_down_seg(int count, int& idx, float& val, bool want_max) {
+__device__ __forceinline__ void reduce_down_max(int count, int& idx, float& val) {
     int amount = count / 2;
     while (count > 1) {
         const int oi = __shfl_down_sync(0xffffffffu, idx, amount, W);
         const float ov = __shfl_down_sync(0xffffffffu, val, amount, W);
-        if (want_max ? (ov > val) : (ov < val)) {
+        if (ov > val) {
             val = ov;
             idx = oi;
         }
@@ -468,7 +469,7 @@ __device__ __forceinline__ int largest_leaf(int count, float area, const uint8_t
     if (__any_sync(0xffffffffu, in && area != area)) {  // a NaN area: the reference's own steps
         int idx = in ? sl : -1;
         float a = in ? area : -FLT_MAX;
-        reduce_down_seg<W>(count, idx, a, true);
+        reduce_down_max<W>(count, idx, a);
         return __shfl_sync(0xffffffffu, idx, 0, W);
     }
     const uint32_t key = in ? f2key(area) : 0u;

@@ -7,8 +7,9 @@
 // sets of a batch are planned once on the host into a task queue, and one
 // kernel whose CTAs pull tasks from an atomic counter fits them all:
 //
-//   warp task   - up to 8 (16) small sets, one warp each (both passes, the candidate
-//                 search and the final box by the same warp);
+//   warp task   - up to 8 small sets (16 in a CTA of 512 threads), one warp each
+//                 (both passes, the candidate search and the final box by the
+//                 same warp);
 //   CTA task    - one medium set, both passes by one CTA;
 //   pass-1 task - one chunk of a large set: extremal points of the chunk into a
 //                 record; the last chunk to finish reduces the records and runs
@@ -24,8 +25,9 @@
 // released before anyone waits and its points are still in L2 when pass 2
 // reads them.  Small and medium sets are read twice by the same warp or CTA
 // and their second pass hits L1/L2.  Results are the single-set fit's
-// (dito.cu), bit for bit: the same first-index extremal points, the same
-// candidate search and the same final test.
+// (dito.cu), bit for bit: the same first-index extremal points, each extreme
+// with its point's own zero sign (candidate_warp), the same candidate search
+// and the same final test.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -517,7 +519,8 @@ kr_error check_tuning(const obvh_dito_batch_tuning& t) {
 // many to narrow ones, which overlap one set's serial steps with another's
 // points.  Measured (us, narrow / wide): 100 sets of 64..100,000 points 53 /
 // 39, 500 of 64..262,144 115 / 98, 1,000 of 64..60,000 54 / 72, 4,096 of
-// 64..262,144 499 / 606.
+// 64..262,144 499 / 606.  (ctas_per_sm = 2 fills the SM either way; the
+// autotuner times each setting with the width this rule gives it.)
 double longest_cta(const Batch& B, const std::vector<uint32_t>& large, const std::vector<uint32_t>& cta,
                    const std::vector<uint32_t>& warp, size_t ctas, int threads) {
     const double speed = threads == kWide ? 1.65 : 1.0, fixed = 25000.0;

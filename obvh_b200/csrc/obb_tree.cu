@@ -636,9 +636,7 @@ __global__ void __launch_bounds__(kThreads) dfs_rank_kernel(const kr_bvh_node* n
     }
 }
 
-// `points` is the packed xyz array the summary's vertex ids index: the mesh
-// vertices, or the depth-first triangle slots of the fused build.
-// Tiled: a thread per node, extents in tiles; listed: those of chain.list
+// The nodes that a candidate launch takes.  Tiled: a thread per node, extents in tiles; listed: those of chain.list
 // (FrameNodes::kAcross), extents in tiles; planned: a thread per node, extents
 // by plan_node's lists.
 enum class Nodes { kTiled, kListed, kPlanned };

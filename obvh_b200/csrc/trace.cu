@@ -8,19 +8,20 @@
 // Each ray follows exactly the reference's per-ray sequence, so results are
 // bit-identical: at an internal node both children's 4x3 transforms map the
 // ray into the unit cube's frame, the nearer hit child is taken first (ties
-// to the left) and the farther pushed; a leaf met during the descent is
-// intersected after the next node is popped; triangles are tested in the
-// leaf's order and a hit replaces the closest one only if strictly nearer.
+// to the left) and the farther pushed; the triangles of a leaf are tested in
+// its order when the descent reaches it, and a hit replaces the closest one
+// only if strictly nearer; then the next node is popped (the reference pops it
+// first, which changes nothing).
 // The reference's warp ballots only decide when a warp leaves its loops, so
 // the scheduling is free, and what sets the time is how many lanes of a warp
 // step together: lane by lane, a warp of incoherent rays ran 7.7 of 32 lanes
 // wide.  Here a warp visits nodes only while most of its lanes stand at one
 // (25 lanes wide), tests the triangles of all waiting lanes as one dealt-out
 // batch, and finished lanes take new rays together.  2,000,003 probe rays into
-// the 2M-triangle soup: 6.71 -> 4.74 ms, now waiting for node rows (58 of 100
-// sectors miss L1); 1920 x 1080 camera rays into the 917K-triangle knot: 1.26
-// -> 0.31 ms.  The 64-entry stack lives in local memory as in the
-// reference.  Indices are checked: a node, leaf, primitive
+// the 2M-triangle soup: 6.62 -> 4.76 ms, now waiting for node rows (58 of 100
+// sectors miss L1); 1920 x 1080 camera rays into the 917K-triangle knot: 1.15
+// -> 0.38 ms; the same with an infinite tmax.  The 64-entry stack lives in local
+// memory as in the reference.  Indices are checked: a node, leaf, primitive
 // slot or face outside its array, or a stack deeper than 64, stops that ray
 // with its miss record and sets the error word.
 #include <cuda_runtime.h>
@@ -379,9 +380,9 @@ __device__ __forceinline__ void visit_leaves(const kr_ivec4* __restrict__ meta, 
 // A warp visits nodes while at least kNodeLanes of 32 lanes with a ray stand
 // at one; the lanes that meanwhile reached a leaf wait and test their leaves
 // together.  Finished lanes wait until kRefillLanes of them write their
-// records and take new rays together.  Measured (probe / camera, us): 20 of 32
-// 4,829 / 494, 24 4,808 / 505, 28 4,866 / 534; 4 or 8 finished lanes 5,044 /
-// 577 and 5,171 / 567 on an earlier form.
+// records and take new rays together.  Measured (2,000,003 probe rays / 1920 x
+// 1080 camera rays, us): 20 of 32 4,800 / 376, 24 4,760 / 386, 28 4,728 / 403;
+// 2, 4 and 8 finished lanes 4,710 / 384, 4,760 / 386 and 4,865 / 385.
 constexpr int kNodeLanes = 24;
 constexpr int kRefillLanes = 4;
 

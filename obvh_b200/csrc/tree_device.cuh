@@ -120,7 +120,8 @@ struct M4 {
 // the last row (0, 0, 0, 1), a pure frame (kFrame) a zero last column too.
 // With finite entries whose products do not overflow, a term with a zero
 // factor adds a zero and a factor 1 changes nothing, so those drop out and the
-// rest is evaluated in the same order: 150 operations a box instead of 560.
+// rest is evaluated in the same order (a sum that is zero may have the other
+// sign): 150 operations a box instead of 560.
 enum class Shape { kAny, kAffine, kFrame };
 
 template <Shape S>
@@ -243,7 +244,7 @@ __device__ inline void write_box(kr_obb3* obb, kr_mat4* xf, f3 a0, f3 a1, f3 a2,
     o[9] = a2.x; o[10] = a2.y; o[11] = a2.z;
     o[12] = ext.x; o[13] = ext.y; o[14] = ext.z;
     // T R S: the axes scaled by twice the extents, then mid (finite factors:
-    // the products with zeros and ones change nothing)
+    // the products with zeros and ones change nothing but a zero's sign)
     const f3 c0 = mulv(a0, ext.x * 2.0f), c1 = mulv(a1, ext.y * 2.0f), c2 = mulv(a2, ext.z * 2.0f);
     M4 inv;
     if (plain_entries(c0, c1, c2, mid) && plain_entries(a0, a1, a2, ext)) {
