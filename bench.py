@@ -1260,8 +1260,8 @@ def bench_batch_ours(a, dist):
         "kernels": kernel_table(prof, a.steps, batch_bytes, peak),
         "gpu_launches": sum(v[0] for v in prof.values()), "roofline": roof,
         "per_call": {"value": round(pc_value, 3), "unit": "Mpoints/s", "ms_per_batch": round(pc_ms, 3),
-                     "api": "obvh_dito_fit_async per set (2 kernels per set, grid sized to the set's 2,048-point "
-                            "tiles), same device buffer, the 4,096 calls replayed from one CUDA graph",
+                     "api": "obvh_dito_fit_async per set (one cluster launch per set), same device buffer, the "
+                            "4,096 calls replayed from one CUDA graph",
                      "speedup": round(value / pc_value, 2),
                      "host_loop_ms_per_batch": round(host_loop_ms, 3),
                      "host_loop_speedup": round(value / (total / (host_loop_ms / 1e3) / 1e6), 2)},
