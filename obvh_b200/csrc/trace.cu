@@ -239,21 +239,24 @@ __device__ __forceinline__ void visit_node(const Boxes& boxes, const kr_ivec4* _
     const float limit = fminf(st.hit_t, FLT_MAX);
     const bool sure_l = sl && apart(l0, l1) && apart(l0, limit);
     const bool sure_r = sr && apart(r0, r1) && apart(r0, limit);
-    // which child is nearer: decided only where both distances have the bound
-    const bool close = (tl || !sure_l) && (tr || !sure_r) && (sl != sr || !apart(l0, r0));
+    const bool close = (tl || !sure_l) && (tr || !sure_r) && !apart(l0, r0);
     bool exact_l = !sure_l || close, exact_r = !sure_r || close;
-    while (exact_l || exact_r) {
-        const float2 e = unit_slabs(exact_l ? l : r);
-        const bool hit = e.y >= e.x && e.y >= 0.0f && e.x <= st.hit_t;
-        if (exact_l) {
-            tl = hit;
-            l0 = e.x;
-            exact_l = false;
-        } else {
-            tr = hit;
-            r0 = e.x;
-            exact_r = false;
-        }
+    if (exact_l || exact_r) {
+        // which child is nearer needs both distances with the bound, or both exact
+        if (sl != sr) exact_l = exact_r = true;
+        do {
+            const float2 e = unit_slabs(exact_l ? l : r);
+            const bool hit = e.y >= e.x && e.y >= 0.0f && e.x <= st.hit_t;
+            if (exact_l) {
+                tl = hit;
+                l0 = e.x;
+                exact_l = false;
+            } else {
+                tr = hit;
+                r0 = e.x;
+                exact_r = false;
+            }
+        } while (exact_l || exact_r);
     }
     const bool swap = r0 < l0;
     if (tl && tr) {
