@@ -18,7 +18,7 @@
 // wide.  Here a warp visits nodes only while most of its lanes stand at one
 // (25 lanes wide), tests the triangles of all waiting lanes as one dealt-out
 // batch, and finished lanes take new rays together.  2,000,003 probe rays into
-// the 2M-triangle soup: 6.62 -> 4.76 ms, now waiting for node rows (58 of 100
+// the 2M-triangle soup: 6.62 -> 4.75 ms, now waiting for node rows (58 of 100
 // sectors miss L1); 1920 x 1080 camera rays into the 917K-triangle knot: 1.15
 // -> 0.38 ms; the same with an infinite tmax.  The 64-entry stack lives in local
 // memory as in the reference.  Indices are checked: a node, leaf, primitive
@@ -384,8 +384,8 @@ __device__ __forceinline__ void visit_leaves(const kr_ivec4* __restrict__ meta, 
 // at one; the lanes that meanwhile reached a leaf wait and test their leaves
 // together.  Finished lanes wait until kRefillLanes of them write their
 // records and take new rays together.  Measured (2,000,003 probe rays / 1920 x
-// 1080 camera rays, us): 20 of 32 4,800 / 376, 24 4,760 / 386, 28 4,728 / 403;
-// 2, 4 and 8 finished lanes 4,710 / 384, 4,760 / 386 and 4,865 / 385.
+// 1080 camera rays, us): 20 of 32 4,785 / 367, 24 4,750 / 379, 28 4,716 / 402;
+// 2, 4 and 8 finished lanes 4,690 / 376, 4,750 / 379 and 4,859 / 378.
 constexpr int kNodeLanes = 24;
 constexpr int kRefillLanes = 4;
 
